@@ -219,7 +219,7 @@ long long nsa_topk_sparse_attn_bwd_workspace(int total_len, int batch, int num_q
  * Replaces _topk_sparse_attention_bwd: backward_sum_o_do, count_query, reorder_topk_idx (argsort + 4 host
  * syncs), backward_dkdv with its [G, N, Hkv, d] buffers and .sum(0), backward_dq,
  * native_sparse_attention/ops/triton/topk_sparse_attention.py:176-477,480-825,912-1109.
- *   cu_seqblocks int32 [batch+1]: prefix sum of ceil(seqlen / block_size).
+ *   cu_seqblocks int32 [batch+1]: prefix sum of ceil(seqlen / block_size), or NULL: computed by this call.
  *   strides[19] = the 16 of nsa_varlen_attn_bwd followed by {idx_h, idx_n, idx_k}. */
 int nsa_topk_sparse_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
                              const float* lse, const int* topk_idx, const int* cu_seqlens,

@@ -4,13 +4,17 @@ The library is built in-tree by ``make -C csrc`` (see ``build``); there is no CP
 if the shared object is missing or a call fails, a RuntimeError is raised.
 """
 import ctypes
+import importlib
 import os
 import subprocess
+import sys
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libnsa_b200.so")
+HOST_PATH = os.path.join(_HERE, "_nsa_host.so")
 _lib = None
+_host = None
 
 DTYPE_BF16, DTYPE_FP16 = 0, 1
 
@@ -66,13 +70,14 @@ _SIZE_QUERIES = {
 
 
 def build(verbose: bool = False) -> str:
-    """Compile every CUDA source for sm_100a into libnsa_b200.so (nvcc cross-compiles without a GPU)."""
-    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), "-j", str(min(8, os.cpu_count() or 1))]
+    """Compile every CUDA source for sm_100a into libnsa_b200.so (nvcc cross-compiles without a GPU) and the operators' host
+    side, the Python extension _nsa_host.so, against the installed torch."""
+    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), "-j", str(min(8, os.cpu_count() or 1)), f"PYTHON={sys.executable}"]
     res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or res.returncode:
         print(res.stdout)
     if res.returncode:
-        raise RuntimeError("building libnsa_b200.so failed")
+        raise RuntimeError("building libnsa_b200.so and _nsa_host.so failed")
     return LIB_PATH
 
 
@@ -96,6 +101,17 @@ def lib() -> ctypes.CDLL:
             fn.restype = c_longlong
         _lib = handle
     return _lib
+
+
+def host():
+    """The extension module with the operators' host side (csrc/host/torch_ops.cpp), which calls the same libnsa_b200.so."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
+        _host = importlib.import_module("._nsa_host", __package__)
+    return _host
 
 
 def exported_symbols():

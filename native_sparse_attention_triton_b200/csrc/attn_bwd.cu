@@ -268,6 +268,34 @@ struct IndexParams {
   Status st;
 };
 
+// cu_blocks[b] = sum over the sequences before b of ceil(length / block_size): one CTA, 256 sequences per round
+__global__ void __launch_bounds__(256) block_prefix_kernel(const int* __restrict__ cu, int batch, int block_size, int* __restrict__ cu_blocks) {
+  __shared__ int warp_sum[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry = 0;
+  if (threadIdx.x == 0) cu_blocks[0] = 0;
+  for (int base = 0; base < batch; base += 256) {
+    const int b = base + threadIdx.x;
+    int v = b < batch ? (__ldg(cu + b + 1) - __ldg(cu + b) + block_size - 1) / block_size : 0;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v, off);
+      if (lane >= off) v += t;
+    }
+    if (lane == 31) warp_sum[warp] = v;
+    __syncthreads();
+    int before = carry, total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += warp_sum[w];
+      total += warp_sum[w];
+    }
+    if (b < batch) cu_blocks[b + 1] = before + v;
+    carry += total;
+    __syncthreads();
+  }
+}
+
 template <bool FILL>
 __global__ void index_scatter_kernel(IndexParams p) {
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -648,7 +676,7 @@ static int launch_dkdv(const void* q, const void* dout, const void* k, const voi
   const size_t smem = 1024 + 2 * TILE_BYTES + kBwdStages * STAGE_BYTES + (2 * kBwdStages + 1) * sizeof(uint64_t) +
                       kBwdStages * kSlots * (16 * sizeof(float2) + sizeof(int)) + 64;
   auto kern = dkdv_kernel<T, D, SPARSE>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   { LaunchScope ls_(SPARSE ? "sparse_dkdv" : "dense_dkdv", stream); kern<<<grid, 160, smem, stream>>>(tmQ, tmDO, tmK, tmV, p); }
   return cuda_rc(cudaGetLastError());
@@ -737,6 +765,7 @@ static size_t sparse_ws_bytes(int N, int batch, int Hq, int Hkv, int D, int topk
   const size_t x = (size_t)Hkv * sparse_windows(N, Hq / Hkv, D).second * TB + 1;
   return align_up((size_t)N * Hq * sizeof(float2), 256) + 2 * align_up((size_t)N * Hkv * D * sizeof(float), 256) +
          4 * align_up(x * sizeof(int), 256) + align_up((size_t)Hkv * N * topk * sizeof(int), 256) +
+         align_up(((size_t)batch + 1) * sizeof(int), 256) +
          align_up(((size_t)Hkv * N * topk / kSparseChunk + x) * sizeof(int), 256) +
          (sparse_fused_dq(Hq / Hkv, D) ? align_up((size_t)N * Hq * D * sizeof(float), 256) : 0);
 }
@@ -770,6 +799,13 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   w += align_up((size_t)Hkv * N * topk * sizeof(int), 256);
   int* item_bin = reinterpret_cast<int*>(w);   // one entry per possible work item (the grid's upper bound below)
   w += align_up(((size_t)Hkv * N * topk / kSparseChunk + X) * sizeof(int), 256);
+  if (!cu_blocks) {  // the caller left the prefix sum of blocks to this call
+    int* own = reinterpret_cast<int*>(w);
+    LaunchScope ls_("block_prefix", stream);
+    block_prefix_kernel<<<1, 256, 0, stream>>>(cu, batch, block_size, own);
+    cu_blocks = own;
+  }
+  w += align_up(((size_t)batch + 1) * sizeof(int), 256);
   const bool fused = sparse_fused_dq(G, D);  // dQ comes out of the tcgen05 dK/dV pass; otherwise the per-token dQ kernel runs
   float* dq32 = fused ? reinterpret_cast<float*>(w) : nullptr;
   // dk32, dv32, count, cursor are contiguous: one memset
@@ -820,7 +856,7 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
     if (rc) return rc;
     const size_t smem = 1024 + WARPS * (KBUFS + 1) * TILE_BYTES + (KBUFS + 1) * WARPS * sizeof(uint64_t) + WARPS * kMaxTilesBwd * sizeof(int);
     auto kern = sparse_dq_kernel<T, D, WARPS, KBUFS>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     dim3 grid((N + WARPS - 1) / WARPS, Hkv);
     { LaunchScope ls_("sparse_dq", stream); kern<<<grid, WARPS * 32, smem, stream>>>(tmK, tmV, p); }
@@ -918,7 +954,7 @@ extern "C" int nsa_topk_sparse_attn_bwd(const void* q, const void* k, const void
                                         int num_kv_heads, int head_dim, int topk, int block_size, const long long* strides,
                                         float sm_scale, int dtype, void* stream) {
   using namespace nsa;
-  if (!q || !k || !v || !o || !dout || !lse || !topk_idx || !cu_seqlens || !cu_seqblocks || !dq || !dk || !dv || !workspace ||
+  if (!q || !k || !v || !o || !dout || !lse || !topk_idx || !cu_seqlens || !dq || !dk || !dv || !workspace ||
       !strides)
     return kInvalid;
   if (total_len <= 0 || batch <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return kInvalid;

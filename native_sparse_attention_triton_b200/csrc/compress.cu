@@ -327,7 +327,7 @@ static int launch_linear_fwd(LinFwdParams p, const void* pe, void* bias_scratch,
   }
   const size_t smem = 1024 + 2 * (64 * D * 2 + D * D * 2);
   auto kern = linear_fwd_kernel<T, D>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_ylen + 63) / 64, B, p.H);
   { LaunchScope ls_("linear_compress_fwd", stream); kern<<<grid, 128, smem, stream>>>(p); }

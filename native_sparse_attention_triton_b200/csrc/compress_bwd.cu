@@ -355,14 +355,14 @@ static int run_linear_bwd(LinBwdParams p, void* dpe, float* dbias, int total_y, 
   {
     const size_t smem = 1024 + 4 * 64 * D * 2;
     auto kern = linear_dw_kernel<T, D>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     { LaunchScope ls_("linear_dw", stream); kern<<<dim3(p.ks, p.H), D * 2, smem, stream>>>(p); }
   }
   {
     const size_t smem = 1024 + D * D * 2;
     auto kern = linear_dx_kernel<T, D>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     const int chunks = (max_len + p.stride - 1) / p.stride;
     { LaunchScope ls_("linear_dx", stream); kern<<<dim3((chunks + 63) / 64, p.stride, p.B * p.H), 128, smem, stream>>>(p); }

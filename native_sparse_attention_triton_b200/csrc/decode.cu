@@ -374,15 +374,11 @@ static int launch_decode(const void* k, const void* v, const long long* kv_strid
     if (mode == kDecodeCompressed) p.logits = f;
   }
   const size_t smem = 1024 + WARPS * 2 * TILE_BYTES + WARPS * 2 * sizeof(uint64_t) + WARPS * kMaxTilesPerDecodeQuery * sizeof(int);
-  int sms = 148;
-  {
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
+  const int sms = num_sms();
   const int ctas_all = (p.total_tasks + WARPS - 1) / WARPS;
   const int grid = p.ctrl ? (ctas_all < sms ? ctas_all : sms) : ctas_all;  // persistent when tasks are handed out dynamically
   auto launch = [&](auto kern, const char* name) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     LaunchScope ls_(name, stream);
     kern<<<grid, WARPS * 32, smem, stream>>>(tmK, tmV, p);

@@ -370,7 +370,7 @@ int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const v
   if (rc) return rc;
   const size_t smem = (size_t)(2 + kQStages + kDoStages) * kTileBytes + 4 * 128 * sizeof(float) + 24 * sizeof(uint64_t) + 16;
   auto kern = dense_dkdv_tc_kernel<T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_k + 127) / 128, (max_q + p.chunk - 1) / p.chunk, batch * p.Hkv);
   { LaunchScope ls_("dense_dkdv_tc", stream); kern<<<grid, 320, smem, stream>>>(tmQ, tmDO, tmK, tmV, p, logG); }

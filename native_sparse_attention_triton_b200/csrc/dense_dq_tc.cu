@@ -383,7 +383,7 @@ static int launch_dense_dq_tc(const void* k, const void* v, long long k_sn, long
   if (rc) return rc;
   const size_t smem = (size_t)(2 + kDqKStages + kDqVStages) * (128 * D * 2) + 256 * sizeof(float) + 24 * sizeof(uint64_t) + 16;
   auto kern = dense_dq_tc_kernel<T, D>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_seqlen_q + QT - 1) / QT, p.B, p.Hkv);
   { LaunchScope ls_("dense_dq_tc", stream); kern<<<grid, 320, smem, stream>>>(tmQ, tmDO, tmO, tmK, tmV, tmDQ, p); }

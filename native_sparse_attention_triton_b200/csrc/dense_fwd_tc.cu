@@ -445,7 +445,7 @@ static int launch_dense_fwd_tc(const void* q, const void* k, const void* v, cons
   if (rc) return rc;
   const size_t smem = 2 * 128 * D * 2 + (kTcKStages + kTcVStages) * kTcKeyTile * D * 2 + 32 * sizeof(uint64_t);
   auto kern = dense_fwd_tc_kernel<T, D>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_seqlen_q + 2 * QT - 1) / (2 * QT), p.B, p.Hkv);
   { LaunchScope ls_("dense_fwd_tc", stream); kern<<<grid, 320, smem, stream>>>(tmQ, tmK, tmV, tmO, p); }

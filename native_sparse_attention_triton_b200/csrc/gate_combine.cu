@@ -123,11 +123,8 @@ __global__ void __launch_bounds__(256) gate_combine_bwd_kernel(CombineParams p) 
 
 // Enough CTAs to keep every SM's load queues full; the grid-stride loops cover the rest.
 static int combine_grid(long long threads_needed) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = (threads_needed + 255) / 256;
-  const long long cap = (long long)sms * 16;
+  const long long cap = (long long)num_sms() * 16;
   return (int)(want < cap ? (want > 0 ? want : 1) : cap);
 }
 

@@ -53,22 +53,61 @@ int make_tmap_4d(CUtensorMap* out, CUtensorMapDataType dt, const void* base, uin
   return r == CUDA_SUCCESS ? kOk : kInvalid;
 }
 
+namespace {
+struct SmemGrant {
+  std::atomic<const void*> kernel{nullptr};
+  std::atomic<int> bytes[16];  // by device
+};
+constexpr int kGrants = 512;  // open addressing; the library has about a hundred kernels with dynamic shared memory
+SmemGrant g_grants[kGrants];
+std::atomic<int> g_sms[64];
+}  // namespace
+
+cudaError_t allow_smem(const void* kernel, int bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  SmemGrant* g = nullptr;
+  if (dev < 16) {
+    size_t at = (reinterpret_cast<uintptr_t>(kernel) >> 4) % kGrants;
+    for (int i = 0; i < kGrants && !g; ++i, at = (at + 1) % kGrants) {
+      const void* seen = g_grants[at].kernel.load(std::memory_order_acquire);
+      if (!seen && g_grants[at].kernel.compare_exchange_strong(seen, kernel)) seen = kernel;
+      if (seen == kernel) g = &g_grants[at];
+    }
+    if (g && g->bytes[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+  }
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && g) g->bytes[dev].store(bytes, std::memory_order_release);
+  return e;
+}
+
+int num_sms() {
+  int dev = 0, n = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return n;
+  if (dev < 64) {
+    const int seen = g_sms[dev].load(std::memory_order_relaxed);
+    if (seen) return seen;
+  }
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && dev < 64) g_sms[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // One status word per device that loads the library (a module-scope device variable, zero at load).
 __device__ int g_status_word;
 
-static int* g_status[64] = {};
+static std::atomic<int*> g_status[64];
 static std::mutex g_status_mu;
 
 int* status_word() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (int* seen = g_status[dev].load(std::memory_order_acquire)) return seen;
   std::lock_guard<std::mutex> lk(g_status_mu);
-  if (!g_status[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
-    g_status[dev] = static_cast<int*>(p);
-  }
-  return g_status[dev];
+  void* p = nullptr;
+  if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
+  g_status[dev].store(static_cast<int*>(p), std::memory_order_release);
+  return static_cast<int*>(p);
 }
 
 int read_status(cudaStream_t stream) {

@@ -28,6 +28,17 @@ int make_tmap_4d(CUtensorMap* out, CUtensorMapDataType dt, const void* base, uin
                  uint64_t n3, uint64_t stride1, uint64_t stride2, uint64_t stride3, uint32_t b0, uint32_t b2,
                  uint32_t b3 = 1);
 
+// Opt `kernel` in to `bytes` of dynamic shared memory on the current device.  The runtime call costs about a microsecond of
+// host time, so what has been granted is remembered per (kernel, device) and asked for once.
+cudaError_t allow_smem(const void* kernel, int bytes);
+template <typename K>
+cudaError_t allow_smem(K* kernel, size_t bytes) {
+  return allow_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(bytes));
+}
+
+// multiprocessors of the current device (remembered)
+int num_sms();
+
 // device status word of the current device (allocated on first use, zero-initialised)
 int* status_word();
 // read-and-clear; returns the OR of error bits raised by kernels since the last call

@@ -195,7 +195,7 @@ static int launch_linear_fwd_tc(const void* x, const void* w, int batch, int max
   if (rc) return rc;
   const size_t smem = 2 * kLinStages * kLinTile + (2 * kLinStages + 1) * sizeof(uint64_t) + 16;
   auto kern = linear_fwd_tc_kernel<T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_y_len + kLinRows - 1) / kLinRows, batch, p.H);
   { LaunchScope ls_("linear_compress_fwd", stream); kern<<<grid, 192, smem, stream>>>(tmXa, tmXb, tmW, p); }

@@ -270,7 +270,7 @@ static int launch_pool_bwd_stream(const void* x, int* slots_out, int batch, int 
   }
   const size_t smem = (dw ? (size_t)p.groups * p.slots * chunk : 0) + 2 * kPbMaxBars * sizeof(uint64_t) + (size_t)p.hb * p.ks * sizeof(float);
   auto launch = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     { LaunchScope ls_(dw ? "pool_dx_dw" : "pool_dx", stream); kern<<<grid, kPbConsumers + 32, smem, stream>>>(tmX, p); }
     return cuda_rc(cudaGetLastError());

@@ -227,7 +227,7 @@ static int launch_pool_fwd_stream(const void* x, int batch, int total_len, int t
   const size_t smem = (size_t)p.groups * p.slots * chunk + 2 * kPoolMaxBars * sizeof(uint64_t) + (size_t)p.hb * p.ks * sizeof(float);
   const dim3 grid((max_y_len + p.run - 1) / p.run, batch, (p.H + p.hb - 1) / p.hb);
   auto launch = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     { LaunchScope ls_("pool_compress_fwd", stream); kern<<<grid, kPoolConsumers + 32, smem, stream>>>(tmX, p); }
     return cuda_rc(cudaGetLastError());

@@ -112,11 +112,8 @@ static int launch_rope3(Rope3Params p, cudaStream_t stream) {
 template <typename T, int D>
 static int launch_rope(RopeParams p, cudaStream_t stream) {
   constexpr int TOK = 256 / (D / 2);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = ((long long)p.N + TOK - 1) / TOK;
-  const long long cap = (long long)sms * 8;  // 8 resident CTAs of 256 threads per SM
+  const long long cap = (long long)num_sms() * 8;  // 8 resident CTAs of 256 threads per SM
   LaunchScope ls_("rope", stream);
   rope_kernel<T, D><<<(int)(want < cap ? want : cap), 256, 0, stream>>>(p);
   return cuda_rc(cudaGetLastError());

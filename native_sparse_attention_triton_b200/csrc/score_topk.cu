@@ -190,7 +190,7 @@ static int launch_score_topk(const void* k, long long k_sn, long long k_sh, int 
   p.nwarps = nwarps;
   const size_t smem = smem_for(nwarps);
   auto kern = score_topk_kernel<T, D, STAGES>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   const int QT = nwarps * QPW;
   dim3 grid((max_seqlen_q + QT - 1) / QT, p.B, p.Hkv);

@@ -219,7 +219,7 @@ static int launch_score_topk_tc(const void* q, const void* k, long long k_sn, lo
   rc = make_tmap_3d(&tmK, DT<T>::kTmapType, k, D, p.Hkv, Nk, k_sh, k_sn, 64, 1, kScKeyTile);
   if (rc) return rc;
   auto kern = p.logG == 4 ? score_topk_tc_kernel<T, D, 4> : (p.logG == 3 ? score_topk_tc_kernel<T, D, 3> : score_topk_tc_kernel<T, D, 2>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_seqlen_q + TPT - 1) / TPT, p.B, p.Hkv);
   { LaunchScope ls_("score_topk_tc", stream); kern<<<grid, 320, smem, stream>>>(tmQ, tmK, p); }

@@ -628,13 +628,12 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
   if (rc) return rc;
   const size_t smem = 2 * kSpKvBytes + 2 * kSpPdBytes + (kSpQStages + kSpDoStages) * kSpRowBytes + 48 * sizeof(uint64_t) + 64;
   auto launch = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
     LaunchScope ls_("sparse_dkdv_tc", stream);
     // persistent CTAs: one per SM (shared memory and the 512 TMEM columns allow no more), each taking work items from a
     // grid-wide counter; grid.x * grid.y on entry is the upper bound of their number
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = num_sms();
     const unsigned long long bound = (unsigned long long)grid.x * grid.y;   // (list entries) x (tiles per block)
     grid = dim3((unsigned)std::min<unsigned long long>(bound, (unsigned long long)sms), 1, 1);
     kern<<<grid, kSpThreads, smem, stream>>>(tmK, tmV, static_cast<const T*>(q), static_cast<const T*>(dout), strides[0], strides[1],

@@ -143,7 +143,7 @@ static int launch_sparse_fwd(const void* k, const void* v, long long k_sn, long 
   if (rc) return rc;
   const size_t smem = 1024 + WARPS * 2 * TILE_BYTES + WARPS * 2 * sizeof(uint64_t) + WARPS * kMaxTilesPerQuery * sizeof(int);
   auto kern = sparse_fwd_kernel<T, D, WARPS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((p.N + WARPS - 1) / WARPS, p.Hkv);
   { LaunchScope ls_("sparse_fwd", stream); kern<<<grid, WARPS * 32, smem, stream>>>(tmK, tmV, p); }

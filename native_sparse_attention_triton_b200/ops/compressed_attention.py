@@ -10,51 +10,6 @@ from typing import Tuple, Union
 import torch
 
 from .. import _lib
-from ._common import default_scale, dtype_code, host_seqlens, inner_contiguous, ptr, require_cuda, stream_ptr
-from .dense_attention import varlen_attention_backward, varlen_attention_forward
-
-
-class CompressedAttention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, kernel_size, kernel_stride, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, sm_scale):
-        assert q.dtype == torch.bfloat16 or q.dtype == torch.float16
-        assert q.dtype == k.dtype and k.dtype == v.dtype
-        assert cu_seqlens_q.dtype == torch.int32 and cu_seqlens_k.dtype == torch.int32
-        if sm_scale is None:
-            sm_scale = default_scale(q.shape[-1])
-        q, k, v = inner_contiguous(q), inner_contiguous(k), inner_contiguous(v)
-        o, lse = varlen_attention_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, True, kernel_size,
-                                          kernel_stride, sm_scale)
-        ctx.save_for_backward(q, k, v, o, lse, cu_seqlens_q, cu_seqlens_k)
-        ctx.meta = (sm_scale, max_seqlen_q, max_seqlen_k, kernel_size, kernel_stride)
-        ctx.mark_non_differentiable(lse)
-        return o, lse
-
-    @staticmethod
-    def backward(ctx, do, *args):
-        q, k, v, o, lse, cu_q, cu_k = ctx.saved_tensors
-        sm_scale, max_q, max_k, kernel_size, kernel_stride = ctx.meta
-        dq, dk, dv = varlen_attention_backward(q, k, v, o, lse, do, cu_q, cu_k, max_q, max_k, True, kernel_size,
-                                               kernel_stride, sm_scale)
-        return dq, dk, dv, None, None, None, None, None, None, None
-
-
-def select_topk_blocks(q, k, lse, kernel_size, kernel_stride, block_size, topk, cu_seqlens_q, cu_seqlens_k,
-                       max_seqlen_q, sm_scale, init_blocks, local_blocks) -> torch.Tensor:
-    """topk_idx int32 [num_kv_heads, total_q, min(topk, ceil(max_seqlen_q / block_size))]."""
-    total_q, num_q_heads, head_dim = q.shape
-    total_k, num_kv_heads, _ = k.shape
-    batch = cu_seqlens_q.shape[0] - 1
-    max_blocks = (max_seqlen_q + block_size - 1) // block_size
-    t_out = min(topk, max_blocks)
-    topk_idx = torch.empty(num_kv_heads, total_q, t_out, dtype=torch.int32, device=q.device)
-    strides = _lib.strides_array(q.stride(0), q.stride(1), k.stride(0), k.stride(1), *topk_idx.stride())
-    rc = _lib.lib().nsa_compressed_attn_topk(
-        ptr(q), ptr(k), ptr(lse), ptr(cu_seqlens_q), ptr(cu_seqlens_k), ptr(topk_idx), total_q, total_k, batch,
-        max_seqlen_q, num_q_heads, num_kv_heads, head_dim, kernel_size, kernel_stride, block_size, topk, init_blocks,
-        local_blocks, strides, sm_scale, dtype_code(q), stream_ptr(q.device))
-    _lib.check(rc, "nsa_compressed_attn_topk")
-    return topk_idx
 
 
 def compressed_attention(
@@ -90,30 +45,7 @@ def compressed_attention(
     Returns:
         (attention output like q, topk_idx int32 [num_kv_heads, total_q_len, min(topk, num_blocks)])
     """
-    require_cuda(q, k, v, cu_seqlens_q, cu_seqlens_k)
-    if max_seqlen_q is None:
-        cq = host_seqlens(cu_seqlens_q)
-        max_seqlen_q = max(cq[i + 1] - cq[i] for i in range(len(cq) - 1))
-    if max_seqlen_k is None:
-        ck = host_seqlens(cu_seqlens_k)
-        max_seqlen_k = max(ck[i + 1] - ck[i] for i in range(len(ck) - 1))
-    max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
-    assert k.shape[0] == v.shape[0] and q.shape[0] > k.shape[0]
-    assert k.shape[1] == v.shape[1] and q.shape[1] % k.shape[1] == 0
-    attn_output, lse = CompressedAttention.apply(q, k, v, kernel_size, kernel_stride, cu_seqlens_q, cu_seqlens_k,
-                                                 max_seqlen_q, max_seqlen_k, sm_scale)
     if topk <= 0:
         warnings.warn("topk <= 0, returned topk_idx will be None")
-        return attn_output, None
-    assert topk >= init_blocks + local_blocks
-    assert block_size % kernel_stride == 0 and kernel_size % kernel_stride == 0
-    with torch.no_grad():
-        if sm_scale is None:
-            sm_scale = default_scale(q.shape[-1])
-        if k.shape[0] == 0:
-            # no compressed key anywhere: scores are all zero, only forced blocks and the lowest ids are taken
-            k = torch.zeros(1, k.shape[1], k.shape[2], dtype=q.dtype, device=q.device)
-        topk_idx = select_topk_blocks(inner_contiguous(q.detach()), inner_contiguous(k.detach()), lse, kernel_size,
-                                      kernel_stride, block_size, topk, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
-                                      sm_scale, init_blocks, local_blocks)
-    return attn_output, topk_idx
+    return _lib.host().compressed_attention(q, k, v, kernel_size, kernel_stride, block_size, topk, cu_seqlens_q, cu_seqlens_k,
+                                            max_seqlen_q, max_seqlen_k, sm_scale, init_blocks, local_blocks)
