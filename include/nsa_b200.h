@@ -96,17 +96,6 @@ int nsa_pool_compress_fwd(const void* x, const void* w, const void* pe, const in
                           int total_y, int max_y_len, int num_heads, int head_dim, int kernel_size,
                           int kernel_stride, long long x_stride_n, long long x_stride_h, int dtype, void* stream);
 
-/* The compression of a decode step for both pooling modes, K and V in one launch: every sequence contributes exactly
- * one window, the kernel_size rows of its staging buffer (x_k, x_v: [batch, kernel_size, H, d] views with strides
- * x_stride_b, x_stride_n, x_stride_h), so no cu_seqlens is read.  w_k / w_v [H, kernel_size] or NULL (average); bias_k /
- * bias_v [H, d] (the position embedding folded through the weights by nsa_pool_bias, which does not change between steps)
- * or NULL; y_k, y_v [batch, H, d] contiguous.  Replaces the two compress_func calls on the staging buffers in
- * native_sparse_attention/infer/inference_func.py:56-87 when both are pooling operators. */
-int nsa_pool_compress_decode_pair(const void* x_k, const void* x_v, const void* w_k, const void* w_v, const void* bias_k,
-                                  const void* bias_v, void* y_k, void* y_v, int batch, int num_heads, int head_dim,
-                                  int kernel_size, long long x_stride_b, long long x_stride_n, long long x_stride_h,
-                                  int dtype, void* stream);
-
 /* bias[h, :] = sum_k w[h, k] * pe[h, k, :] (w == NULL: the mean over k), in the storage type: the term the pooling
  * operators add to every compressed row (native_sparse_attention/ops/triton/weighted_pool.py:301-363). */
 int nsa_pool_bias(const void* pe, const void* w, void* bias, int num_heads, int head_dim, int kernel_size, int dtype,
@@ -156,7 +145,7 @@ int nsa_flash_attn_decode_static(const void* q, const void* k, const void* v, co
 
 /* Single-token attention over the selected blocks of a dense cache.
  * Replaces forward_kernel, native_sparse_attention/ops/triton/topk_sparse_attention_decode.py:22-237.
- *   topk_idx int32 [Hkv, B, topk]. */
+ *   topk_idx int32 [Hkv, B, topk].  Needs no scratch: scratch, scratch_floats and num_splits are ignored. */
 int nsa_topk_sparse_attn_decode(const void* q, const void* k, const void* v, const int* topk_idx,
                                 const int* seqlens, void* o, float* scratch, long long scratch_floats,
                                 int num_splits, int batch, int cache_len, int num_q_heads, int num_kv_heads,
@@ -335,6 +324,39 @@ int nsa_rope_decode(const void* x, void* y, const float* inv_freq, const int* le
 int nsa_rope_decode3(const void* q, void* yq, const void* k, void* yk, const void* ck, void* yck, const float* inv_freq,
                      const int* lengths_qk, const int* lengths_ck, int batch, int num_q_heads, int num_kv_heads, int head_dim,
                      int stride_ck, float attention_scaling, const long long* strides, int dtype, void* stream);
+
+/* One decode step of a layer on its caches in one launch: stage the new token (nsa_kv_cache_stage_decode), pool the window it
+ * completes, rotate query, key and compressed key (nsa_rope_decode3), append them (nsa_kv_cache_append_decode), compressed
+ * attention with block selection, selected-block and sliding-window attention, gated sum (nsa_gate_combine_fwd): the decode
+ * branch of nsa_infer, native_sparse_attention/infer/nsa_inference.py:77-150, with every position and length read from the
+ * caches' counters on the device.
+ *   q [batch, Hq, d], k, v [batch, Hkv, d]: the new token, before rotation; gate [batch, Hq, 3]; out like q.
+ *   caches and counters as in the functions above; ticket int32 [batch], zero before the first step (left at zero).
+ *   w_k, w_v [Hkv, kernel_size] pooling weights or NULL (average); bias_k [Hkv, d] (nsa_pool_bias / nsa_linear_bias) or NULL;
+ *   linear_taps: NULL for pooling; else the output of nsa_linear_decode_taps for this step.
+ *   strides[26]: q_b q_h | k_b k_h | v_b v_h | gate_b gate_h | out_b out_h | (kv, sequence, row, head) of the selected-block,
+ *   compressed, staging and sliding-window caches.
+ * Returns -2 for a group of more than 16 query heads, more than 64 selected 64-key tiles or head_dim other than 64 and 128. */
+int nsa_decode_step(const void* q, const void* k, const void* v, const void* gate, void* out, void* sparse_cache, int* sparse_len,
+                    void* compress_cache, int* compress_len, void* stage_cache, int* stage_len, void* sliding_cache,
+                    int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* bias_k, const float* linear_taps,
+                    const float* inv_freq, float attention_scaling, int batch, int num_q_heads, int num_kv_heads, int head_dim,
+                    int kernel_size, int kernel_stride, int block_size, int topk, int init_blocks, int local_blocks,
+                    int sparse_rows, int compress_rows, int sliding_rows, const long long* strides, float sm_scale, int dtype,
+                    void* stream);
+
+/* Linear compression of the windows the coming decode step completes: taps[tap][b][key, value][h][:] = row `tap` of the
+ * staged window (with the new token k, v appended) times its [d, d] slice of w_k / w_v [Hkv, kernel_size * d, d], for every
+ * sequence whose window the new token completes; other sequences' entries are left alone.  Reads the staging cache as it is
+ * before the step.  taps: kernel_size * batch * 2 * Hkv * d floats.
+ *   strides[8]: k_b k_h | v_b v_h | (kv, sequence, row, head) of the staging cache. */
+int nsa_linear_decode_taps(const void* k, const void* v, const void* w_k, const void* w_v, const void* stage_cache,
+                           const int* stage_len, float* taps, int batch, int num_kv_heads, int head_dim, int kernel_size,
+                           int kernel_stride, const long long* strides, int dtype, void* stream);
+
+/* bias[h, :] = concat_k(pe[h, k, :]) @ w[h], in the storage type: the term linear compression adds to every row. */
+int nsa_linear_bias(const void* pe, const void* w, void* bias, int num_heads, int head_dim, int kernel_size, int dtype,
+                    void* stream);
 
 #ifdef __cplusplus
 }

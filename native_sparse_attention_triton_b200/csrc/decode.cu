@@ -1,15 +1,17 @@
 // Single-token (decode) attention against dense KV caches [batch, cache_len, kv_heads, d].
 //
 //  * flash decode            : every cache row below seqlens[b]
-//  * top-k sparse decode     : the rows of the selected blocks below seqlens[b]
+//  * top-k sparse decode     : the rows of the selected blocks below seqlens[b] (decode_cluster.cu)
 //  * compressed decode       : every compressed row below compress_seqlens[b], plus block scores
 //                              and top-k block selection for the current token
 //
-// All three are bound by HBM: the cache rows are read once, through TMA, into per-warp
-// shared-memory tiles; the G query heads of a KV head form the rows of the mma tile so the rows
-// are shared by the whole group.  Long rows are split across warps/CTAs (split-KV); partial
-// (max, sum, output) triples go through a caller-provided scratch buffer and a combine kernel.
+// This file has the entry points and the split-KV kernel for large batches, where HBM is the bound: the cache rows are read
+// once, through TMA, into per-warp shared-memory tiles; the G query heads of a KV head form the rows of the mma tile so the
+// rows are shared by the whole group.  Long rows are split across warps/CTAs; partial (max, sum, output) triples go through a
+// caller-provided scratch buffer and are merged by the warp that finishes a pair last.  Smaller batches, bound by latency, run
+// on the cluster kernels of decode_cluster.cu.
 #include "attn_tile.cuh"
+#include "decode_cluster.h"
 #include "dispatch.h"
 #include "host_util.h"
 #include "nsa_b200.h"
@@ -23,14 +25,13 @@ constexpr int kMaxTilesPerDecodeQuery = 64;
 constexpr int kMaxDecodeSplits = 64;  // upper bound on the partial results combined per row
 constexpr int kDecodeWarps = 6;       // warps (= concurrent tasks) per CTA; each owns one K and one V tile buffer
 
-enum DecodeMode { kDecodeDense = 0, kDecodeSparse = 1, kDecodeCompressed = 2 };
+enum DecodeMode { kDecodeDense = 0, kDecodeCompressed = 2 };
 
 struct DecodeParams {
   const void* q;
   void* o;
-  const int* seqlens;      // dense / sparse: valid cache rows; compressed: sequence length including the current token
+  const int* seqlens;      // dense: valid cache rows; compressed: sequence length including the current token
   const int* cmp_seqlens;  // compressed: valid compressed rows
-  const int* topk_idx;     // sparse: selected blocks (input)
   int* topk_out_idx;       // compressed: selected blocks (output) or nullptr
   // scratch (caller memory): ctrl[0] = next task, ctrl[1 + b*Hkv + h] = splits of that pair finished so far
   int* ctrl;
@@ -39,7 +40,7 @@ struct DecodeParams {
   float* logits;           // compressed: [pairs][16][lc_pad] scaled base-2 logits (-inf where masked)
   long long q_sb, q_sh, o_sb, o_sh;
   long long t_sh, t_sb, t_sk;
-  int B, Hq, Hkv, G, T, block_size;
+  int B, Hq, Hkv, G, block_size;
   int S, tiles_per_split, total_tasks;
   int window, stride, topk_out, init_blocks, local_blocks, lc_pad, nb_pad;
   float scale2;
@@ -72,7 +73,6 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WARPS * 2 * TILE_BYTES);
   uint64_t* barK = bars + 2 * warp;
   uint64_t* barV = barK + 1;
-  int* tiles = reinterpret_cast<int*>(bars + 2 * WARPS) + warp * kMaxTilesPerDecodeQuery;
   if (lane == 0) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
@@ -106,40 +106,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     // ---- the pair's tiles and this split's share ----
     const int len = __ldg(p.seqlens + b);
     int ntiles, rows;  // rows: valid cache rows of this pair
-    if constexpr (MODE == kDecodeSparse) {
-      const int BS = p.block_size, nsub = BS / kKeyTile;
-      const int bq = len > 0 ? (len - 1) / BS : -1;
-      rows = len;
-      ntiles = 0;
-      const int* tptr = p.topk_idx + h * p.t_sh + (long long)b * p.t_sb;
-      __syncwarp();
-      for (int base = 0; base < p.T; base += 32) {
-        const int j = base + lane;
-        const int idx = (j < p.T) ? __ldg(tptr + j * p.t_sk) : -1;
-        const bool valid = idx >= 0 && idx <= bq;
-        const int cnt = valid ? min(nsub, (len - 1 - idx * BS) / kKeyTile + 1) : 0;
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int excl = incl - cnt;
-        for (int s = 0; s < cnt; ++s) {
-          const int pos = ntiles + excl + s;
-          if (pos < kMaxTilesPerDecodeQuery) tiles[pos] = idx * BS + s * kKeyTile;
-        }
-        ntiles += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (ntiles > kMaxTilesPerDecodeQuery) {
-        p.st.raise(kErrBadIndex);
-        ntiles = kMaxTilesPerDecodeQuery;
-      }
-      __syncwarp();
-    } else {
-      rows = (MODE == kDecodeCompressed) ? __ldg(p.cmp_seqlens + b) : len;
-      ntiles = (rows + kKeyTile - 1) / kKeyTile;
-    }
+    rows = (MODE == kDecodeCompressed) ? __ldg(p.cmp_seqlens + b) : len;
+    ntiles = (rows + kKeyTile - 1) / kKeyTile;
     const int s_eff = max(1, min(p.S, (ntiles + p.tiles_per_split - 1) / p.tiles_per_split));  // splits of this pair that have tiles
     if (split >= s_eff) continue;
     const int t_begin = min(ntiles, split * p.tiles_per_split);
@@ -154,7 +122,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       for (int pn = 0; pn < PANELS; ++pn) tma_load_4d(buf + pn * (kKeyTile * 128), tm, bar, pn * 64, h, kpos, b);
     };
     auto tile_at = [&](int i, int& kpos, int& limv) {
-      kpos = (MODE == kDecodeSparse) ? tiles[t_begin + i] : (t_begin + i) * kKeyTile;
+      kpos = (t_begin + i) * kKeyTile;
       limv = min(kKeyTile, rows - kpos);
     };
     float* lrow = (MODE == kDecodeCompressed) ? p.logits + (size_t)pair * 16 * p.lc_pad : nullptr;
@@ -373,7 +341,7 @@ static int launch_decode(const void* k, const void* v, const long long* kv_strid
     }
     if (mode == kDecodeCompressed) p.logits = f;
   }
-  const size_t smem = 1024 + WARPS * 2 * TILE_BYTES + WARPS * 2 * sizeof(uint64_t) + WARPS * kMaxTilesPerDecodeQuery * sizeof(int);
+  const size_t smem = 1024 + WARPS * 2 * TILE_BYTES + WARPS * 2 * sizeof(uint64_t);
   const int sms = num_sms();
   const int ctas_all = (p.total_tasks + WARPS - 1) / WARPS;
   const int grid = p.ctrl ? (ctas_all < sms ? ctas_all : sms) : ctas_all;  // persistent when tasks are handed out dynamically
@@ -386,7 +354,6 @@ static int launch_decode(const void* k, const void* v, const long long* kv_strid
   };
   switch (mode) {
     case kDecodeDense: return launch(decode_attn_kernel<T, D, kDecodeDense>, "decode_attn");
-    case kDecodeSparse: return launch(decode_attn_kernel<T, D, kDecodeSparse>, "decode_attn_sparse");
     default: return launch(decode_attn_kernel<T, D, kDecodeCompressed>, "decode_attn_compressed");
   }
 }
@@ -437,6 +404,23 @@ extern "C" long long nsa_compressed_decode_scratch_floats(int batch, int num_kv_
 }
 
 namespace nsa {
+// Which kernel: clusters (decode_cluster.cu) or the split-KV tasks of this file, which are handed out dynamically.  Measured on
+// ragged batches (rows of 1 to the cache's length, d = 128), clusters / tasks in us:
+//   dense       8 pairs x 8256: 13 / 34; 64 x 4096: 19 / 28; 128 x 8192: 55 / 53; 160 x 8192: 69 / 61; 192 x 8192: 78 / 71;
+//               304 x 8192: 112 / 112; 304 x 2000: 34 / 36; 608 x 8192: 198 / 206; 1024 x 2048: 95 / 107
+//   compressed  8 x 515: 9 / 23; 128 x 255: 11 / 17; 304 x 511: 21 / 25; 1024 x 127: 35 / 21
+// so tasks stay for dense rows of more than 4096 when the pairs are between one and two CTAs per SM (one long row per place and
+// nothing to follow it), and for compressed rows beyond three pairs per SM, where a CTA per pair mostly waits at its barriers.
+static bool dense_by_cluster(long long pairs, int cache_len) { return cache_len <= 4096 || pairs < 120 || pairs >= 288; }
+static bool compressed_by_cluster(long long pairs) { return pairs <= 444; }
+
+static DecodeOpArgs op_args(const void* q, const void* k, const void* v, void* o, const int* seqlens, int batch, int cache_len,
+                            int num_q_heads, int num_kv_heads, int head_dim, const long long* strides, float sm_scale, int dtype) {
+  DecodeOpArgs a{};
+  a.q = q; a.k = k; a.v = v; a.o = o; a.seqlens = seqlens; a.batch = batch; a.cache_len = cache_len; a.num_q_heads = num_q_heads;
+  a.num_kv_heads = num_kv_heads; a.head_dim = head_dim; a.strides = strides; a.sm_scale = sm_scale; a.dtype = dtype;
+  return a;
+}
 static void set_splits(DecodeParams& p, int num_splits, int max_tiles) {
   p.S = num_splits < 1 ? 1 : (num_splits > max_tiles ? max_tiles : num_splits);
   if (p.S > kMaxDecodeSplits) p.S = kMaxDecodeSplits;
@@ -454,10 +438,15 @@ extern "C" int nsa_flash_attn_decode(const void* q, const void* k, const void* v
   if (!seqlens) return kInvalid;
   int rc = decode_common_checks(q, k, v, o, strides, batch, cache_len, num_q_heads, num_kv_heads);
   if (rc) return rc;
+  if (dense_by_cluster((long long)batch * num_kv_heads, cache_len)) {
+    const DecodeOpArgs a = op_args(q, k, v, o, seqlens, batch, cache_len, num_q_heads, num_kv_heads, head_dim, strides, sm_scale, dtype);
+    rc = decode_cluster_dense(a, static_cast<cudaStream_t>(stream));
+    if (rc != kUnsupported) return rc;
+  }
   DecodeParams p{};
   p.q = q; p.o = o; p.seqlens = seqlens;
   p.q_sb = strides[0]; p.q_sh = strides[1]; p.o_sb = strides[8]; p.o_sh = strides[9];
-  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.T = 0; p.block_size = kKeyTile;
+  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.block_size = kKeyTile;
   set_splits(p, num_splits, (cache_len + kKeyTile - 1) / kKeyTile);
   const long long need = decode_scratch_floats((long long)batch * num_kv_heads, p.S, head_dim, 0);
   if (need > 0 && (!scratch || scratch_floats < need)) return kWorkspace;
@@ -479,19 +468,9 @@ extern "C" int nsa_topk_sparse_attn_decode(const void* q, const void* k, const v
   if (rc) return rc;
   if (block_size < kKeyTile || block_size % kKeyTile) return kUnsupported;
   if (topk <= 0 || (long long)topk * (block_size / kKeyTile) > kMaxTilesPerDecodeQuery) return kUnsupported;
-  DecodeParams p{};
-  p.q = q; p.o = o; p.seqlens = seqlens; p.topk_idx = topk_idx;
-  p.q_sb = strides[0]; p.q_sh = strides[1]; p.o_sb = strides[8]; p.o_sh = strides[9];
-  p.t_sh = strides[10]; p.t_sb = strides[11]; p.t_sk = strides[12];
-  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.T = topk; p.block_size = block_size;
-  set_splits(p, num_splits, topk * (block_size / kKeyTile));
-  const long long need = decode_scratch_floats((long long)batch * num_kv_heads, p.S, head_dim, 0);
-  if (need > 0 && (!scratch || scratch_floats < need)) return kWorkspace;
-  p.scale2 = sm_scale * kLog2e;
-  p.st.word = status_word();
-  const long long kvs[6] = {strides[2], strides[3], strides[4], strides[5], strides[6], strides[7]};
-  return NSA_DISPATCH_T_D(dtype, head_dim, launch_decode, k, v, kvs, cache_len, p, kDecodeSparse, need > 0 ? scratch : nullptr,
-                          static_cast<cudaStream_t>(stream));
+  DecodeOpArgs a = op_args(q, k, v, o, seqlens, batch, cache_len, num_q_heads, num_kv_heads, head_dim, strides, sm_scale, dtype);
+  a.topk_idx = topk_idx; a.topk = topk; a.block_size = block_size;
+  return decode_cluster_sparse(a, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nsa_compressed_attn_decode(const void* q, const void* k, const void* v, const int* seqlens,
@@ -506,11 +485,19 @@ extern "C" int nsa_compressed_attn_decode(const void* q, const void* k, const vo
   if (rc) return rc;
   if (kernel_size % kernel_stride || block_size % kernel_stride || kernel_stride < 1) return kInvalid;
   if (topk_idx && (topk < 1 || topk < init_blocks + local_blocks || max_seqlen < 1)) return kInvalid;
+  if (compressed_by_cluster((long long)batch * num_kv_heads)) {
+    DecodeOpArgs a = op_args(q, k, v, o, seqlens, batch, cache_len, num_q_heads, num_kv_heads, head_dim, strides, sm_scale, dtype);
+    a.cmp_seqlens = compress_seqlens; a.topk_out_idx = topk_idx; a.topk = topk; a.block_size = block_size; a.kernel_size = kernel_size;
+    a.kernel_stride = kernel_stride; a.init_blocks = init_blocks; a.local_blocks = local_blocks;
+    a.max_blocks = topk_idx ? (max_seqlen + block_size - 1) / block_size : 1;
+    rc = decode_cluster_compressed(a, static_cast<cudaStream_t>(stream));
+    if (rc != kUnsupported) return rc;
+  }
   DecodeParams p{};
   p.q = q; p.o = o; p.topk_out_idx = topk_idx; p.seqlens = seqlens; p.cmp_seqlens = compress_seqlens;
   p.q_sb = strides[0]; p.q_sh = strides[1]; p.o_sb = strides[8]; p.o_sh = strides[9];
   p.t_sh = strides[10]; p.t_sb = strides[11]; p.t_sk = strides[12];
-  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.T = 0; p.block_size = block_size;
+  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.block_size = block_size;
   p.window = kernel_size; p.stride = kernel_stride;
   const int max_blocks = topk_idx ? (max_seqlen + block_size - 1) / block_size : 1;
   p.topk_out = topk < max_blocks ? topk : max_blocks;
@@ -587,6 +574,9 @@ extern "C" int nsa_flash_attn_decode_static(const void* q, const void* k, const 
     while (splits > 1 && decode_scratch_floats(pairs, splits, head_dim, 0) > kStaticScratchFloats) --splits;
   const long long need = decode_scratch_floats(pairs, splits, head_dim, 0);
   if (need > kStaticScratchFloats) return kWorkspace;  // an explicit split count that does not fit: ask for fewer
+  if (dense_by_cluster(pairs, cache_len))  // that kernel uses no scratch
+    return nsa_flash_attn_decode(q, k, v, seqlens, o, nullptr, 0, splits, batch, cache_len, num_q_heads, num_kv_heads, head_dim, strides,
+                                 sm_scale, dtype, stream);
   float* scratch = nullptr;
   const int rc = static_scratch(&scratch);
   if (rc) return rc;

@@ -804,12 +804,11 @@ Tensor topk_sparse_attention_decode(const Tensor& q_in, const Tensor& k_in, cons
   if (L == 0) return at::zeros_like(q);
   Tensor o = empty_like_rows(q);
   Launch run(q);
-  const ScratchUse u = take_scratch((int)B, (int)Hkv, (int)D, (int)T * std::max(1, block_size / 64), q.device());
   const DecodeStrides st(q, k, v, o, &idx);
-  check_decode_rc(nsa_topk_sparse_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(idx), ptr<int>(seqlens), ptr(o), u.p, u.n, u.splits, (int)B,
-                                              (int)L, (int)Hq, (int)Hkv, (int)D, (int)T, block_size, st.s,
-                                              (float)sm_scale.value_or(default_scale(D)), dtype_code(q), run.stream),
-                  "nsa_topk_sparse_attn_decode", u);
+  check_rc(nsa_topk_sparse_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(idx), ptr<int>(seqlens), ptr(o), nullptr, 0, 1, (int)B, (int)L, (int)Hq,
+                                       (int)Hkv, (int)D, (int)T, block_size, st.s, (float)sm_scale.value_or(default_scale(D)), dtype_code(q),
+                                       run.stream),
+           "nsa_topk_sparse_attn_decode");
   return o;
 }
 
@@ -839,6 +838,154 @@ std::tuple<Tensor, Tensor> compressed_attention_decode(const Tensor& q_in, const
   return {o, idx};
 }
 
+// ------------------------------------------------------------------------------------------------------- inference step
+// The position embedding folded through a compression's weights, [H, d]: it changes only when the parameters do, so it is
+// computed once per (weight, pe) pair and version and not once per decode step.
+struct BiasEntry {
+  c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> w, pe;
+  uint32_t w_version = 0, pe_version = 0;
+  Tensor bias;
+  BiasEntry(const Tensor& w_, const Tensor& pe_) : w(w_.getIntrusivePtr()), pe(pe_.getIntrusivePtr()) {}
+};
+std::mutex g_bias_mu;
+std::unordered_map<uint64_t, BiasEntry> g_bias;
+constexpr size_t kBiasEntries = 256;
+
+Tensor position_bias(const Tensor& w, const Tensor& pe, int mode, void* stream) {
+  uint32_t wv = 0, pv = 0;
+  const bool counted = (!w.defined() || version_of(w, wv)) && version_of(pe, pv);
+  const uint64_t key = reinterpret_cast<uint64_t>(w.unsafeGetTensorImpl()) * 0x9E3779B97F4A7C15ull ^
+                       reinterpret_cast<uint64_t>(pe.unsafeGetTensorImpl()) ^ (uint64_t)mode;
+  if (counted) {
+    std::lock_guard<std::mutex> lk(g_bias_mu);
+    auto it = g_bias.find(key);
+    if (it != g_bias.end() && it->second.w_version == wv && it->second.pe_version == pv &&
+        it->second.w._unsafe_get_target() == w.unsafeGetTensorImpl() && it->second.pe._unsafe_get_target() == pe.unsafeGetTensorImpl())
+      return it->second.bias;
+  }
+  const int64_t H = pe.size(0), ks = pe.size(1), D = pe.size(2);
+  Tensor bias = empty({H, D}, pe.scalar_type(), pe.device());
+  const Tensor pec = pe.contiguous(), wc = w.defined() ? w.contiguous() : Tensor();
+  if (mode == kLinear)
+    check_rc(nsa_linear_bias(ptr(pec), ptr(wc), ptr(bias), (int)H, (int)D, (int)ks, dtype_code(pe), stream), "nsa_linear_bias");
+  else
+    check_rc(nsa_pool_bias(ptr(pec), wc.defined() ? ptr(wc) : nullptr, ptr(bias), (int)H, (int)D, (int)ks, dtype_code(pe), stream),
+             "nsa_pool_bias");
+  if (counted && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+    std::lock_guard<std::mutex> lk(g_bias_mu);
+    if (g_bias.size() >= kBiasEntries) g_bias.clear();
+    BiasEntry e(w, pe);
+    e.w_version = wv;
+    e.pe_version = pv;
+    e.bias = bias;
+    g_bias.insert_or_assign(key, std::move(e));
+  }
+  return bias;
+}
+
+// The caches of a layer as NSACache holds them: [2, batch, rows, heads, d] tensors and int32 counters.
+struct CacheRefs {
+  Tensor sel, sel_len, cmp, cmp_len, stage, stage_len, win, win_len, ticket;
+};
+CacheRefs cache_refs(const std::vector<Tensor>& c) {
+  NSA_ASSERT(c.size() == 9, "nine cache tensors");
+  return CacheRefs{c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8]};
+}
+
+// One decode step of nsa_infer in one launch (two for linear compression).  Returns nothing when the shapes are not the fused
+// kernel's, before anything has been launched; the caller then takes the operators one by one.
+std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& gate_in,
+                                  const std::vector<Tensor>& caches, const OptTensor& w_k, const OptTensor& w_v, const OptTensor& pe,
+                                  int mode, const Tensor& inv_freq, double rope_scaling, int ks, int st, int block_size, int topk,
+                                  int init_blocks, int local_blocks, const OptTensor& out) {
+  const CacheRefs c = cache_refs(caches);
+  require_cuda(q_in, k_in, v_in, gate_in, inv_freq);
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView guard;
+  const int64_t B = k_in.size(0), Hkv = k_in.size(1), D = k_in.size(2), Hq = q_in.size(1);
+  NSA_ASSERT(q_in.size(0) == B && k_in.sizes() == v_in.sizes() && B <= c.sel.size(1), "one row per sequence, no more than the cache holds");
+  NSA_ASSERT(Hkv == c.sel.size(3) && D == c.sel.size(4) && q_in.size(2) == D && Hq % Hkv == 0, "heads and head_dim must be the cache's");
+  NSA_ASSERT(is_16bit(q_in) && q_in.scalar_type() == k_in.scalar_type() && q_in.scalar_type() == v_in.scalar_type() &&
+                 q_in.scalar_type() == gate_in.scalar_type() && q_in.scalar_type() == c.sel.scalar_type(),
+             "query, key, value, gate and caches must have the same 16-bit dtype");
+  NSA_ASSERT(gate_in.size(0) == B && gate_in.size(1) == Hq && gate_in.size(2) == 3, "gate must be [batch, query heads, 3]");
+  if ((D != 64 && D != 128) || Hq / Hkv > 16 || inv_freq.size(0) != D / 2) return std::nullopt;
+  const Tensor q = inner_contiguous(q_in), k = inner_contiguous(k_in), v = inner_contiguous(v_in), gate = gate_in.contiguous();
+  Launch run(q);
+  Tensor bias, wk, wv;
+  if (w_k) wk = w_k->contiguous();
+  if (w_v) wv = w_v->contiguous();
+  if (pe) bias = position_bias(w_k.value_or(Tensor()), *pe, mode, run.stream);
+  Tensor o = out ? *out : empty_like_rows(q);
+  Tensor taps;
+  if (mode == kLinear) {
+    taps = empty({ks, B, 2, Hkv, D}, at::kFloat, q.device());
+    const long long s[8] = {k.stride(0), k.stride(1), v.stride(0), v.stride(1), c.stage.stride(0), c.stage.stride(1), c.stage.stride(2),
+                            c.stage.stride(3)};
+    check_rc(nsa_linear_decode_taps(ptr(k), ptr(v), ptr(wk), ptr(wv), ptr(c.stage), ptr<int>(c.stage_len), ptr<float>(taps), (int)B, (int)Hkv,
+                                    (int)D, ks, st, s, dtype_code(q), run.stream),
+             "nsa_linear_decode_taps");
+  }
+  QkvStrides s;
+  long long strides[26];
+  s.add(q).add(k).add(v).add(gate).add(o);
+  std::copy(s.s, s.s + 10, strides);
+  int n = 10;
+  for (const Tensor* t : {&c.sel, &c.cmp, &c.stage, &c.win})
+    for (int i = 0; i < 4; ++i) strides[n++] = t->stride(i);
+  const auto p = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
+  const int rc = nsa_decode_step(ptr(q), ptr(k), ptr(v), ptr(gate), ptr(o), ptr(c.sel), ptr<int>(c.sel_len), ptr(c.cmp), ptr<int>(c.cmp_len),
+                                 ptr(c.stage), ptr<int>(c.stage_len), ptr(c.win), ptr<int>(c.win_len), ptr<int>(c.ticket), p(wk), p(wv),
+                                 p(bias), static_cast<float*>(p(taps)), ptr<float>(inv_freq), (float)rope_scaling, (int)B, (int)Hq, (int)Hkv,
+                                 (int)D, ks, st, block_size, topk, init_blocks, local_blocks, (int)c.sel.size(2), (int)c.cmp.size(2),
+                                 (int)c.win.size(2), strides, (float)default_scale(D), dtype_code(q), run.stream);
+  if (rc == -2) return std::nullopt;
+  check_rc(rc, "nsa_decode_step");
+  return o;
+}
+
+void cache_fill(const Tensor& cache, const Tensor& len, const Tensor& key, const Tensor& value, const Tensor& cu, int mode, int window, int hop,
+                void* stream) {
+  const long long s[8] = {cache.stride(0), cache.stride(1), cache.stride(2), cache.stride(3), key.stride(0), key.stride(1), value.stride(0),
+                          value.stride(1)};
+  check_rc(nsa_kv_cache_fill(ptr(cache), ptr<int>(len), ptr(key), ptr(value), ptr<int>(cu), mode, window, hop, (int)key.size(0),
+                             (int)cu.size(0) - 1, (int)cache.size(2), (int)key.size(1), (int)key.size(2), s, stream),
+           "nsa_kv_cache_fill");
+}
+
+// The prefill of nsa_infer with the library's own compression and rotary embedding.  The lengths come from the host copy of
+// cu_seqlens, so nothing waits for the device once that tensor has been seen.
+Tensor prefill(const Tensor& cu, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& gate, const std::vector<Tensor>& caches,
+               const OptTensor& w_k, const OptTensor& w_v, const OptTensor& pe, int mode_k, int mode_v, const Tensor& inv_freq,
+               double rope_scaling, int ks, int st, int block_size, int topk, int init_blocks, int local_blocks, int window) {
+  const CacheRefs c = cache_refs(caches);
+  at::NoGradGuard no_grad;
+  require_cuda(q_in, k_in, v_in, gate, cu);
+  NSA_ASSERT(k_in.sizes() == v_in.sizes() && k_in.scalar_type() == c.sel.scalar_type() && v_in.scalar_type() == c.sel.scalar_type(),
+             "key and value must have the same shape and the cache's dtype");
+  NSA_ASSERT(k_in.size(1) == c.sel.size(3) && k_in.size(2) == c.sel.size(4), "heads and head_dim must be the cache's");
+  NSA_ASSERT(is_int32(cu) && cu.size(0) - 1 <= c.sel.size(1), "cu_seqlens must be int32, with no more sequences than the cache holds");
+  const Tensor k = inner_contiguous(k_in), v = inner_contiguous(v_in);
+  const auto info = seq_info(cu);
+  const Layout l = layout_of(*info, ks, st, k.device());
+  Launch run(k);
+  cache_fill(c.stage, c.stage_len, k, v, cu, 2, ks, st, run.stream);
+  auto [ck, cu_k] = compress(k, w_k, cu, ks, st, pe, mode_k);
+  const Tensor cv = std::get<0>(compress(v, w_v, cu, ks, st, std::nullopt, mode_v));
+  const Tensor q = rope(q_in, inv_freq, cu, 0, 1, rope_scaling);
+  ck = rope(ck, inv_freq, cu_k, 0, st, rope_scaling);
+  const Tensor kr = rope(k, inv_freq, cu, 0, 1, rope_scaling);
+  cache_fill(c.cmp, c.cmp_len, ck, cv, cu_k, 0, 0, 0, run.stream);
+  cache_fill(c.sel, c.sel_len, kr, v, cu, 0, 0, 0, run.stream);
+  cache_fill(c.win, c.win_len, kr, v, cu, 1, window, 0, run.stream);
+  auto [o_cmp, idx] = compressed_attention(q, ck, cv, ks, st, block_size, topk, cu, cu_k, info->longest, l.longest, std::nullopt, init_blocks,
+                                           local_blocks);
+  NSA_ASSERT(idx.has_value(), "topk must be positive");
+  const Tensor o_sel = topk_sparse_attention(q, kr, v, *idx, block_size, cu, std::nullopt);
+  const Tensor o_win = sliding_window_attention(q, kr, v, cu, info->longest, window, std::nullopt);
+  return gate_combine(gate, o_cmp, o_sel, o_win);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_nsa_host, m) {
@@ -853,4 +1000,6 @@ PYBIND11_MODULE(_nsa_host, m) {
   m.def("flash_attention_decode", &flash_attention_decode);
   m.def("topk_sparse_attention_decode", &topk_sparse_attention_decode);
   m.def("compressed_attention_decode", &compressed_attention_decode);
+  m.def("decode_step", &decode_step);
+  m.def("prefill", &prefill);
 }

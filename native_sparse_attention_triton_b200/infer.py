@@ -82,77 +82,29 @@ def _device_rope_of(rope):
     return mine
 
 
+_MODES = {ops.linear_compress: 0, ops.weightedpool_compress: 1, ops.avgpool_compress: 2}   # as csrc/host/torch_ops.cpp counts them
+
+
 def _compress_staged(cache: NSACache, batch: int, which: int, func: Callable, weight, pe):
-    """One compressed row per sequence from the staging buffers [batch * kernel_size, heads, d] (the reference runs its
-    compress function over them with an arange cu_seqlens, infer/inference_func.py:56-87).  The library's own compress
-    functions go through the C interface directly (no host copy of cu_seqlens); any other callable is called as given."""
+    """One compressed row per sequence from the staging buffers [batch * kernel_size, heads, d], the way the reference does it:
+    the compress function run over them with an arange cu_seqlens (infer/inference_func.py:56-87)."""
     x = cache.before_compress_kv_cache[which, :batch].view(batch * cache.kernel_size, cache.num_kv_heads, cache.head_dim)
-    cu, ycu = cache.stage_cu_seqlens[:batch + 1], cache.stage_out_cu_seqlens[:batch + 1]
-    mode = {ops.linear_compress: "linear", ops.weightedpool_compress: "weighted", ops.avgpool_compress: "avg"}.get(func)
-    if mode is None:
-        return func(x, weight, cu, cache.kernel_size, cache.kernel_stride, pe)[0]
-    y = torch.empty(batch, cache.num_kv_heads, cache.head_dim, dtype=x.dtype, device=x.device)
-    bias = torch.empty(cache.num_kv_heads, cache.head_dim, dtype=x.dtype, device=x.device) if pe is not None else None
-    w = weight.contiguous() if weight is not None else None
-    pec = pe.contiguous() if pe is not None else None
-    lib = _lib.lib()
-    torch.cuda.set_device(x.device)
-    if mode == "linear":
-        rc = lib.nsa_linear_compress_fwd(ptr(x), ptr(w), ptr(pec), ptr(cu), ptr(ycu), ptr(y), ptr(bias), x.shape[0], batch, batch, 1,
-                                         cache.num_kv_heads, cache.head_dim, cache.kernel_size, cache.kernel_stride, x.stride(0),
-                                         x.stride(1), dtype_code(x), stream_ptr(x.device))
-        _lib.check(rc, "nsa_linear_compress_fwd")
-    else:
-        rc = lib.nsa_pool_compress_fwd(ptr(x), ptr(w), ptr(pec), ptr(cu), ptr(ycu), ptr(y), ptr(bias), x.shape[0], batch, batch, 1,
-                                       cache.num_kv_heads, cache.head_dim, cache.kernel_size, cache.kernel_stride, x.stride(0),
-                                       x.stride(1), dtype_code(x), stream_ptr(x.device))
-        _lib.check(rc, "nsa_pool_compress_fwd")
-    return y
+    return func(x, weight, cache.stage_cu(batch), cache.kernel_size, cache.kernel_stride, pe)[0]
 
 
-_pool_bias_cache = {}   # (id(w), id(pe)) -> (weakref w, weakref pe, versions, bias tensor)
-
-
-def _pool_bias(weight, pe):
-    """The position embedding folded through the pooling weights, [H, d]: it changes only when the parameters do, so it is
-    computed once per (weight, pe) pair and version, not once per decode step."""
-    import weakref
-
-    key = (id(weight), id(pe))
-    versions = (weight._version if weight is not None else -1, pe._version)
-    hit = _pool_bias_cache.get(key)
-    if hit is not None and hit[0]() is weight and hit[1]() is pe and hit[2] == versions:
-        return hit[3]
-    bias = torch.empty(pe.shape[0], pe.shape[2], dtype=pe.dtype, device=pe.device)
-    w = weight.contiguous() if weight is not None else None
-    rc = _lib.lib().nsa_pool_bias(ptr(pe.contiguous()), ptr(w), ptr(bias), pe.shape[0], pe.shape[2], pe.shape[1], dtype_code(pe),
-                                  stream_ptr(pe.device))
-    _lib.check(rc, "nsa_pool_bias")
-    if len(_pool_bias_cache) > 256:
-        _pool_bias_cache.clear()
-    _pool_bias_cache[key] = (weakref.ref(weight) if weight is not None else (lambda: None), weakref.ref(pe), versions, bias)
-    return bias
-
-
-_POOL_FUNCS = (ops.weightedpool_compress, ops.avgpool_compress)
-
-
-def _compress_staged_pair(cache: NSACache, batch: int, funcs, weights, pe):
-    """Both staging buffers pooled in one launch (nsa_pool_compress_decode_pair): one compressed key row and one compressed
-    value row per sequence; the key's position-embedding bias comes from the cache above."""
-    stage = cache.before_compress_kv_cache
-    xk, xv = stage[0, :batch], stage[1, :batch]            # [batch, kernel_size, H, d]
-    wk = weights[0].contiguous() if funcs[0] is ops.weightedpool_compress else None
-    wv = weights[1].contiguous() if funcs[1] is ops.weightedpool_compress else None
-    bias_k = _pool_bias(wk, pe) if pe is not None else None
-    yk = torch.empty(batch, cache.num_kv_heads, cache.head_dim, dtype=stage.dtype, device=stage.device)
-    yv = torch.empty_like(yk)
-    torch.cuda.set_device(stage.device)
-    rc = _lib.lib().nsa_pool_compress_decode_pair(ptr(xk), ptr(xv), ptr(wk), ptr(wv), ptr(bias_k), None, ptr(yk), ptr(yv), batch,
-                                                  cache.num_kv_heads, cache.head_dim, cache.kernel_size, xk.stride(0), xk.stride(1),
-                                                  xk.stride(2), dtype_code(stage), stream_ptr(stage.device))
-    _lib.check(rc, "nsa_pool_compress_decode_pair")
-    return yk, yv
+def _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weight, compress_func, pe, block_size, topk, init_blocks,
+                       local_blocks, out=None):
+    """The decode step as one launch (two with linear compression); None where it needs one of the caller's own functions, a
+    mixture of linear and pooling compression, or a shape the fused kernel does not have."""
+    mode_k, mode_v = _MODES.get(compress_func[0]), _MODES.get(compress_func[1])
+    if mode_k is None or mode_v is None or (mode_k == 0) != (mode_v == 0):
+        return None
+    mine = rope if type(rope) is RotaryEmbedding else _device_rope_of(rope)
+    if mine is None:
+        return None
+    return _lib.host().decode_step(query, key, value, gate_value, cache._tensors(), compress_weight[0] if mode_k != 2 else None,
+                                   compress_weight[1] if mode_v != 2 else None, pe, mode_k, mine.inv_freq, mine.attention_scaling,
+                                   cache.kernel_size, cache.kernel_stride, block_size, topk, init_blocks, local_blocks, out)
 
 
 @torch.no_grad()
@@ -168,6 +120,12 @@ def nsa_infer(cu_seqlens: torch.Tensor, step: int, query: torch.Tensor, key: tor
     batch = cu_seqlens.shape[0] - 1
     if step == 0:
         cache.reset()
+        mode_k, mode_v = _MODES.get(compress_func[0]), _MODES.get(compress_func[1])
+        if mode_k is not None and mode_v is not None and type(rope) is RotaryEmbedding:
+            return _lib.host().prefill(cu_seqlens, query, key, value, gate_value, cache._tensors(), compress_weight[0] if mode_k != 2 else None,
+                                       compress_weight[1] if mode_v != 2 else None, intra_block_pe, mode_k, mode_v, rope.inv_freq,
+                                       rope.attention_scaling, kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks,
+                                       window_size)
         cache.prepare_compress(cu_seqlens, 0, key, value)
         compress_key, compress_cu_seqlens = compress_func[0](key, compress_weight[0], cu_seqlens, kernel_size, kernel_stride,
                                                              intra_block_pe)
@@ -187,12 +145,13 @@ def nsa_infer(cu_seqlens: torch.Tensor, step: int, query: torch.Tensor, key: tor
         return ops.gate_combine(gate_value, o_cmp, o_sel, o_win)
 
     # ---- decode: nothing below reads a device value on the host ----
+    out = _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weight, compress_func, intra_block_pe, block_size, topk,
+                             init_blocks, local_blocks)
+    if out is not None:
+        return out
     cache.prepare_compress(cu_seqlens, step, key, value)
-    if compress_func[0] in _POOL_FUNCS and compress_func[1] in _POOL_FUNCS:
-        compress_key, compress_value = _compress_staged_pair(cache, batch, compress_func, compress_weight, intra_block_pe)
-    else:
-        compress_key = _compress_staged(cache, batch, 0, compress_func[0], compress_weight[0], intra_block_pe)
-        compress_value = _compress_staged(cache, batch, 1, compress_func[1], compress_weight[1], None)
+    compress_key = _compress_staged(cache, batch, 0, compress_func[0], compress_weight[0], intra_block_pe)
+    compress_value = _compress_staged(cache, batch, 1, compress_func[1], compress_weight[1], None)
     fast_rope = rope if hasattr(rope, "decode_at3") else _device_rope_of(rope)
     if fast_rope is not None:
         # the new token's index is the number of tokens cached so far; the compressed token's, the compressed count
@@ -241,28 +200,40 @@ def _side_stream(device):
 
 
 class DecodeGraph:
-    """One decode step of ``nsa_infer`` captured in a CUDA graph: ``graph(query, key, value, gate_value)`` copies the four
-    inputs into fixed buffers, replays the launches and returns the (fixed) output tensor.  Capture after prefill; the
-    cache object, weights and shapes are fixed at capture."""
+    """Decode steps of ``nsa_infer`` with everything fixed but the inputs' values: ``graph(query, key, value, gate_value)`` runs
+    one step and returns the (fixed) output tensor.  Made after prefill; the cache object, weights and shapes are fixed here.
+
+    A step that is one launch is launched as such, straight from the caller's tensors: a CUDA graph around it would add the copy
+    of four inputs into fixed buffers (5 us) and save nothing.  A step that needs the separate kernels is captured in a CUDA
+    graph and replayed."""
 
     def __init__(self, cu_seqlens, query, key, value, gate_value, **nsa_args):
         self.inputs = [t.clone() for t in (query, key, value, gate_value)]
         self.args = dict(nsa_args)
         self.cu_seqlens = cu_seqlens
+        self.output = torch.empty_like(query, memory_format=torch.contiguous_format)
+        self.graph = None
         cache: NSACache = nsa_args["cache"]
-        # The warm-up step below (which also performs every lazy one-time initialisation of the library outside the capture)
-        # and the capture itself both advance the cache: snapshot its state and restore it afterwards.
+        # The trial step below and the capture advance the cache: its state is put back afterwards.
         state = [t.clone() for t in self._state(cache)]
         side = torch.cuda.Stream(device=query.device)
         side.wait_stream(torch.cuda.current_stream(query.device))
         with torch.cuda.stream(side):
-            nsa_infer(cu_seqlens, 1, *self.inputs, **self.args)
+            fused = self._step(self.inputs) is not None
+            if not fused:
+                nsa_infer(cu_seqlens, 1, *self.inputs, **self.args)   # every lazy one-time initialisation, outside the capture
         torch.cuda.current_stream(query.device).wait_stream(side)
-        self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph, stream=side):   # the warm-up stream: its decode scratch is reused by the capture
-            self.output = nsa_infer(cu_seqlens, 1, *self.inputs, **self.args)
+        if not fused:
+            self.graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(self.graph, stream=side):   # the warm-up stream: its decode scratch is reused by the capture
+                self.output = nsa_infer(cu_seqlens, 1, *self.inputs, **self.args)
         for dst, src in zip(self._state(cache), state):
             dst.copy_(src)
+
+    def _step(self, inputs):
+        a = self.args
+        return _fused_decode_step(a["cache"], *inputs, a["rope"], a["compress_weight"], a["compress_func"], a["intra_block_pe"],
+                                  a["block_size"], a["topk"], a["init_blocks"], a["local_blocks"], self.output)
 
     @staticmethod
     def _state(cache):
@@ -273,10 +244,17 @@ class DecodeGraph:
 
     def __call__(self, query, key, value, gate_value):
         srcs = [query, key, value, gate_value]
-        if all(s.dtype == d.dtype and s.device == d.device and s.shape == d.shape for s, d in zip(srcs, self.inputs)):
+        same = all(s.dtype == d.dtype and s.device == d.device and s.shape == d.shape for s, d in zip(srcs, self.inputs))
+        if same and self.graph is None:
+            self._step(srcs)
+            return self.output
+        if same:
             torch._foreach_copy_(self.inputs, srcs)   # one launch for the four inputs
         else:
             for dst, src in zip(self.inputs, srcs):
                 dst.copy_(src)
-        self.graph.replay()
+        if self.graph is None:
+            self._step(self.inputs)
+        else:
+            self.graph.replay()
         return self.output

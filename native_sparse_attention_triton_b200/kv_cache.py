@@ -32,23 +32,44 @@ class NSACache:
         self.device = torch.device(device)
         self.max_comp_length = (max_length - kernel_size) // kernel_stride + 1
 
-        def alloc(rows):
-            cache = torch.zeros(2, max_batch_size, rows, num_kv_heads, head_dim, dtype=dtype, device=self.device)
-            return cache, torch.zeros(max_batch_size, dtype=torch.int32, device=self.device)
-
-        self.sparse_kv_cache, self.sparse_kv_len = alloc(max_length)
-        self.compress_kv_cache, self.compress_kv_len = alloc(self.max_comp_length)
-        self.before_compress_kv_cache, self.before_compress_kv_len = alloc(kernel_size)
-        self.sliding_kv_cache, self.sliding_kv_len = alloc(window_size)
+        # caches and counters in one allocation, so that reset() is one memset
+        rows = (max_length, self.max_comp_length, kernel_size, window_size)
+        sizes = [2 * max_batch_size * r * num_kv_heads * head_dim * 2 for r in rows] + [max_batch_size * 4] * 5
+        starts = [0]
+        for n in sizes:
+            starts.append(starts[-1] + (n + 255) // 256 * 256)
+        self._storage = torch.zeros(starts[-1], dtype=torch.uint8, device=self.device)
+        part = lambda i, dt: self._storage[starts[i]:starts[i] + sizes[i]].view(dt)
+        caches = [part(i, dtype).view(2, max_batch_size, r, num_kv_heads, head_dim) for i, r in enumerate(rows)]
+        lens = [part(4 + i, torch.int32) for i in range(5)]
+        self.sparse_kv_cache, self.sparse_kv_len = caches[0], lens[0]
+        self.compress_kv_cache, self.compress_kv_len = caches[1], lens[1]
+        self.before_compress_kv_cache, self.before_compress_kv_len = caches[2], lens[2]
+        self.sliding_kv_cache, self.sliding_kv_len = caches[3], lens[3]
+        self._step_ticket = lens[4]   # zero between decode steps
+        self._allocated = self._tensors()
         self.device = self.sparse_kv_cache.device  # with its index
-        # cu_seqlens of the staging buffers seen as a varlen batch (every sequence kernel_size rows, one compressed row)
-        self.stage_cu_seqlens = torch.arange(max_batch_size + 1, dtype=torch.int32, device=self.device) * kernel_size
-        self.stage_out_cu_seqlens = torch.arange(max_batch_size + 1, dtype=torch.int32, device=self.device)
+        self._stage_cu = {}
+
+    def stage_cu(self, batch: int) -> torch.Tensor:
+        """cu_seqlens of the staging buffers seen as a varlen batch: `batch` sequences of kernel_size rows.  One tensor per batch
+        size, kept, so that its host copy is made once."""
+        if batch not in self._stage_cu:
+            self._stage_cu[batch] = torch.arange(batch + 1, dtype=torch.int32, device=self.device) * self.kernel_size
+        return self._stage_cu[batch]
+
+    def _tensors(self):
+        """What the fused prefill and decode step take, in the order csrc/host/torch_ops.cpp expects."""
+        return [self.sparse_kv_cache, self.sparse_kv_len, self.compress_kv_cache, self.compress_kv_len, self.before_compress_kv_cache,
+                self.before_compress_kv_len, self.sliding_kv_cache, self.sliding_kv_len, self._step_ticket]
 
     def reset(self):
-        for t in (self.compress_kv_cache, self.compress_kv_len, self.before_compress_kv_cache, self.before_compress_kv_len,
-                  self.sparse_kv_cache, self.sparse_kv_len, self.sliding_kv_cache, self.sliding_kv_len):
-            t.zero_()
+        now = self._tensors()
+        if all(a is b for a, b in zip(now, self._allocated)):
+            self._storage.zero_()
+        else:   # a caller has put tensors of its own in place of some
+            for t in now:
+                t.zero_()
 
     # ------------------------------------------------------------------ helpers
     def _fill(self, cache, length, key, value, cu_seqlens, mode, window, hop):
