@@ -14,7 +14,7 @@
 //               dimension, so no per-head dK/dV copies exist.  Partial results of the CTAs that
 //               share a key tile are added with fp32 red.global into a zeroed accumulator and
 //               converted to the storage type at the end.
-#include <cstdlib>
+#include <algorithm>
 #include <utility>
 
 #include "attn_tile.cuh"
@@ -251,7 +251,6 @@ sparse_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 struct IndexParams {
   const int* topk_idx;
   const int* cu_seqlens;
-  const int* cu_blocks;  // [B+1] prefix sum of ceil(len / block_size)
   // A bin is (kv head, token window, global block): bin = (head * NW + window) * TB + block.  Binning the tokens of a
   // block's list by window, with the window as the slower index, makes CTAs that run at the same time gather Q/dO rows
   // of the same few thousand tokens, so the rows are read from DRAM once and then served by L2.
@@ -268,58 +267,54 @@ struct IndexParams {
   Status st;
 };
 
-// cu_blocks[b] = sum over the sequences before b of ceil(length / block_size): one CTA, 256 sequences per round
-__global__ void __launch_bounds__(256) block_prefix_kernel(const int* __restrict__ cu, int batch, int block_size, int* __restrict__ cu_blocks) {
-  __shared__ int warp_sum[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int carry = 0;
-  if (threadIdx.x == 0) cu_blocks[0] = 0;
-  for (int base = 0; base < batch; base += 256) {
-    const int b = base + threadIdx.x;
-    int v = b < batch ? (__ldg(cu + b + 1) - __ldg(cu + b) + block_size - 1) / block_size : 0;
+// A block of a sequence is numbered block_base(b) + its index; the bases leave a gap of at most one number per sequence and need
+// no prefix sum over the batch (attn_bwd.h).
+//
+// One thread per (head, token); the lanes of a warp are 32 consecutive tokens, many of which chose the same blocks (every token
+// its first block, 64 neighbours their own): lanes that hit the same bin share one atomic.  Without that the counter of a
+// sequence's first block serialised the kernel (7097 tokens x 8 heads: 60 us per pass, 57 us for 65 536 tokens x 4).
+template <bool FILL>
+__device__ __forceinline__ void index_scatter(const IndexParams& p, long long gid) {
+  const bool live = gid < (long long)p.Hkv * p.N;
+  const int h = live ? (int)(gid / p.N) : 0, n = live ? (int)(gid % p.N) : 0;
+  const int b = find_sequence(p.cu_seqlens, p.B, n);
+  const int s0 = __ldg(p.cu_seqlens + b);
+  const int bq = (n - s0) / p.block_size;
+  const int blk0 = block_base(s0, b, p.block_size);
+  const int x0 = (h * p.NW + n / p.W) * p.TB + blk0;
+  const int* tptr = p.topk_idx + h * p.t_sh + (long long)n * p.t_sn;
+  const int lane = threadIdx.x & 31;
+  constexpr int U = 4;
+  for (int j0 = 0; j0 < p.T; j0 += U) {
+    int x[U], old[U];
+    unsigned same[U];
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, v, off);
-      if (lane >= off) v += t;
+    for (int u = 0; u < U; ++u) {
+      const int idx = (live && j0 + u < p.T) ? __ldg(tptr + (j0 + u) * p.t_sk) : -1;
+      x[u] = (idx >= 0 && idx <= bq) ? x0 + idx : -1;
     }
-    if (lane == 31) warp_sum[warp] = v;
-    __syncthreads();
-    int before = carry, total = 0;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      if (w < warp) before += warp_sum[w];
-      total += warp_sum[w];
+    for (int u = 0; u < U; ++u) same[u] = __match_any_sync(0xffffffffu, x[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      old[u] = 0;
+      if (x[u] >= 0 && lane == __ffs(same[u]) - 1) old[u] = atomicAdd((FILL ? p.cursor : p.count) + x[u], __popc(same[u]));
     }
-    if (b < batch) cu_blocks[b + 1] = before + v;
-    carry += total;
-    __syncthreads();
+    if (FILL) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int first = __shfl_sync(0xffffffffu, old[u], __ffs(same[u]) - 1);
+        if (x[u] < 0) continue;
+        const long long dst = (long long)__ldg(p.offsets + x[u]) + first + __popc(same[u] & ((1u << lane) - 1u));
+        if (dst < p.capacity) p.list[dst] = n; else p.st.raise(kErrBadIndex);
+      }
+    }
   }
 }
 
 template <bool FILL>
-__global__ void index_scatter_kernel(IndexParams p) {
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)p.Hkv * p.N;
-  if (gid >= total) return;
-  const int h = gid / p.N, n = gid % p.N;
-  const int b = find_sequence(p.cu_seqlens, p.B, n);
-  const int t = n - __ldg(p.cu_seqlens + b);
-  const int bq = t / p.block_size;
-  const int blk0 = __ldg(p.cu_blocks + b);
-  const int* tptr = p.topk_idx + h * p.t_sh + (long long)n * p.t_sn;
-  for (int j = 0; j < p.T; ++j) {
-    const int idx = __ldg(tptr + j * p.t_sk);
-    if (idx < 0 || idx > bq) continue;
-    const int x = (h * p.NW + n / p.W) * p.TB + blk0 + idx;
-    if (blk0 + idx >= p.TB) { p.st.raise(kErrBadIndex); continue; }
-    if (!FILL) {
-      atomicAdd(p.count + x, 1);
-    } else {
-      const int pos = atomicAdd(p.cursor + x, 1);
-      const long long dst = (long long)p.offsets[x] + pos;
-      if (dst < p.capacity) p.list[dst] = n; else p.st.raise(kErrBadIndex);
-    }
-  }
+__global__ void __launch_bounds__(128) index_scatter_kernel(IndexParams p) {
+  index_scatter<FILL>(p, (long long)blockIdx.x * 128 + threadIdx.x);
 }
 
 // single CTA: exclusive scans of count and of the per-bin item count, 1024 bins per round (warp shuffles, then the 32 warp
@@ -405,10 +400,10 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     const int x = __ldg(p.item_bin + item);  // item_base[x] <= item < item_base[x + 1]
     h = x / (p.NW * p.TB);
     const int gb = x % p.TB;
-    const int b = find_sequence(p.cu_blocks, p.B, gb);
+    const int b = find_block_sequence(p.cu_q, p.B, gb, p.block_size);
     qs = __ldg(p.cu_q + b);
     Lq = __ldg(p.cu_q + b + 1) - qs;
-    const int blk = gb - __ldg(p.cu_blocks + b);
+    const int blk = gb - block_base(qs, b, p.block_size);
     kpos = blk * p.block_size + blockIdx.y * kKeyTile;
     krow0 = qs + kpos;
     kvalid = min(kKeyTile, Lq - kpos);
@@ -596,40 +591,71 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
 // kConvertUnroll float4 pieces, 256 pieces apart, and issues all of its loads before the first store: one 16-byte load in
 // flight per thread left HBM two thirds busy.
 constexpr int kConvertUnroll = 4;
+struct ConvertSegment {
+  const float* src;    // [rows, H, D] contiguous
+  void* dst;
+  long long d_sn, d_sh;
+  long long total;     // float4 pieces
+  int H;
+  unsigned first_block;
+};
+struct ConvertParams {
+  ConvertSegment seg[3];
+  int n, D;
+};
 template <typename T>
-__global__ void __launch_bounds__(256) convert_rows_kernel(const float* __restrict__ src, void* dst, long long rows, int Hkv, int D,
-                                                           long long d_sn, long long d_sh) {
-  const int CH = D / 4;
-  const long long total = rows * Hkv * CH;
-  const long long base = (long long)blockIdx.x * (256 * kConvertUnroll) + threadIdx.x;
+__global__ void __launch_bounds__(256) convert_rows_kernel(const __grid_constant__ ConvertParams p) {
+  int si = 0;
+  while (si + 1 < p.n && blockIdx.x >= p.seg[si + 1].first_block) ++si;
+  const ConvertSegment& g = p.seg[si];
+  const int CH = p.D / 4;
+  const long long base = (long long)(blockIdx.x - g.first_block) * (256 * kConvertUnroll) + threadIdx.x;
   float4 v[kConvertUnroll];
 #pragma unroll
   for (int u = 0; u < kConvertUnroll; ++u) {
     const long long idx = base + u * 256;
-    v[u] = idx < total ? __ldcs(reinterpret_cast<const float4*>(src) + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[u] = idx < g.total ? __ldcs(reinterpret_cast<const float4*>(g.src) + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
   for (int u = 0; u < kConvertUnroll; ++u) {
     const long long idx = base + u * 256;
-    if (idx >= total) continue;
+    if (idx >= g.total) continue;
     const int c = idx % CH;
-    const int h = (idx / CH) % Hkv;
-    const long long n = idx / ((long long)CH * Hkv);
+    const int h = (idx / CH) % g.H;
+    const long long n = idx / ((long long)CH * g.H);
     uint2 out;
     out.x = DT<T>::pack(v[u].x, v[u].y);
     out.y = DT<T>::pack(v[u].z, v[u].w);
-    *reinterpret_cast<uint2*>(static_cast<T*>(dst) + n * d_sn + (long long)h * d_sh + c * 4) = out;
+    *reinterpret_cast<uint2*>(static_cast<T*>(g.dst) + n * g.d_sn + (long long)h * g.d_sh + c * 4) = out;
   }
 }
+
+// One launch for all accumulators of a pass.
+struct Converter {
+  ConvertParams p{};
+  unsigned blocks = 0;
+  void add(const float* src, void* dst, long long rows, int H, int D, long long d_sn, long long d_sh) {
+    ConvertSegment& g = p.seg[p.n++];
+    g.src = src; g.dst = dst; g.d_sn = d_sn; g.d_sh = d_sh; g.H = H; g.total = rows * H * (D / 4); g.first_block = blocks;
+    blocks += (unsigned)((g.total + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll));
+    p.D = D;
+  }
+  template <typename T>
+  int run(cudaStream_t stream) {
+    LaunchScope ls_("convert_rows", stream);
+    convert_rows_kernel<T><<<blocks, 256, 0, stream>>>(p);
+    return cuda_rc(cudaGetLastError());
+  }
+};
 
 // (lse, delta) per (token, query head) for the backward passes: delta = sum_d o * dO in fp32.  16 lanes per row of
 // D 16-bit elements (16 bytes each for D = 128); one pass over o and dO.
 template <typename T, int D>
-__global__ void row_stats_kernel(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
-                                 float2* __restrict__ ld, long long rows, int Hq, long long o_sn, long long o_sh, long long do_sn,
-                                 long long do_sh) {
+__device__ __forceinline__ void row_stats(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
+                                          float2* __restrict__ ld, long long rows, int Hq, long long o_sn, long long o_sh, long long do_sn,
+                                          long long do_sh, long long thread) {
   constexpr int EPL = D / 16;  // elements per lane
-  const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  const long long row = thread >> 4;
   const int sub = threadIdx.x & 15;
   float acc = 0.f;
   if (row < rows) {
@@ -654,6 +680,17 @@ __global__ void row_stats_kernel(const T* __restrict__ o, const T* __restrict__ 
 #pragma unroll
   for (int off = 8; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (row < rows && sub == 0) ld[row] = make_float2(__ldg(lse + row), acc);
+}
+
+// The histogram of the inverted index and the row statistics in one launch: they depend on nothing the other makes.
+template <typename T, int D>
+__global__ void __launch_bounds__(128) index_count_stats_kernel(IndexParams ip, unsigned count_blocks, SparseBwdParams p) {
+  if (blockIdx.x < count_blocks) {
+    index_scatter<false>(ip, (long long)blockIdx.x * 128 + threadIdx.x);
+    return;
+  }
+  row_stats<T, D>(static_cast<const T*>(p.o), static_cast<const T*>(p.dout), p.lse, p.ld, (long long)p.N * p.Hq, p.Hq, p.o_sn, p.o_sh,
+                  p.do_sn, p.do_sh, (long long)(blockIdx.x - count_blocks) * 128 + threadIdx.x);
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -685,7 +722,19 @@ static int launch_dkdv(const void* q, const void* dout, const void* k, const voi
 // ------------------------------------------------------------------------------------------------
 // host drivers
 // ------------------------------------------------------------------------------------------------
-struct DenseBwdWs { float2* ld; float* dk32; float* dv32; };
+// Tokens per CTA of the dense dK/dV pass.  Long chunks amortise a key tile's loads and the adding of its sums; a small problem is
+// cut finer, down to four row tiles per CTA, until there are two CTAs for every SM (777 tokens x 2 heads, window 512: 48 CTAs of up
+// to 32 row tiles, 61 us, at 256 tokens).
+static int dense_chunk(int max_q, int max_k, int heads, int G, int D, int left) {
+  int chunk = 256;
+  while (chunk < 1024 && chunk * 16 < max_q) chunk <<= 1;
+  const int key_tile = D == 128 ? 128 : kKeyTile, least = D == 128 ? std::max(32, 4 * (128 / G)) : 32;
+  const long long tiles = (long long)((max_k + key_tile - 1) / key_tile) * heads;
+  // tokens that see a key tile: all of them, half of them on average under the causal mask, a window
+  const int span = left >= 0 ? std::min(max_q, left + key_tile) : (max_q + 1) / 2;
+  while (chunk > least && tiles * ((span + chunk - 1) / chunk) < 2 * 148) chunk >>= 1;
+  return chunk;
+}
 
 static size_t dense_ws_bytes(int total_q, int total_k, int Hq, int Hkv, int D) {
   return align_up((size_t)total_q * Hq * sizeof(float2), 256) + 2 * align_up((size_t)total_k * Hkv * D * sizeof(float), 256);
@@ -724,11 +773,10 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   }
   DkdvParams d;
   d.ld = ld; d.dk32 = dk32; d.dv32 = dv32; d.cu_q = cu_q; d.cu_k = cu_k;
-  d.cu_blocks = nullptr; d.offsets = nullptr; d.item_base = nullptr; d.item_bin = nullptr; d.item_counter = nullptr; d.list = nullptr;
+  d.offsets = nullptr; d.item_base = nullptr; d.item_bin = nullptr; d.item_counter = nullptr; d.list = nullptr;
   d.B = batch; d.Hq = Hq; d.Hkv = Hkv; d.G = G; d.TB = 0; d.NW = 1; d.block_size = kKeyTile;
-  int chunk = 256;
-  while (chunk < 1024 && chunk * 16 < max_q) chunk <<= 1;
-  d.chunk = chunk;
+  d.chunk = dense_chunk(max_q, max_k, batch * Hkv, G, D, left);
+  const int chunk = d.chunk;
   d.window = window; d.stride = stride; d.causal = causal; d.left = left;
   d.scale2 = p.scale2; d.sm_scale = sm_scale; d.st = p.st;
   const long long ds[8] = {S[0], S[1], S[2], S[3], S[4], S[5], S[8], S[9]};
@@ -740,13 +788,20 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
     rc = launch_dkdv<T, D, false>(q, dout, k, v, ds, total_q, total_k, grid, d, stream);
   }
   if (rc) return rc;
-  const long long n4 = (long long)total_k * Hkv * (D / 4);
-  { LaunchScope ls_("convert_dk", stream); convert_rows_kernel<T><<<(unsigned)((n4 + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll)), 256, 0, stream>>>(dk32, dk, total_k, Hkv, D, S[12], S[13]); }
-  { LaunchScope ls_("convert_dv", stream); convert_rows_kernel<T><<<(unsigned)((n4 + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll)), 256, 0, stream>>>(dv32, dv, total_k, Hkv, D, S[14], S[15]); }
-  return cuda_rc(cudaGetLastError());
+  Converter cv;
+  cv.add(dk32, dk, total_k, Hkv, D, S[12], S[13]);
+  cv.add(dv32, dv, total_k, Hkv, D, S[14], S[15]);
+  return cv.run<T>(stream);
 }
 
-constexpr int kSparseChunk = 512;  // tokens of one block's list handled by one CTA
+// Tokens of one block's list per work item.  512 where there is work enough (an item carries its block's K/V tile and the read-out
+// of its dK/dV sums); fewer where that would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads
+// x top-8 are 30 items of up to 64 tiles (148 us) at 512, 244 of 8 (see the figures in sparse_dkdv_tc.cu) at 64.
+static int sparse_chunk(int N, int Hkv, int topk) {
+  int chunk = 512;
+  while (chunk > 64 && (long long)Hkv * N * topk / chunk < 4 * 148) chunk >>= 1;
+  return chunk;
+}
 
 // Token windows of the inverted index: as many tokens as keep the Q and dO rows of one KV-head group (G heads) within
 // about half of the L2 cache, a power of two, at least 1024.  Returns (tokens per window, windows).
@@ -765,24 +820,28 @@ static size_t sparse_ws_bytes(int N, int batch, int Hq, int Hkv, int D, int topk
   const size_t x = (size_t)Hkv * sparse_windows(N, Hq / Hkv, D).second * TB + 1;
   return align_up((size_t)N * Hq * sizeof(float2), 256) + 2 * align_up((size_t)N * Hkv * D * sizeof(float), 256) +
          4 * align_up(x * sizeof(int), 256) + align_up((size_t)Hkv * N * topk * sizeof(int), 256) +
-         align_up(((size_t)batch + 1) * sizeof(int), 256) +
-         align_up(((size_t)Hkv * N * topk / kSparseChunk + x) * sizeof(int), 256) +
+         align_up(((size_t)Hkv * N * topk / sparse_chunk(N, Hkv, topk) + x) * sizeof(int), 256) +
          (sparse_fused_dq(Hq / Hkv, D) ? align_up((size_t)N * Hq * D * sizeof(float), 256) : 0);
 }
 
 template <typename T, int D>
 static int run_sparse_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
-                          const int* topk_idx, const int* cu, const int* cu_blocks, void* dq, void* dk, void* dv, void* ws,
+                          const int* topk_idx, const int* cu, void* dq, void* dk, void* dv, void* ws,
                           int N, int batch, int Hq, int Hkv, int topk, int block_size, const long long* S, float sm_scale,
                           cudaStream_t stream) {
   // S: q_n q_h k_n k_h v_n v_h o_n o_h do_n do_h dq_n dq_h dk_n dk_h dv_n dv_h idx_h idx_n idx_k
   const int G = Hq / Hkv;
   const int TB = N / block_size + batch;
   const auto [W, NW] = sparse_windows(N, G, D);
+  const int chunk = sparse_chunk(N, Hkv, topk);
   const size_t X = (size_t)Hkv * NW * TB + 1;
   uint8_t* w = static_cast<uint8_t*>(ws);
   float2* ld = reinterpret_cast<float2*>(w);
   w += align_up((size_t)N * Hq * sizeof(float2), 256);
+  const bool fused = sparse_fused_dq(G, D);  // dQ comes out of the tcgen05 dK/dV pass; otherwise the per-token dQ kernel runs
+  uint8_t* const zero_begin = w;
+  float* dq32 = fused ? reinterpret_cast<float*>(w) : nullptr;
+  if (fused) w += align_up((size_t)N * Hq * D * sizeof(float), 256);
   float* dk32 = reinterpret_cast<float*>(w);
   w += align_up((size_t)N * Hkv * D * sizeof(float), 256);
   float* dv32 = reinterpret_cast<float*>(w);
@@ -798,23 +857,10 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   int* list = reinterpret_cast<int*>(w);
   w += align_up((size_t)Hkv * N * topk * sizeof(int), 256);
   int* item_bin = reinterpret_cast<int*>(w);   // one entry per possible work item (the grid's upper bound below)
-  w += align_up(((size_t)Hkv * N * topk / kSparseChunk + X) * sizeof(int), 256);
-  if (!cu_blocks) {  // the caller left the prefix sum of blocks to this call
-    int* own = reinterpret_cast<int*>(w);
-    LaunchScope ls_("block_prefix", stream);
-    block_prefix_kernel<<<1, 256, 0, stream>>>(cu, batch, block_size, own);
-    cu_blocks = own;
-  }
-  w += align_up(((size_t)batch + 1) * sizeof(int), 256);
-  const bool fused = sparse_fused_dq(G, D);  // dQ comes out of the tcgen05 dK/dV pass; otherwise the per-token dQ kernel runs
-  float* dq32 = fused ? reinterpret_cast<float*>(w) : nullptr;
-  // dk32, dv32, count, cursor are contiguous: one memset
-  cudaError_t e = cudaMemsetAsync(dk32, 0, reinterpret_cast<uint8_t*>(offsets) - reinterpret_cast<uint8_t*>(dk32), stream);
+  w += align_up(((size_t)Hkv * N * topk / chunk + X) * sizeof(int), 256);
+  // dq32, dk32, dv32, count, cursor are contiguous: one memset
+  cudaError_t e = cudaMemsetAsync(zero_begin, 0, reinterpret_cast<uint8_t*>(offsets) - zero_begin, stream);
   if (e != cudaSuccess) return cuda_rc(e);
-  if (fused) {
-    e = cudaMemsetAsync(dq32, 0, (size_t)N * Hq * D * sizeof(float), stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-  }
 
   SparseBwdParams p;
   p.q = q; p.o = o; p.dout = dout; p.lse = lse; p.ld = ld; p.dq = dq; p.topk_idx = topk_idx; p.cu_seqlens = cu;
@@ -825,25 +871,26 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   p.st.word = status_word();
 
   IndexParams ip;
-  ip.topk_idx = topk_idx; ip.cu_seqlens = cu; ip.cu_blocks = cu_blocks; ip.count = count; ip.cursor = cursor;
+  ip.topk_idx = topk_idx; ip.cu_seqlens = cu; ip.count = count; ip.cursor = cursor;
   ip.offsets = offsets; ip.item_base = item_base; ip.item_bin = item_bin; ip.list = list;
   ip.t_sh = S[16]; ip.t_sn = S[17]; ip.t_sk = S[18];
-  ip.N = N; ip.B = batch; ip.Hkv = Hkv; ip.T = topk; ip.block_size = block_size; ip.TB = TB; ip.chunk = kSparseChunk; ip.W = W; ip.NW = NW;
+  ip.N = N; ip.B = batch; ip.Hkv = Hkv; ip.T = topk; ip.block_size = block_size; ip.TB = TB; ip.chunk = chunk; ip.W = W; ip.NW = NW;
   ip.capacity = (long long)Hkv * N * topk;
   ip.st = p.st;
   const long long hn = (long long)Hkv * N;
-  { LaunchScope ls_("index_count", stream); index_scatter_kernel<false><<<(unsigned)((hn + 255) / 256), 256, 0, stream>>>(ip); }
-  { LaunchScope ls_("index_scan", stream); index_scan_kernel<<<1, 1024, 0, stream>>>(ip); }
-  { LaunchScope ls_("index_fill", stream); index_scatter_kernel<true><<<(unsigned)((hn + 255) / 256), 256, 0, stream>>>(ip); }
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_rc(e);
+  const unsigned scatter_blocks = (unsigned)((hn + 127) / 128);
   if (fused) {
-    const long long rows = (long long)N * Hq;
-    LaunchScope ls_("row_stats", stream);
-    row_stats_kernel<T, D><<<(unsigned)((rows * 16 + 255) / 256), 256, 0, stream>>>(
-        static_cast<const T*>(o), static_cast<const T*>(dout), lse, ld, rows, Hq, S[6], S[7], S[8], S[9]);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_rc(e);
-  } else
-  {
+    const unsigned stat_blocks = (unsigned)(((long long)N * Hq * 16 + 127) / 128);
+    LaunchScope ls_("index_count_stats", stream);
+    index_count_stats_kernel<T, D><<<scatter_blocks + stat_blocks, 128, 0, stream>>>(ip, scatter_blocks, p);
+  } else {
+    LaunchScope ls_("index_count", stream);
+    index_scatter_kernel<false><<<scatter_blocks, 128, 0, stream>>>(ip);
+  }
+  { LaunchScope ls_("index_scan", stream); index_scan_kernel<<<1, 1024, 0, stream>>>(ip); }
+  { LaunchScope ls_("index_fill", stream); index_scatter_kernel<true><<<scatter_blocks, 128, 0, stream>>>(ip); }
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_rc(e);
+  if (!fused) {
     // one K buffer and as many warps as shared memory holds: measured 11.7 ms with 6 warps, 10.2 ms with 7, 12.0 ms with
     // 4 warps and two K buffers (64 K tokens) -- the kernel is bound by latency, and warps are what hides it
     constexpr int KBUFS = 1;
@@ -864,14 +911,14 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   }
   DkdvParams d;
   d.ld = ld; d.dk32 = dk32; d.dv32 = dv32; d.dq32 = dq32; d.cu_q = cu; d.cu_k = cu;
-  d.cu_blocks = cu_blocks; d.offsets = offsets; d.item_base = item_base; d.item_bin = item_bin; d.list = list;
+  d.offsets = offsets; d.item_base = item_base; d.item_bin = item_bin; d.list = list;
   d.item_counter = cursor + (X - 1);   // the spare last word of the zeroed cursor array
-  d.B = batch; d.Hq = Hq; d.Hkv = Hkv; d.G = G; d.TB = TB; d.NW = NW; d.chunk = kSparseChunk; d.block_size = block_size;
+  d.B = batch; d.Hq = Hq; d.Hkv = Hkv; d.G = G; d.TB = TB; d.NW = NW; d.chunk = chunk; d.block_size = block_size;
   d.window = 1; d.stride = 1; d.causal = 1; d.left = -1;
   d.scale2 = p.scale2; d.sm_scale = sm_scale; d.st = p.st;
   const long long ds[8] = {S[0], S[1], S[2], S[3], S[4], S[5], S[8], S[9]};
   // upper bound on work items: every selection in a full chunk, plus one partial chunk per (head, block)
-  const long long max_items = ((long long)Hkv * N * topk) / kSparseChunk + (long long)Hkv * NW * TB;
+  const long long max_items = ((long long)Hkv * N * topk) / chunk + (long long)Hkv * NW * TB;
   dim3 grid((unsigned)max_items, block_size / kKeyTile, 1);
   int rc;
   if constexpr (D == 128) {
@@ -881,15 +928,11 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
     rc = launch_dkdv<T, D, true>(q, dout, k, v, ds, N, N, grid, d, stream);
   }
   if (rc) return rc;
-  if (fused) {
-    const long long q4 = (long long)N * Hq * (D / 4);
-    LaunchScope ls_("convert_dq", stream);
-    convert_rows_kernel<T><<<(unsigned)((q4 + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll)), 256, 0, stream>>>(dq32, dq, N, Hq, D, S[10], S[11]);
-  }
-  const long long n4 = (long long)N * Hkv * (D / 4);
-  { LaunchScope ls_("convert_dk", stream); convert_rows_kernel<T><<<(unsigned)((n4 + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll)), 256, 0, stream>>>(dk32, dk, N, Hkv, D, S[12], S[13]); }
-  { LaunchScope ls_("convert_dv", stream); convert_rows_kernel<T><<<(unsigned)((n4 + 256 * kConvertUnroll - 1) / (256 * kConvertUnroll)), 256, 0, stream>>>(dv32, dv, N, Hkv, D, S[14], S[15]); }
-  return cuda_rc(cudaGetLastError());
+  Converter cv;
+  if (fused) cv.add(dq32, dq, N, Hq, D, S[10], S[11]);
+  cv.add(dk32, dk, N, Hkv, D, S[12], S[13]);
+  cv.add(dv32, dv, N, Hkv, D, S[14], S[15]);
+  return cv.run<T>(stream);
 }
 
 }  // namespace nsa
@@ -966,7 +1009,7 @@ extern "C" int nsa_topk_sparse_attn_bwd(const void* q, const void* k, const void
     if (strides[i] % 8) return kInvalid;
   if (workspace_bytes < (long long)sparse_ws_bytes(total_len, batch, num_q_heads, num_kv_heads, head_dim, topk, block_size))
     return kWorkspace;
-  return NSA_DISPATCH_T_D(dtype, head_dim, run_sparse_bwd, q, k, v, o, dout, lse, topk_idx, cu_seqlens, cu_seqblocks, dq, dk, dv,
+  return NSA_DISPATCH_T_D(dtype, head_dim, run_sparse_bwd, q, k, v, o, dout, lse, topk_idx, cu_seqlens, dq, dk, dv,
                           workspace, total_len, batch, num_q_heads, num_kv_heads, topk, block_size, strides, sm_scale,
                           static_cast<cudaStream_t>(stream));
 }

@@ -7,6 +7,20 @@
 
 namespace nsa {
 
+// Numbers of the selection blocks over a varlen batch: block i of sequence b is block_base(cu[b], b) + i.  floor(cu / size) + b
+// leaves room for ceil(length / size) blocks per sequence, at most one number in excess, without a prefix sum over the batch;
+// all numbers are below floor(total / size) + batch.
+__device__ __forceinline__ int block_base(int cu_b, int b, int block_size) { return cu_b / block_size + b; }
+// the sequence that block number gb belongs to
+__device__ __forceinline__ int find_block_sequence(const int* __restrict__ cu, int nseq, int gb, int block_size) {
+  int lo = 0, hi = nseq;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (block_base(__ldg(cu + mid), mid, block_size) <= gb) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 struct DkdvParams {
   const float2* ld;    // [Nq, Hq]
   float* dk32;         // [Nk, Hkv, D] fp32 accumulators (zeroed)
@@ -15,7 +29,6 @@ struct DkdvParams {
   const int* cu_q;
   const int* cu_k;      // dense: compressed cu; sparse: same as cu_q
   // sparse
-  const int* cu_blocks;
   const int* offsets;
   const int* item_base;
   const int* item_bin;   // [items] bin of every work item

@@ -19,49 +19,82 @@
 
 namespace nsa {
 
-// dbias[h, n] = sum_m dy[m, h, n]   (fp32).  One CTA of 256 threads per (head, 8 columns): a thread walks the rows
-// m = tid, tid + 256, ... with one 16-byte load per row; fixed-order reduction (deterministic).
+// dbias[c] = sum_m dy[m, c] over the M rows of H * D columns (fp32), in a fixed order (deterministic).  A cluster of eight CTAs
+// takes 32 columns, an eighth of the rows each; a thread sums every 64th row of its CTA's eighth with eight 16-byte loads in
+// flight, the CTA's 64 partial sums are added in shared memory and rank 0 adds the eight CTAs'. 
+constexpr int kColsumCluster = 8;
 template <typename T>
-__global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, int M, int H, int D) {
-  __shared__ float red[8][8];
-  const int h = blockIdx.x, n0 = blockIdx.y * 8;
+__global__ void __cluster_dims__(kColsumCluster, 1, 1) __launch_bounds__(256)
+colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, int M, int C) {
+  __shared__ float red[64][33];
+  __shared__ float sum[kColsumCluster][32];   // rank 0's: one row per CTA of the cluster
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  const int c4 = threadIdx.x & 3, rl = threadIdx.x >> 2;
+  const int col = blockIdx.y * 32 + c4 * 8;
+  const int per = (M + kColsumCluster - 1) / kColsumCluster;
+  const int m_end = min(M, (int)(rank + 1) * per);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int m = threadIdx.x; m < M; m += 256) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(dy + ((size_t)m * H + h) * D + n0));
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+  for (int m = rank * per + rl; m < m_end; m += 512) {
+    uint4 v[8];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = DT<T>::unpack(u[e]);
-      acc[2 * e] += f.x;
-      acc[2 * e + 1] += f.y;
+    for (int u = 0; u < 8; ++u)
+      v[u] = m + 64 * u < m_end ? __ldg(reinterpret_cast<const uint4*>(dy + (size_t)(m + 64 * u) * C + col)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = DT<T>::unpack(w[e]);
+        acc[2 * e] += f.x;
+        acc[2 * e + 1] += f.y;
+      }
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[threadIdx.x >> 5][j] = acc[j];
+  for (int e = 0; e < 8; ++e) red[rl][c4 * 8 + e] = acc[e];
   __syncthreads();
-  if (threadIdx.x < 8) {
-    float sum = 0.f;
+  if (threadIdx.x < 32) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int r = 0; r < 64; ++r) s += red[r][threadIdx.x];
+    uint32_t dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"(smem_u32(&sum[rank][threadIdx.x])));
+    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(dst), "f"(s) : "memory");
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (rank == 0 && threadIdx.x < 32) {
+    float s = 0.f;
 #pragma unroll
-    for (int wp = 0; wp < 8; ++wp) sum += red[wp][threadIdx.x];
-    dbias[h * D + n0 + threadIdx.x] = sum;
+    for (int r = 0; r < kColsumCluster; ++r) s += sum[r][threadIdx.x];
+    dbias[blockIdx.y * 32 + threadIdx.x] = s;
   }
 }
 
-// dpe[h, r] = sum_n dbias[h, n] * W[h, r, n]
 template <typename T>
-__global__ void linear_dpe_kernel(const float* __restrict__ dbias, const T* __restrict__ w, T* __restrict__ dpe, int H, int R, int D) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)H * R) return;
-  const int h = idx / R;
-  const T* wr = w + (size_t)idx * D;
+static void launch_colsum(const void* dy, float* dbias, int M, int H, int D, cudaStream_t stream) {
+  LaunchScope ls_("colsum", stream);
+  colsum_kernel<T><<<dim3(kColsumCluster, H * D / 32), 256, 0, stream>>>(static_cast<const T*>(dy), dbias, M, H * D);
+}
+
+// dpe[h, r] = sum_n dbias[h, n] * W[h, r, n]: D / 8 lanes per row of W, 16 bytes each
+template <typename T, int D>
+__global__ void __launch_bounds__(256) linear_dpe_kernel(const float* __restrict__ dbias, const T* __restrict__ w, T* __restrict__ dpe, int H, int R) {
+  constexpr int CH = D / 8;
+  const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) / CH;
+  const int c = threadIdx.x % CH;
+  const bool live = row < (long long)H * R;
   float acc = 0.f;
-  for (int n = 0; n < D; ++n) acc += dbias[h * D + n] * DT<T>::to_float(wr[n]);
-  dpe[idx] = DT<T>::from_float(acc);
+  if (live) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(w + (size_t)row * D + c * 8));
+    const float4 b0 = __ldg(reinterpret_cast<const float4*>(dbias + (row / R) * D + c * 8)), b1 = __ldg(reinterpret_cast<const float4*>(dbias + (row / R) * D + c * 8) + 1);
+    const float2 f0 = DT<T>::unpack(v.x), f1 = DT<T>::unpack(v.y), f2 = DT<T>::unpack(v.z), f3 = DT<T>::unpack(v.w);
+    acc = b0.x * f0.x + b0.y * f0.y + b0.z * f1.x + b0.w * f1.y + b1.x * f2.x + b1.y * f2.y + b1.z * f3.x + b1.w * f3.y;
+  }
+#pragma unroll
+  for (int off = CH / 2; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (live && c == 0) dpe[row] = DT<T>::from_float(acc);
 }
 
 struct LinBwdParams {
@@ -346,11 +379,11 @@ __global__ void __launch_bounds__(256) pool_dw_finish_kernel(PoolBwdParams p, co
 template <typename T, int D>
 static int run_linear_bwd(LinBwdParams p, void* dpe, float* dbias, int total_y, int max_len, cudaStream_t stream) {
   if (p.pe) {
-    { LaunchScope ls_("colsum", stream); colsum_kernel<T><<<dim3(p.H, D / 8), 256, 0, stream>>>(static_cast<const T*>(p.dy), dbias, total_y, p.H, D); }
+    launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
     p.dbias = dbias;
-    const long long hr = (long long)p.H * p.ks * D;
-    { LaunchScope ls_("linear_dpe", stream); linear_dpe_kernel<T><<<(unsigned)((hr + 255) / 256), 256, 0, stream>>>(dbias, static_cast<const T*>(p.w),
-                                                                          static_cast<T*>(dpe), p.H, p.ks * D, D); }
+    const long long lanes = (long long)p.H * p.ks * D * (D / 8);
+    LaunchScope ls_("linear_dpe", stream);
+    linear_dpe_kernel<T, D><<<(unsigned)((lanes + 255) / 256), 256, 0, stream>>>(dbias, static_cast<const T*>(p.w), static_cast<T*>(dpe), p.H, p.ks * D);
   }
   {
     const size_t smem = 1024 + 4 * 64 * D * 2;
@@ -374,7 +407,7 @@ template <typename T, int D>
 static int run_pool_bwd(PoolBwdParams p, float* dbias, float* partial, long long partial_floats, int total_y, int max_seqlen,
                         int dtype, cudaStream_t stream) {
   if (p.pe) {
-    { LaunchScope ls_("colsum", stream); colsum_kernel<T><<<dim3(p.H, D / 8), 256, 0, stream>>>(static_cast<const T*>(p.dy), dbias, total_y, p.H, D); }
+    launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
     p.dbias = dbias;
   }
   // long inputs: one streaming pass writes dx and (weighted pooling) the partial rows of dw

@@ -143,10 +143,10 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     const int base = ld_i32_here(p.item_base + x), off0 = ld_i32_here(p.offsets + x), off1 = ld_i32_here(p.offsets + x + 1);
     it.h = x / (p.NW * p.TB);
     const int gb = x % p.TB;
-    const int b = find_sequence(p.cu_blocks, p.B, gb);
+    const int b = find_block_sequence(p.cu_q, p.B, gb, p.block_size);
     it.qs = ld_i32_here(p.cu_q + b);
     const int Lq = ld_i32_here(p.cu_q + b + 1) - it.qs;
-    const int blk = gb - ld_i32_here(p.cu_blocks + b);
+    const int blk = gb - block_base(it.qs, b, p.block_size);
     it.kpos = blk * p.block_size + ysub * KT;
     it.krow0 = it.qs + it.kpos;
     it.kvalid = min(KT, Lq - it.kpos);
