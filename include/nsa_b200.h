@@ -45,6 +45,13 @@ int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const 
                              int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
                              const long long* strides, float sm_scale, int dtype, void* stream);
 
+/* The same with an upper bound on the sequence lengths (max_seqlen; nsa_topk_sparse_attn_fwd assumes total_len), which spares
+ * launches and empty CTAs for batches of short sequences. */
+int nsa_topk_sparse_attn_fwd_bounded(const void* q, const void* k, const void* v, const int* topk_idx,
+                                     const int* cu_seqlens, void* o, float* lse, int total_len, int batch, int max_seqlen,
+                                     int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
+                                     const long long* strides, float sm_scale, int dtype, void* stream);
+
 /* Forward of dense varlen GQA attention with the strided-causal mask
  *     query at in-sequence position t sees key i  iff  t >= i*stride + window - 1   (causal != 0)
  * window = kernel_size, stride = kernel_stride: attention over compressed keys, replaces
@@ -208,7 +215,7 @@ long long nsa_topk_sparse_attn_bwd_workspace(int total_len, int batch, int num_q
  * Replaces _topk_sparse_attention_bwd: backward_sum_o_do, count_query, reorder_topk_idx (argsort + 4 host
  * syncs), backward_dkdv with its [G, N, Hkv, d] buffers and .sum(0), backward_dq,
  * native_sparse_attention/ops/triton/topk_sparse_attention.py:176-477,480-825,912-1109.
- *   cu_seqblocks int32 [batch+1]: prefix sum of ceil(seqlen / block_size), or NULL: computed by this call.
+ *   cu_seqblocks is not used (NULL will do): blocks are numbered from cu_seqlens alone.
  *   strides[19] = the 16 of nsa_varlen_attn_bwd followed by {idx_h, idx_n, idx_k}. */
 int nsa_topk_sparse_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
                              const float* lse, const int* topk_idx, const int* cu_seqlens,

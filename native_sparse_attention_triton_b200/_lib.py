@@ -27,6 +27,7 @@ _SIGNATURES = {
     "nsa_profile_enable": [_I],
     "nsa_profile_collect": [ctypes.c_char_p, _I],
     "nsa_topk_sparse_attn_fwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P],
+    "nsa_topk_sparse_attn_fwd_bounded": [_P, _P, _P, _P, _P, _P, _P] + [_I] * 8 + [_P, _F, _I, _P],
     "nsa_varlen_attn_fwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P],
     "nsa_window_attn_fwd": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P],
     "nsa_compressed_attn_topk": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _F,

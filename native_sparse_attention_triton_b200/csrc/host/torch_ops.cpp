@@ -166,6 +166,17 @@ std::shared_ptr<SeqInfo> seq_info(const Tensor& cu) {
   return info;
 }
 
+// The longest sequence where that is known without a synchronisation, else the bound `total`.
+int longest_if_known(const Tensor& cu, int64_t total) {
+  uint32_t version = 0;
+  if (version_of(cu, version)) {
+    std::lock_guard<std::mutex> lk(g_seq_mu);
+    auto it = g_seq.find(cu.unsafeGetTensorImpl());
+    if (it != g_seq.end() && it->second->version == version) return it->second->longest;
+  }
+  return (int)total;
+}
+
 Layout layout_of(SeqInfo& info, int ks, int st, const at::Device& device) {
   std::lock_guard<std::mutex> lk(info.mu);
   for (const auto& l : info.layouts) {
@@ -555,8 +566,8 @@ Tensor topk_sparse_attention(const Tensor& q_in, const Tensor& k_in, const Tenso
     st.add(q).add(k).add(v).add(o);
     for (int i = 0; i < 3; ++i) st.s[st.n++] = idx.stride(i);
     Launch run(q);
-    check_rc(nsa_topk_sparse_attn_fwd(ptr(q), ptr(k), ptr(v), ptr<int>(idx), ptr<int>(cu), ptr(o), ptr<float>(lse), (int)N,
-                                      (int)cu.size(0) - 1, (int)Hq, (int)k.size(1), (int)D, (int)idx.size(2), block_size, st.s, (float)scale,
+    check_rc(nsa_topk_sparse_attn_fwd_bounded(ptr(q), ptr(k), ptr(v), ptr<int>(idx), ptr<int>(cu), ptr(o), ptr<float>(lse), (int)N,
+                                      (int)cu.size(0) - 1, std::max(1, longest_if_known(cu, N)), (int)Hq, (int)k.size(1), (int)D, (int)idx.size(2), block_size, st.s, (float)scale,
                                       dtype_code(q), run.stream),
              "nsa_topk_sparse_attn_fwd");
   }

@@ -6,28 +6,18 @@
 // turned into a list of 64-key tiles, K and V tiles are fetched with cp.async.bulk.tensor
 // straight from the [tokens, kv_heads, d] tensors into 128B-swizzled shared memory, and the
 // next tile of each kind is in flight while the current one is used.
-// The kernel is bound by L2 -> shared-memory tile fill (16 flop per byte fetched at G = 16).
+// The kernel is bound by L2 -> shared-memory tile fill (16 flop per byte fetched at G = 16).  It takes the tokens whose neighbours
+// choose other blocks; those near the start of a sequence, where a few neighbours touch nearly every block, go to
+// sparse_fwd_union_tc.cu.
 #include "attn_tile.cuh"
 #include "dispatch.h"
 #include "host_util.h"
 #include "nsa_b200.h"
+#include "sparse_fwd.h"
 
 namespace nsa {
 
 constexpr int kMaxTilesPerQuery = 64;
-
-struct SparseFwdParams {
-  const void* q;
-  void* o;
-  float* lse;  // [N, Hq], base-2 log-sum-exp of the scaled logits
-  const int* topk_idx;
-  const int* cu_seqlens;
-  long long q_sn, q_sh, o_sn, o_sh;
-  long long t_sh, t_sn, t_sk;
-  int N, B, Hq, Hkv, G, T, block_size;
-  float scale2;
-  Status st;
-};
 
 template <typename T, int D, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
@@ -47,6 +37,10 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const int n = blockIdx.x * WARPS + warp;
   if (n >= p.N) return;  // warps are independent: no block-wide barrier below
   const int h = blockIdx.y;
+  const int b = find_sequence(p.cu_seqlens, p.B, n);
+  const int s0 = __ldg(p.cu_seqlens + b);
+  const int t = n - s0;
+  if (t < p.first) return;
   if (lane == 0) {
     mbar_init(barK, 1);
     mbar_init(barV, 1);
@@ -54,9 +48,6 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   }
   __syncwarp();
 
-  const int b = find_sequence(p.cu_seqlens, p.B, n);
-  const int s0 = __ldg(p.cu_seqlens + b);
-  const int t = n - s0;
   const int BS = p.block_size;
   const int bq = t / BS;
   const int nsub = BS / kKeyTile;
@@ -152,13 +143,13 @@ static int launch_sparse_fwd(const void* k, const void* v, long long k_sn, long 
 
 }  // namespace nsa
 
-extern "C" int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const int* topk_idx,
-                                        const int* cu_seqlens, void* o, float* lse, int total_len, int batch,
-                                        int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
-                                        const long long* strides, float sm_scale, int dtype, void* stream) {
+extern "C" int nsa_topk_sparse_attn_fwd_bounded(const void* q, const void* k, const void* v, const int* topk_idx,
+                                                const int* cu_seqlens, void* o, float* lse, int total_len, int batch, int max_seqlen,
+                                                int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
+                                                const long long* strides, float sm_scale, int dtype, void* stream) {
   using namespace nsa;
   if (!q || !k || !v || !topk_idx || !cu_seqlens || !o || !lse || !strides) return kInvalid;
-  if (total_len <= 0 || batch <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return kInvalid;
+  if (total_len <= 0 || batch <= 0 || max_seqlen <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return kInvalid;
   const int G = num_q_heads / num_kv_heads;
   if (G > 16) return kUnsupported;
   if (block_size < kKeyTile || block_size % kKeyTile) return kUnsupported;
@@ -172,6 +163,22 @@ extern "C" int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void
   p.scale2 = sm_scale * kLog2e;
   p.st.word = status_word();
   if ((p.q_sn | p.q_sh | p.o_sn | p.o_sh) % 8 || !aligned16(q) || !aligned16(o)) return kInvalid;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (max_seqlen > total_len) max_seqlen = total_len;
+  p.first = sparse_fwd_union_limit(G, topk, block_size, head_dim);
+  if (p.first > 0) {
+    const int rc = sparse_fwd_union(q, k, v, strides, p, max_seqlen, p.first, head_dim, dtype, st);
+    if (rc == kInvalid || rc == kUnsupported) p.first = 0;   // a view no tensor map describes: every token below
+    else if (rc || max_seqlen <= p.first) return rc;
+  }
   return NSA_DISPATCH_T_D(dtype, head_dim, launch_sparse_fwd, k, v, strides[2], strides[3], strides[4], strides[5], p,
-                          static_cast<cudaStream_t>(stream));
+                          st);
+}
+
+extern "C" int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const int* topk_idx,
+                                        const int* cu_seqlens, void* o, float* lse, int total_len, int batch,
+                                        int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
+                                        const long long* strides, float sm_scale, int dtype, void* stream) {
+  return nsa_topk_sparse_attn_fwd_bounded(q, k, v, topk_idx, cu_seqlens, o, lse, total_len, batch, total_len, num_q_heads, num_kv_heads,
+                                          head_dim, topk, block_size, strides, sm_scale, dtype, stream);
 }
