@@ -8,7 +8,10 @@
 // next tile of each kind is in flight while the current one is used.
 // The kernel is bound by L2 -> shared-memory tile fill (16 flop per byte fetched at G = 16).  It takes the tokens whose neighbours
 // choose other blocks; those near the start of a sequence, where a few neighbours touch nearly every block, go to
-// sparse_fwd_union_tc.cu.
+// sparse_fwd_union_tc.cu.  There a key or value that is not finite reaches rows that did not select it (0 * inf); the pairs it
+// spoils are marked and walked here, where a row meets its own tiles only.
+#include <algorithm>
+
 #include "attn_tile.cuh"
 #include "dispatch.h"
 #include "host_util.h"
@@ -34,23 +37,39 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   uint64_t* barV = barK + 1;
   int* tiles = reinterpret_cast<int*>(bars + 2 * WARPS) + warp * kMaxTilesPerQuery;
 
-  const int n = blockIdx.x * WARPS + warp;
-  if (n >= p.N) return;  // warps are independent: no block-wide barrier below
   const int h = blockIdx.y;
+  const int BS = p.block_size;
+  const int nsub = BS / kKeyTile;
+  uint32_t phase = 0;
+  bool ready = false;
+  // Warps are independent: no block-wide barrier below.  With a span of 1 the grid has a warp for every token; with 32 a few CTAs
+  // look through all of them for the pairs that were left to this kernel.
+  for (int base_n = (blockIdx.x * WARPS + warp) * p.span; base_n < p.N; base_n += gridDim.x * WARPS * p.span) {
+  unsigned todo = 1u;
+  if (p.first > 0) {
+    bool take = false;
+    if (lane < p.span && base_n + lane < p.N) {
+      const int pos = base_n + lane - __ldg(p.cu_seqlens + find_sequence(p.cu_seqlens, p.B, base_n + lane));
+      take = pos >= p.first || isnan(__ldcg(p.lse + (long long)(base_n + lane) * p.Hq + h * p.G));
+    }
+    todo = __ballot_sync(0xffffffffu, take);
+  }
+  for (; todo; todo &= todo - 1u) {
+  const int n = base_n + __ffs(todo) - 1;
   const int b = find_sequence(p.cu_seqlens, p.B, n);
   const int s0 = __ldg(p.cu_seqlens + b);
   const int t = n - s0;
-  if (t < p.first) return;
-  if (lane == 0) {
-    mbar_init(barK, 1);
-    mbar_init(barV, 1);
-    fence_barrier_init();
+  if (!ready) {
+    if (lane == 0) {
+      mbar_init(barK, 1);
+      mbar_init(barV, 1);
+      fence_barrier_init();
+    }
+    ready = true;
   }
   __syncwarp();
 
-  const int BS = p.block_size;
   const int bq = t / BS;
-  const int nsub = BS / kKeyTile;
 
   // ---- selected blocks -> list of 64-key tiles (in-sequence position of the first key) ----
   int ntiles = 0;
@@ -101,7 +120,6 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
   for (int j = 0; j < D / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  uint32_t phase = 0;
   warp_attend_tiles<T, D>(qf, o, m, l, ntiles, smem_u32(kbuf), smem_u32(vbuf), barK, barV, phase, p.scale2, p.st, tile_at,
                           issue);
 
@@ -120,11 +138,15 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   }
   T* obase = static_cast<T*>(p.o) + (long long)n * p.o_sn + (long long)h * p.G * p.o_sh;
   store_rows_staged<T, D>(o, rs, reinterpret_cast<T*>(kbuf), [&](int r) -> T* { return r < p.G ? obase + r * p.o_sh : nullptr; });
+  fence_proxy_async();  // the staged rows have been read; the next pair's tiles overwrite them through the async proxy
+  __syncwarp();
+  }
+  }
 }
 
 template <typename T, int D>
 static int launch_sparse_fwd(const void* k, const void* v, long long k_sn, long long k_sh, long long v_sn, long long v_sh,
-                             SparseFwdParams p, cudaStream_t stream) {
+                             SparseFwdParams p, bool sweep, cudaStream_t stream) {
   constexpr int WARPS = (D == 128) ? 7 : 8;  // as many private K+V tile pairs as shared memory holds
   constexpr int TILE_BYTES = kKeyTile * D * 2;
   CUtensorMap tmK, tmV;
@@ -136,7 +158,10 @@ static int launch_sparse_fwd(const void* k, const void* v, long long k_sn, long 
   auto kern = sparse_fwd_kernel<T, D, WARPS>;
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
-  dim3 grid((p.N + WARPS - 1) / WARPS, p.Hkv);
+  p.span = sweep ? 32 : 1;
+  int ctas = (p.N + WARPS * p.span - 1) / (WARPS * p.span);
+  if (sweep) ctas = std::min(ctas, std::max(1, num_sms() / p.Hkv));
+  dim3 grid(ctas, p.Hkv);
   { LaunchScope ls_("sparse_fwd", stream); kern<<<grid, WARPS * 32, smem, stream>>>(tmK, tmV, p); }
   return cuda_rc(cudaGetLastError());
 }
@@ -164,15 +189,17 @@ extern "C" int nsa_topk_sparse_attn_fwd_bounded(const void* q, const void* k, co
   p.st.word = status_word();
   if ((p.q_sn | p.q_sh | p.o_sn | p.o_sh) % 8 || !aligned16(q) || !aligned16(o)) return kInvalid;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (max_seqlen > total_len) max_seqlen = total_len;
   p.first = sparse_fwd_union_limit(G, topk, block_size, head_dim);
   if (p.first > 0) {
-    const int rc = sparse_fwd_union(q, k, v, strides, p, max_seqlen, p.first, head_dim, dtype, st);
+    const int rc = sparse_fwd_union(q, k, v, strides, p, p.first, head_dim, dtype, st);
     if (rc == kInvalid || rc == kUnsupported) p.first = 0;   // a view no tensor map describes: every token below
-    else if (rc || max_seqlen <= p.first) return rc;
+    else if (rc) return rc;
   }
+  // No token is expected beyond the division: a few CTAs look through all of them for what the union kernel left (and for tokens
+  // of sequences longer than the caller said, so that the result does not depend on max_seqlen).
+  const bool sweep = p.first > 0 && std::min(max_seqlen, total_len) <= p.first;
   return NSA_DISPATCH_T_D(dtype, head_dim, launch_sparse_fwd, k, v, strides[2], strides[3], strides[4], strides[5], p,
-                          st);
+                          sweep, st);
 }
 
 extern "C" int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const int* topk_idx,

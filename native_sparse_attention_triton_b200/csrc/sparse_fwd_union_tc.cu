@@ -66,11 +66,41 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     if (threadIdx.x == 0) p.st.raise(kErrSmemLayout);
     return;
   }
-  const int b = blockIdx.y, h = blockIdx.z;
-  const int qs = __ldg(p.cu_seqlens + b), L = __ldg(p.cu_seqlens + b + 1) - qs;
+  const int h = blockIdx.y;
   const int QT = 128 >> logG;                  // tokens per row tile
-  const int q0 = (gridDim.x - 1 - blockIdx.x) * 2 * QT;
-  if (q0 >= min(L, limit)) return;
+  // The CTA's row tiles: those before the limit of all sequences are counted through, so that the grid need not know any length
+  // (it has room for tokens / (2 QT) + sequences of them); the last ones, with the most blocks, start first.
+  int b = 0, qs = 0, L = 0, q0 = -1;
+  {
+    int want = gridDim.x - 1 - blockIdx.x;
+    for (int b0 = 0; b0 < p.B && q0 < 0; b0 += 32) {
+      const int mine = b0 + lane;
+      int start = 0, len = 0;
+      if (mine < p.B) {
+        start = __ldg(p.cu_seqlens + mine);
+        len = __ldg(p.cu_seqlens + mine + 1) - start;
+      }
+      const int tiles = (min(max(len, 0), limit) + 2 * QT - 1) / (2 * QT);
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, incl > want);
+      const int src = hit ? __ffs(hit) - 1 : 31;
+      const int before = __shfl_sync(0xffffffffu, incl - tiles, src);
+      if (hit) {
+        b = b0 + src;
+        qs = __shfl_sync(0xffffffffu, start, src);
+        L = __shfl_sync(0xffffffffu, len, src);
+        q0 = (want - before) * 2 * QT;
+      } else {
+        want -= __shfl_sync(0xffffffffu, incl, 31);
+      }
+    }
+  }
+  if (q0 < 0) return;
   const int t_hi = min(q0 + 2 * QT, L) - 1;    // the limit is a multiple of 2 * QT: no row tile straddles it
   const int BS = p.block_size, nsub = BS / 64;
   const int nblk = t_hi / BS + 1, mw = (2 * QT + 31) / 32;
@@ -394,10 +424,10 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       tc_fence_after_sync();
     }
     const float inv = l > 0.f ? 1.f / l : 0.f;
-    if (valid) p.lse[(long long)(qs + tpos) * p.Hq + head] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
     // A row tile whose tokens all belong to the sequence leaves through shared memory (its own Q buffer, free since its
     // last S product, in the swizzled panel layout) and one TMA store per panel; otherwise row by row.
     const bool staged = ntiles > 0 && q0 + g * QT + QT <= L;
+    float probe = l;  // becomes NaN with any output of the row
     T* orow = static_cast<T*>(p.o) + (long long)(qs + tpos) * p.o_sn + (long long)head * p.o_sh;
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
@@ -409,6 +439,8 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
         for (int j = 0; j < 32; ++j) r[j] = 0u;
       }
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) probe = fmaf(0.f, __uint_as_float(r[j]) + __uint_as_float(r[j + 1]), probe);
       if (staged) {
         const uint32_t stage = smem_u32(q_sm + g * Q_BYTES);
 #pragma unroll
@@ -433,6 +465,11 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
       }
     }
+    // one row of the pair not finite: its first lse says so, and sparse_fwd.cu does the pair again after this kernel
+    const unsigned bad = __ballot_sync(0xffffffffu, valid && isnan(probe));
+    const unsigned pair_rows = ((1u << p.G) - 1u) << (lane & ~(p.G - 1));  // G <= 16
+    const bool redo = (bad & pair_rows) != 0u && (row & (p.G - 1)) == 0;
+    if (valid) p.lse[(long long)(qs + tpos) * p.Hq + head] = redo ? __int_as_float(0x7fffffff) : l > 0.f ? m_ref + log2f(l) : -INFINITY;
     if (staged) {
       fence_proxy_async();  // the TMA engine reads the tile through the async proxy
       asm volatile("bar.sync %0, 128;\n" ::"r"(1 + g) : "memory");
@@ -475,8 +512,7 @@ int union_limit(int G, int T, int block_size, int head_dim) {
 }
 
 template <typename T, int D>
-int launch_union(const void* q, const void* k, const void* v, const long long* S, SparseFwdParams p, int max_seqlen, int limit,
-                 cudaStream_t stream) {
+int launch_union(const void* q, const void* k, const void* v, const long long* S, SparseFwdParams p, int limit, cudaStream_t stream) {
   // S: q_n q_h k_n k_h v_n v_h o_n o_h
   const int QT = 128 / p.G;
   CUtensorMap tmQ, tmK, tmV, tmO;
@@ -494,9 +530,10 @@ int launch_union(const void* q, const void* k, const void* v, const long long* S
   auto kern = sparse_fwd_union_kernel<T, D>;
   const cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
-  const int longest = std::min(max_seqlen, limit);
+  const long long per_seq = (std::min(p.N, limit) + 2 * QT - 1) / (2 * QT);
+  const long long ctas = std::min((long long)p.N / (2 * QT) + p.B, per_seq * p.B);
   LaunchScope ls_("sparse_fwd_union", stream);
-  kern<<<dim3((longest + 2 * QT - 1) / (2 * QT), p.B, p.Hkv), 320, smem, stream>>>(tmQ, tmK, tmV, tmO, p, logG, limit);
+  kern<<<dim3((unsigned)ctas, p.Hkv), 320, smem, stream>>>(tmQ, tmK, tmV, tmO, p, logG, limit);
   return cuda_rc(cudaGetLastError());
 }
 
@@ -506,9 +543,9 @@ int sparse_fwd_union_limit(int G, int T, int block_size, int head_dim) {
   return (G & (G - 1)) ? 0 : union_limit(G, T, block_size, head_dim);
 }
 
-int sparse_fwd_union(const void* q, const void* k, const void* v, const long long* strides, SparseFwdParams p, int max_seqlen, int limit,
-                     int head_dim, int dtype, cudaStream_t stream) {
-  return NSA_DISPATCH_T_D(dtype, head_dim, launch_union, q, k, v, strides, p, max_seqlen, limit, stream);
+int sparse_fwd_union(const void* q, const void* k, const void* v, const long long* strides, SparseFwdParams p, int limit, int head_dim,
+                     int dtype, cudaStream_t stream) {
+  return NSA_DISPATCH_T_D(dtype, head_dim, launch_union, q, k, v, strides, p, limit, stream);
 }
 
 }  // namespace nsa
