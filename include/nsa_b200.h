@@ -45,8 +45,8 @@ int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const 
                              int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
                              const long long* strides, float sm_scale, int dtype, void* stream);
 
-/* The same with an upper bound on the sequence lengths (max_seqlen; nsa_topk_sparse_attn_fwd assumes total_len), which spares
- * launches and empty CTAs for batches of short sequences. */
+/* The same with the length of the longest sequence where the caller knows it (max_seqlen; nsa_topk_sparse_attn_fwd assumes
+ * total_len): it chooses the grid, and a value that is too small costs time and no result. */
 int nsa_topk_sparse_attn_fwd_bounded(const void* q, const void* k, const void* v, const int* topk_idx,
                                      const int* cu_seqlens, void* o, float* lse, int total_len, int batch, int max_seqlen,
                                      int num_q_heads, int num_kv_heads, int head_dim, int topk, int block_size,
@@ -102,6 +102,17 @@ int nsa_pool_compress_fwd(const void* x, const void* w, const void* pe, const in
                           const int* y_cu_seqlens, void* y, void* bias_scratch, int total_len, int batch,
                           int total_y, int max_y_len, int num_heads, int head_dim, int kernel_size,
                           int kernel_stride, long long x_stride_n, long long x_stride_h, int dtype, void* stream);
+
+/* The compression of a decode step for both pooling modes, K and V in one launch: every sequence contributes exactly
+ * one window, the kernel_size rows of its staging buffer (x_k, x_v: [batch, kernel_size, H, d] views with strides
+ * x_stride_b, x_stride_n, x_stride_h), so no cu_seqlens is read.  w_k / w_v [H, kernel_size] or NULL (average); bias_k /
+ * bias_v [H, d] (the position embedding folded through the weights by nsa_pool_bias, which does not change between steps)
+ * or NULL; y_k, y_v [batch, H, d] contiguous.  Replaces the two compress_func calls on the staging buffers in
+ * native_sparse_attention/infer/inference_func.py:56-87 when both are pooling operators. */
+int nsa_pool_compress_decode_pair(const void* x_k, const void* x_v, const void* w_k, const void* w_v, const void* bias_k,
+                                  const void* bias_v, void* y_k, void* y_v, int batch, int num_heads, int head_dim,
+                                  int kernel_size, long long x_stride_b, long long x_stride_n, long long x_stride_h,
+                                  int dtype, void* stream);
 
 /* bias[h, :] = sum_k w[h, k] * pe[h, k, :] (w == NULL: the mean over k), in the storage type: the term the pooling
  * operators add to every compressed row (native_sparse_attention/ops/triton/weighted_pool.py:301-363). */
@@ -339,31 +350,27 @@ int nsa_rope_decode3(const void* q, void* yq, const void* k, void* yk, const voi
  * caches' counters on the device.
  *   q [batch, Hq, d], k, v [batch, Hkv, d]: the new token, before rotation; gate [batch, Hq, 3]; out like q.
  *   caches and counters as in the functions above; ticket int32 [batch], zero before the first step (left at zero).
- *   w_k, w_v [Hkv, kernel_size] pooling weights or NULL (average); bias_k [Hkv, d] (nsa_pool_bias / nsa_linear_bias) or NULL;
- *   linear_taps: NULL for pooling; else the output of nsa_linear_decode_taps for this step.
+ *   w_k, w_v [Hkv, kernel_size] pooling weights or NULL (average); pe [Hkv, kernel_size, d]: position embedding of the keys'
+ *   windows, or NULL; linear_taps: NULL for pooling; else the output of nsa_linear_decode_taps for this step (which takes pe then).
  *   strides[26]: q_b q_h | k_b k_h | v_b v_h | gate_b gate_h | out_b out_h | (kv, sequence, row, head) of the selected-block,
  *   compressed, staging and sliding-window caches.
  * Returns -2 for a group of more than 16 query heads, more than 64 selected 64-key tiles or head_dim other than 64 and 128. */
 int nsa_decode_step(const void* q, const void* k, const void* v, const void* gate, void* out, void* sparse_cache, int* sparse_len,
                     void* compress_cache, int* compress_len, void* stage_cache, int* stage_len, void* sliding_cache,
-                    int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* bias_k, const float* linear_taps,
+                    int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* pe, const float* linear_taps,
                     const float* inv_freq, float attention_scaling, int batch, int num_q_heads, int num_kv_heads, int head_dim,
                     int kernel_size, int kernel_stride, int block_size, int topk, int init_blocks, int local_blocks,
                     int sparse_rows, int compress_rows, int sliding_rows, const long long* strides, float sm_scale, int dtype,
                     void* stream);
 
 /* Linear compression of the windows the coming decode step completes: taps[tap][b][key, value][h][:] = row `tap` of the
- * staged window (with the new token k, v appended) times its [d, d] slice of w_k / w_v [Hkv, kernel_size * d, d], for every
+ * staged window (with the new token k, v appended; plus pe [Hkv, kernel_size, d] for keys, unless NULL) times its [d, d] slice of w_k / w_v [Hkv, kernel_size * d, d], for every
  * sequence whose window the new token completes; other sequences' entries are left alone.  Reads the staging cache as it is
  * before the step.  taps: kernel_size * batch * 2 * Hkv * d floats.
  *   strides[8]: k_b k_h | v_b v_h | (kv, sequence, row, head) of the staging cache. */
-int nsa_linear_decode_taps(const void* k, const void* v, const void* w_k, const void* w_v, const void* stage_cache,
-                           const int* stage_len, float* taps, int batch, int num_kv_heads, int head_dim, int kernel_size,
+int nsa_linear_decode_taps(const void* k, const void* v, const void* w_k, const void* w_v, const void* pe,
+                           const void* stage_cache, const int* stage_len, float* taps, int batch, int num_kv_heads, int head_dim, int kernel_size,
                            int kernel_stride, const long long* strides, int dtype, void* stream);
-
-/* bias[h, :] = concat_k(pe[h, k, :]) @ w[h], in the storage type: the term linear compression adds to every row. */
-int nsa_linear_bias(const void* pe, const void* w, void* bias, int num_heads, int head_dim, int kernel_size, int dtype,
-                    void* stream);
 
 #ifdef __cplusplus
 }

@@ -62,7 +62,7 @@ struct Params {
   Cache sel, cmp, stage, win;
   int* ticket;  // [B] zero between steps
   const void* w[2];
-  const void* bias_k;
+  const void* pe;        // [Hkv, window, D] position embedding of the keys' windows (pooling), or nullptr
   const float* partial;  // linear compression: [window][B][2][Hkv][D] per-tap products, or nullptr
   const float* inv_freq;
   float rope_scaling;
@@ -246,13 +246,13 @@ __device__ __forceinline__ void cta_merge(uint8_t* smem, int br, int w0, int nw,
   for (int w = 0; w < nw; ++w) mx = fmaxf(mx, mlw[w * 16].x);
   float sum = 0.f;
   for (int w = 0; w < nw; ++w)
-    if (mlw[w * 16].x != -INFINITY) sum += mlw[w * 16].y * fast_exp2(mlw[w * 16].x - mx);
+    if (mlw[w * 16].y != 0.f) sum += mlw[w * 16].y * fast_exp2(mlw[w * 16].x - mx);
   float* part = reinterpret_cast<float*>(smem + L::kPart) + (br * 16 + row) * D;
   for (int v = c; v < D / 4; v += tpr) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int w = 0; w < nw; ++w) {
       const float mw = mlw[w * 16].x;
-      if (mw == -INFINITY) continue;
+      if (mlw[w * 16].y == 0.f) continue;  // saw no key (a NaN row has a NaN here)
       const float wt = fast_exp2(mw - mx);
       const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem + (w0 + w) * L::kWarpBuf) + row * L::kOStride + v * 4);
       acc.x += x.x * wt; acc.y += x.y * wt; acc.z += x.z * wt; acc.w += x.w * wt;
@@ -283,7 +283,7 @@ __device__ __forceinline__ void cluster_weights(uint8_t* smem, int S, int branch
 #pragma unroll
     for (int s = 0; s < kMaxCluster; ++s)
       if (s < S) {
-        const float w = ml[s].x == -INFINITY ? 0.f : fast_exp2(ml[s].x - mx);
+        const float w = ml[s].y == 0.f ? 0.f : fast_exp2(ml[s].x - mx);
         sum += ml[s].y * w;
         ml[s].x = w;
       }
@@ -388,7 +388,24 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
         // staging buffer: drop the first `stride` rows if it was full, append the new row, pool it if that completes a window
         const T* w = static_cast<const T*>(p.w[kv]);
         const bool weighted = w != nullptr && p.partial == nullptr;
-        float a1 = 0.f, a2 = 0.f;
+        const T* pe = kv == 0 && full ? static_cast<const T*>(p.pe) : nullptr;  // summed apart and rounded, as the operators do
+        float a1 = 0.f, a2 = 0.f, e1 = 0.f, e2 = 0.f;
+        if (pe) {
+          pe += (long long)h * p.window * D + j;
+          for (int r0 = 0; r0 < p.window; r0 += 16) {
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+              if (r0 + u < p.window) {
+                const float wv = weighted ? DT<T>::to_float(w[h * p.window + r0 + u]) : 1.f;
+                e1 += wv * DT<T>::to_float(pe[(r0 + u) * D]);
+                e2 += wv * DT<T>::to_float(pe[(r0 + u) * D + D / 2]);
+              }
+          }
+          if (!weighted) {
+            e1 /= (float)p.window;
+            e2 /= (float)p.window;
+          }
+        }
         if (shift || full) {
           const int off = shift ? p.stride : 0;
           for (int r0 = 0; r0 < kept; r0 += 16) {
@@ -439,10 +456,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
               a2 *= inv;
             }
           }
-          if (kv == 0 && p.bias_k) {
-            const T* bias = static_cast<const T*>(p.bias_k) + h * D;
-            a1 = round16<T>(a1) + DT<T>::to_float(bias[j]);
-            a2 = round16<T>(a2) + DT<T>::to_float(bias[j + D / 2]);
+          if (pe) {
+            a1 = round16<T>(a1) + round16<T>(e1);
+            a2 = round16<T>(a2) + round16<T>(e2);
           }
           a1 = round16<T>(a1);
           a2 = round16<T>(a2);
@@ -692,6 +708,7 @@ struct LinearTapParams {
   const void* x[2];  // the new token's key and value rows [B, Hkv, D]
   long long x_sb[2], x_sh[2];
   const void* w[2];  // [Hkv, window * D, D]
+  const void* pe;    // [Hkv, window, D] added to the keys' rows, or nullptr
   Cache stage;
   float* partial;    // [window][B][2][Hkv][D]
   int B, Hkv, window, stride;
@@ -713,7 +730,9 @@ __global__ void __launch_bounds__(256) linear_tap_kernel(LinearTapParams p) {
     if (threadIdx.x < D) {
       const T* src = tap == kept ? static_cast<const T*>(p.x[kv]) + b * p.x_sb[kv] + h * p.x_sh[kv]
                                  : cache_ptr<T, D>(p.stage, kv, b, tap + (shift ? p.stride : 0), h);
-      xs[threadIdx.x] = DT<T>::to_float(src[threadIdx.x]);
+      float x = DT<T>::to_float(src[threadIdx.x]);
+      if (kv == 0 && p.pe) x += DT<T>::to_float(static_cast<const T*>(p.pe)[((size_t)h * p.window + tap) * D + threadIdx.x]);
+      xs[threadIdx.x] = x;
     }
     __syncthreads();
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -907,7 +926,7 @@ int decode_cluster_compressed(const DecodeOpArgs& a, cudaStream_t stream) {
 // compressed, staging and window caches: 26 entries, elements
 extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, const void* gate, void* out, void* sparse_cache, int* sparse_len,
                                void* compress_cache, int* compress_len, void* stage_cache, int* stage_len, void* sliding_cache,
-                               int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* bias_k, const float* linear_taps,
+                               int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* pe, const float* linear_taps,
                                const float* inv_freq, float attention_scaling, int batch, int num_q_heads, int num_kv_heads, int head_dim,
                                int kernel_size, int kernel_stride, int block_size, int topk, int init_blocks, int local_blocks,
                                int sparse_rows, int compress_rows, int sliding_rows, const long long* strides, float sm_scale, int dtype,
@@ -931,7 +950,7 @@ extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, cons
   p.stage = make_cache(stage_cache, stage_len, strides + 18, kernel_size);
   p.win = make_cache(sliding_cache, sliding_len, strides + 22, sliding_rows);
   if (!cache_ok(p.sel) || !cache_ok(p.cmp) || !cache_ok(p.stage) || !cache_ok(p.win)) return kInvalid;
-  p.ticket = ticket; p.w[0] = w_k; p.w[1] = w_v; p.bias_k = bias_k; p.partial = linear_taps; p.inv_freq = inv_freq;
+  p.ticket = ticket; p.w[0] = w_k; p.w[1] = w_v; p.pe = linear_taps ? nullptr : pe; p.partial = linear_taps; p.inv_freq = inv_freq;
   p.rope_scaling = attention_scaling;
   p.B = batch; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.block_size = block_size; p.window = kernel_size;
   p.stride = kernel_stride; p.init_blocks = init_blocks; p.local_blocks = local_blocks;
@@ -945,14 +964,14 @@ extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, cons
 }
 
 // strides: k_b k_h | v_b v_h | (kv, sequence, row, head) of the staging cache
-extern "C" int nsa_linear_decode_taps(const void* k, const void* v, const void* w_k, const void* w_v, const void* stage_cache,
-                                      const int* stage_len, float* taps, int batch, int num_kv_heads, int head_dim, int kernel_size,
+extern "C" int nsa_linear_decode_taps(const void* k, const void* v, const void* w_k, const void* w_v, const void* pe,
+                                      const void* stage_cache, const int* stage_len, float* taps, int batch, int num_kv_heads, int head_dim, int kernel_size,
                                       int kernel_stride, const long long* strides, int dtype, void* stream) {
   using namespace nsa;
   if (!k || !v || !w_k || !w_v || !stage_cache || !stage_len || !taps || !strides || batch <= 0 || num_kv_heads <= 0) return kInvalid;
   if (kernel_size <= 0 || kernel_stride <= 0 || kernel_size % kernel_stride || !aligned16(w_k) || !aligned16(w_v)) return kInvalid;
   LinearTapParams p;
-  p.x[0] = k; p.x[1] = v; p.w[0] = w_k; p.w[1] = w_v;
+  p.x[0] = k; p.x[1] = v; p.w[0] = w_k; p.w[1] = w_v; p.pe = pe;
   p.x_sb[0] = strides[0]; p.x_sh[0] = strides[1]; p.x_sb[1] = strides[2]; p.x_sh[1] = strides[3];
   p.stage = make_cache(const_cast<void*>(stage_cache), const_cast<int*>(stage_len), strides + 4, kernel_size);
   if (!cache_ok(p.stage)) return kInvalid;

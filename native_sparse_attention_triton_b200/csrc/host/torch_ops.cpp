@@ -221,6 +221,9 @@ struct SavingNode : Node {
 };
 
 bool needs_graph(std::initializer_list<Tensor> inputs) {
+  for (const auto& t : inputs)  // a tangent would be dropped in silence below the autograd dispatch keys
+    if (t.defined() && t._fw_grad(/*level=*/0).defined())
+      throw std::runtime_error("forward-mode differentiation is not implemented for native_sparse_attention_triton_b200 operators");
   if (!at::GradMode::is_enabled()) return false;
   for (const auto& t : inputs)
     if (t.defined() && t.requires_grad()) return true;
@@ -850,50 +853,6 @@ std::tuple<Tensor, Tensor> compressed_attention_decode(const Tensor& q_in, const
 }
 
 // ------------------------------------------------------------------------------------------------------- inference step
-// The position embedding folded through a compression's weights, [H, d]: it changes only when the parameters do, so it is
-// computed once per (weight, pe) pair and version and not once per decode step.
-struct BiasEntry {
-  c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> w, pe;
-  uint32_t w_version = 0, pe_version = 0;
-  Tensor bias;
-  BiasEntry(const Tensor& w_, const Tensor& pe_) : w(w_.getIntrusivePtr()), pe(pe_.getIntrusivePtr()) {}
-};
-std::mutex g_bias_mu;
-std::unordered_map<uint64_t, BiasEntry> g_bias;
-constexpr size_t kBiasEntries = 256;
-
-Tensor position_bias(const Tensor& w, const Tensor& pe, int mode, void* stream) {
-  uint32_t wv = 0, pv = 0;
-  const bool counted = (!w.defined() || version_of(w, wv)) && version_of(pe, pv);
-  const uint64_t key = reinterpret_cast<uint64_t>(w.unsafeGetTensorImpl()) * 0x9E3779B97F4A7C15ull ^
-                       reinterpret_cast<uint64_t>(pe.unsafeGetTensorImpl()) ^ (uint64_t)mode;
-  if (counted) {
-    std::lock_guard<std::mutex> lk(g_bias_mu);
-    auto it = g_bias.find(key);
-    if (it != g_bias.end() && it->second.w_version == wv && it->second.pe_version == pv &&
-        it->second.w._unsafe_get_target() == w.unsafeGetTensorImpl() && it->second.pe._unsafe_get_target() == pe.unsafeGetTensorImpl())
-      return it->second.bias;
-  }
-  const int64_t H = pe.size(0), ks = pe.size(1), D = pe.size(2);
-  Tensor bias = empty({H, D}, pe.scalar_type(), pe.device());
-  const Tensor pec = pe.contiguous(), wc = w.defined() ? w.contiguous() : Tensor();
-  if (mode == kLinear)
-    check_rc(nsa_linear_bias(ptr(pec), ptr(wc), ptr(bias), (int)H, (int)D, (int)ks, dtype_code(pe), stream), "nsa_linear_bias");
-  else
-    check_rc(nsa_pool_bias(ptr(pec), wc.defined() ? ptr(wc) : nullptr, ptr(bias), (int)H, (int)D, (int)ks, dtype_code(pe), stream),
-             "nsa_pool_bias");
-  if (counted && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
-    std::lock_guard<std::mutex> lk(g_bias_mu);
-    if (g_bias.size() >= kBiasEntries) g_bias.clear();
-    BiasEntry e(w, pe);
-    e.w_version = wv;
-    e.pe_version = pv;
-    e.bias = bias;
-    g_bias.insert_or_assign(key, std::move(e));
-  }
-  return bias;
-}
-
 // The caches of a layer as NSACache holds them: [2, batch, rows, heads, d] tensors and int32 counters.
 struct CacheRefs {
   Tensor sel, sel_len, cmp, cmp_len, stage, stage_len, win, win_len, ticket;
@@ -920,20 +879,39 @@ std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const 
                  q_in.scalar_type() == gate_in.scalar_type() && q_in.scalar_type() == c.sel.scalar_type(),
              "query, key, value, gate and caches must have the same 16-bit dtype");
   NSA_ASSERT(gate_in.size(0) == B && gate_in.size(1) == Hq && gate_in.size(2) == 3, "gate must be [batch, query heads, 3]");
-  if ((D != 64 && D != 128) || Hq / Hkv > 16 || inv_freq.size(0) != D / 2) return std::nullopt;
+  NSA_ASSERT(block_size % ks == 0 && ks % st == 0, "block_size must be a multiple of kernel_size, kernel_size of kernel_stride");
+  if ((D != 64 && D != 128) || Hq / Hkv > 16 || c.cmp.size(2) == 0 || c.win.size(2) == 0) return std::nullopt;
+  if (inv_freq.scalar_type() != at::kFloat || inv_freq.dim() != 1 || inv_freq.size(0) != D / 2 || !inv_freq.is_contiguous()) return std::nullopt;
+  if (mode != kAverage) {
+    NSA_ASSERT(w_k.has_value() && w_v.has_value(), "this compression needs weights");
+    for (const Tensor* w : {&*w_k, &*w_v}) {
+      require_cuda(*w);
+      NSA_ASSERT(w->scalar_type() == c.sel.scalar_type(), "w must have the caches' dtype");
+    }
+  }
+  const auto check_weight = [&](const OptTensor& w, bool linear) {
+    if (w) NSA_ASSERT(w->size(0) == Hkv && w->numel() == Hkv * ks * (linear ? D * D : 1), "w must be [num_heads, kernel_size * head_dim, head_dim] or [num_heads, kernel_size]");
+  };
+  check_weight(w_k, mode == kLinear);
+  check_weight(w_v, mode == kLinear);
+  if (pe) {
+    require_cuda(*pe);
+    NSA_ASSERT(pe->scalar_type() == c.sel.scalar_type() && pe->numel() == Hkv * ks * D, "pe must be [num_heads, kernel_size, head_dim] of the caches' dtype");
+  }
   const Tensor q = inner_contiguous(q_in), k = inner_contiguous(k_in), v = inner_contiguous(v_in), gate = gate_in.contiguous();
   Launch run(q);
-  Tensor bias, wk, wv;
+  Tensor pec, wk, wv;
   if (w_k) wk = w_k->contiguous();
   if (w_v) wv = w_v->contiguous();
-  if (pe) bias = position_bias(w_k.value_or(Tensor()), *pe, mode, run.stream);
+  if (pe) pec = pe->contiguous();
+  const auto p = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
   Tensor o = out ? *out : empty_like_rows(q);
   Tensor taps;
   if (mode == kLinear) {
     taps = empty({ks, B, 2, Hkv, D}, at::kFloat, q.device());
     const long long s[8] = {k.stride(0), k.stride(1), v.stride(0), v.stride(1), c.stage.stride(0), c.stage.stride(1), c.stage.stride(2),
                             c.stage.stride(3)};
-    check_rc(nsa_linear_decode_taps(ptr(k), ptr(v), ptr(wk), ptr(wv), ptr(c.stage), ptr<int>(c.stage_len), ptr<float>(taps), (int)B, (int)Hkv,
+    check_rc(nsa_linear_decode_taps(ptr(k), ptr(v), ptr(wk), ptr(wv), p(pec), ptr(c.stage), ptr<int>(c.stage_len), ptr<float>(taps), (int)B, (int)Hkv,
                                     (int)D, ks, st, s, dtype_code(q), run.stream),
              "nsa_linear_decode_taps");
   }
@@ -944,10 +922,9 @@ std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const 
   int n = 10;
   for (const Tensor* t : {&c.sel, &c.cmp, &c.stage, &c.win})
     for (int i = 0; i < 4; ++i) strides[n++] = t->stride(i);
-  const auto p = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
   const int rc = nsa_decode_step(ptr(q), ptr(k), ptr(v), ptr(gate), ptr(o), ptr(c.sel), ptr<int>(c.sel_len), ptr(c.cmp), ptr<int>(c.cmp_len),
                                  ptr(c.stage), ptr<int>(c.stage_len), ptr(c.win), ptr<int>(c.win_len), ptr<int>(c.ticket), p(wk), p(wv),
-                                 p(bias), static_cast<float*>(p(taps)), ptr<float>(inv_freq), (float)rope_scaling, (int)B, (int)Hq, (int)Hkv,
+                                 p(pec), static_cast<float*>(p(taps)), ptr<float>(inv_freq), (float)rope_scaling, (int)B, (int)Hq, (int)Hkv,
                                  (int)D, ks, st, block_size, topk, init_blocks, local_blocks, (int)c.sel.size(2), (int)c.cmp.size(2),
                                  (int)c.win.size(2), strides, (float)default_scale(D), dtype_code(q), run.stream);
   if (rc == -2) return std::nullopt;

@@ -77,6 +77,10 @@ cudaError_t allow_smem(const void* kernel, int bytes) {
     }
     if (g && g->bytes[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
   }
+  // one at a time: a smaller request that passes a larger one on the way would take that one's grant back
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (g && g->bytes[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess && g) g->bytes[dev].store(bytes, std::memory_order_release);
   return e;

@@ -88,18 +88,47 @@ _MODES = {ops.linear_compress: 0, ops.weightedpool_compress: 1, ops.avgpool_comp
 def _compress_staged(cache: NSACache, batch: int, which: int, func: Callable, weight, pe):
     """One compressed row per sequence from the staging buffers [batch * kernel_size, heads, d], the way the reference does it:
     the compress function run over them with an arange cu_seqlens (infer/inference_func.py:56-87)."""
-    x = cache.before_compress_kv_cache[which, :batch].view(batch * cache.kernel_size, cache.num_kv_heads, cache.head_dim)
+    x = cache.before_compress_kv_cache[which, :batch].reshape(batch * cache.kernel_size, cache.num_kv_heads, cache.head_dim)
     return func(x, weight, cache.stage_cu(batch), cache.kernel_size, cache.kernel_stride, pe)[0]
+
+
+def _compress_staged_pair(cache: NSACache, batch: int, funcs, weights, pe):
+    """Both staging buffers pooled in one launch (nsa_pool_compress_decode_pair): one compressed key row and one compressed
+    value row per sequence."""
+    stage = cache.before_compress_kv_cache
+    xk, xv = stage[0, :batch], stage[1, :batch]            # [batch, kernel_size, H, d]
+    wk = weights[0].contiguous() if funcs[0] is ops.weightedpool_compress else None
+    wv = weights[1].contiguous() if funcs[1] is ops.weightedpool_compress else None
+    yk = torch.empty(batch, cache.num_kv_heads, cache.head_dim, dtype=stage.dtype, device=stage.device)
+    yv, bias_k = torch.empty_like(yk), None
+    torch.cuda.set_device(stage.device)
+    if pe is not None:
+        bias_k, pec = torch.empty_like(yk[0]), pe.contiguous()
+        rc = _lib.lib().nsa_pool_bias(ptr(pec), ptr(wk), ptr(bias_k), pe.shape[0], pe.shape[2], pe.shape[1], dtype_code(pe),
+                                      stream_ptr(stage.device))
+        _lib.check(rc, "nsa_pool_bias")
+    rc = _lib.lib().nsa_pool_compress_decode_pair(ptr(xk), ptr(xv), ptr(wk), ptr(wv), ptr(bias_k), None, ptr(yk), ptr(yv), batch,
+                                                  cache.num_kv_heads, cache.head_dim, cache.kernel_size, xk.stride(0), xk.stride(1),
+                                                  xk.stride(2), dtype_code(stage), stream_ptr(stage.device))
+    _lib.check(rc, "nsa_pool_compress_decode_pair")
+    return yk, yv
+
+
+def _is_plain(cache):
+    """A cache whose decode bookkeeping is NSACache's own (a subclass that replaces a part of it takes the operators one by one)."""
+    t = type(cache)
+    return t is NSACache or (issubclass(t, NSACache) and t.prepare_compress is NSACache.prepare_compress
+                             and t.update_kv is NSACache.update_kv and t._fill is NSACache._fill)
 
 
 def _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weight, compress_func, pe, block_size, topk, init_blocks,
                        local_blocks, out=None):
-    """The decode step as one launch (two with linear compression); None where it needs one of the caller's own functions, a
-    mixture of linear and pooling compression, or a shape the fused kernel does not have."""
+    """The decode step as one launch (two with linear compression); None where it needs one of the caller's own functions or
+    classes, a mixture of linear and pooling compression, or a shape the fused kernel does not have."""
     mode_k, mode_v = _MODES.get(compress_func[0]), _MODES.get(compress_func[1])
-    if mode_k is None or mode_v is None or (mode_k == 0) != (mode_v == 0):
+    if mode_k is None or mode_v is None or (mode_k == 0) != (mode_v == 0) or not _is_plain(cache):
         return None
-    mine = rope if type(rope) is RotaryEmbedding else _device_rope_of(rope)
+    mine = rope if type(rope) is RotaryEmbedding else None if hasattr(rope, "decode_at3") else _device_rope_of(rope)
     if mine is None:
         return None
     return _lib.host().decode_step(query, key, value, gate_value, cache._tensors(), compress_weight[0] if mode_k != 2 else None,
@@ -121,7 +150,7 @@ def nsa_infer(cu_seqlens: torch.Tensor, step: int, query: torch.Tensor, key: tor
     if step == 0:
         cache.reset()
         mode_k, mode_v = _MODES.get(compress_func[0]), _MODES.get(compress_func[1])
-        if mode_k is not None and mode_v is not None and type(rope) is RotaryEmbedding:
+        if mode_k is not None and mode_v is not None and type(rope) is RotaryEmbedding and _is_plain(cache):
             return _lib.host().prefill(cu_seqlens, query, key, value, gate_value, cache._tensors(), compress_weight[0] if mode_k != 2 else None,
                                        compress_weight[1] if mode_v != 2 else None, intra_block_pe, mode_k, mode_v, rope.inv_freq,
                                        rope.attention_scaling, kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks,
@@ -145,13 +174,17 @@ def nsa_infer(cu_seqlens: torch.Tensor, step: int, query: torch.Tensor, key: tor
         return ops.gate_combine(gate_value, o_cmp, o_sel, o_win)
 
     # ---- decode: nothing below reads a device value on the host ----
+    assert key.shape[0] == batch, "a decode step has one row per sequence of the prefill"
     out = _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weight, compress_func, intra_block_pe, block_size, topk,
                              init_blocks, local_blocks)
     if out is not None:
         return out
     cache.prepare_compress(cu_seqlens, step, key, value)
-    compress_key = _compress_staged(cache, batch, 0, compress_func[0], compress_weight[0], intra_block_pe)
-    compress_value = _compress_staged(cache, batch, 1, compress_func[1], compress_weight[1], None)
+    if _MODES.get(compress_func[0]) and _MODES.get(compress_func[1]):
+        compress_key, compress_value = _compress_staged_pair(cache, batch, compress_func, compress_weight, intra_block_pe)
+    else:
+        compress_key = _compress_staged(cache, batch, 0, compress_func[0], compress_weight[0], intra_block_pe)
+        compress_value = _compress_staged(cache, batch, 1, compress_func[1], compress_weight[1], None)
     fast_rope = rope if hasattr(rope, "decode_at3") else _device_rope_of(rope)
     if fast_rope is not None:
         # the new token's index is the number of tokens cached so far; the compressed token's, the compressed count
@@ -214,6 +247,9 @@ class DecodeGraph:
         self.output = torch.empty_like(query, memory_format=torch.contiguous_format)
         self.graph = None
         cache: NSACache = nsa_args["cache"]
+        assert key.shape[0] == cu_seqlens.shape[0] - 1, "a decode step has one row per sequence of the prefill"
+        for arg in ("kernel_size", "kernel_stride", "window_size"):
+            assert nsa_args[arg] == getattr(cache, arg), f"{arg} must be the cache's"
         # The trial step below and the capture advance the cache: its state is put back afterwards.
         state = [t.clone() for t in self._state(cache)]
         side = torch.cuda.Stream(device=query.device)

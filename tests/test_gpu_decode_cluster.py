@@ -99,3 +99,54 @@ def test_fused_step_equals_operators(monkeypatch, mode, lens, Hq, Hkv, d, ks, st
     assert torch.equal(a.before_compress_kv_cache, b.before_compress_kv_cache)
     assert float((a.compress_kv_cache.float() - b.compress_kv_cache.float()).abs().max()) <= (2e-2 if dtype == torch.bfloat16 else 3e-3) * 4
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["weighted", "avg", "linear"])
+def test_step_reads_the_parameters_it_is_given(mode):
+    """Weights and position embedding overwritten behind the version counter between two steps that complete a window, and calls
+    that the separate operators refuse."""
+    import native_sparse_attention_triton_b200 as pkg
+    from native_sparse_attention_triton_b200 import infer
+    from native_sparse_attention_triton_b200.kv_cache import NSACache
+    ops = pkg.ops
+    B, Hq, Hkv, d, ks, st = 2, 8, 2, 128, 16, 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, generator=g, device="cuda") * scale).bfloat16()
+    fn = {"linear": ops.linear_compress, "weighted": ops.weightedpool_compress, "avg": ops.avgpool_compress}[mode]
+    w = {"linear": lambda: rnd(Hkv, ks * d, d, scale=(ks * d) ** -0.5), "weighted": lambda: rnd(Hkv, ks, scale=ks ** -0.5), "avg": lambda: None}[mode]
+    wk, wv, pe = w(), w(), rnd(Hkv, ks, d)
+    rope = infer.RotaryEmbedding(torch.zeros(d // 2, device="cuda"))    # no rotation: the cached rows are the compressed ones
+    cache = NSACache(B, 128, Hkv, d, ks, st, 32, torch.bfloat16)
+    args = dict(rope=rope, cache=cache, compress_weight=(wk, wv), compress_func=(fn, fn), intra_block_pe=pe, kernel_size=ks, kernel_stride=st,
+                block_size=64, topk=4, init_blocks=1, local_blocks=2, window_size=32)
+    cu = torch.zeros(B + 1, dtype=torch.int32, device="cuda")
+    keys = []
+    for step in range(1, 2 * ks + 1):
+        if step == ks + 1:
+            for t in (wk, pe):
+                if t is not None:
+                    t.data.copy_(rnd(*t.shape, scale=float(t.float().std())))
+        rows = [rnd(B, Hq, d), rnd(B, Hkv, d), rnd(B, Hkv, d), rnd(B, Hq, 3)]
+        keys.append(rows[1])
+        infer.nsa_infer(cu, step, *rows, **args)
+    x = torch.stack(keys[ks:], 1).reshape(B * ks, Hkv, d)
+    want = fn(x, wk, torch.arange(B + 1, dtype=torch.int32, device="cuda") * ks, ks, st, pe)[0]
+    got = cache.compress_kv_cache[0, :B, 1]
+    # both round a sum of about 1 + |pe| to 16 bits once or twice
+    assert float((got.float() - want.float()).abs().max()) <= 4e-2
+    with pytest.raises(AssertionError):
+        infer.nsa_infer(cu, 1, *[r[:1] for r in rows], **args)            # fewer rows than sequences
+    with pytest.raises(AssertionError):
+        infer.nsa_infer(cu, 1, *rows, **{**args, "block_size": 40})       # no multiple of kernel_size
+
+
+def test_forward_mode_is_refused():
+    import native_sparse_attention_triton_b200 as pkg
+    import torch.autograd.forward_ad as fwAD
+    x = torch.randn(64, 2, 64, device="cuda").half()
+    cu = torch.tensor([0, 64], dtype=torch.int32, device="cuda")
+    with fwAD.dual_level():
+        with pytest.raises(RuntimeError):
+            pkg.ops.avgpool_compress(fwAD.make_dual(x, torch.ones_like(x)), None, cu, 32, 16, None)
+        with pytest.raises(RuntimeError):
+            pkg.ops.rope(fwAD.make_dual(x, torch.ones_like(x)), torch.ones(32, device="cuda"), cu)
