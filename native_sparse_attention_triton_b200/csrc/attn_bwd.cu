@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(1024) index_scan_kernel(IndexParams p) {
 constexpr int kSlots = 2;        // tokens per pipeline stage
 constexpr int kBwdStages = 4;
 
-template <typename T, int D, bool SPARSE>
+template <typename T, int D>
 __global__ void __launch_bounds__(160, 1)
 dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
             const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, DkdvParams p) {
@@ -390,42 +390,21 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   int* tok_sh = reinterpret_cast<int*>(ld_sh + kBwdStages * kSlots * 16);  // [stages][slots] in-sequence position or -1
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // ---- which key tile and which tokens ----
-  int h, qs, Lq, krow0, kpos, kvalid;   // krow0: global K row of the tile's first key; kpos: its in-sequence index
-  int tok_begin, tok_count;             // dense: first token position and count; sparse: list offset and count
-  if (SPARSE) {
-    const int item = blockIdx.x;
-    const int total_x = p.Hkv * p.NW * p.TB;
-    if (item >= __ldg(p.item_base + total_x)) return;
-    const int x = __ldg(p.item_bin + item);  // item_base[x] <= item < item_base[x + 1]
-    h = x / (p.NW * p.TB);
-    const int gb = x % p.TB;
-    const int b = find_block_sequence(p.cu_q, p.B, gb, p.block_size);
-    qs = __ldg(p.cu_q + b);
-    Lq = __ldg(p.cu_q + b + 1) - qs;
-    const int blk = gb - block_base(qs, b, p.block_size);
-    kpos = blk * p.block_size + blockIdx.y * kKeyTile;
-    krow0 = qs + kpos;
-    kvalid = min(kKeyTile, Lq - kpos);
-    const int c = item - __ldg(p.item_base + x);
-    const int cnt = __ldg(p.offsets + x + 1) - __ldg(p.offsets + x);
-    tok_begin = __ldg(p.offsets + x) + c * p.chunk;
-    tok_count = min(p.chunk, cnt - c * p.chunk);
-  } else {
-    const int b = blockIdx.z / p.Hkv;
-    h = blockIdx.z % p.Hkv;
-    qs = __ldg(p.cu_q + b);
-    Lq = __ldg(p.cu_q + b + 1) - qs;
-    const int ks0 = __ldg(p.cu_k + b), Lk = __ldg(p.cu_k + b + 1) - ks0;
-    kpos = blockIdx.x * kKeyTile;  // key tiles vary fastest: CTAs that run together share a token chunk in L2
-    if (kpos >= Lk) return;
-    krow0 = ks0 + kpos;
-    kvalid = min(kKeyTile, Lk - kpos);
-    const int t_first = p.causal ? kpos * p.stride + p.window - 1 : 0;
-    const int c_lo = blockIdx.y * p.chunk;
-    tok_begin = max(c_lo, t_first);
-    tok_count = min(c_lo + p.chunk, Lq) - tok_begin;
-  }
+  // ---- which key tile (krow0: global K row of its first key, kpos: in-sequence index) and which tokens of the list ----
+  const int item = blockIdx.x;
+  const int total_x = p.Hkv * p.NW * p.TB;
+  if (item >= __ldg(p.item_base + total_x)) return;
+  const int x = __ldg(p.item_bin + item);  // item_base[x] <= item < item_base[x + 1]
+  const int h = x / (p.NW * p.TB);
+  const int gb = x % p.TB;
+  const int b = find_block_sequence(p.cu_q, p.B, gb, p.block_size);
+  const int qs = __ldg(p.cu_q + b), Lq = __ldg(p.cu_q + b + 1) - qs;
+  const int blk = gb - block_base(qs, b, p.block_size);
+  const int kpos = blk * p.block_size + blockIdx.y * kKeyTile, krow0 = qs + kpos;
+  const int kvalid = min(kKeyTile, Lq - kpos);
+  const int c = item - __ldg(p.item_base + x);
+  const int cnt = __ldg(p.offsets + x + 1) - __ldg(p.offsets + x);
+  const int tok_begin = __ldg(p.offsets + x) + c * p.chunk, tok_count = min(p.chunk, cnt - c * p.chunk);
   if (kvalid <= 0 || tok_count <= 0) return;
 
   if (threadIdx.x == 0) {
@@ -462,8 +441,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
       const int ti = g * kSlots + slot;
       int n = -1, tpos = -1;
       if (ti < tok_count) {
-        if (SPARSE) { n = __ldg(p.list + tok_begin + ti); tpos = n - qs; }
-        else { tpos = tok_begin + ti; n = qs + tpos; }
+        n = __ldg(p.list + tok_begin + ti);
+        tpos = n - qs;
       }
       float2 ldv = make_float2(INFINITY, 0.f);
       if (n >= 0 && head < p.G) ldv = __ldg(p.ld + (long long)n * p.Hq + h * p.G + head);
@@ -504,7 +483,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   for (int r = 0; r < 2; ++r) {
     const int row = warp * 16 + r_lo + 8 * r;
     const int kidx = kpos + row;
-    need[r] = (row < kvalid) ? (p.causal ? kidx * p.stride + p.window - 1 : 0) : 0x7fffffff;
+    need[r] = (row < kvalid) ? kidx : 0x7fffffff;
   }
   const uint32_t kt = smem_u32(ktile), vt = smem_u32(vtile);
   const int a_row = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), a_ch = lane >> 4;   // A-fragment addressing
@@ -673,8 +652,10 @@ __device__ __forceinline__ void row_stats(const T* __restrict__ o, const T* __re
         acc = fmaf(x.y, y.y, acc);
       }
     } else {
-#pragma unroll
-      for (int j = 0; j < EPL; ++j) acc = fmaf(DT<T>::to_float(po[j]), DT<T>::to_float(pd[j]), acc);
+      static_assert(EPL == 4, "head_dim 64 or 128");
+      const uint2 a = *reinterpret_cast<const uint2*>(po), b = *reinterpret_cast<const uint2*>(pd);
+      const float2 x0 = DT<T>::unpack(a.x), y0 = DT<T>::unpack(b.x), x1 = DT<T>::unpack(a.y), y1 = DT<T>::unpack(b.y);
+      acc = fmaf(x1.y, y1.y, fmaf(x1.x, y1.x, fmaf(x0.y, y0.y, x0.x * y0.x)));
     }
   }
 #pragma unroll
@@ -695,7 +676,7 @@ __global__ void __launch_bounds__(128) index_count_stats_kernel(IndexParams ip, 
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-template <typename T, int D, bool SPARSE>
+template <typename T, int D>
 static int launch_dkdv(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk,
                        dim3 grid, DkdvParams p, cudaStream_t stream) {
   // strides: q_n q_h k_n k_h v_n v_h do_n do_h
@@ -712,10 +693,10 @@ static int launch_dkdv(const void* q, const void* dout, const void* k, const voi
   constexpr int STAGE_BYTES = kSlots * 2 * 16 * D * 2;
   const size_t smem = 1024 + 2 * TILE_BYTES + kBwdStages * STAGE_BYTES + (2 * kBwdStages + 1) * sizeof(uint64_t) +
                       kBwdStages * kSlots * (16 * sizeof(float2) + sizeof(int)) + 64;
-  auto kern = dkdv_kernel<T, D, SPARSE>;
+  auto kern = dkdv_kernel<T, D>;
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
-  { LaunchScope ls_(SPARSE ? "sparse_dkdv" : "dense_dkdv", stream); kern<<<grid, 160, smem, stream>>>(tmQ, tmDO, tmK, tmV, p); }
+  { LaunchScope ls_("sparse_dkdv", stream); kern<<<grid, 160, smem, stream>>>(tmQ, tmDO, tmK, tmV, p); }
   return cuda_rc(cudaGetLastError());
 }
 
@@ -725,10 +706,10 @@ static int launch_dkdv(const void* q, const void* dout, const void* k, const voi
 // Tokens per CTA of the dense dK/dV pass.  Long chunks amortise a key tile's loads and the adding of its sums; a small problem is
 // cut finer, down to four row tiles per CTA, until there are two CTAs for every SM (777 tokens x 2 heads, window 512: 48 CTAs of up
 // to 32 row tiles, 61 us, at 256 tokens).
-static int dense_chunk(int max_q, int max_k, int heads, int G, int D, int left) {
+static int dense_chunk(int max_q, int max_k, int heads, int G, int left) {
   int chunk = 256;
   while (chunk < 1024 && chunk * 16 < max_q) chunk <<= 1;
-  const int key_tile = D == 128 ? 128 : kKeyTile, least = D == 128 ? std::max(32, 4 * (128 / G)) : 32;
+  const int key_tile = 128, least = std::max(32, 4 * (128 / G));
   const long long tiles = (long long)((max_k + key_tile - 1) / key_tile) * heads;
   // tokens that see a key tile: all of them, half of them on average under the causal mask, a window
   const int span = left >= 0 ? std::min(max_q, left + key_tile) : (max_q + 1) / 2;
@@ -765,7 +746,7 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   p.window = window; p.stride = stride; p.causal = causal; p.left = left;
   p.scale2 = sm_scale * kLog2e; p.sm_scale = sm_scale;
   p.st.word = status_word();
-  if (left >= 0 && D != 128) return kUnsupported;  // the sliding window needs the tcgen05 dK/dV pass (head_dim 128)
+  if (left >= 0 && D != 128) return kUnsupported;  // the sliding window is built for head_dim 128
   {
     const int dt = DT<T>::kTmapType == CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 ? NSA_DTYPE_BF16 : NSA_DTYPE_FP16;
     const int rc = dense_dq_tc(k, v, S[2], S[3], S[4], S[5], total_q, total_k, max_q, D, dt, p, stream);
@@ -775,18 +756,11 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   d.ld = ld; d.dk32 = dk32; d.dv32 = dv32; d.cu_q = cu_q; d.cu_k = cu_k;
   d.offsets = nullptr; d.item_base = nullptr; d.item_bin = nullptr; d.item_counter = nullptr; d.list = nullptr;
   d.B = batch; d.Hq = Hq; d.Hkv = Hkv; d.G = G; d.TB = 0; d.NW = 1; d.block_size = kKeyTile;
-  d.chunk = dense_chunk(max_q, max_k, batch * Hkv, G, D, left);
-  const int chunk = d.chunk;
+  d.chunk = dense_chunk(max_q, max_k, batch * Hkv, G, left);
   d.window = window; d.stride = stride; d.causal = causal; d.left = left;
   d.scale2 = p.scale2; d.sm_scale = sm_scale; d.st = p.st;
   const long long ds[8] = {S[0], S[1], S[2], S[3], S[4], S[5], S[8], S[9]};
-  dim3 grid((max_k + kKeyTile - 1) / kKeyTile, (max_q + chunk - 1) / chunk, batch * Hkv);
-  int rc;
-  if constexpr (D == 128) {
-    rc = launch_dense_dkdv_tc<T>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream);
-  } else {
-    rc = launch_dkdv<T, D, false>(q, dout, k, v, ds, total_q, total_k, grid, d, stream);
-  }
+  const int rc = launch_dense_dkdv_tc<T, D>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream);
   if (rc) return rc;
   Converter cv;
   cv.add(dk32, dk, total_k, Hkv, D, S[12], S[13]);
@@ -805,11 +779,11 @@ static int sparse_chunk(int N, int Hkv, int topk) {
 
 // Token windows of the inverted index: as many tokens as keep the Q and dO rows of one KV-head group (G heads) within
 // about half of the L2 cache, a power of two, at least 1024.  Returns (tokens per window, windows).
-static bool sparse_fused_dq(int G, int D) { return D == 128 && G >= 4 && (G & (G - 1)) == 0; }
+static bool sparse_fused_dq(int G) { return G >= 4 && (G & (G - 1)) == 0; }
 
 static std::pair<int, int> sparse_windows(int N, int G, int D) {
   // Q and dO rows (16-bit) and, where the tcgen05 pass also produces dQ, the fp32 dQ accumulator rows it reduces into
-  const long long bytes_per_token = 2ll * G * D * 2 + (sparse_fused_dq(G, D) ? 4ll * G * D : 0);
+  const long long bytes_per_token = 2ll * G * D * 2 + (sparse_fused_dq(G) ? 4ll * G * D : 0);
   int W = 1024;
   while (2ll * W * bytes_per_token <= (64ll << 20)) W <<= 1;
   return {W, (N + W - 1) / W};
@@ -821,7 +795,7 @@ static size_t sparse_ws_bytes(int N, int batch, int Hq, int Hkv, int D, int topk
   return align_up((size_t)N * Hq * sizeof(float2), 256) + 2 * align_up((size_t)N * Hkv * D * sizeof(float), 256) +
          4 * align_up(x * sizeof(int), 256) + align_up((size_t)Hkv * N * topk * sizeof(int), 256) +
          align_up(((size_t)Hkv * N * topk / sparse_chunk(N, Hkv, topk) + x) * sizeof(int), 256) +
-         (sparse_fused_dq(Hq / Hkv, D) ? align_up((size_t)N * Hq * D * sizeof(float), 256) : 0);
+         (sparse_fused_dq(Hq / Hkv) ? align_up((size_t)N * Hq * D * sizeof(float), 256) : 0);
 }
 
 template <typename T, int D>
@@ -838,7 +812,7 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   uint8_t* w = static_cast<uint8_t*>(ws);
   float2* ld = reinterpret_cast<float2*>(w);
   w += align_up((size_t)N * Hq * sizeof(float2), 256);
-  const bool fused = sparse_fused_dq(G, D);  // dQ comes out of the tcgen05 dK/dV pass; otherwise the per-token dQ kernel runs
+  const bool fused = sparse_fused_dq(G);  // dQ comes out of the tcgen05 dK/dV pass; otherwise the per-token dQ kernel runs
   uint8_t* const zero_begin = w;
   float* dq32 = fused ? reinterpret_cast<float*>(w) : nullptr;
   if (fused) w += align_up((size_t)N * Hq * D * sizeof(float), 256);
@@ -920,13 +894,8 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   // upper bound on work items: every selection in a full chunk, plus one partial chunk per (head, block)
   const long long max_items = ((long long)Hkv * N * topk) / chunk + (long long)Hkv * NW * TB;
   dim3 grid((unsigned)max_items, block_size / kKeyTile, 1);
-  int rc;
-  if constexpr (D == 128) {
-    rc = (G >= 4 && (G & (G - 1)) == 0) ? launch_sparse_dkdv_tc<T>(q, dout, k, v, ds, N, grid, d, stream)
-                                                         : launch_dkdv<T, D, true>(q, dout, k, v, ds, N, N, grid, d, stream);
-  } else {
-    rc = launch_dkdv<T, D, true>(q, dout, k, v, ds, N, N, grid, d, stream);
-  }
+  const int rc = fused ? launch_sparse_dkdv_tc<T, D>(q, dout, k, v, ds, N, grid, d, stream)
+                       : launch_dkdv<T, D>(q, dout, k, v, ds, N, N, grid, d, stream);
   if (rc) return rc;
   Converter cv;
   if (fused) cv.add(dq32, dq, N, Hq, D, S[10], S[11]);

@@ -66,15 +66,15 @@ struct DenseBwdParams {
 int dense_dq_tc(const void* k, const void* v, long long k_sn, long long k_sh, long long v_sn, long long v_sh, int total_q,
                 int total_k, int max_seqlen_q, int head_dim, int dtype, DenseBwdParams p, cudaStream_t stream);
 
-// tcgen05 dK/dV pass of the top-k sparse attention (sparse_dkdv_tc.cu); head_dim 128, group size a power of two.
+// tcgen05 dK/dV pass of the top-k sparse attention (sparse_dkdv_tc.cu); head_dim 64 and 128, group size 4, 8 or 16.
 // strides: q_n q_h k_n k_h v_n v_h do_n do_h (elements); grid = (work items, 64-key tiles per block).
-template <typename T>
+template <typename T, int D>
 int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nk, dim3 grid,
                           DkdvParams p, cudaStream_t stream);
 
-// tcgen05 dK/dV pass of the dense attention with the keys as the M dimension (dense_dkdv_tc.cu); head_dim 128,
-// group size a power of two <= 16.  p.chunk = tokens per CTA (a multiple of 128).
-template <typename T>
+// tcgen05 dK/dV pass of the dense attention with the keys as the M dimension (dense_dkdv_tc.cu); head_dim 64 and
+// 128, group size a power of two <= 16.  p.chunk = tokens per CTA.
+template <typename T, int D>
 int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk,
                          int max_q, int max_k, int batch, DkdvParams p, cudaStream_t stream);
 

@@ -1,4 +1,4 @@
-// dK/dV pass of dense strided-causal attention on the 5th-generation tensor cores (head_dim 128),
+// dK/dV pass of dense strided-causal attention on the 5th-generation tensor cores (head_dim 64 and 128),
 // transposed formulation: the KEYS are the M dimension of every product.
 //
 // CTA = one tile of 128 keys (K and V tiles resident in SMEM) x a stream of row tiles; a row tile is
@@ -11,6 +11,9 @@
 // accumulating products read their A operand from tensor memory and the only shared-memory traffic of the
 // tensor pipe is one 128 x 128 operand per product.  A thread owns one key (TMEM lane); the per-row
 // statistics (lse, delta) are broadcast reads from a small SMEM table the producer warp fills.
+// At head_dim 64 the operands are one panel instead of two and the accumulating products have N = 64; the softmax threads, which
+// bound it there (the products of a tile take 900 clocks against 1900 of softmax), work on the same 128 x 128 logits.  It replaced
+// a kernel of mma.sync warps that owned 16 keys each and took tokens in pairs: 7833 tokens, 16q/2kv, 137 -> 38 us.
 //   warps 0..7 : two threads per key (64 of the 128 row columns each)
 //   warp 8     : TMA producer (Q ring of 3 tiles, dO ring of 2) and the per-row table
 //   warp 9     : TMEM allocation, MMA issue (one thread polls four queues: S, dP, dV, dK)
@@ -23,26 +26,25 @@ namespace nsa {
 namespace {
 constexpr int kQStages = 3;
 constexpr int kDoStages = 2;
-constexpr int kTileBytes = 128 * 128 * 2;  // any 128 x 128 operand tile of 16-bit elements: two panels of [128][64]
-constexpr int kPanelBytes = 128 * 128;
+constexpr int kPanelBytes = 128 * 128;  // [128][64] 16-bit elements; an operand tile of 128 x D is D / 64 of them
 
 __device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 }  // namespace
 
-template <typename T>
+template <typename T, int D>
 __global__ void __launch_bounds__(320, 1)
 dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, DkdvParams p, int logG) {
-  constexpr int D = 128;
   constexpr int KT = 128;
+  constexpr int PANELS = D / 64, TILE_BYTES = PANELS * kPanelBytes;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* k_sm = smem;
-  uint8_t* v_sm = k_sm + kTileBytes;
-  uint8_t* q_ring = v_sm + kTileBytes;
-  uint8_t* do_ring = q_ring + kQStages * kTileBytes;
-  float* nlse_sh = reinterpret_cast<float*>(do_ring + kDoStages * kTileBytes);  // [2][128]  -lse (base 2)
+  uint8_t* v_sm = k_sm + TILE_BYTES;
+  uint8_t* q_ring = v_sm + TILE_BYTES;
+  uint8_t* do_ring = q_ring + kQStages * TILE_BYTES;
+  float* nlse_sh = reinterpret_cast<float*>(do_ring + kDoStages * TILE_BYTES);  // [2][128]  -lse (base 2)
   float* dsc_sh = nlse_sh + 2 * 128;                                              // [2][128]  delta * sm_scale
   uint64_t* bars = reinterpret_cast<uint64_t*>(dsc_sh + 2 * 128);
   uint64_t* kv_full = bars;
@@ -119,9 +121,9 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 8) {
     // ===================== producer =====================
     if (lane == 0) {
-      mbar_expect_tx(kv_full, 2 * kTileBytes);
+      mbar_expect_tx(kv_full, 2 * TILE_BYTES);
 #pragma unroll
-      for (int pn = 0; pn < 2; ++pn) {
+      for (int pn = 0; pn < PANELS; ++pn) {
         tma_load_3d(k_sm + pn * kPanelBytes, &tmK, kv_full, pn * 64, h, krow0);
         tma_load_3d(v_sm + pn * kPanelBytes, &tmV, kv_full, pn * 64, h, krow0);
       }
@@ -131,10 +133,10 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (lane == 0) {
         const int s = i % kQStages;
         if (i >= kQStages) mbar_wait(q_empty + s, ((i / kQStages) - 1) & 1, p.st);
-        mbar_expect_tx(q_full + s, kTileBytes);
+        mbar_expect_tx(q_full + s, TILE_BYTES);
 #pragma unroll
-        for (int pn = 0; pn < 2; ++pn)
-          tma_load_3d(q_ring + s * kTileBytes + pn * kPanelBytes, &tmQ, q_full + s, pn * 64, h * p.G, qs + tok0);
+        for (int pn = 0; pn < PANELS; ++pn)
+          tma_load_3d(q_ring + s * TILE_BYTES + pn * kPanelBytes, &tmQ, q_full + s, pn * 64, h * p.G, qs + tok0);
       }
       {
         const int s = i & 1;
@@ -154,10 +156,10 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (lane == 0) {
         const int s = i % kDoStages;
         if (i >= kDoStages) mbar_wait(do_empty + s, ((i / kDoStages) - 1) & 1, p.st);
-        mbar_expect_tx(do_full + s, kTileBytes);
+        mbar_expect_tx(do_full + s, TILE_BYTES);
 #pragma unroll
-        for (int pn = 0; pn < 2; ++pn)
-          tma_load_3d(do_ring + s * kTileBytes + pn * kPanelBytes, &tmDO, do_full + s, pn * 64, h * p.G, qs + tok0);
+        for (int pn = 0; pn < PANELS; ++pn)
+          tma_load_3d(do_ring + s * TILE_BYTES + pn * kPanelBytes, &tmDO, do_full + s, pn * 64, h * p.G, qs + tok0);
       }
       __syncwarp();
     }
@@ -166,7 +168,7 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // The whole warp runs the control flow (so that it stays warp-uniform and cheap); one elected lane issues.
     {
       const uint32_t idesc_s = umma_idesc<T>(128, 128, false, false);
-      const uint32_t idesc_t = umma_idesc<T>(128, 128, false, true);
+      const uint32_t idesc_t = umma_idesc<T>(128, D, false, true);
       const uint32_t k_addr = smem_u32(k_sm), v_addr = smem_u32(v_sm), q_base = smem_u32(q_ring), do_base = smem_u32(do_ring);
       auto issue_logits = [&](uint32_t a_addr, uint32_t b_addr, uint32_t d_tmem, uint64_t* bar) {
         if (elect_one()) {
@@ -192,25 +194,25 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         bool progressed = false;
         if (nv < ns && nv < np && mbar_test(p_full, nv & 1)) {
           tc_fence_after_sync();
-          issue_grad(tmem + 256, do_base + (nv % kDoStages) * kTileBytes, tmem, nv == 0, do_empty + (nv % kDoStages));
+          issue_grad(tmem + 256, do_base + (nv % kDoStages) * TILE_BYTES, tmem, nv == 0, do_empty + (nv % kDoStages));
           ++nv;
           progressed = true;
         }
         if (ns < ntiles && ns == nv && mbar_test(q_full + (ns % kQStages), (ns / kQStages) & 1)) {
           tc_fence_after_sync();
-          issue_logits(k_addr, q_base + (ns % kQStages) * kTileBytes, tmem + 256, s_full);
+          issue_logits(k_addr, q_base + (ns % kQStages) * TILE_BYTES, tmem + 256, s_full);
           ++ns;
           progressed = true;
         }
         if (nk < np && mbar_test(ds_full, nk & 1)) {
           tc_fence_after_sync();
-          issue_grad(tmem + 384, q_base + (nk % kQStages) * kTileBytes, tmem + 128, nk == 0, q_empty + (nk % kQStages));
+          issue_grad(tmem + 384, q_base + (nk % kQStages) * TILE_BYTES, tmem + 128, nk == 0, q_empty + (nk % kQStages));
           ++nk;
           progressed = true;
         }
         if (np < ntiles && np == nk && mbar_test(do_full + (np % kDoStages), (np / kDoStages) & 1)) {
           tc_fence_after_sync();
-          issue_logits(v_addr, do_base + (np % kDoStages) * kTileBytes, tmem + 384, dp_full);
+          issue_logits(v_addr, do_base + (np % kDoStages) * TILE_BYTES, tmem + 384, dp_full);
           ++np;
           progressed = true;
         }
@@ -327,16 +329,16 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         mbar_arrive(meta_empty + ms);
       }
     }
-    // ---- drain: thread (key, half) adds 64 of the 128 d columns of its key's dV and dK rows ----
+    // ---- drain: thread (key, half) adds half of the d columns of its key's dV and dK rows ----
     mbar_wait(all_done, 0, p.st);
     tc_fence_after_sync();
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
-      float* dst = (which == 0 ? p.dv32 : p.dk32) + ((size_t)(krow0 + key) * p.Hkv + h) * D + half * 64;
+      float* dst = (which == 0 ? p.dv32 : p.dk32) + ((size_t)(krow0 + key) * p.Hkv + h) * D + half * (D / 2);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < D / 64; ++c) {
         uint32_t r[32];
-        tmem_ld32(lane_base + which * 128 + half * 64 + c * 32, r);
+        tmem_ld32(lane_base + which * 128 + half * (D / 2) + c * 32, r);
         tmem_ld_wait();
         if (key_ok) {
 #pragma unroll
@@ -352,10 +354,10 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
-template <typename T>
+template <typename T, int D>
 int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk,
                          int max_q, int max_k, int batch, DkdvParams p, cudaStream_t stream) {
-  constexpr int D = 128;
+  constexpr int TILE_BYTES = D / 64 * kPanelBytes;
   int logG = 0;
   while ((1 << logG) < p.G) ++logG;
   const int TPT = 128 >> logG;
@@ -368,8 +370,8 @@ int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const v
   if (rc) return rc;
   rc = make_tmap_3d(&tmV, DT<T>::kTmapType, v, D, p.Hkv, Nk, strides[5], strides[4], 64, 1, 128);
   if (rc) return rc;
-  const size_t smem = (size_t)(2 + kQStages + kDoStages) * kTileBytes + 4 * 128 * sizeof(float) + 24 * sizeof(uint64_t) + 16;
-  auto kern = dense_dkdv_tc_kernel<T>;
+  const size_t smem = (size_t)(2 + kQStages + kDoStages) * TILE_BYTES + 4 * 128 * sizeof(float) + 24 * sizeof(uint64_t) + 16;
+  auto kern = dense_dkdv_tc_kernel<T, D>;
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_k + 127) / 128, (max_q + p.chunk - 1) / p.chunk, batch * p.Hkv);
@@ -377,9 +379,13 @@ int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const v
   return cuda_rc(cudaGetLastError());
 }
 
-template int launch_dense_dkdv_tc<__nv_bfloat16>(const void*, const void*, const void*, const void*, const long long*, int, int, int,
-                                                 int, int, DkdvParams, cudaStream_t);
-template int launch_dense_dkdv_tc<__half>(const void*, const void*, const void*, const void*, const long long*, int, int, int, int,
-                                          int, DkdvParams, cudaStream_t);
+#define NSA_INSTANTIATE(T, D)                                                                                                         \
+  template int launch_dense_dkdv_tc<T, D>(const void*, const void*, const void*, const void*, const long long*, int, int, int, int, int, \
+                                          DkdvParams, cudaStream_t)
+NSA_INSTANTIATE(__nv_bfloat16, 64);
+NSA_INSTANTIATE(__nv_bfloat16, 128);
+NSA_INSTANTIATE(__half, 64);
+NSA_INSTANTIATE(__half, 128);
+#undef NSA_INSTANTIATE
 
 }  // namespace nsa

@@ -1,4 +1,4 @@
-// dK/dV pass of the top-k sparse attention on the 5th-generation tensor cores (head_dim 128).
+// dK/dV pass of the top-k sparse attention on the 5th-generation tensor cores (head_dim 64 and 128).
 //
 // Work item = one tile of 64 keys of a selected block (K and V tile resident in SMEM) x a stream of row tiles taken from
 // the block's inverted index (the tokens that selected it); a row tile is 128 rows = (128/G tokens) x (G query
@@ -41,6 +41,14 @@
 //                 phases behind every full reduction queue and the two costs added up (11.6 ms at 64 K tokens; 10.1 ms
 //                 with these warps, of which 8.5 ms remain when the reductions are left out).
 // TMEM columns: S0 [0,64) S1 [64,128) dP0 [128,192) dP1 [192,256) dV^T [256,320) dK^T [320,384) dQ [384,512).
+//
+// head_dim 64: d alone is half a row dimension, so two operands are stacked to fill it.  A stage holds a tile's dO and Q rows as
+// two panels of one 128-row operand and a P/dS pair its two tiles as panels of one 128-column operand, and ONE product
+//     [dO^T; Q^T] [P dS]     [128 x 128]           dV^T is its upper left quadrant, dK^T its lower right one
+// takes the place of two with M = 64 (512 clocks; the other two quadrants are computed and never read); [K^T; V^T] dS^T gives
+// dQ^T in its upper half.  Tiles and stages are half as large, so P/dS pairs are double-buffered and both row rings have three
+// stages.  Measured against the mma.sync kernels that served head_dim 64 before (16 rows per warp, dQ by a per-token kernel of its
+// own): 7833 tokens, 16q/2kv, top-8: 516 -> 128 us.
 #include <algorithm>
 
 #include "attn_bwd.h"
@@ -50,13 +58,20 @@
 namespace nsa {
 
 namespace {
-constexpr int kSpQStages = 3;
-constexpr int kSpDoStages = 2;
-constexpr int kSpRowBytes = 128 * 128 * 2;  // Q or dO rows of one tile: 32 KB, 2 panels of [128 rows][64 d]
-constexpr int kSpRowPanel = 128 * 128;
-constexpr int kSpKvBytes = 64 * 128 * 2;    // K or V tile: 16 KB, 2 panels of [64 keys][64 d]
-constexpr int kSpKvPanel = 64 * 128;
+constexpr int kSpRowPanel = 128 * 128;      // [128 rows][64 d]
+constexpr int kSpKvPanel = 64 * 128;        // [64 keys][64 d]
 constexpr int kSpPdBytes = 128 * 64 * 2;    // P or dS tile [128 rows][64 keys]: one panel
+template <int D>
+struct SpCfg {
+  static constexpr int kPanels = D / 64;
+  static constexpr int kQStages = 3, kDoStages = D == 128 ? 2 : 3;
+  static constexpr int kPdBufs = D == 128 ? 1 : 2;             // P/dS pairs
+  static constexpr int kRowBytes = kPanels * kSpRowPanel;      // Q or dO rows of one tile
+  static constexpr int kKvBytes = kPanels * kSpKvPanel;        // K or V tile
+  static constexpr int kQStride = D == 128 ? kRowBytes : 2 * kRowBytes, kDoStride = kQStride;  // from a stage to the next
+  static constexpr int kRings = (kQStages + kDoStages) * kRowBytes;
+  static constexpr size_t kSmem = 2 * kKvBytes + kPdBufs * 2 * kSpPdBytes + kRings + 48 * sizeof(uint64_t) + 64;
+};
 constexpr int kSpThreads = 17 * 32;
 constexpr int kSpItemQ = 4;                // entries of a CTA's queue of work items
 
@@ -79,36 +94,38 @@ __device__ __forceinline__ int ld_i32_here(const int* ptr) {
   return v;
 }
 
-template <typename T, int LOGG>
+template <typename T, int LOGG, int D>
 __global__ void __launch_bounds__(kSpThreads, 1)
 sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const T* __restrict__ q,
                       const T* __restrict__ dout, long long q_sn, long long q_sh, long long do_sn, long long do_sh, DkdvParams p) {
   constexpr int logG = LOGG;
   constexpr int G = 1 << LOGG;
-  constexpr int D = 128;
   constexpr int KT = 64;
+  using C = SpCfg<D>;
+  constexpr int PANELS = C::kPanels, NB = C::kPdBufs;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* k_sm = smem;
-  uint8_t* v_sm = k_sm + kSpKvBytes;
-  uint8_t* p_sm = v_sm + kSpKvBytes;
+  uint8_t* v_sm = k_sm + C::kKvBytes;
+  uint8_t* p_sm = v_sm + C::kKvBytes;              // [NB] pairs of a P and a dS tile
   uint8_t* ds_sm = p_sm + kSpPdBytes;
-  uint8_t* q_ring = ds_sm + kSpPdBytes;
-  uint8_t* do_ring = q_ring + kSpQStages * kSpRowBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(do_ring + kSpDoStages * kSpRowBytes);
+  uint8_t* rings = p_sm + NB * 2 * kSpPdBytes;
+  uint8_t* q_ring = D == 128 ? rings : rings + C::kRowBytes;                      // head_dim 64: dO and Q of a stage side by side
+  uint8_t* do_ring = D == 128 ? rings + C::kQStages * C::kRowBytes : rings;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(rings + C::kRings);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;
-  uint64_t* q_empty = q_full + kSpQStages;
-  uint64_t* do_full = q_empty + kSpQStages;
-  uint64_t* do_empty = do_full + kSpDoStages;
-  uint64_t* s_full = do_empty + kSpDoStages;  // [2]
+  uint64_t* q_empty = q_full + C::kQStages;
+  uint64_t* do_full = q_empty + C::kQStages;
+  uint64_t* do_empty = do_full + C::kDoStages;
+  uint64_t* s_full = do_empty + C::kDoStages;  // [2]
   uint64_t* s_empty = s_full + 2;             // [2]
   uint64_t* dp_full = s_empty + 2;            // [2]
   uint64_t* dp_empty = dp_full + 2;           // [2]
-  uint64_t* p_full = dp_empty + 2;
-  uint64_t* p_empty = p_full + 1;
-  uint64_t* ds_full = p_empty + 1;
-  uint64_t* ds_empty = ds_full + 1;
-  uint64_t* all_done = ds_empty + 1;
+  uint64_t* p_full = dp_empty + 2;            // [NB] each
+  uint64_t* p_empty = p_full + NB;
+  uint64_t* ds_full = p_empty + NB;
+  uint64_t* ds_empty = ds_full + NB;
+  uint64_t* all_done = ds_empty + NB;
   uint64_t* dq_full = all_done + 1;
   uint64_t* dq_empty = dq_full + 1;
   uint64_t* acc_free = dq_empty + 1;          // the dV / dK accumulators of the previous item have been read out
@@ -159,11 +176,11 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < kSpQStages; ++s) {
+    for (int s = 0; s < C::kQStages; ++s) {
       mbar_init(q_full + s, 64);
       mbar_init(q_empty + s, 1);
     }
-    for (int s = 0; s < kSpDoStages; ++s) {
+    for (int s = 0; s < C::kDoStages; ++s) {
       mbar_init(do_full + s, 64);
       mbar_init(do_empty + s, 1);
     }
@@ -173,13 +190,15 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       mbar_init(dp_full + s, 1);
       mbar_init(dp_empty + s, 8);
     }
-    mbar_init(p_full, 8);
-    mbar_init(p_empty, 1);
-    mbar_init(ds_full, 8);
-    mbar_init(ds_empty, with_dq ? 2 : 1);  // dK, and dQ when it is produced, read the dS tile
+    for (int s = 0; s < NB; ++s) {
+      mbar_init(p_full + s, 8);
+      mbar_init(p_empty + s, 1);
+      mbar_init(ds_full + s, 8);
+      mbar_init(ds_empty + s, with_dq ? 2 : 1);  // dK, and dQ when it is produced, read the dS tile
+    }
     mbar_init(all_done, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 4);
+    mbar_init(dq_empty, D / 32);  // the warps that drain it
     mbar_init(acc_free, 8);
     for (int s = 0; s < kSpItemQ; ++s) {
       mbar_init(iq_full + s, 1);
@@ -224,8 +243,8 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     // ===================== loaders: group 0 (warps 8,9) tiles with even j, group 1 (warps 10,11) odd j =====================
     const int grp = (warp - 8) >> 1;
     const int tl = threadIdx.x - (8 + 2 * grp) * 32;  // 0..63
-    const int chunk16 = tl & 15;                      // which 16 bytes of the row's 256
-    const int row_in_step = tl >> 4;                  // 4 rows per step
+    const int chunk16 = tl % (D / 8);                 // which 16 bytes of the row
+    const int row_in_step = tl / (D / 8);             // 4 rows per step (head_dim 64: 8)
     const uint32_t pn_off = (chunk16 >> 3) * kSpRowPanel;
     const int c8 = chunk16 & 7;
     int gt = 0;
@@ -260,26 +279,37 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
           // not depend on the token is folded into constants so that a copy costs a handful of instructions.
           auto gather = [&](const T* src, long long sn, long long sh, long long row0, uint32_t dst_base) {
             const uint32_t dst0 = dst_base + pn_off + row_in_step * 128;
-            const uint32_t sw0 = (uint32_t)((c8 ^ row_in_step) << 4), sw1 = (uint32_t)((c8 ^ (row_in_step + 4)) << 4);
-            const T* src0 = src + row0 + (long long)row_in_step * sh;
+            if constexpr (D == 64) {
+              const uint32_t sw = (uint32_t)((c8 ^ row_in_step) << 4);
 #pragma unroll 4
-            for (int slot = 0; slot < (128 >> LOGG); ++slot) {
-              const int n = __shfl_sync(0xffffffffu, my_n, slot);
-              const bool ok = n >= 0;
-              const T* g = src0 + (long long)(ok ? n : 0) * sn;
+              for (int st = 0; st < 16; ++st) {
+                const int r = st * 8 + row_in_step;
+                const int n = __shfl_sync(0xffffffffu, my_n, r >> LOGG);
+                const bool ok = n >= 0;
+                cp_async16(dst0 + st * 1024 + sw, src + row0 + (long long)(ok ? n : 0) * sn + (long long)(r & (G - 1)) * sh, ok);
+              }
+            } else {
+              const uint32_t sw0 = (uint32_t)((c8 ^ row_in_step) << 4), sw1 = (uint32_t)((c8 ^ (row_in_step + 4)) << 4);
+              const T* src0 = src + row0 + (long long)row_in_step * sh;
+#pragma unroll 4
+              for (int slot = 0; slot < (128 >> LOGG); ++slot) {
+                const int n = __shfl_sync(0xffffffffu, my_n, slot);
+                const bool ok = n >= 0;
+                const T* g = src0 + (long long)(ok ? n : 0) * sn;
 #pragma unroll
-              for (int jj = 0; jj < G / 4; ++jj) {
-                const int jr = slot * (G / 4) + jj;  // r = 4 jr + row_in_step; r & 7 = row_in_step + 4 (jr & 1)
-                cp_async16(dst0 + jr * 512 + ((jr & 1) ? sw1 : sw0), g + (long long)(4 * jj) * sh, ok);  // missing tokens: zero fill
+                for (int jj = 0; jj < G / 4; ++jj) {
+                  const int jr = slot * (G / 4) + jj;  // r = 4 jr + row_in_step; r & 7 = row_in_step + 4 (jr & 1)
+                  cp_async16(dst0 + jr * 512 + ((jr & 1) ? sw1 : sw0), g + (long long)(4 * jj) * sh, ok);  // missing tokens: zero fill
+                }
               }
             }
           };
-          const int sq = j % kSpQStages, sd = j % kSpDoStages;
-          if (j >= kSpQStages) mbar_wait(q_empty + sq, ((j / kSpQStages) - 1) & 1, p.st);
-          gather(q, q_sn, q_sh, q_row0, smem_u32(q_ring + sq * kSpRowBytes));
+          const int sq = j % C::kQStages, sd = j % C::kDoStages;
+          if (j >= C::kQStages) mbar_wait(q_empty + sq, ((j / C::kQStages) - 1) & 1, p.st);
+          gather(q, q_sn, q_sh, q_row0, smem_u32(q_ring + sq * C::kQStride));
           cp_async_commit();
-          if (j >= kSpDoStages) mbar_wait(do_empty + sd, ((j / kSpDoStages) - 1) & 1, p.st);
-          gather(dout, do_sn, do_sh, do_row0, smem_u32(do_ring + sd * kSpRowBytes));
+          if (j >= C::kDoStages) mbar_wait(do_empty + sd, ((j / C::kDoStages) - 1) & 1, p.st);
+          gather(dout, do_sn, do_sh, do_row0, smem_u32(do_ring + sd * C::kDoStride));
           cp_async_commit();
           cp_async_wait<1>();
           fence_proxy_async();  // the tensor pipe reads these bytes through the async proxy
@@ -297,7 +327,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   } else if (warp == 12) {
     // ===================== K/V load and MMA issue (converged warp, elected lane issues) =====================
     const uint32_t idesc_s = umma_idesc<T>(128, KT, false, false);
-    const uint32_t idesc_t = umma_idesc<T>(128, KT, true, true);
+    const uint32_t idesc_t = umma_idesc<T>(128, D == 128 ? KT : 2 * KT, true, true);
     const uint32_t k_addr = smem_u32(k_sm), v_addr = smem_u32(v_sm), p_addr = smem_u32(p_sm), ds_addr = smem_u32(ds_sm);
     const uint32_t q_base = smem_u32(q_ring), do_base = smem_u32(do_ring);
     // S/dP: A = rows (two [128][64] panels), B = K or V tile (two [64][64] panels)
@@ -324,15 +354,29 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       }
       __syncwarp();
     };
-    // dQ^T = K^T dS^T: A = K tile MN-major (d as M over two panels, 16 keys = 2048 bytes), B = dS tile K-major (one panel)
+    // dQ^T = K^T dS^T: A = K tile MN-major (d as M over two panels, 16 keys = 2048 bytes; head_dim 64: the K tile and the V tile
+    // behind it), B = dS tile K-major (one panel)
     const uint32_t idesc_q = umma_idesc<T>(128, 128, true, false);
-    auto issue_dq = [&](uint32_t d_tmem) {
+    auto issue_dq = [&](uint32_t d_tmem, uint32_t ds_addr, uint64_t* bar_tile) {
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk)
           umma_ss(d_tmem, umma_desc_mnmajor(k_addr + kk * 2048, kSpKvPanel), umma_desc_kmajor(ds_addr + kk * 32), idesc_q, kk > 0);
         umma_commit(dq_full);
-        umma_commit(ds_empty);
+        umma_commit(bar_tile);
+      }
+      __syncwarp();
+    };
+    auto issue_pair = [&](uint32_t a_addr, uint32_t b_addr, bool first, int stage, int buf) {
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 128 / 16; ++kk)
+          umma_ss(tmem + 256, umma_desc_mnmajor(a_addr + kk * 2048, kSpRowPanel), umma_desc_mnmajor(b_addr + kk * 2048, kSpPdBytes), idesc_t,
+                  !first || kk > 0);
+        umma_commit(do_empty + stage);
+        umma_commit(q_empty + stage);
+        umma_commit(p_empty + buf);
+        umma_commit(ds_empty + buf);
       }
       __syncwarp();
     };
@@ -350,9 +394,9 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       if (cur.ntiles > 0) {
         // every product of the item before has completed (waited for at its end): its K/V tile can be replaced
         if (elect_one()) {
-          mbar_expect_tx(kv_full, 2 * kSpKvBytes);
+          mbar_expect_tx(kv_full, 2 * C::kKvBytes);
 #pragma unroll
-          for (int pn = 0; pn < 2; ++pn) {
+          for (int pn = 0; pn < PANELS; ++pn) {
             tma_load_3d(k_sm + pn * kSpKvPanel, &tmK, kv_full, pn * 64, cur.h, cur.krow0);
             tma_load_3d(v_sm + pn * kSpKvPanel, &tmV, kv_full, pn * 64, cur.h, cur.krow0);
           }
@@ -368,35 +412,40 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         while (alive && (nk < end || nq < end)) {
           bool progressed = false;
           if (!acc_ok) acc_ok = mbar_test(acc_free, (n_done - 1) & 1);
-          if (nq < np && nq < end && mbar_test(ds_full, nq & 1) && (nq == 0 || mbar_test(dq_empty, (nq - 1) & 1))) {
+          if (nq < np && nq < end && mbar_test(ds_full + nq % NB, (nq / NB) & 1) && (nq == 0 || mbar_test(dq_empty, (nq - 1) & 1))) {
             tc_fence_after_sync();
-            issue_dq(tmem + 384);
+            issue_dq(tmem + 384, ds_addr + (nq % NB) * 2 * kSpPdBytes, ds_empty + nq % NB);
             ++nq;
             progressed = true;
           }
-          if (acc_ok && nv < np && mbar_test(p_full, nv & 1)) {
-            tc_fence_after_sync();
-            issue_grad(do_base + (nv % kSpDoStages) * kSpRowBytes, p_addr, tmem + 256, nv == gt, do_empty + (nv % kSpDoStages), p_empty);
-            ++nv;
-            progressed = true;
+          if constexpr (D == 128) {
+            if (acc_ok && nv < np && mbar_test(p_full, nv & 1)) {
+              tc_fence_after_sync();
+              issue_grad(do_base + (nv % C::kDoStages) * C::kDoStride, p_addr, tmem + 256, nv == gt, do_empty + (nv % C::kDoStages), p_empty);
+              ++nv;
+              progressed = true;
+            }
           }
-          if (ns < end && mbar_test(q_full + (ns % kSpQStages), (ns / kSpQStages) & 1) &&
+          if (ns < end && mbar_test(q_full + (ns % C::kQStages), (ns / C::kQStages) & 1) &&
               (ns < 2 || mbar_test(s_empty + (ns & 1), ((ns >> 1) - 1) & 1))) {
             tc_fence_after_sync();
-            issue_logits(q_base + (ns % kSpQStages) * kSpRowBytes, k_addr, tmem + (ns & 1) * KT, s_full + (ns & 1));
+            issue_logits(q_base + (ns % C::kQStages) * C::kQStride, k_addr, tmem + (ns & 1) * KT, s_full + (ns & 1));
             ++ns;
             progressed = true;
           }
-          if (acc_ok && nk < np && nk < end && mbar_test(ds_full, nk & 1)) {
+          if (acc_ok && nk < np && nk < end && mbar_test(ds_full + nk % NB, (nk / NB) & 1)) {
             tc_fence_after_sync();
-            issue_grad(q_base + (nk % kSpQStages) * kSpRowBytes, ds_addr, tmem + 320, nk == gt, q_empty + (nk % kSpQStages), ds_empty);
+            if constexpr (D == 128)
+              issue_grad(q_base + (nk % C::kQStages) * C::kQStride, ds_addr, tmem + 320, nk == gt, q_empty + (nk % C::kQStages), ds_empty);
+            else  // dS written, P is too (by the same threads, before it): both gradients in one product over the stacked operands
+              issue_pair(do_base + (nk % C::kDoStages) * C::kDoStride, p_addr + (nk % NB) * 2 * kSpPdBytes, nk == gt, nk % C::kQStages, nk % NB);
             ++nk;
             progressed = true;
           }
-          if (np < ns && mbar_test(do_full + (np % kSpDoStages), (np / kSpDoStages) & 1) &&
+          if (np < ns && mbar_test(do_full + (np % C::kDoStages), (np / C::kDoStages) & 1) &&
               (np < 2 || mbar_test(dp_empty + (np & 1), ((np >> 1) - 1) & 1))) {
             tc_fence_after_sync();
-            issue_logits(do_base + (np % kSpDoStages) * kSpRowBytes, v_addr, tmem + 128 + (np & 1) * KT, dp_full + (np & 1));
+            issue_logits(do_base + (np % C::kDoStages) * C::kDoStride, v_addr, tmem + 128 + (np & 1) * KT, dp_full + (np & 1));
             ++np;
             progressed = true;
           }
@@ -424,7 +473,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
   } else if (warp >= 13) {
     // ===================== dQ drain: lane = d, 128 columns = the rows of the tile =====================
-    if (with_dq) {
+    if (with_dq && (D == 128 || (warp & 3) < 2)) {  // head_dim 64: the upper half of the lanes holds dQ^T
       constexpr int SPC = 32 >> LOGG;  // tokens (slots) per chunk of 32 columns
       const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 384;
       int gt = 0;
@@ -485,7 +534,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     const int row = (warp & 3) * 32 + lane;
     const int slot = row >> logG;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t prow = smem_u32(p_sm) + row * 128, dsrow = smem_u32(ds_sm) + row * 128;
+    const uint32_t prow0 = smem_u32(p_sm) + row * 128;
     int gt = 0, n_done = 0;
     bool alive = true;
     int item = take(0);
@@ -505,6 +554,8 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         for (int i = 0; i < ntiles && alive; ++i) {
           const int j = gt + i;
           const int bsel = j & 1;
+          const int pd = j % NB;
+          const uint32_t prow = prow0 + pd * 2 * kSpPdBytes, dsrow = prow + kSpPdBytes;
           const int n_next2 = token_of(i + 2);
           const float2 ld_next = stats_of(n_next);
           // keys of this tile the row may see: those at or before its own position
@@ -539,7 +590,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             uint32_t pw[16];
 #pragma unroll
             for (int c2 = 0; c2 < 16; ++c2) pw[c2] = DT<T>::pack(pf[2 * c2], pf[2 * c2 + 1]);
-            if (j > 0) mbar_wait(p_empty, (j - 1) & 1, p.st);  // dV of the previous tile has read the P tile
+            if (j >= NB) mbar_wait(p_empty + pd, (j / NB - 1) & 1, p.st);  // dV of the tile that had the P buffer has read it
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4)
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(prow + (((half * 4 + c4) ^ (row & 7)) << 4)), "r"(pw[c4 * 4]),
@@ -547,7 +598,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
           }
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0) mbar_arrive(p_full);
+          if (lane == 0) mbar_arrive(p_full + pd);
 
           // ---- dS phase ----
           if (!mbar_wait(dp_full + bsel, (j >> 1) & 1, p.st)) { alive = false; break; }
@@ -567,7 +618,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
               const float2 d2 = fmul2(make_float2(pf[c2], pf[c2 + 1]), t2);
               dw[c2 >> 1] = DT<T>::pack(d2.x, d2.y);
             }
-            if (j > 0) mbar_wait(ds_empty, (j - 1) & 1, p.st);  // dK (and dQ) of the previous tile have read the dS tile
+            if (j >= NB) mbar_wait(ds_empty + pd, (j / NB - 1) & 1, p.st);  // dK (and dQ) have read the dS buffer
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4)
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(dsrow + (((half * 4 + c4) ^ (row & 7)) << 4)), "r"(dw[c4 * 4]),
@@ -575,7 +626,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
           }
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0) mbar_arrive(ds_full);
+          if (lane == 0) mbar_arrive(ds_full + pd);
           n_cur = n_next;
           n_next = n_next2;
           ld_cur = ld_next;
@@ -584,23 +635,39 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         // ---- read out dV and dK of this item: thread (d, half) holds column d for 32 of the 64 keys ----
         if (!mbar_wait(all_done, n_done & 1, p.st)) { alive = false; break; }
         tc_fence_after_sync();
-        const int d = row;
-        uint32_t rv[32], rk[32];
-        tmem_ld32(lane_base + 256 + half * 32, rv);
-        tmem_ld32(lane_base + 320 + half * 32, rk);
-        tmem_ld_wait();
-        // the accumulators are in registers: the next item's dV / dK products may start
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_free);
-        float* dstv = p.dv32 + ((size_t)krow0 * p.Hkv + h) * D + d;
-        float* dstk = p.dk32 + ((size_t)krow0 * p.Hkv + h) * D + d;
+        if constexpr (D == 128) {
+          const int d = row;
+          uint32_t rv[32], rk[32];
+          tmem_ld32(lane_base + 256 + half * 32, rv);
+          tmem_ld32(lane_base + 320 + half * 32, rk);
+          tmem_ld_wait();
+          // the accumulators are in registers: the next item's dV / dK products may start
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_free);
+          float* dstv = p.dv32 + ((size_t)krow0 * p.Hkv + h) * D + d;
+          float* dstk = p.dk32 + ((size_t)krow0 * p.Hkv + h) * D + d;
 #pragma unroll
-        for (int c2 = 0; c2 < 32; ++c2) {
-          const int key = half * 32 + c2;
-          if (key < kvalid) {
-            atomicAdd(dstv + (size_t)key * p.Hkv * D, __uint_as_float(rv[c2]));
-            atomicAdd(dstk + (size_t)key * p.Hkv * D, __uint_as_float(rk[c2]));
+          for (int c2 = 0; c2 < 32; ++c2) {
+            const int key = half * 32 + c2;
+            if (key < kvalid) {
+              atomicAdd(dstv + (size_t)key * p.Hkv * D, __uint_as_float(rv[c2]));
+              atomicAdd(dstk + (size_t)key * p.Hkv * D, __uint_as_float(rk[c2]));
+            }
+          }
+        } else {  // lanes below 64 hold a column of dV in the left half of the product, lanes above one of dK in the right half
+          const bool is_v = (warp & 3) < 2;
+          uint32_t r[32];
+          tmem_ld32(lane_base + (is_v ? 256 : 320) + half * 32, r);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_free);
+          float* dst = (is_v ? p.dv32 : p.dk32) + ((size_t)krow0 * p.Hkv + h) * D + (row & 63);
+#pragma unroll
+          for (int c2 = 0; c2 < 32; ++c2) {
+            const int key = half * 32 + c2;
+            if (key < kvalid) atomicAdd(dst + (size_t)key * p.Hkv * D, __uint_as_float(r[c2]));
           }
         }
         gt += ntiles;
@@ -615,10 +682,9 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   if (warp == 12) tmem_dealloc(tmem, 512);
 }
 
-template <typename T>
+template <typename T, int D>
 int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nk, dim3 grid,
                           DkdvParams p, cudaStream_t stream) {
-  constexpr int D = 128;
   int logG = 0;
   while ((1 << logG) < p.G) ++logG;
   CUtensorMap tmK, tmV;
@@ -626,7 +692,7 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
   if (rc) return rc;
   rc = make_tmap_3d(&tmV, DT<T>::kTmapType, v, D, p.Hkv, Nk, strides[5], strides[4], 64, 1, 64);
   if (rc) return rc;
-  const size_t smem = 2 * kSpKvBytes + 2 * kSpPdBytes + (kSpQStages + kSpDoStages) * kSpRowBytes + 48 * sizeof(uint64_t) + 64;
+  const size_t smem = SpCfg<D>::kSmem;
   auto launch = [&](auto kern) -> int {
     cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
@@ -641,16 +707,19 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
     return cuda_rc(cudaGetLastError());
   };
   switch (logG) {
-    case 2: return launch(sparse_dkdv_tc_kernel<T, 2>);
-    case 3: return launch(sparse_dkdv_tc_kernel<T, 3>);
-    case 4: return launch(sparse_dkdv_tc_kernel<T, 4>);
+    case 2: return launch(sparse_dkdv_tc_kernel<T, 2, D>);
+    case 3: return launch(sparse_dkdv_tc_kernel<T, 3, D>);
+    case 4: return launch(sparse_dkdv_tc_kernel<T, 4, D>);
     default: return kUnsupported;
   }
 }
 
-template int launch_sparse_dkdv_tc<__nv_bfloat16>(const void*, const void*, const void*, const void*, const long long*, int, dim3,
-                                                  DkdvParams, cudaStream_t);
-template int launch_sparse_dkdv_tc<__half>(const void*, const void*, const void*, const void*, const long long*, int, dim3, DkdvParams,
-                                           cudaStream_t);
+#define NSA_INSTANTIATE(T, D) \
+  template int launch_sparse_dkdv_tc<T, D>(const void*, const void*, const void*, const void*, const long long*, int, dim3, DkdvParams, cudaStream_t)
+NSA_INSTANTIATE(__nv_bfloat16, 64);
+NSA_INSTANTIATE(__nv_bfloat16, 128);
+NSA_INSTANTIATE(__half, 64);
+NSA_INSTANTIATE(__half, 128);
+#undef NSA_INSTANTIATE
 
 }  // namespace nsa
