@@ -18,6 +18,7 @@
 //     parts.  The length counters, shared by the heads of a sequence, are advanced by the last of its clusters to have read
 //     them.
 #include "attn_tile.cuh"
+#include "cluster.cuh"
 #include "decode_cluster.h"
 #include "dispatch.h"
 #include "host_util.h"
@@ -69,42 +70,6 @@ struct Params {
   Status st;
 };
 
-// ---- cluster primitives ----
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-// every thread of the cluster has arrived; global and (distributed) shared memory written before is visible after
-__device__ __forceinline__ void cluster_barrier() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ float2 ld_peer2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_peer4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ int ld_peer_i(uint32_t a) {
-  int v;
-  asm volatile("ld.shared::cluster.b32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_peer(uint32_t a, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory");
-}
-
 template <int D, int NW>
 struct Layout {
   static constexpr int kTile = kSub * D * 2;               // K or V sub-tile
@@ -117,8 +82,9 @@ struct Layout {
   static constexpr int kWts = kMlc + 2 * 16 * 8;           // float [2][kMaxCluster][16]: weight of every CTA's partial output
   static constexpr int kLse = kWts + 2 * kMaxCluster * 16 * 4;  // float [16]
   static constexpr int kList = kLse + 64;                  // int [kMaxList + kMaxSelTiles]: sub-tile rows; selected blocks
-  static constexpr int kQ = (kList + (kMaxList + kMaxSelTiles) * 4 + 127) / 128 * 128;  // step: [16][D] rotated query, 16-bit
-  static constexpr int kTrig = kQ + 16 * D * 2;            // step: float [4][D / 2] cos / sin of the two positions
+  static constexpr int kQ = (kList + (kMaxList + kMaxSelTiles) * 4 + 127) / 128 * 128;  // step: [16][kQLd] rotated query, 16-bit
+  static constexpr int kQLd = D + 8;                       // elements per row of the rotated query: fragment loads hit 32 banks
+  static constexpr int kTrig = kQ + 16 * kQLd * 2;         // step: float [4][D / 2] cos / sin of the two positions
   static constexpr int kVar = kTrig + 4 * (D / 2) * 4;     // logits [G][slots * 32], key scores [lc_pad], block scores [nb_pad]
 };
 
@@ -267,31 +233,18 @@ __device__ __forceinline__ void cta_merge(uint8_t* smem, int br, int w0, int nw,
 template <int D, int NW>
 __device__ __forceinline__ void cluster_weights(uint8_t* smem, int S, int branches) {
   using L = Layout<D, NW>;
-  const int t = threadIdx.x;
-  if (t < 16 * branches) {
-    const float2* mlc = reinterpret_cast<const float2*>(smem + L::kMlc) + t;
-    float* wts = reinterpret_cast<float*>(smem + L::kWts) + (t >> 4) * kMaxCluster * 16 + (t & 15);
-    float mx = -INFINITY;
-    float2 ml[kMaxCluster];
-#pragma unroll
-    for (int s = 0; s < kMaxCluster; ++s)
-      if (s < S) ml[s] = ld_peer2(peer_addr(mlc, s));
-#pragma unroll
-    for (int s = 0; s < kMaxCluster; ++s)
-      if (s < S) mx = fmaxf(mx, ml[s].x);
-    float sum = 0.f;
-#pragma unroll
-    for (int s = 0; s < kMaxCluster; ++s)
-      if (s < S) {
-        const float w = ml[s].y == 0.f ? 0.f : fast_exp2(ml[s].x - mx);
-        sum += ml[s].y * w;
-        ml[s].x = w;
-      }
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
-#pragma unroll
-    for (int s = 0; s < kMaxCluster; ++s)
-      if (s < S) wts[s * 16] = ml[s].x * inv;
-    if (t < 16) reinterpret_cast<float*>(smem + L::kLse)[t] = sum > 0.f ? mx + log2f(sum) : INFINITY;
+  // S lanes per row (S is a power of two): one load each, then shuffles
+  for (int t = threadIdx.x; t < 16 * branches * S; t += NW * 32) {
+    const int s = t & (S - 1), row = t / S;  // row: branch * 16 + row
+    const float2 ml = ld_peer2(peer_addr(reinterpret_cast<const float2*>(smem + L::kMlc) + row, s));
+    float mx = ml.x;
+    for (int o = S >> 1; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float w = ml.y == 0.f ? 0.f : fast_exp2(ml.x - mx);
+    float sum = ml.y * w;
+    for (int o = S >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    w *= sum > 0.f ? 1.f / sum : 0.f;
+    reinterpret_cast<float*>(smem + L::kWts)[((row >> 4) * kMaxCluster + s) * 16 + (row & 15)] = w;
+    if (s == 0 && row < 16) reinterpret_cast<float*>(smem + L::kLse)[row] = sum > 0.f ? mx + log2f(sum) : INFINITY;
   }
 }
 
@@ -361,23 +314,33 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
     cmp_rows = lc + (has_cmp ? 1 : 0);
     win_rows = min(lw + 1, p.win.rows);
     float* trig = reinterpret_cast<float*>(smem + L::kTrig);
+    // the query elements are on their way while the counters arrive and the angles are computed
+    constexpr int QPT = 16 * (D / 2) / NT;
+    T qx1[QPT], qx2[QPT];
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const int g = (tid + u * NT) / (D / 2), j = (tid + u * NT) % (D / 2);
+      const T* src = static_cast<const T*>(p.q) + b * p.q_sb + (long long)(h * p.G + min(g, p.G - 1)) * p.q_sh;
+      qx1[u] = src[j];
+      qx2[u] = src[j + D / 2];
+    }
     if (tid < D / 2) trig_table<T, D>(trig, trig + D / 2, p.inv_freq, ls, p.rope_scaling, tid);
     else if (tid >= 64 && tid < 64 + D / 2 && rank == 0 && full)
       trig_table<T, D>(trig + D, trig + 3 * D / 2, p.inv_freq, lc * p.stride, p.rope_scaling, tid - 64);
     __syncthreads();
     // rotated query: 16 rows of D in shared memory (rows beyond the group are zero); every CTA makes its own copy
     T* qs = reinterpret_cast<T*>(smem + L::kQ);
-    for (int i = tid; i < 16 * (D / 2); i += NT) {
-      const int g = i / (D / 2), j = i % (D / 2);
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const int g = (tid + u * NT) / (D / 2), j = (tid + u * NT) % (D / 2);
       float y1 = 0.f, y2 = 0.f;
       if (g < p.G) {
-        const T* src = static_cast<const T*>(p.q) + b * p.q_sb + (long long)(h * p.G + g) * p.q_sh;
-        const float x1 = DT<T>::to_float(src[j]), x2 = DT<T>::to_float(src[j + D / 2]);
+        const float x1 = DT<T>::to_float(qx1[u]), x2 = DT<T>::to_float(qx2[u]);
         y1 = fmaf(x1, trig[j], -x2 * trig[D / 2 + j]);
         y2 = fmaf(x2, trig[j], x1 * trig[D / 2 + j]);
       }
-      qs[g * D + j] = DT<T>::from_float(y1);
-      qs[g * D + j + D / 2] = DT<T>::from_float(y2);
+      qs[g * L::kQLd + j] = DT<T>::from_float(y1);
+      qs[g * L::kQLd + j + D / 2] = DT<T>::from_float(y2);
     }
     if (rank == 0) {
       // one thread per pair of columns (j, j + D / 2) of the key or value: it owns them in every row it touches
@@ -388,49 +351,47 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
         // staging buffer: drop the first `stride` rows if it was full, append the new row, pool it if that completes a window
         const T* w = static_cast<const T*>(p.w[kv]);
         const bool weighted = w != nullptr && p.partial == nullptr;
-        const T* pe = kv == 0 && full ? static_cast<const T*>(p.pe) : nullptr;  // summed apart and rounded, as the operators do
+        const bool pool = full && !p.partial;
+        // (the position embedding's sum is kept apart and rounded, as the operators do)
+        const T* pe = kv == 0 && pool && p.pe ? static_cast<const T*>(p.pe) + (long long)h * p.window * D + j : nullptr;
         float a1 = 0.f, a2 = 0.f, e1 = 0.f, e2 = 0.f;
-        if (pe) {
-          pe += (long long)h * p.window * D + j;
-          for (int r0 = 0; r0 < p.window; r0 += 16) {
-#pragma unroll
-            for (int u = 0; u < 16; ++u)
-              if (r0 + u < p.window) {
-                const float wv = weighted ? DT<T>::to_float(w[h * p.window + r0 + u]) : 1.f;
-                e1 += wv * DT<T>::to_float(pe[(r0 + u) * D]);
-                e2 += wv * DT<T>::to_float(pe[(r0 + u) * D + D / 2]);
-              }
-          }
-          if (!weighted) {
-            e1 /= (float)p.window;
-            e2 /= (float)p.window;
-          }
-        }
         if (shift || full) {
+          // Sixteen rows at a time, every load of them before the first store: a store to the buffer in between holds back the
+          // loads behind it, and 32 weights fetched one by one were 10 of the 30 us of a step that completes a window.
           const int off = shift ? p.stride : 0;
-          for (int r0 = 0; r0 < kept; r0 += 16) {
-            T x1[16], x2[16];
+          const int n_rows = pe ? p.window : kept;
+          for (int r0 = 0; r0 < n_rows; r0 += 16) {
+            T x1[16], x2[16], z1[16], z2[16], wr[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
-              if (r0 + u < kept) {
-                const T* row = cache_ptr<T, D>(p.stage, kv, b, r0 + u + off, h);
-                x1[u] = row[j];
-                x2[u] = row[j + D / 2];
+            for (int u = 0; u < 16; ++u) {
+              const int r = min(r0 + u, n_rows - 1), rk = max(min(r, kept - 1), 0);
+              const T* row = cache_ptr<T, D>(p.stage, kv, b, rk + off, h);
+              x1[u] = row[j];
+              x2[u] = row[j + D / 2];
+              wr[u] = pool && weighted ? w[h * p.window + r] : DT<T>::from_float(1.f);
+              z1[u] = z2[u] = DT<T>::from_float(0.f);
+              if (pe) {
+                z1[u] = pe[r * D];
+                z2[u] = pe[r * D + D / 2];
               }
+            }
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
+            for (int u = 0; u < 16; ++u) {
+              const float wv = DT<T>::to_float(wr[u]);
               if (r0 + u < kept) {
                 if (shift) {
                   T* row = cache_ptr<T, D>(p.stage, kv, b, r0 + u, h);
                   row[j] = x1[u];
                   row[j + D / 2] = x2[u];
                 }
-                if (full && !p.partial) {
-                  const float wv = weighted ? DT<T>::to_float(w[h * p.window + r0 + u]) : 1.f;
-                  a1 += wv * DT<T>::to_float(x1[u]);
-                  a2 += wv * DT<T>::to_float(x2[u]);
-                }
+                a1 += wv * DT<T>::to_float(x1[u]);
+                a2 += wv * DT<T>::to_float(x2[u]);
               }
+              if (r0 + u < n_rows) {
+                e1 += wv * DT<T>::to_float(z1[u]);
+                e2 += wv * DT<T>::to_float(z2[u]);
+              }
+            }
           }
         }
         {
@@ -442,6 +403,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
           if (p.partial) {  // linear compression: the taps' products, summed in order
             const long long tap = (long long)p.B * 2 * p.Hkv * D;
             const float* pt = p.partial + (((long long)b * 2 + kv) * p.Hkv + h) * D;
+            a1 = a2 = 0.f;
+#pragma unroll 8
             for (int r = 0; r < p.window; ++r) {
               a1 += __ldcg(pt + r * tap + j);
               a2 += __ldcg(pt + r * tap + j + D / 2);
@@ -454,6 +417,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
               const float inv = 1.f / (float)p.window;
               a1 *= inv;
               a2 *= inv;
+              e1 /= (float)p.window;
+              e2 /= (float)p.window;
             }
           }
           if (pe) {
@@ -509,10 +474,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
       const int r = lane >> 2, c = (lane & 3) * 2;
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
-        qf[kk][0] = *reinterpret_cast<const uint32_t*>(q0 + r * D + kk * 16 + c);
-        qf[kk][1] = *reinterpret_cast<const uint32_t*>(q0 + (r + 8) * D + kk * 16 + c);
-        qf[kk][2] = *reinterpret_cast<const uint32_t*>(q0 + r * D + kk * 16 + c + 8);
-        qf[kk][3] = *reinterpret_cast<const uint32_t*>(q0 + (r + 8) * D + kk * 16 + c + 8);
+        qf[kk][0] = *reinterpret_cast<const uint32_t*>(q0 + r * L::kQLd + kk * 16 + c);
+        qf[kk][1] = *reinterpret_cast<const uint32_t*>(q0 + (r + 8) * L::kQLd + kk * 16 + c);
+        qf[kk][2] = *reinterpret_cast<const uint32_t*>(q0 + r * L::kQLd + kk * 16 + c + 8);
+        qf[kk][3] = *reinterpret_cast<const uint32_t*>(q0 + (r + 8) * L::kQLd + kk * 16 + c + 8);
       }
     }
   } else {
