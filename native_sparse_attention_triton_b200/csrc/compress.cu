@@ -11,6 +11,7 @@
 // x[s + m*stride + k] gathered with cp.async into 128B-swizzled shared memory, the B tile is the
 // tap's [d, d] slice of W.  Pooling is a vectorised streaming kernel.
 #include "attn_tile.cuh"
+#include "cluster.cuh"
 #include "dispatch.h"
 #include "host_util.h"
 #include "linear_fwd_tc.h"
@@ -82,8 +83,16 @@ struct LinFwdParams {
   const int* ycu;
   long long x_sn, x_sh;
   int H, ks, stride;
+  int S;             // CTAs per cluster: they share the taps of one tile of windows
 };
 
+// The taps of a tile are a serial chain of ks weight slices (48 KB of loads per tap at d = 128), and short inputs have a handful of
+// tiles: the S CTAs of a cluster take ks / S consecutive taps each, meet in distributed shared memory (every CTA adds up and writes
+// its share of the rows, in rank order), and the chain is S times shorter.  Microseconds with S = 1 / 2 / 4 / 8, 32 taps:
+//   d = 64    up to 60 tiles: 21 / 14 / 9 / 6..9     68 tiles: 21 / 14 / 11 / 11     132: 22 / 18 / 15 / 20     264: 28 / 25 / 27 / 32
+//   d = 128   up to 12 tiles: 59 / 34 / 20 / 12      20: 59 / 34 / 20 / 15           36: 60 / 34 / 24 / 26      64: 60 / 35 / 25 / 29
+// hence the limits in launch_linear_fwd: places for four CTAs per SM (32 KB of tiles each) at d = 64, for two at d = 128.  The
+// tcgen05 kernel takes 17.5 us from one CTA to one per SM: it is the better one beyond 20 tiles of d = 128.
 template <typename T, int D>
 __global__ void __launch_bounds__(128) linear_fwd_kernel(LinFwdParams p) {
   constexpr int MT = 64;                      // output rows per CTA
@@ -96,10 +105,13 @@ __global__ void __launch_bounds__(128) linear_fwd_kernel(LinFwdParams p) {
   const int b = blockIdx.y, h = blockIdx.z;
   const int s0 = __ldg(p.cu + b);
   const int y0 = __ldg(p.ycu + b), Mb = __ldg(p.ycu + b + 1) - y0;
-  const int m0 = blockIdx.x * MT;
-  if (m0 >= Mb) return;
+  const int S = p.S;
+  const uint32_t rank = S > 1 ? cluster_rank() : 0;
+  const int m0 = blockIdx.x / S * MT;
+  if (m0 >= Mb) return;  // all CTAs of the cluster
   const T* x = static_cast<const T*>(p.x);
   const T* w = static_cast<const T*>(p.w) + (size_t)h * p.ks * D * D;
+  const int k_first = p.ks / S * (int)rank, k_end = k_first + p.ks / S;
 
   auto load_stage = [&](int k, int stg) {
     const uint32_t a_base = smem_u32(smem + stg * (A_BYTES + B_BYTES));
@@ -122,10 +134,10 @@ __global__ void __launch_bounds__(128) linear_fwd_kernel(LinFwdParams p) {
 #pragma unroll
   for (int j = 0; j < D / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
 
-  load_stage(0, 0);
-  for (int k = 0; k < p.ks; ++k) {
-    const int stg = k & 1;
-    if (k + 1 < p.ks) {
+  load_stage(k_first, 0);
+  for (int k = k_first; k < k_end; ++k) {
+    const int stg = (k - k_first) & 1;
+    if (k + 1 < k_end) {
       load_stage(k + 1, stg ^ 1);
       cp_async_wait<1>();
     } else {
@@ -141,6 +153,39 @@ __global__ void __launch_bounds__(128) linear_fwd_kernel(LinFwdParams p) {
 
   // epilogue: round, add the bias in the storage type, store
   const int l = lane_id();
+  if (S > 1) {
+    constexpr int LD = D + 8;  // floats per row: the fragment stores of a half-warp fall on different banks
+    float* part = reinterpret_cast<float*>(smem);
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) {
+      const int r = warp * 16 + (l >> 2), c = j * 8 + (l & 3) * 2;
+      *reinterpret_cast<float2*>(part + r * LD + c) = make_float2(acc[j][0], acc[j][1]);
+      *reinterpret_cast<float2*>(part + (r + 8) * LD + c) = make_float2(acc[j][2], acc[j][3]);
+    }
+    cluster_barrier();
+    const T* bias = p.bias ? static_cast<const T*>(p.bias) + (size_t)h * D : nullptr;
+    const int rows = MT / S;
+    for (int i = threadIdx.x; i < rows * (D / 4); i += 128) {
+      const int r = (int)rank * rows + i / (D / 4), c = i % (D / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) {
+        const float4 t = ld_peer4(peer_addr(part + r * LD + c, s));
+        v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+      }
+      if (m0 + r < Mb) {
+        uint2 out = make_uint2(DT<T>::pack(v.x, v.y), DT<T>::pack(v.z, v.w));
+        if (bias) {
+          const float2 a = DT<T>::unpack(out.x), b2 = DT<T>::unpack(out.y);
+          out.x = DT<T>::pack(a.x + DT<T>::to_float(bias[c]), a.y + DT<T>::to_float(bias[c + 1]));
+          out.y = DT<T>::pack(b2.x + DT<T>::to_float(bias[c + 2]), b2.y + DT<T>::to_float(bias[c + 3]));
+        }
+        *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + ((size_t)(y0 + m0 + r) * p.H + h) * D + c) = out;
+      }
+    }
+    cluster_barrier();  // no CTA leaves while its shared memory is being read
+    return;
+  }
   if (p.bias) {
     const T* bias = static_cast<const T*>(p.bias) + (size_t)h * D;
 #pragma unroll
@@ -320,7 +365,10 @@ static int launch_linear_fwd(LinFwdParams p, const void* pe, void* bias_scratch,
   } else {
     p.bias = nullptr;
   }
-  if (linear_fwd_tc_eligible(D, max_ylen, total_len, p.ks, p.stride)) {
+  const long long tiles = (long long)((max_ylen + 63) / 64) * B * p.H, places = (D == 128 ? 2ll : 4ll) * num_sms();
+  p.S = 1;
+  while (p.S < 8 && p.ks % (2 * p.S) == 0 && tiles * p.S * 2 <= places) p.S <<= 1;
+  if (tiles * 7 > num_sms() && linear_fwd_tc_eligible(D, max_ylen, total_len, p.ks, p.stride)) {
     const int rc = linear_fwd_tc(p.x, p.w, p.bias, p.y, p.cu, p.ycu, B, max_ylen, total_len, p.H, p.ks, p.stride, p.x_sn, p.x_sh,
                                  dtype, stream);
     if (rc != kInvalid && rc != kUnsupported) return rc;   // a view of x no tensor map describes: the gathering kernel below
@@ -329,9 +377,19 @@ static int launch_linear_fwd(LinFwdParams p, const void* pe, void* bias_scratch,
   auto kern = linear_fwd_kernel<T, D>;
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
-  dim3 grid((max_ylen + 63) / 64, B, p.H);
-  { LaunchScope ls_("linear_compress_fwd", stream); kern<<<grid, 128, smem, stream>>>(p); }
-  return cuda_rc(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((max_ylen + 63) / 64 * p.S, B, p.H);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)p.S;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  LaunchScope ls_("linear_compress_fwd", stream);
+  return cuda_rc(cudaLaunchKernelEx(&cfg, kern, p));
 }
 
 template <typename T, int D>
