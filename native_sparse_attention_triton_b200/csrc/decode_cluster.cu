@@ -17,6 +17,10 @@
 //     appending them, the three branches, the gated sum -- so the step is this one kernel with a cluster barrier between its
 //     parts.  The length counters, shared by the heads of a sequence, are advanced by the last of its clusters to have read
 //     them.
+// Measured (8 pairs of 8256 rows): dense 13 us, compressed with selection 8.5, selected blocks 7; a whole step 18 us (34 k clocks:
+// counters, angles and rotation 3 k, staging and append 1 k -- 4 k where a window completes --, compressed and window branches 4 k,
+// their merge and weights 4 k, key scores and output slices 3 k, selection 2-4 k, list and selected blocks 5 k, merge, weights and
+// output 5 k, six cluster barriers of about 1 k each).
 #include "attn_tile.cuh"
 #include "cluster.cuh"
 #include "decode_cluster.h"
