@@ -296,7 +296,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
           bsc[bb] = acc;
         }
         __syncwarp();
-        warp_select_topk(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks,
+        warp_select_topk<false>(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks,
                          p.topk_out_idx + h * p.t_sh + (long long)b * p.t_sb, p.t_sk);
         __syncwarp();
       }

@@ -582,8 +582,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 2 : 1) decode_cluster_kerne
       }
       __syncthreads();
       if (warp == 0) {
-        if constexpr (MODE == kStep) warp_select_topk(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks, sel, 1);
-        else warp_select_topk(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks,
+        if constexpr (MODE == kStep) warp_select_topk<false>(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks, sel, 1);
+        else warp_select_topk<false>(bsc, min(bq, p.nb_pad - 1), p.topk_out, p.init_blocks, p.local_blocks,
                               p.topk_out_idx + h * p.t_sh + (long long)b * p.t_sb, p.t_sk);
       }
     }

@@ -4,6 +4,77 @@
 
 namespace nsa {
 
+// The selection below for at most 32 U candidates: they sit in registers and the threshold is found from the top bit down, two bits
+// per warp reduction (the counts of three trial thresholds packed in one word), until exactly Tout candidates reach it.  A round per
+// taken block costs two dependent reductions, 13 rounds for top-16, and with a few warps per SM nothing hides that latency.
+// Score pass of a layer: 32q/8kv, 7097 tokens, top-16, 138 -> 121 us; 64q/4kv, ragged 16 K, 353 -> 305 us.  A decode step runs the
+// selection once per launch, with cold instructions, and gains nothing from the longer code (24.9 against 23.8 us a step before the
+// clusters' kernel went back to rounds): it stays with the rounds.
+// Same result: candidates are the finite non-negative scores, forced blocks come first, ties go to the lower id.
+template <int U>
+__device__ __forceinline__ void warp_select_bits(const float* sc, int ncand, int n_init, int lo, int Tout, int* out, long long out_stride) {
+  const int lane = lane_id();
+  int v[U];
+  int mx = -1, live = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int x = lane + 32 * u;
+    int val = x < ncand ? __float_as_int(sc[x]) : -1;
+    if (val == static_cast<int>(0x80000000u)) val = 0;
+    if (val >= 0x7f800000 || val < 0) val = -1;  // neither infinities nor NaN
+    mx = max(mx, val);
+    if (x < ncand && (x < n_init || x >= lo)) val = 0x7f800000;
+    v[u] = val;
+    live += val >= 0;
+  }
+  live = __reduce_add_sync(0xffffffffu, live);
+  int t = 0;             // every candidate with v >= t is taken ...
+  bool ties = false;     // ... but of those with v == t only the first ones
+  if (live > Tout) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    ties = true;
+    // forced blocks are fewer than Tout, so the threshold is at most mx
+    for (int bit = mx > 0 ? ((31 - __clz(mx)) | 1) : -1; bit > 0; bit -= 2) {
+      // (scores from 2 on start at bit 31, the sign: trial values with it are beyond every candidate)
+      const int t1 = t | (1 << (bit - 1));
+      const int t2 = (int)min((unsigned)t | (2u << (bit - 1)), 0x7fffffffu), t3 = (int)min((unsigned)t | (3u << (bit - 1)), 0x7fffffffu);
+      unsigned n = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) n += (v[u] >= t1 ? 1u : 0u) + (v[u] >= t2 ? 1u << 10 : 0u) + (v[u] >= t3 ? 1u << 20 : 0u);
+      n = __reduce_add_sync(0xffffffffu, n);
+      const int n1 = n & 1023u, n2 = (n >> 10) & 1023u, n3 = n >> 20;
+      int at = -1;
+      if (n3 >= Tout) { t = t3; at = n3; }
+      else if (n2 >= Tout) { t = t2; at = n2; }
+      else if (n1 >= Tout) { t = t1; at = n1; }
+      if (at == Tout) { ties = false; break; }
+    }
+  }
+  int quota = 0;  // candidates equal to t that may still be taken
+  if (ties) {
+    int above = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) above += v[u] > t;
+    quota = Tout - __reduce_add_sync(0xffffffffu, above);
+  }
+  const unsigned lt_mask = (1u << lane) - 1u;
+  int base = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    bool sel = v[u] >= t;
+    if (ties) {
+      const unsigned eq = __ballot_sync(0xffffffffu, v[u] == t);
+      if (v[u] == t) sel = __popc(eq & lt_mask) < quota;
+      quota -= min(quota, __popc(eq));
+    }
+    const unsigned mk = __ballot_sync(0xffffffffu, sel);
+    if (sel) out[(base + __popc(mk & lt_mask)) * out_stride] = lane + 32 * u;
+    base += __popc(mk);
+  }
+  for (int j = base + lane; j < Tout; j += 32) out[j * out_stride] = -1;
+  __syncwarp();
+}
+
 // sc[0..bq] : finite, non-negative block scores of one token in shared memory (modified in place: taken blocks are
 // overwritten with +inf, candidates a lane has pulled into its cache with -1).  Writes `Tout` ids to out[j*out_stride]:
 // the taken blocks in ascending order, then -1.  Forced blocks: b < init_blocks and b > bq - local_blocks.
@@ -13,6 +84,7 @@ namespace nsa {
 // rolled scan of its candidates), so a selection round is two warp reductions and a cache pop; a lane rescans only
 // after it has won C rounds.  The code is deliberately compact (rolled loops, candidates left in shared memory): the
 // selection runs once per CTA, and a fully unrolled register version spent its time fetching instructions.
+template <bool BITS = true>
 __device__ __forceinline__ void warp_select_topk(float* sc, int bq, int Tout, int init_blocks, int local_blocks, int* out,
                                                  long long out_stride) {
   constexpr int C = 4;
@@ -27,6 +99,13 @@ __device__ __forceinline__ void warp_select_topk(float* sc, int bq, int Tout, in
   const int n_init = min(init_blocks, ncand);
   const int lo = max(n_init, bq - local_blocks + 1);
   const int nforced = n_init + (bq - lo + 1);
+  if (BITS && ncand <= 256 && nforced < Tout) {
+    __syncwarp();
+    if (ncand <= 64) warp_select_bits<2>(sc, ncand, n_init, lo, Tout, out, out_stride);
+    else if (ncand <= 128) warp_select_bits<4>(sc, ncand, n_init, lo, Tout, out, out_stride);
+    else warp_select_bits<8>(sc, ncand, n_init, lo, Tout, out, out_stride);
+    return;
+  }
   for (int bb = lane; bb < n_init; bb += 32) sc[bb] = INFINITY;
   for (int bb = lo + lane; bb <= bq; bb += 32) sc[bb] = INFINITY;
   const int need = max(0, Tout - nforced);
