@@ -35,6 +35,11 @@ __device__ __forceinline__ int ld_peer_i(uint32_t a) {
   asm volatile("ld.shared::cluster.b32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ float ld_peer(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_peer(uint32_t a, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory");
 }

@@ -12,6 +12,7 @@
 //   dx[t] = sum_i w[h, j + i*stride] dy[t/stride - i],  dw[h,k] = sum_m <x[s+m*stride+k,h,:], dy[m,h,:]> + <pe[h,k,:], dbias[h,:]>,
 //   dpe[h,k,:] = w[h,k] dbias[h,:]
 #include "attn_tile.cuh"
+#include "cluster.cuh"
 #include "dispatch.h"
 #include "host_util.h"
 #include "nsa_b200.h"
@@ -21,15 +22,15 @@ namespace nsa {
 
 // dbias[c] = sum_m dy[m, c] over the M rows of H * D columns (fp32), in a fixed order (deterministic).  A cluster of eight CTAs
 // takes 32 columns, an eighth of the rows each; a thread sums every 64th row of its CTA's eighth with eight 16-byte loads in
-// flight, the CTA's 64 partial sums are added in shared memory and rank 0 adds the eight CTAs'. 
+// flight, the CTA's 64 partial sums are added in its shared memory, and rank 0 reads and adds the eight CTAs' behind a cluster
+// barrier: a CTA whose share of the rows is empty gets there long before the others have started.
 constexpr int kColsumCluster = 8;
 template <typename T>
 __global__ void __cluster_dims__(kColsumCluster, 1, 1) __launch_bounds__(256)
 colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, int M, int C) {
   __shared__ float red[64][33];
-  __shared__ float sum[kColsumCluster][32];   // rank 0's: one row per CTA of the cluster
-  uint32_t rank;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  __shared__ float sum[32];
+  const uint32_t rank = cluster_rank();
   const int c4 = threadIdx.x & 3, rl = threadIdx.x >> 2;
   const int col = blockIdx.y * 32 + c4 * 8;
   const int per = (M + kColsumCluster - 1) / kColsumCluster;
@@ -58,18 +59,16 @@ colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, int M, int C)
     float s = 0.f;
 #pragma unroll 8
     for (int r = 0; r < 64; ++r) s += red[r][threadIdx.x];
-    uint32_t dst;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"(smem_u32(&sum[rank][threadIdx.x])));
-    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(dst), "f"(s) : "memory");
+    sum[threadIdx.x] = s;
   }
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  cluster_barrier();
   if (rank == 0 && threadIdx.x < 32) {
     float s = 0.f;
 #pragma unroll
-    for (int r = 0; r < kColsumCluster; ++r) s += sum[r][threadIdx.x];
+    for (int r = 0; r < kColsumCluster; ++r) s += ld_peer(peer_addr(sum + threadIdx.x, r));
     dbias[blockIdx.y * 32 + threadIdx.x] = s;
   }
+  cluster_barrier();  // no CTA leaves while its shared memory is being read
 }
 
 template <typename T>
