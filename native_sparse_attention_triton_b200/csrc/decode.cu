@@ -365,7 +365,8 @@ static int decode_common_checks(const void* q, const void* k, const void* v, con
   if (num_q_heads / num_kv_heads > 16) return kUnsupported;
   for (int i = 0; i < 10; ++i)
     if (strides[i] % 8) return kInvalid;
-  if (!aligned16(q) || !aligned16(o)) return kInvalid;
+  // the cluster kernels copy cache rows 16 bytes at a time (the tensor maps of the split-KV kernel ask for the same)
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return kInvalid;
   return kOk;
 }
 
