@@ -6,9 +6,17 @@
 // groups the private tile serves four rows or one.  Here a CTA takes two row tiles of 128 rows (2 x 128 / G consecutive tokens),
 // forms the UNION of their selections and walks it like dense attention: two 64-key tiles of the union make a 128-key step, a
 // row that did not select one of them gets its exponentials biased by -inf, a warp none of whose rows selected it skips them.
-// A tile is fetched once per 256 rows; what bounds the kernel is the tensor pipe (1024 clocks per 128 keys and row tile) and, where
-// most rows do select, the softmax.  Which tokens gain follows from their position in the sequence (union_limit below, with the
-// measurements): this kernel takes the tokens before the limit in every sequence and sparse_fwd.cu those behind it.
+// A tile is fetched once per 256 rows; what bounds the kernel is the softmax (two reads of the logits, 16 exponentials per clock;
+// 2150 clocks per 64-key tile of the union at head_dim 128 against 1024 of products).  Which tokens gain follows from their
+// position in the sequence (union_limit below, with the measurements): this kernel takes the tokens before the limit in every
+// sequence and sparse_fwd.cu those behind it.
+//
+// The result is no less exact than the private walk's.  The reference maximum of a row is its running maximum, so that the largest
+// probability is an exact 1 (raised only when outgrown by 2^8, as in dense_fwd_tc.cu, it costs 1.8 % of the error against 64 bits:
+// 32q/8kv bf16 2.120e-3 against 2.083e-3), all exponentials come from the exponential unit (one pair in three as a cubic would put
+// 7.5e-5 into the fp32 row sum and the lse), and the output is divided by the sum of the ROUNDED probabilities, those the product
+// with V saw: with 128 keys per update instead of 64 fewer of them are exact, which alone would leave 2.087e-3; so it is 2.072e-3.
+// The lse comes from the unrounded sum.
 //   warp 8      : TMA producer: Q of both row tiles, then K and V tiles of the union (ring of 2 each)
 //   warp 9      : tensor memory, MMA issue (as in dense_fwd_tc.cu: S of a row tile, then P V, alternating between the row tiles)
 //   warps 0..7  : softmax, one thread per row (0..3 row tile A, 4..7 row tile B)
@@ -27,7 +35,6 @@
 namespace nsa {
 namespace {
 
-constexpr int kUnPolyEvery = 3;     // in tiles every row sees in full, one pair of exponentials in three is a polynomial
 constexpr int kUnKeys = 128;        // keys per step: two 64-key tiles of the union
 constexpr int kUnStages = 2;        // K tiles, and V tiles, in flight
 constexpr int kUnMaskWords = 4096;  // 32-bit words of selection masks per CTA
@@ -254,7 +261,7 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const unsigned* my_mask = mask + (tt >> 5);
     const uint32_t s_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 128);
     const uint32_t o_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 256u + (uint32_t)(g * 128);
-    float m_ref = -INFINITY, l = 0.f;
+    float m_ref = -INFINITY, l = 0.f, l_rounded = 0.f;
     for (int i = 0; i < ntiles; ++i) {
       // visible keys of the step's two tiles: 0 where the row's token did not select the block (or sees none of the tile)
       int lim[2];
@@ -268,152 +275,96 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
       }
       const bool any0 = __any_sync(0xffffffffu, lim[0] > 0), any1 = __any_sync(0xffffffffu, lim[1] > 0);
-      const bool full = __all_sync(0xffffffffu, lim[0] == 64 && lim[1] == 64);
       // every row takes a tile whole or not at all: no mask per element, the rows that do not take it are biased by -inf
       const bool whole = __all_sync(0xffffffffu, (lim[0] & 63) == 0 && (lim[1] & 63) == 0);
       mbar_wait(s_full + g, i & 1, p.st);
       tc_fence_after_sync();
       auto none_of = [&](int c) { return c < 2 ? !any0 : !any1; };   // no row of the warp takes the tile of chunk c
-      auto two_pass = [&]() {
-        // ---- pass 1: row maximum of the raw logits (the scale is positive) ----
-        float mh[2] = {-INFINITY, -INFINITY};
-        auto pass1 = [&](auto masked_tag) {
-          constexpr bool MASKED = decltype(masked_tag)::value;
+      // ---- pass 1: row maximum of the raw logits (the scale is positive) ----
+      float mh[2] = {-INFINITY, -INFINITY};
+      auto pass1 = [&](auto masked_tag) {
+        constexpr bool MASKED = decltype(masked_tag)::value;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (none_of(c)) continue;
+        for (int c = 0; c < 4; ++c) {
+          if (none_of(c)) continue;
+          uint32_t su[32];
+          tmem_ld32(s_base + c * 32, su);
+          tmem_ld_wait();
+          const int lm = lim[c >> 1] - (c & 1) * 32;
+          float mx2[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float v0 = (!MASKED || j < lm) ? __uint_as_float(su[j]) : -INFINITY;
+            const float v1 = (!MASKED || j + 1 < lm) ? __uint_as_float(su[j + 1]) : -INFINITY;
+            mx2[(j >> 1) & 1] = fmax3(mx2[(j >> 1) & 1], v0, v1);
+          }
+          mh[c >> 1] = fmax3(mh[c >> 1], mx2[0], mx2[1]);
+        }
+      };
+      if (whole) pass1(std::false_type{}); else pass1(std::true_type{});
+      const float mt = fmaxf(lim[0] > 0 ? mh[0] : -INFINITY, lim[1] > 0 ? mh[1] : -INFINITY) * p.scale2;
+      const bool need = mt > m_ref;
+      float factor = 1.f;
+      if (need) {
+        factor = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mt);
+        m_ref = mt;
+        l *= factor;
+        l_rounded *= factor;
+      }
+      if (i > 0 && __any_sync(0xffffffffu, need)) {
+        mbar_wait(pv_done + g, (i - 1) & 1, p.st);  // P V of the previous step is complete: O is stable
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(o_base + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 y = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(factor, factor));
+            r[j] = __float_as_uint(y.x);
+            r[j + 1] = __float_as_uint(y.y);
+          }
+          tmem_st32(o_base + c * 32, r);
+        }
+        tmem_st_wait();
+      }
+      // ---- pass 2: P = exp2(S * scale - m_ref) as 16-bit pairs over the logits (chunk c's 16 packed columns lie inside chunk
+      // c / 2, already consumed) ----
+      const float nm = (m_ref == -INFINITY) ? 0.f : -m_ref;
+      float2 ls2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, lr2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      auto pass2 = [&](auto masked_tag) {
+        constexpr bool MASKED = decltype(masked_tag)::value;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+          if (none_of(c)) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) pk[j] = 0u;
+          } else {
             uint32_t su[32];
             tmem_ld32(s_base + c * 32, su);
             tmem_ld_wait();
             const int lm = lim[c >> 1] - (c & 1) * 32;
-            float mx2[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float v0 = (!MASKED || j < lm) ? __uint_as_float(su[j]) : -INFINITY;
-              const float v1 = (!MASKED || j + 1 < lm) ? __uint_as_float(su[j + 1]) : -INFINITY;
-              mx2[(j >> 1) & 1] = fmax3(mx2[(j >> 1) & 1], v0, v1);
-            }
-            mh[c >> 1] = fmax3(mh[c >> 1], mx2[0], mx2[1]);
-          }
-        };
-        if (whole) pass1(std::false_type{}); else pass1(std::true_type{});
-        const float mt = fmaxf(lim[0] > 0 ? mh[0] : -INFINITY, lim[1] > 0 ? mh[1] : -INFINITY) * p.scale2;
-        const bool need = mt > m_ref + 8.f;
-        float factor = 1.f;
-        if (need) {
-          factor = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mt);
-          m_ref = mt;
-          l *= factor;
-        }
-        if (i > 0 && __any_sync(0xffffffffu, need)) {
-          mbar_wait(pv_done + g, (i - 1) & 1, p.st);  // P V of the previous step is complete: O is stable
-          tc_fence_after_sync();
-#pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld32(o_base + c * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float2 y = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(factor, factor));
-              r[j] = __float_as_uint(y.x);
-              r[j + 1] = __float_as_uint(y.y);
-            }
-            tmem_st32(o_base + c * 32, r);
-          }
-          tmem_st_wait();
-        }
-        // ---- pass 2: P = exp2(S * scale - m_ref) as 16-bit pairs over the logits (chunk c's 16 packed columns lie inside chunk
-        // c / 2, already consumed) ----
-        const float nm = (m_ref == -INFINITY) ? 0.f : -m_ref;
-        float2 ls2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        auto pass2 = [&](auto masked_tag) {
-          constexpr bool MASKED = decltype(masked_tag)::value;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pk[16];
-            if (none_of(c)) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) pk[j] = 0u;
-            } else {
-              uint32_t su[32];
-              tmem_ld32(s_base + c * 32, su);
-              tmem_ld_wait();
-              const int lm = lim[c >> 1] - (c & 1) * 32;
-              const float bias = lim[c >> 1] > 0 ? nm : -INFINITY;
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float2 x = ffma2(make_float2(__uint_as_float(su[2 * j]), __uint_as_float(su[2 * j + 1])), make_float2(p.scale2, p.scale2),
-                                       make_float2(bias, bias));
-                const float p0 = MASKED ? masked_exp2(2 * j < lm, x.x) : fast_exp2(x.x);
-                const float p1 = MASKED ? masked_exp2(2 * j + 1 < lm, x.y) : fast_exp2(x.y);
-                ls2[j & 1] = fadd2(ls2[j & 1], make_float2(p0, p1));
-                pk[j] = DT<T>::pack(p0, p1);
-              }
-            }
-            tmem_st16(s_base + c * 16, pk);
-          }
-        };
-        if (whole) pass2(std::false_type{}); else pass2(std::true_type{});
-        tmem_st_wait();
-        l += (ls2[0].x + ls2[0].y) + (ls2[1].x + ls2[1].y);
-      };
-      // As in dense_fwd_tc.cu: with a reference maximum at hand the exponentials are tried in one pass; if some row outgrew its
-      // reference by more than 2^8 nothing has been written yet and the step is redone in two.
-      bool done = false;
-      if (whole && __all_sync(0xffffffffu, m_ref != -INFINITY || lim[0] + lim[1] == 0)) {
-        const float nm = (m_ref == -INFINITY) ? 0.f : -m_ref;
-        uint32_t pk[64];
-        float2 ls2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        auto one_pass = [&](auto full_tag) {
-          constexpr bool FULL = decltype(full_tag)::value;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (!FULL && none_of(c)) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) pk[c * 16 + j] = 0u;
-              continue;
-            }
-            uint32_t su[32];
-            tmem_ld32(s_base + c * 32, su);
-            tmem_ld_wait();
-            const float bias = FULL || lim[c >> 1] > 0 ? nm : -INFINITY;
+            const float bias = lim[c >> 1] > 0 ? nm : -INFINITY;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const float2 x = ffma2(make_float2(__uint_as_float(su[2 * j]), __uint_as_float(su[2 * j + 1])), make_float2(p.scale2, p.scale2),
                                      make_float2(bias, bias));
-              mx4[j & 3] = fmax3(mx4[j & 3], x.x, x.y);
-              float p0, p1;
-              if (FULL && j % kUnPolyEvery == kUnPolyEvery - 1) {  // (a biased row needs exact zeros, which the polynomial does not give)
-                const float2 e = exp2_poly2(x);
-                p0 = e.x;
-                p1 = e.y;
-              } else {
-                p0 = fast_exp2(x.x);
-                p1 = fast_exp2(x.y);
-              }
+              const float p0 = MASKED ? masked_exp2(2 * j < lm, x.x) : fast_exp2(x.x);
+              const float p1 = MASKED ? masked_exp2(2 * j + 1 < lm, x.y) : fast_exp2(x.y);
               ls2[j & 1] = fadd2(ls2[j & 1], make_float2(p0, p1));
-              pk[c * 16 + j] = DT<T>::pack(p0, p1);
+              pk[j] = DT<T>::pack(p0, p1);
+              lr2[j & 1] = fadd2(lr2[j & 1], DT<T>::unpack(pk[j]));
             }
           }
-        };
-        if (full) one_pass(std::true_type{}); else one_pass(std::false_type{});
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        if (!__any_sync(0xffffffffu, mx > 8.f)) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pc[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) pc[j] = pk[c * 16 + j];
-            tmem_st16(s_base + c * 16, pc);
-          }
-          tmem_st_wait();
-          l += (ls2[0].x + ls2[0].y) + (ls2[1].x + ls2[1].y);
-          done = true;
+          tmem_st16(s_base + c * 16, pk);
         }
-      }
-      if (!done) two_pass();
+      };
+      if (whole) pass2(std::false_type{}); else pass2(std::true_type{});
+      tmem_st_wait();
+      l += (ls2[0].x + ls2[0].y) + (ls2[1].x + ls2[1].y);
+      l_rounded += (lr2[0].x + lr2[0].y) + (lr2[1].x + lr2[1].y);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full + g);
@@ -423,7 +374,7 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       mbar_wait(pv_done + g, (ntiles - 1) & 1, p.st);
       tc_fence_after_sync();
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const float inv = l_rounded > 0.f ? 1.f / l_rounded : 0.f;
     // A row tile whose tokens all belong to the sequence leaves through shared memory (its own Q buffer, free since its
     // last S product, in the swizzled panel layout) and one TMA store per panel; otherwise row by row.
     const bool staged = ntiles > 0 && q0 + g * QT + QT <= L;
@@ -491,12 +442,14 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // T - 3 free choices as uniform over the nb blocks before it (neighbours that agree more only make the union smaller), 2 QT tokens
 // touch U = 3 + nb (1 - (1 - (T - 3) / nb)^(2 QT)) of them; the union wins while U * (clocks per union tile) < 2 QT * T * (clocks per
 // private tile).  Measured with such selections, all tokens private / all in unions / split by this rule, us:
-//   32q/2kv d128 top-8   1024 tokens: 37 / 25 / 25    4096: 136 / 117    8192: 273 / 296
-//   64q/4kv d128 top-16  1024: 93 / 39    4096: 445 / 271    8192: 925 / 813   16384: 1912 / 2540
-//   32q/8kv d128 top-16  1024: 165 / 27   4096: 841 / 176    8192: 1760 / 501  16384: 3637 / 1826
-//   16q/2kv d64  top-8   1024: 29 / 25    4096: 95 / 68      8192: 173 / 181
-// From the increments between the lengths: about 1850 clocks per union tile (64 keys, both row tiles) against 530 per private one at
-// head_dim 128, 1950 against 370 at 64.
+//   32q/2kv d128 top-8   1024 tokens: 43 / 40 / 40    4096: 150 / 161 / 149    8192: 290 / 388 / 292
+//   64q/4kv d128 top-16  1024: 99 / 56 / 56   4096: 459 / 359 / 359   8192: 934 / 1033 / 882   16384: 1886 / 2882 / 1848
+//   32q/8kv d128 top-16  1024: 167 / 42 / 42  4096: 860 / 239 / 239   8192: 1775 / 656 / 656   16384: 3618 / 2217 / 2217
+//   16q/2kv d64  top-8   1024: 31 / 34 / 34   4096: 94 / 87 / 91      8192: 176 / 230 / 179
+// From the increments between the lengths: about 2150 clocks per union tile (64 keys, both row tiles) against 530 per private one at
+// head_dim 128, 1950 against 370 at 64.  The rule counts 1850 at 128: the second kernel's start and its last wave count against a
+// division that leaves it few tokens (with 2150 32q/2kv 2048 tokens: 79 us against 67, 64q/4kv 4096: 384 against 359, 8192: 876
+// against 882).
 int union_limit(int G, int T, int block_size, int head_dim) {
   const double union_clocks = head_dim == 128 ? 1850. : 1950., private_clocks = head_dim == 128 ? 530. : 370.;
   const int tokens = 2 * (128 / G), nsub = block_size / 64, mw = (tokens + 31) / 32;

@@ -100,3 +100,78 @@ def test_non_finite_rows_stay_with_those_who_selected_them(where, value):
     assert int(seen.sum()) > 50
     if value != float("-inf"):
         assert not torch.isfinite(o[seen.repeat_interleave(Hq // Hkv, 0).T]).all()
+
+
+def private_walk(q, k, v, idx, bs, lens):
+    """The walk of sparse_fwd.cu, one (token, KV head) pair at a time in fp32 torch: 64 keys per step in the order of the selection, the
+    running maximum as reference, probabilities rounded to 16 bits before the product with V, the sum of the unrounded ones."""
+    N, Hq, d = q.shape
+    Hkv = k.shape[1]
+    G, T = Hq // Hkv, idx.shape[-1]
+    out, at = torch.zeros_like(q), 0
+    for n in lens:
+        pos = torch.arange(n, device=q.device)
+        for h in range(Hkv):
+            qf, kf, vf = q[at:at + n, h * G:(h + 1) * G].float(), k[at:at + n, h].float(), v[at:at + n, h].float()
+            m = torch.full((n, G), -float("inf"), device=q.device)
+            l, o = torch.zeros(n, G, device=q.device), torch.zeros(n, G, d, device=q.device)
+            for j in range(T):
+                for half in range(bs // 64):
+                    key = idx[h, at:at + n, j].long()[:, None] * bs + half * 64 + torch.arange(64, device=q.device)
+                    seen = (idx[h, at:at + n, j] >= 0)[:, None] & (key <= pos[:, None])
+                    key = key.clamp(0, n - 1)
+                    s = torch.einsum("ngd,nkd->ngk", qf, kf[key]) * (d ** -0.5 * 1.4426950408889634)
+                    s = s.masked_fill(~seen[:, None], -float("inf"))
+                    mn = torch.maximum(m, s.amax(-1))
+                    ref = torch.where(mn == -float("inf"), torch.zeros_like(mn), mn)
+                    p, c = torch.exp2(s - ref[..., None]), torch.exp2(m - ref)
+                    l, o, m = l * c + p.sum(-1), o * c[..., None] + torch.einsum("ngk,nkd->ngd", p.to(q.dtype).float(), vf[key]), mn
+            out[at:at + n, h * G:(h + 1) * G] = torch.where(l[..., None] > 0, o / l[..., None], torch.zeros_like(o)).to(q.dtype)
+        at += n
+    return out
+
+
+@pytest.mark.parametrize("Hq,Hkv,d,topk,lens,dtype", [
+    (8, 2, 128, 8, [900, 700], torch.bfloat16),
+    (8, 2, 128, 8, [900, 700], torch.float16),
+    (16, 1, 64, 6, [1500], torch.bfloat16),
+])
+def test_unions_are_no_less_exact_than_private_walks(Hq, Hkv, d, topk, lens, dtype):
+    """Error of the output against 64 bits beside that of the private walk, and of the lse, which the backward reads."""
+    import native_sparse_attention_triton_b200 as pkg
+    from native_sparse_attention_triton_b200 import _lib
+    g = torch.Generator().manual_seed(11)
+    N, bs, G = sum(lens), 64, Hq // Hkv
+    rnd = lambda h: torch.randn(N, h, d, generator=g).to(dtype).cuda()
+    q, k, v = rnd(Hq), rnd(Hkv), rnd(Hkv)
+    idx = selection(g, lens, Hkv, bs, topk).cuda()
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    o, lse = torch.empty_like(q), torch.empty(N, Hq, device="cuda")
+    strides = _lib.strides_array(*[x for t in (q, k, v, o) for x in t.stride()[:2]], *idx.stride())
+    rc = _lib.lib().nsa_topk_sparse_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), idx.data_ptr(), cu.data_ptr(), o.data_ptr(),
+                                             lse.data_ptr(), N, len(lens), Hq, Hkv, d, topk, bs, strides, d ** -0.5,
+                                             _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_FP16,
+                                             torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    exact, exact_lse = torch.zeros(N, Hq, d, device="cuda", dtype=torch.float64), torch.zeros(N, Hq, device="cuda", dtype=torch.float64)
+    at = 0
+    for n in lens:
+        nb = (n + bs - 1) // bs
+        for h in range(Hkv):
+            ids = idx[h, at:at + n].long()
+            took = torch.zeros(n, nb + 1, dtype=torch.bool, device="cuda").scatter_(1, torch.where(ids < 0, nb, ids), True)
+            mask = took[:, :nb].repeat_interleave(bs, 1)[:, :n] & torch.ones(n, n, dtype=torch.bool, device="cuda").tril()
+            s = torch.einsum("ngd,md->ngm", q[at:at + n, h * G:(h + 1) * G].double(), k[at:at + n, h].double()) * d ** -0.5
+            s = s.masked_fill(~mask[:, None], -float("inf"))
+            exact[at:at + n, h * G:(h + 1) * G] = s.softmax(-1).nan_to_num(0.0) @ v[at:at + n, h].double()
+            exact_lse[at:at + n, h * G:(h + 1) * G] = torch.logsumexp(s, -1) * 1.4426950408889634
+        at += n
+    rel = lambda x: float((x.double() - exact).norm() / exact.norm())
+    # the same roundings of other sums: over a million outputs the two norms agree to a few parts in ten thousand
+    assert rel(o) <= 1.002 * rel(private_walk(q, k, v, idx, bs, lens)), (rel(o), rel(private_walk(q, k, v, idx, bs, lens)))
+    seen = torch.isfinite(exact_lse)
+    assert torch.equal(seen, torch.isfinite(lse))
+    # fp32: logits of magnitude 8 to 2^-21, exponentials of the unit to 2^-22, a sum of up to 512 terms
+    worst = float((lse.double() - exact_lse)[seen].abs().max())
+    assert worst <= 6e-6, worst
+    assert pkg.device_status() == 0
