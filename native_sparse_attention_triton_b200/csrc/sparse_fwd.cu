@@ -8,8 +8,8 @@
 // next tile of each kind is in flight while the current one is used.
 // The kernel is bound by L2 -> shared-memory tile fill (16 flop per byte fetched at G = 16).  It takes the tokens whose neighbours
 // choose other blocks; those near the start of a sequence, where a few neighbours touch nearly every block, go to
-// sparse_fwd_union_tc.cu.  There a key or value that is not finite reaches rows that did not select it (0 * inf); the pairs it
-// spoils are marked and walked here, where a row meets its own tiles only.
+// sparse_fwd_union_tc.cu.  There a key or value that is not finite reaches rows that did not select it (0 * inf), and a block that a
+// token gave twice is met once; such pairs are marked and walked here, where a row meets its own tiles only, each as often as given.
 #include <algorithm>
 
 #include "attn_tile.cuh"

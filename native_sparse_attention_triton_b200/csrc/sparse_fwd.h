@@ -16,7 +16,8 @@ struct SparseFwdParams {
   long long t_sh, t_sn, t_sk;
   int N, B, Hq, Hkv, G, T, block_size;
   int first;   // in-sequence position of the first token sparse_fwd.cu takes; the union kernel takes those before it, and leaves
-               // a NaN in the first lse of a (token, KV head) pair whose result is not finite, which sparse_fwd.cu then redoes
+               // a NaN in the first lse of a (token, KV head) pair whose result is not finite or whose selection has a block twice,
+               // which sparse_fwd.cu then redoes
   int span;    // tokens a warp of sparse_fwd.cu looks at per round (1 or 32)
   float scale2;
   Status st;

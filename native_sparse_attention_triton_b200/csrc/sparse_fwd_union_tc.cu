@@ -38,6 +38,7 @@ namespace {
 constexpr int kUnKeys = 128;        // keys per step: two 64-key tiles of the union
 constexpr int kUnStages = 2;        // K tiles, and V tiles, in flight
 constexpr int kUnMaskWords = 4096;  // 32-bit words of selection masks per CTA
+constexpr int kUnMaxTokens = 256;   // tokens of a CTA (groups of one)
 constexpr int kUnMaxBlocks = 2048;  // blocks, and 64-key tiles of the union
 
 template <typename T, int D>
@@ -65,7 +66,8 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* pv_done = p_full + 2;              // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   int* list_n = reinterpret_cast<int*>(tmem_slot + 1);
-  unsigned* mask = reinterpret_cast<unsigned*>(tmem_slot + 4);               // [blocks][mw]: which tokens of the CTA selected a block
+  unsigned* twice = reinterpret_cast<unsigned*>(tmem_slot + 4);              // [kUnMaxTokens / 32]: tokens that gave a block twice
+  unsigned* mask = twice + kUnMaxTokens / 32;                                // [blocks][mw]: which tokens of the CTA selected a block
   uint16_t* list = reinterpret_cast<uint16_t*>(mask + kUnMaskWords);         // 64-key tiles of the union, ascending
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -132,6 +134,7 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     tmem_relinquish();
   }
   for (int i = threadIdx.x; i < nblk * mw; i += 320) mask[i] = 0u;
+  if (threadIdx.x < kUnMaxTokens / 32) twice[threadIdx.x] = 0u;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -150,7 +153,10 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const int tt = i / p.T, j = i - tt * p.T;
     if (q0 + tt < L) {
       const int idx = __ldg(p.topk_idx + h * p.t_sh + (long long)(qs + q0 + tt) * p.t_sn + j * p.t_sk);
-      if (idx >= 0 && idx <= (q0 + tt) / BS) atomicOr(mask + idx * mw + (tt >> 5), 1u << (tt & 31));
+      if (idx >= 0 && idx <= (q0 + tt) / BS) {
+        const unsigned bit = 1u << (tt & 31);
+        if (atomicOr(mask + idx * mw + (tt >> 5), bit) & bit) atomicOr(twice + (tt >> 5), bit);
+      }
     }
   }
   __syncthreads();
@@ -416,8 +422,10 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
       }
     }
-    // one row of the pair not finite: its first lse says so, and sparse_fwd.cu does the pair again after this kernel
-    const unsigned bad = __ballot_sync(0xffffffffu, valid && isnan(probe));
+    // one row of the pair not finite, or a block given twice (it counts twice; a mask holds it once): the pair's first lse says so,
+    // and sparse_fwd.cu does the pair again after this kernel
+    const bool again = isnan(probe) || ((twice[tt >> 5] >> (tt & 31)) & 1u);
+    const unsigned bad = __ballot_sync(0xffffffffu, valid && again);
     const unsigned pair_rows = ((1u << p.G) - 1u) << (lane & ~(p.G - 1));  // G <= 16
     const bool redo = (bad & pair_rows) != 0u && (row & (p.G - 1)) == 0;
     if (valid) p.lse[(long long)(qs + tpos) * p.Hq + head] = redo ? __int_as_float(0x7fffffff) : l > 0.f ? m_ref + log2f(l) : -INFINITY;

@@ -16,7 +16,8 @@ def topk_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, top
     Args:
         q: [total_len, num_q_heads, head_dim]
         k, v: [total_len, num_kv_heads, head_dim]
-        topk_idx: int32 [num_kv_heads, total_len, topk], valid block ids first, -1 padding
+        topk_idx: int32 [num_kv_heads, total_len, topk], valid block ids first, -1 padding; the keys of an id given twice
+            count twice, forward and backward, as in the single-token operator
         block_size: keys per block (multiple of 64)
         cu_seqlens: int32 [batch + 1]
         softmax_scale: default 1/sqrt(head_dim)

@@ -175,3 +175,53 @@ def test_unions_are_no_less_exact_than_private_walks(Hq, Hkv, d, topk, lens, dty
     worst = float((lse.double() - exact_lse)[seen].abs().max())
     assert worst <= 6e-6, worst
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("Hq,Hkv,d,topk,lens,dtype", [
+    (8, 2, 128, 5, [300, 200], torch.bfloat16),
+    (3, 3, 64, 4, [257], torch.float16),        # groups of one: 256 tokens per CTA
+    (16, 1, 64, 4, [2600], torch.bfloat16),     # crosses the division
+])
+def test_blocks_given_twice_count_twice(Hq, Hkv, d, topk, lens, dtype):
+    """Some tokens give a block two or three times: output and gradients against attention whose logits carry the logarithm of the
+    number of times, and the single-token operator on the last token's row."""
+    import native_sparse_attention_triton_b200 as pkg
+    g = torch.Generator().manual_seed(23)
+    N, bs, G = sum(lens), 64, Hq // Hkv
+    rnd = lambda h: torch.randn(N, h, d, generator=g).to(dtype).cuda()
+    q, k, v, do = rnd(Hq), rnd(Hkv), rnd(Hkv), rnd(Hq)
+    idx = selection(g, lens, Hkv, bs, topk)
+    for t in range(N):
+        if t % 3 == 0 or t == N - 1:
+            for h in range(Hkv):
+                ids = [x for x in idx[h, t].tolist() if x >= 0]
+                ids = (ids + ids[-1:] * (1 + t % 2) + ids)[:topk]
+                idx[h, t] = torch.tensor(ids + [-1] * (topk - len(ids)), dtype=torch.int32)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    a = [x.clone().requires_grad_(True) for x in (q, k, v)]
+    o = pkg.ops.topk_sparse_attention(*a, idx.cuda(), bs, cu)
+    grads = torch.autograd.grad(o, a, do)
+    b = [x.double().requires_grad_(True) for x in (q, k, v)]
+    outs, at = [], 0
+    for n in lens:
+        nb = (n + bs - 1) // bs
+        ids = idx[:, at:at + n].long().cuda()
+        times = torch.zeros(Hkv, n, nb + 1, device="cuda").scatter_add_(2, torch.where(ids < 0, nb, ids), torch.ones(ids.shape, device="cuda"))
+        times = times[..., :nb].repeat_interleave(bs, 2)[..., :n] * torch.ones(n, n, device="cuda").tril()
+        s = torch.einsum("nhgd,mhd->hgnm", b[0][at:at + n].view(n, Hkv, G, d), b[1][at:at + n]) * d ** -0.5
+        s = s + times.double().log()[:, None]
+        empty = (times.sum(-1) == 0)[:, None, :, None]
+        p = torch.where(empty, 0.0, s.masked_fill(empty, 0.0).softmax(-1))
+        outs.append(torch.einsum("hgnm,mhd->nhgd", p, b[2][at:at + n]).reshape(n, Hq, d))
+        at += n
+    want = torch.cat(outs)
+    for name, x, y in zip(("o", "dq", "dk", "dv"), (o,) + grads, (want,) + torch.autograd.grad(want, b, do.double())):
+        rel = float((x.detach().double() - y.detach()).norm() / y.detach().norm())
+        # P, dS and the results are rounded to 16 bits: 2^-9 (2^-12 in fp16) each, two or three times; once instead of twice is 0.1
+        assert rel <= (8e-3 if dtype == torch.bfloat16 else 1e-3), (name, rel)
+    n = lens[-1]
+    last = pkg.ops.topk_sparse_attention_decode(q[-1:], k[N - n:][None], v[N - n:][None], idx[:, -1:].cuda(), bs,
+                                                torch.tensor([n], dtype=torch.int32).cuda())
+    err = (last[0].double() - want[-1].detach()).abs() / want[-1].detach().abs().clamp(min=1.0)
+    assert float(err.max()) <= 2e-2
+    assert pkg.device_status() == 0
