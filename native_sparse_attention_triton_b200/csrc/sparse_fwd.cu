@@ -49,8 +49,9 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   if (p.first > 0) {
     bool take = false;
     if (lane < p.span && base_n + lane < p.N) {
-      const int pos = base_n + lane - __ldg(p.cu_seqlens + find_sequence(p.cu_seqlens, p.B, base_n + lane));
-      take = pos >= p.first || isnan(__ldcg(p.lse + (long long)(base_n + lane) * p.Hq + h * p.G));
+      // (rows in front of the first sequence and behind the last, which cu_seqlens leaves out, are this kernel's)
+      const int n = base_n + lane, pos = n - __ldg(p.cu_seqlens + find_sequence(p.cu_seqlens, p.B, n));
+      take = pos < 0 || pos >= p.first || n >= __ldg(p.cu_seqlens + p.B) || isnan(__ldcg(p.lse + (long long)n * p.Hq + h * p.G));
     }
     todo = __ballot_sync(0xffffffffu, take);
   }

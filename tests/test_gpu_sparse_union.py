@@ -225,3 +225,28 @@ def test_blocks_given_twice_count_twice(Hq, Hkv, d, topk, lens, dtype):
     err = (last[0].double() - want[-1].detach()).abs() / want[-1].detach().abs().clamp(min=1.0)
     assert float(err.max()) <= 2e-2
     assert pkg.device_status() == 0
+
+
+def test_rows_outside_the_sequences_are_written():
+    """Padding rows behind the last sequence: they continue it, as they do where the private walk takes every token."""
+    import native_sparse_attention_triton_b200 as pkg
+    from native_sparse_attention_triton_b200 import _lib
+    Hq, Hkv, d, bs, topk, N, used = 8, 2, 128, 64, 4, 700, 530
+    g = torch.Generator().manual_seed(29)
+    rnd = lambda h: torch.randn(N, h, d, generator=g).bfloat16().cuda()
+    q, k, v = rnd(Hq), rnd(Hkv), rnd(Hkv)
+    idx = selection(g, [200, N - 200], Hkv, bs, topk).cuda()
+    out = []
+    for end in (used, N):
+        cu = torch.tensor([0, 200, end], dtype=torch.int32).cuda()
+        o, lse = torch.full_like(q, 7.0), torch.full((N, Hq), 7.0, device="cuda")
+        strides = _lib.strides_array(*[x for t in (q, k, v, o) for x in t.stride()[:2]], *idx.stride())
+        rc = _lib.lib().nsa_topk_sparse_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), idx.data_ptr(), cu.data_ptr(), o.data_ptr(),
+                                                 lse.data_ptr(), N, 2, Hq, Hkv, d, topk, bs, strides, d ** -0.5, _lib.DTYPE_BF16,
+                                                 torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        out.append(o.float())
+    err = (out[0] - out[1]).abs() / out[1].abs().clamp(min=1.0)
+    assert float(err.max()) <= 2e-2, float(err.max())
+    assert torch.equal(out[0][:256], out[1][:256])
+    assert pkg.device_status() == 0
