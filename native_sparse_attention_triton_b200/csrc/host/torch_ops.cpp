@@ -203,14 +203,13 @@ Layout layout_of(SeqInfo& info, int ks, int st, const at::Device& device) {
 
 // ----------------------------------------------------------------------------------------------------- autograd nodes
 // Saved tensors behind one lock, freed with the graph like those of torch's own nodes (a second backward without
-// retain_graph raises).
+// retain_graph raises).  They are unpacked with autograd's dispatch keys in place: an unpack hook may run operators that have to be
+// recorded (activation checkpointing computes the forward again in there).
 struct SavingNode : Node {
   std::vector<SavedVariable> saved;
-  bool released = false;
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     for (auto& s : saved) s.reset_data();
-    released = true;
   }
   std::vector<Tensor> unpack() {
     std::vector<Tensor> out;
@@ -267,8 +266,8 @@ struct CompressBackward final : SavingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView guard;
     const auto s = unpack();
+    at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor &x = s[0], &w = s[1], &pe = s[2], &cu = s[3], &ycu = s[4];
     const int64_t N = x.size(0), H = x.size(1), D = x.size(2);
     const Tensor dy = grads[0].contiguous();
@@ -391,8 +390,8 @@ struct DenseAttentionBackward final : SavingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView guard;
     const auto s = unpack();
+    at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor &q = s[0], &k = s[1], &v = s[2], &o = s[3], &lse = s[4], &cu_q = s[5], &cu_k = s[6];
     const int64_t N = q.size(0), Hq = q.size(1), D = q.size(2), Nk = k.size(0), Hkv = k.size(1);
     Tensor dq = empty({N, Hq, D}, q.scalar_type(), q.device()), dk = empty({Nk, Hkv, D}, q.scalar_type(), q.device()),
@@ -518,8 +517,8 @@ struct SparseAttentionBackward final : SavingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView guard;
     const auto s = unpack();
+    at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor &q = s[0], &k = s[1], &v = s[2], &o = s[3], &lse = s[4], &cu = s[5], &idx = s[6];
     const int64_t N = q.size(0), Hq = q.size(1), D = q.size(2), Hkv = k.size(1), topk = idx.size(2);
     const int batch = (int)cu.size(0) - 1;
@@ -593,8 +592,8 @@ struct GateCombineBackward final : SavingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(4);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView guard;
     const auto s = unpack();
+    at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor& gate = s[0];
     const Tensor dout = inner_contiguous(grads[0]);
     for (int i = 0; i < 4; ++i) out[i] = empty_like_rows(s[i]);
@@ -667,8 +666,8 @@ struct RopeBackward final : SavingNode {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    at::AutoDispatchBelowADInplaceOrView guard;
     const auto s = unpack();
+    at::AutoDispatchBelowADInplaceOrView guard;
     out[0] = rope_launch(inner_contiguous(grads[0]), s[0], s[1], m, 1);
     return out;
   }
