@@ -865,8 +865,8 @@ CacheRefs cache_refs(const std::vector<Tensor>& c) {
 // kernel's, before anything has been launched; the caller then takes the operators one by one.
 std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const Tensor& gate_in,
                                   const std::vector<Tensor>& caches, const OptTensor& w_k, const OptTensor& w_v, const OptTensor& pe,
-                                  int mode, const Tensor& inv_freq, double rope_scaling, int ks, int st, int block_size, int topk,
-                                  int init_blocks, int local_blocks, const OptTensor& out) {
+                                  int mode_k, int mode_v, const Tensor& inv_freq, double rope_scaling, int ks, int st, int block_size,
+                                  int topk, int init_blocks, int local_blocks, const OptTensor& out) {
   const CacheRefs c = cache_refs(caches);
   require_cuda(q_in, k_in, v_in, gate_in, inv_freq);
   at::NoGradGuard no_grad;
@@ -881,32 +881,29 @@ std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const 
   NSA_ASSERT(block_size % ks == 0 && ks % st == 0, "block_size must be a multiple of kernel_size, kernel_size of kernel_stride");
   if ((D != 64 && D != 128) || Hq / Hkv > 16 || c.cmp.size(2) == 0 || c.win.size(2) == 0) return std::nullopt;
   if (inv_freq.scalar_type() != at::kFloat || inv_freq.dim() != 1 || inv_freq.size(0) != D / 2 || !inv_freq.is_contiguous()) return std::nullopt;
-  if (mode != kAverage) {
-    NSA_ASSERT(w_k.has_value() && w_v.has_value(), "this compression needs weights");
-    for (const Tensor* w : {&*w_k, &*w_v}) {
-      require_cuda(*w);
-      NSA_ASSERT(w->scalar_type() == c.sel.scalar_type(), "w must have the caches' dtype");
-    }
-  }
-  const auto check_weight = [&](const OptTensor& w, bool linear) {
-    if (w) NSA_ASSERT(w->size(0) == Hkv && w->numel() == Hkv * ks * (linear ? D * D : 1), "w must be [num_heads, kernel_size * head_dim, head_dim] or [num_heads, kernel_size]");
+  NSA_ASSERT((mode_k == kLinear) == (mode_v == kLinear), "linear and pooling compression take separate launches");
+  const bool linear = mode_k == kLinear;
+  const auto weight = [&](const OptTensor& w, int mode) {  // of the keys or the values; average pooling has none
+    if (mode == kAverage) return Tensor();
+    NSA_ASSERT(w.has_value(), "this compression needs weights");
+    require_cuda(*w);
+    NSA_ASSERT(w->scalar_type() == c.sel.scalar_type(), "w must have the caches' dtype");
+    NSA_ASSERT(w->size(0) == Hkv && w->numel() == Hkv * ks * (linear ? D * D : 1), "w must be [num_heads, kernel_size * head_dim, head_dim] or [num_heads, kernel_size]");
+    return w->contiguous();
   };
-  check_weight(w_k, mode == kLinear);
-  check_weight(w_v, mode == kLinear);
+  const Tensor wk = weight(w_k, mode_k), wv = weight(w_v, mode_v);
   if (pe) {
     require_cuda(*pe);
     NSA_ASSERT(pe->scalar_type() == c.sel.scalar_type() && pe->numel() == Hkv * ks * D, "pe must be [num_heads, kernel_size, head_dim] of the caches' dtype");
   }
   const Tensor q = inner_contiguous(q_in), k = inner_contiguous(k_in), v = inner_contiguous(v_in), gate = gate_in.contiguous();
   Launch run(q);
-  Tensor pec, wk, wv;
-  if (w_k) wk = w_k->contiguous();
-  if (w_v) wv = w_v->contiguous();
+  Tensor pec;
   if (pe) pec = pe->contiguous();
   const auto p = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
   Tensor o = out ? *out : empty_like_rows(q);
   Tensor taps;
-  if (mode == kLinear) {
+  if (linear) {
     taps = empty({ks, B, 2, Hkv, D}, at::kFloat, q.device());
     const long long s[8] = {k.stride(0), k.stride(1), v.stride(0), v.stride(1), c.stage.stride(0), c.stage.stride(1), c.stage.stride(2),
                             c.stage.stride(3)};

@@ -131,9 +131,9 @@ def _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weig
     mine = rope if type(rope) is RotaryEmbedding else None if hasattr(rope, "decode_at3") else _device_rope_of(rope)
     if mine is None:
         return None
-    return _lib.host().decode_step(query, key, value, gate_value, cache._tensors(), compress_weight[0] if mode_k != 2 else None,
-                                   compress_weight[1] if mode_v != 2 else None, pe, mode_k, mine.inv_freq, mine.attention_scaling,
-                                   cache.kernel_size, cache.kernel_stride, block_size, topk, init_blocks, local_blocks, out)
+    return _lib.host().decode_step(query, key, value, gate_value, cache._tensors(), compress_weight[0], compress_weight[1], pe, mode_k,
+                                   mode_v, mine.inv_freq, mine.attention_scaling, cache.kernel_size, cache.kernel_stride, block_size,
+                                   topk, init_blocks, local_blocks, out)
 
 
 @torch.no_grad()

@@ -1,0 +1,113 @@
+"""nsa_infer with one compression for the keys and another for the values: prefill and decode steps against the oracle, the fused step
+against the separate operators, and the weights that a step refuses."""
+import math
+
+import pytest
+import torch
+
+from oracle import nsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+HQ, HKV, D, KS, ST, BS, TOPK, W = 8, 2, 128, 32, 16, 64, 4, 64
+FNS = {"linear": O.linear_compress, "weighted": O.weightedpool_compress, "avg": O.avgpool_compress}
+
+
+class Session:
+    """A prefilled cache and what a step takes."""
+
+    def __init__(self, mode_k, mode_v, dtype=torch.bfloat16, lens=(30, 100), max_length=256):
+        import native_sparse_attention_triton_b200 as pkg
+        from native_sparse_attention_triton_b200 import infer
+        from native_sparse_attention_triton_b200.kv_cache import NSACache
+        self.infer, self.dtype, self.lens, self.modes = infer, dtype, list(lens), (mode_k, mode_v)
+        self.g = torch.Generator().manual_seed(17)
+        fns = {"linear": pkg.ops.linear_compress, "weighted": pkg.ops.weightedpool_compress, "avg": pkg.ops.avgpool_compress}
+        self.w = [self.weight(m) for m in (mode_k, mode_v)]
+        self.pe = self.rnd(HKV, KS, D) * 0.02
+        self.inv_freq = 1.0 / (10000.0 ** (torch.arange(0, D, 2, dtype=torch.float32) / D))
+        self.cu = torch.tensor([0] + torch.tensor(self.lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+        self.cache = NSACache(len(lens), max_length, HKV, D, KS, ST, W, dtype)
+        self.args = dict(rope=infer.RotaryEmbedding(self.inv_freq.cuda()), cache=self.cache,
+                         compress_weight=tuple(None if w is None else w.cuda() for w in self.w), compress_func=(fns[mode_k], fns[mode_v]),
+                         intra_block_pe=self.pe.cuda(), kernel_size=KS, kernel_stride=ST, block_size=BS, topk=TOPK, init_blocks=1,
+                         local_blocks=2, window_size=W)
+        n = sum(self.lens)
+        self.prompt = [self.rnd(n, HQ, D), self.rnd(n, HKV, D), self.rnd(n, HKV, D), torch.rand(n, HQ, 3, generator=self.g).to(dtype)]
+        self.hist = [[t[self.cu[b]:self.cu[b + 1]] for b in range(len(lens))] for t in self.prompt[1:3]]
+
+    def rnd(self, *s):
+        return torch.randn(*s, generator=self.g).to(self.dtype)
+
+    def weight(self, mode):
+        if mode == "avg":
+            return None
+        return self.rnd(HKV, KS * D, D) / math.sqrt(KS * D) if mode == "linear" else self.rnd(HKV, KS) / math.sqrt(KS)
+
+    def prefill(self):
+        return self.infer.nsa_infer(self.cu, 0, *[t.cuda() for t in self.prompt], **self.args)
+
+    def rows(self):
+        b = len(self.lens)
+        return [self.rnd(b, HQ, D), self.rnd(b, HKV, D), self.rnd(b, HKV, D), torch.rand(b, HQ, 3, generator=self.g).to(self.dtype)]
+
+    def check(self, out, rows):
+        """The step's output for these rows, appended to the histories, against the oracle."""
+        f32 = lambda t: None if t is None else t.float()
+        for b in range(len(self.lens)):
+            for hist, new in zip(self.hist, rows[1:3]):
+                hist[b] = torch.cat([hist[b], new[b:b + 1]])
+            ref = O.nsa_decode_token(f32(rows[0][b]), f32(self.hist[0][b]), f32(self.hist[1][b]), f32(rows[3][b]), self.inv_freq,
+                                     FNS[self.modes[0]], FNS[self.modes[1]], f32(self.w[0]), f32(self.w[1]), f32(self.pe), KS, ST, BS, TOPK,
+                                     1, 2, W)
+            err = (out[b].float().cpu() - ref).abs() / ref.abs().clamp(min=1.0)
+            # the sum of three branches, each within the single-operator tolerance and of 16-bit rotated rows
+            assert float(err.max()) <= 4e-2 and float(err.mean()) <= 3e-3, (b, float(err.max()), float(err.mean()))
+
+
+@pytest.mark.parametrize("mode_k,mode_v", [("weighted", "avg"), ("avg", "weighted"), ("linear", "avg"), ("weighted", "linear")])
+def test_generation(mode_k, mode_v):
+    import native_sparse_attention_triton_b200 as pkg
+    s = Session(mode_k, mode_v)
+    s.prefill()
+    for step in range(1, 21):
+        rows = s.rows()
+        s.check(s.infer.nsa_infer(s.cu, step, *[t.cuda() for t in rows], **s.args), rows)
+    assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("mode_k,mode_v", [("weighted", "avg"), ("avg", "weighted")])
+def test_fused_step_equals_operators(monkeypatch, mode_k, mode_v):
+    a, b = Session(mode_k, mode_v), Session(mode_k, mode_v)
+    a.prefill(), b.prefill()
+    fused = a.infer._fused_decode_step
+    taken = []
+    monkeypatch.setattr(a.infer, "_fused_decode_step", lambda *x: taken.append(fused(*x)) or taken[-1])
+    for step in range(1, 21):
+        rows = [t.cuda() for t in a.rows()]
+        one = a.infer.nsa_infer(a.cu, step, *rows, **a.args)
+        with monkeypatch.context() as m:
+            m.setattr(b.infer, "_fused_decode_step", lambda *x: None)
+            two = b.infer.nsa_infer(b.cu, step, *rows, **b.args)
+        assert taken[-1] is one
+        err = (one.float() - two.float()).abs() / two.float().abs().clamp(min=1.0)
+        assert float(err.max()) <= 4e-2 and float(err.mean()) <= 4e-3
+    for x, y in zip(a.cache._tensors(), b.cache._tensors()):
+        assert x.dtype != torch.int32 or torch.equal(x, y)
+    # the same fp32 sums, rounded twice: an ulp or two of values around 1
+    assert float((a.cache.compress_kv_cache.float() - b.cache.compress_kv_cache.float()).abs().max()) <= 4e-2
+
+
+@pytest.mark.parametrize("mode_k,mode_v,which", [("weighted", "avg", 0), ("avg", "weighted", 1), ("weighted", "weighted", 1), ("linear", "linear", 1)])
+def test_weights_are_checked_on_their_own_side(mode_k, mode_v, which):
+    s = Session(mode_k, mode_v)
+    s.prefill()
+    rows = [t.cuda() for t in s.rows()]
+    before = [t.clone() for t in s.cache._tensors()]
+    w = s.args["compress_weight"][which]
+    for bad, error in ((w.float(), AssertionError), (w.half(), AssertionError), (w[:1], AssertionError), (None, AssertionError), (w.cpu(), RuntimeError)):
+        given = list(s.args["compress_weight"])
+        given[which] = bad
+        with pytest.raises(error):
+            s.infer.nsa_infer(s.cu, 1, *rows, **{**s.args, "compress_weight": tuple(given)})
+    for x, y in zip(s.cache._tensors(), before):
+        assert torch.equal(x, y)
