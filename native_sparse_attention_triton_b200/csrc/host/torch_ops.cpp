@@ -319,6 +319,8 @@ std::tuple<Tensor, Tensor> compress(const Tensor& x_in, const OptTensor& w_in, c
     else
       NSA_ASSERT(w.size(0) == x_in.size(1) && w.size(1) == ks, "w must be [num_heads, kernel_size]");
     require_cuda(w);
+  } else {
+    NSA_ASSERT(!w.defined(), "don't need additional weight for avgpool");
   }
   require_cuda(x_in, cu);
   if (pe.defined()) require_cuda(pe);

@@ -111,3 +111,12 @@ def test_weights_are_checked_on_their_own_side(mode_k, mode_v, which):
             s.infer.nsa_infer(s.cu, 1, *rows, **{**s.args, "compress_weight": tuple(given)})
     for x, y in zip(s.cache._tensors(), before):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("mode_k,mode_v,which", [("avg", "avg", 0), ("weighted", "avg", 1)])
+def test_prefill_refuses_weights_for_average_pooling(mode_k, mode_v, which):
+    s = Session(mode_k, mode_v)
+    given = list(s.args["compress_weight"])
+    given[which] = torch.ones(HKV, KS, dtype=s.dtype, device="cuda")
+    with pytest.raises(AssertionError):
+        s.infer.nsa_infer(s.cu, 0, *[t.cuda() for t in s.prompt], **{**s.args, "compress_weight": tuple(given)})
