@@ -114,11 +114,14 @@ def _compress_staged_pair(cache: NSACache, batch: int, funcs, weights, pe):
     return yk, yv
 
 
+_OWN_BOOKKEEPING = {name: NSACache.__dict__[name] for name in ("prepare_compress", "update_kv", "_fill")}
+
+
 def _is_plain(cache):
-    """A cache whose decode bookkeeping is NSACache's own (a subclass that replaces a part of it takes the operators one by one)."""
-    t = type(cache)
-    return t is NSACache or (issubclass(t, NSACache) and t.prepare_compress is NSACache.prepare_compress
-                             and t.update_kv is NSACache.update_kv and t._fill is NSACache._fill)
+    """A cache whose bookkeeping is NSACache's own: one that has a part of it replaced, on the object, in a subclass or in the class
+    itself, takes the operators one by one, which call it."""
+    return isinstance(cache, NSACache) and all(getattr(getattr(cache, name), "__func__", None) is own
+                                               for name, own in _OWN_BOOKKEEPING.items())
 
 
 def _fused_decode_step(cache, query, key, value, gate_value, rope, compress_weight, compress_func, pe, block_size, topk, init_blocks,
