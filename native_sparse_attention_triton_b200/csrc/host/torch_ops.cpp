@@ -299,8 +299,9 @@ struct CompressBackward final : SavingNode {
   }
 };
 
-std::tuple<Tensor, Tensor> compress(const Tensor& x_in, const OptTensor& w_in, const Tensor& cu, int ks, int st, const OptTensor& pe_in,
-                                    int mode) {
+// Argument checks of a compression; the weight and the position embedding, undefined where there is none.
+std::pair<Tensor, Tensor> check_compress(const Tensor& x_in, const OptTensor& w_in, const Tensor& cu, int ks, int st, const OptTensor& pe_in,
+                                         int mode) {
   NSA_ASSERT(is_16bit(x_in), "x must be float16 or bfloat16");
   NSA_ASSERT(is_int32(cu), "cu_seqlens must be int32");
   NSA_ASSERT(st > 0 && ks % st == 0, "kernel_size must be a multiple of kernel_stride");
@@ -324,6 +325,12 @@ std::tuple<Tensor, Tensor> compress(const Tensor& x_in, const OptTensor& w_in, c
   }
   require_cuda(x_in, cu);
   if (pe.defined()) require_cuda(pe);
+  return {w, pe};
+}
+
+std::tuple<Tensor, Tensor> compress(const Tensor& x_in, const OptTensor& w_in, const Tensor& cu, int ks, int st, const OptTensor& pe_in,
+                                    int mode) {
+  const auto [w, pe] = check_compress(x_in, w_in, cu, ks, st, pe_in, mode);
   auto info = seq_info(cu);
   const Layout l = layout_of(*info, ks, st, x_in.device());
   const CompressMeta m{mode, ks, st, (int)info->cu.size() - 1, l.total, info->longest};
@@ -345,6 +352,21 @@ std::tuple<Tensor, Tensor> compress(const Tensor& x_in, const OptTensor& w_in, c
     torch::autograd::set_history(y, node);
   }
   return {y, l.cu};
+}
+
+// One row per sequence from staging buffers: every sequence is one window of ks rows, cu and y_cu are its caller's device tensors, and
+// nothing is read on the host or remembered.
+Tensor compress_staged(const Tensor& x, const OptTensor& w_in, const Tensor& cu, const Tensor& y_cu, int ks, int st, const OptTensor& pe_in,
+                       int mode) {
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView guard;
+  const auto [w, pe] = check_compress(x, w_in, cu, ks, st, pe_in, mode);
+  require_cuda(y_cu);
+  const int batch = (int)cu.size(0) - 1;
+  NSA_ASSERT(is_int32(y_cu) && y_cu.size(0) == cu.size(0) && x.size(0) == (int64_t)batch * ks, "kernel_size rows per sequence");
+  const Layout l{ks, st, /*total=*/batch, /*longest=*/1, y_cu, 0};
+  return compress_forward(inner_contiguous(x), w.defined() ? w.contiguous() : w, pe.defined() ? pe.contiguous() : pe, cu, l,
+                          CompressMeta{mode, ks, st, batch, batch, ks});
 }
 
 // ------------------------------------------------------------------------------------- dense varlen and window attention
@@ -977,6 +999,7 @@ Tensor prefill(const Tensor& cu, const Tensor& q_in, const Tensor& k_in, const T
 PYBIND11_MODULE(_nsa_host, m) {
   m.doc() = "Host side of the native_sparse_attention_triton_b200 operators.";
   m.def("compress", &compress);
+  m.def("compress_staged", &compress_staged);
   m.def("compressed_attention", &compressed_attention);
   m.def("flash_attention_varlen", &flash_attention_varlen);
   m.def("sliding_window_attention", &sliding_window_attention);

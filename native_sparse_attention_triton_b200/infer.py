@@ -86,10 +86,14 @@ _MODES = {ops.linear_compress: 0, ops.weightedpool_compress: 1, ops.avgpool_comp
 
 
 def _compress_staged(cache: NSACache, batch: int, which: int, func: Callable, weight, pe):
-    """One compressed row per sequence from the staging buffers [batch * kernel_size, heads, d], the way the reference does it:
-    the compress function run over them with an arange cu_seqlens (infer/inference_func.py:56-87)."""
+    """One compressed row per sequence from the staging buffers [batch * kernel_size, heads, d] (the reference runs its
+    compress function over them with an arange cu_seqlens, infer/inference_func.py:56-87).  The library's own compress functions
+    need no host copy of cu_seqlens here; any other callable is called as given."""
     x = cache.before_compress_kv_cache[which, :batch].reshape(batch * cache.kernel_size, cache.num_kv_heads, cache.head_dim)
-    return func(x, weight, cache.stage_cu(batch), cache.kernel_size, cache.kernel_stride, pe)[0]
+    cu, mode = cache.stage_cu_seqlens[:batch + 1], _MODES.get(func)
+    if mode is None:
+        return func(x, weight, cu, cache.kernel_size, cache.kernel_stride, pe)[0]
+    return _lib.host().compress_staged(x, weight, cu, cache.stage_out_cu_seqlens[:batch + 1], cache.kernel_size, cache.kernel_stride, pe, mode)
 
 
 def _compress_staged_pair(cache: NSACache, batch: int, funcs, weights, pe):

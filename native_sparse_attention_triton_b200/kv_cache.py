@@ -49,14 +49,9 @@ class NSACache:
         self._step_ticket = lens[4]   # zero between decode steps
         self._allocated = self._tensors()
         self.device = self.sparse_kv_cache.device  # with its index
-        self._stage_cu = {}
-
-    def stage_cu(self, batch: int) -> torch.Tensor:
-        """cu_seqlens of the staging buffers seen as a varlen batch: `batch` sequences of kernel_size rows.  One tensor per batch
-        size, kept, so that its host copy is made once."""
-        if batch not in self._stage_cu:
-            self._stage_cu[batch] = torch.arange(batch + 1, dtype=torch.int32, device=self.device) * self.kernel_size
-        return self._stage_cu[batch]
+        # cu_seqlens of the staging buffers seen as a varlen batch (every sequence kernel_size rows, one compressed row)
+        self.stage_cu_seqlens = torch.arange(max_batch_size + 1, dtype=torch.int32, device=self.device) * kernel_size
+        self.stage_out_cu_seqlens = torch.arange(max_batch_size + 1, dtype=torch.int32, device=self.device)
 
     def _tensors(self):
         """What the fused prefill and decode step take, in the order csrc/host/torch_ops.cpp expects."""

@@ -120,3 +120,56 @@ def test_prefill_refuses_weights_for_average_pooling(mode_k, mode_v, which):
     given[which] = torch.ones(HKV, KS, dtype=s.dtype, device="cuda")
     with pytest.raises(AssertionError):
         s.infer.nsa_infer(s.cu, 0, *[t.cuda() for t in s.prompt], **{**s.args, "compress_weight": tuple(given)})
+
+
+@pytest.fixture
+def no_host_copies():
+    """Every synchronising copy raises."""
+    torch.cuda.synchronize()
+    yield lambda: torch.cuda.set_sync_debug_mode("error")
+    torch.cuda.set_sync_debug_mode("default")
+
+
+def test_a_step_of_separate_operators_reads_nothing_on_the_host(no_host_copies):
+    """A mixture of linear and pooling, in inference mode, where tensors carry no version counter and nothing can be remembered by."""
+    with torch.inference_mode():
+        s = Session("linear", "avg")
+        s.prefill()
+        for step in range(1, 4):
+            rows = s.rows()
+            gpu = [t.cuda() for t in rows]
+            no_host_copies()
+            out = s.infer.nsa_infer(s.cu, step, *gpu, **s.args)
+            torch.cuda.set_sync_debug_mode("default")
+            s.check(out, rows)
+
+
+def test_a_first_step_can_be_captured():
+    """No step of this cache has run before the capture, and 80 other cu_seqlens come by before the replays, which cross the end of a
+    compression window."""
+    import native_sparse_attention_triton_b200 as pkg
+    warm = Session("linear", "avg")          # the library's one-time initialisation
+    warm.prefill()
+    warm.infer.nsa_infer(warm.cu, 1, *[t.cuda() for t in warm.rows()], **warm.args)
+    s = Session("linear", "avg")
+    s.prefill()
+    fixed = [t.cuda() for t in s.rows()]
+    state = [t.clone() for t in s.cache._tensors()]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = s.infer.nsa_infer(s.cu, 1, *fixed, **s.args)
+    for dst, src in zip(s.cache._tensors(), state):
+        dst.copy_(src)
+    keep = []
+    for n in range(80):
+        keep.append(torch.tensor([0, 33 + n], dtype=torch.int32).cuda())
+        pkg.ops.avgpool_compress(torch.zeros(33 + n, 1, 64, device="cuda").bfloat16(), None, keep[-1], KS, ST, None)
+    junk = [torch.full((3,), 1 << 20, dtype=torch.int32, device="cuda") for _ in range(200)]
+    for _ in range(20):
+        rows = s.rows()
+        for dst, src in zip(fixed, rows):
+            dst.copy_(src)
+        graph.replay()
+        s.check(out, rows)
+    assert len(junk) == 200 and pkg.device_status() == 0
