@@ -724,10 +724,11 @@ Tensor rope(const Tensor& x, const Tensor& inv_freq, const Tensor& cu, int64_t s
 }
 
 // -------------------------------------------------------------------------------------------------- single-token operators
-// Split-KV scratch, one buffer per (device, stream): calls on one stream cannot overlap.  The kernels leave the control
-// words at the front at zero when they finish, so a buffer zeroed once serves every later call on that stream; it is regrown
-// (and zeroed again) when a call needs more.  A CUDA-graph capture uses the buffer of its capture stream when a warm-up call
-// on that stream has made one, else a fresh zeroed one from the graph's pool.  At most kScratchBuffers are kept.
+// Split-KV scratch, one buffer per (device, stream): calls on one stream cannot overlap.  The kernels leave the control words
+// at the front at zero when they finish, so a buffer zeroed once serves every later call on that stream; it is regrown (and
+// zeroed again) when a call needs more.  At most kScratchBuffers are kept.  A CUDA-graph capture takes none of them: a replay
+// finds its buffer by address, after other calls on the stream may have outgrown it, dirtied control words beyond their own, or had
+// it given back.  It gets one of the graph's pool, zeroed by a captured kernel at every replay.
 struct Scratch {
   Tensor buf;
   long long ctrl = 0;
@@ -740,54 +741,43 @@ uint64_t scratch_key(const at::Device& d, const c10::cuda::CUDAStream& s) {
   return (reinterpret_cast<uint64_t>(s.stream()) << 6) ^ (uint64_t)(d.index() & 63);
 }
 
-struct ScratchUse {
-  int splits = 1;
-  float* p = nullptr;
-  long long n = 0;
-  Tensor hold;
-  uint64_t key = 0;
-};
-
-ScratchUse take_scratch(int batch, int hkv, int d, int max_tiles, const at::Device& device, int compressed_cache_len = -1) {
-  ScratchUse u;
-  u.splits = nsa_decode_num_splits(batch, hkv, max_tiles);
-  u.n = compressed_cache_len < 0 ? nsa_decode_scratch_floats(batch, hkv, d, u.splits)
-                                 : nsa_compressed_decode_scratch_floats(batch, hkv, d, u.splits, compressed_cache_len);
-  const auto stream = c10::cuda::getCurrentCUDAStream(device.index());
-  u.key = scratch_key(device, stream);
-  if (u.n <= 0) {
-    u.n = 0;
-    return u;
-  }
-  const long long ctrl = ((long long)batch * hkv + 1 + 63) / 64 * 64;
-  const auto fresh = [&](long long n) {
+// `pairs`: (sequence, KV head) pairs; `n`: floats
+Tensor take_scratch(long long pairs, long long n, const at::Device& device, uint64_t key) {
+  const long long ctrl = (pairs + 1 + 63) / 64 * 64;
+  const auto fresh = [&] {
     Tensor t = empty({n}, at::kFloat, device);
     t.narrow(0, 0, ctrl).zero_();
     return t;
   };
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return fresh();
   std::lock_guard<std::mutex> lk(g_scratch_mu);
-  auto it = g_scratch.find(u.key);
-  const bool fits = it != g_scratch.end() && it->second.buf.numel() >= u.n;
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None && !(fits && it->second.ctrl >= ctrl)) {
-    u.hold = fresh(u.n);  // zeroed by a captured kernel at every replay
-  } else if (!fits) {
+  auto it = g_scratch.find(key);
+  if (it == g_scratch.end() || it->second.buf.numel() < n) {
     if (it == g_scratch.end() && g_scratch.size() >= kScratchBuffers) g_scratch.clear();  // their tensors go back to the allocator
-    u.hold = fresh(u.n);
-    g_scratch[u.key] = Scratch{u.hold, ctrl};
-  } else {
-    // the control region grows with batch * kv_heads; beyond the previous call's region lie that call's partial results
-    if (it->second.ctrl < ctrl) it->second.buf.narrow(0, 0, ctrl).zero_();
-    it->second.ctrl = ctrl;
-    u.hold = it->second.buf;
+    return (g_scratch[key] = Scratch{fresh(), ctrl}).buf;
   }
-  u.p = u.hold.data_ptr<float>();
-  return u;
+  // the control region grows with the pairs; beyond the previous call's region lie that call's partial results
+  if (it->second.ctrl < ctrl) it->second.buf.narrow(0, 0, ctrl).zero_();
+  it->second.ctrl = ctrl;
+  return it->second.buf;
 }
-// A failed call may have left control words that are not zero: forget the stream's scratch.
-void check_decode_rc(int rc, const char* name, const ScratchUse& u) {
-  if (rc) {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    g_scratch.erase(u.key);
+
+// A decode entry point, call(scratch, floats, splits): first without scratch, which the cluster kernels do not need and for want of
+// which the split-KV kernel's route answers -3 before it launches anything; then with it.
+template <typename Call>
+void with_scratch(const char* name, int batch, int hkv, int d, int cache_len, bool compressed, const at::Device& device, Call call) {
+  const int splits = nsa_decode_num_splits(batch, hkv, (cache_len + 63) / 64);
+  int rc = call(static_cast<float*>(nullptr), 0ll, splits);
+  if (rc == -3) {
+    const long long n = compressed ? nsa_compressed_decode_scratch_floats(batch, hkv, d, splits, cache_len)
+                                   : nsa_decode_scratch_floats(batch, hkv, d, splits);
+    const uint64_t key = scratch_key(device, c10::cuda::getCurrentCUDAStream(device.index()));
+    const Tensor buf = take_scratch((long long)batch * hkv, n, device, key);
+    rc = call(buf.data_ptr<float>(), n, splits);
+    if (rc) {  // a failed call may have left control words that are not zero
+      std::lock_guard<std::mutex> lk(g_scratch_mu);
+      g_scratch.erase(key);
+    }
   }
   check_rc(rc, name);
 }
@@ -821,11 +811,13 @@ Tensor flash_attention_decode(const Tensor& q_in, const Tensor& k_in, const Tens
   if (L == 0) return at::zeros_like(q);
   Tensor o = empty_like_rows(q);  // every row is written: a sequence without visible rows gets zeros from the kernel
   Launch run(q);
-  const ScratchUse u = take_scratch((int)B, (int)Hkv, (int)D, (int)((L + 63) / 64), q.device());
   const DecodeStrides st(q, k, v, o);
-  check_decode_rc(nsa_flash_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(seqlens), ptr(o), u.p, u.n, u.splits, (int)B, (int)L, (int)Hq,
-                                        (int)Hkv, (int)D, st.s, (float)sm_scale.value_or(default_scale(D)), dtype_code(q), run.stream),
-                  "nsa_flash_attn_decode", u);
+  with_scratch("nsa_flash_attn_decode", (int)B, (int)Hkv, (int)D, (int)L, /*compressed=*/false, q.device(),
+               [&](float* scratch, long long floats, int splits) {
+                 return nsa_flash_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(seqlens), ptr(o), scratch, floats, splits, (int)B, (int)L,
+                                              (int)Hq, (int)Hkv, (int)D, st.s, (float)sm_scale.value_or(default_scale(D)), dtype_code(q),
+                                              run.stream);
+               });
   return o;
 }
 
@@ -865,13 +857,14 @@ std::tuple<Tensor, Tensor> compressed_attention_decode(const Tensor& q_in, const
   const int max_blocks = (longest + block_size - 1) / block_size;
   Tensor o = empty_like_rows(q), idx = empty({Hkv, B, std::min(topk, max_blocks)}, at::kInt, q.device());
   Launch run(q);
-  const ScratchUse u = take_scratch((int)B, (int)Hkv, (int)D, (int)((L + 63) / 64), q.device(), (int)L);
   const DecodeStrides st(q, k, v, o, &idx);
-  check_decode_rc(nsa_compressed_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(seqlens), ptr<int>(comp), ptr(o), ptr<int>(idx), u.p, u.n,
-                                             u.splits, (int)B, (int)L, longest, (int)Hq, (int)Hkv, (int)D, ks, st_, block_size, topk,
-                                             init_blocks, local_blocks, st.s, (float)sm_scale.value_or(default_scale(D)), dtype_code(q),
-                                             run.stream),
-                  "nsa_compressed_attn_decode", u);
+  with_scratch("nsa_compressed_attn_decode", (int)B, (int)Hkv, (int)D, (int)L, /*compressed=*/true, q.device(),
+               [&](float* scratch, long long floats, int splits) {
+                 return nsa_compressed_attn_decode(ptr(q), ptr(k), ptr(v), ptr<int>(seqlens), ptr<int>(comp), ptr(o), ptr<int>(idx), scratch,
+                                                   floats, splits, (int)B, (int)L, longest, (int)Hq, (int)Hkv, (int)D, ks, st_, block_size,
+                                                   topk, init_blocks, local_blocks, st.s, (float)sm_scale.value_or(default_scale(D)),
+                                                   dtype_code(q), run.stream);
+               });
   return {o, idx};
 }
 

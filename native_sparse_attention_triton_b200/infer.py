@@ -267,7 +267,7 @@ class DecodeGraph:
         torch.cuda.current_stream(query.device).wait_stream(side)
         if not fused:
             self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph, stream=side):   # the warm-up stream: its decode scratch is reused by the capture
+            with torch.cuda.graph(self.graph, stream=side):
                 self.output = nsa_infer(cu_seqlens, 1, *self.inputs, **self.args)
         for dst, src in zip(self._state(cache), state):
             dst.copy_(src)
