@@ -288,15 +288,18 @@ class DecodeGraph:
         srcs = [query, key, value, gate_value]
         same = all(s.dtype == d.dtype and s.device == d.device and s.shape == d.shape for s, d in zip(srcs, self.inputs))
         if same and self.graph is None:
-            self._step(srcs)
-            return self.output
+            return self._launched(srcs)
         if same:
             torch._foreach_copy_(self.inputs, srcs)   # one launch for the four inputs
         else:
             for dst, src in zip(self.inputs, srcs):
                 dst.copy_(src)
         if self.graph is None:
-            self._step(self.inputs)
-        else:
-            self.graph.replay()
+            return self._launched(self.inputs)
+        self.graph.replay()
+        return self.output
+
+    def _launched(self, inputs):
+        if self._step(inputs) is None:
+            raise RuntimeError("the cache or the rotary embedding was changed so that the fused step no longer takes it")
         return self.output

@@ -173,3 +173,15 @@ def test_a_first_step_can_be_captured():
         graph.replay()
         s.check(out, rows)
     assert len(junk) == 200 and pkg.device_status() == 0
+
+
+def test_a_graph_whose_cache_no_longer_fits_says_so():
+    s = Session("weighted", "avg")
+    s.prefill()
+    rows = [t.cuda() for t in s.rows()]
+    graph = s.infer.DecodeGraph(s.cu, *rows, **s.args)
+    assert graph.graph is None
+    graph(*rows)
+    s.cache.update_kv = lambda *a, **k: None
+    with pytest.raises(RuntimeError):
+        graph(*rows)
