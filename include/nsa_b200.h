@@ -354,7 +354,8 @@ int nsa_rope_decode3(const void* q, void* yq, const void* k, void* yk, const voi
  *   windows, or NULL; linear_taps: NULL for pooling; else the output of nsa_linear_decode_taps for this step (which takes pe then).
  *   strides[26]: q_b q_h | k_b k_h | v_b v_h | gate_b gate_h | out_b out_h | (kv, sequence, row, head) of the selected-block,
  *   compressed, staging and sliding-window caches.
- * Returns -2 for a group of more than 16 query heads, more than 64 selected 64-key tiles or head_dim other than 64 and 128. */
+ * Returns -2 for a group of more than 16 query heads, more than 64 selected 64-key tiles, head_dim other than 64 and 128, or more
+ * compressed rows and blocks than shared memory holds the scores of. */
 int nsa_decode_step(const void* q, const void* k, const void* v, const void* gate, void* out, void* sparse_cache, int* sparse_len,
                     void* compress_cache, int* compress_len, void* stage_cache, int* stage_len, void* sliding_cache,
                     int* sliding_len, int* ticket, const void* w_k, const void* w_v, const void* pe, const float* linear_taps,
@@ -362,6 +363,12 @@ int nsa_decode_step(const void* q, const void* k, const void* v, const void* gat
                     int kernel_size, int kernel_stride, int block_size, int topk, int init_blocks, int local_blocks,
                     int sparse_rows, int compress_rows, int sliding_rows, const long long* strides, float sm_scale, int dtype,
                     void* stream);
+
+/* Whether nsa_decode_step takes these sizes, without launching anything: 0, or the code it would return (-2 also where a cluster's
+ * logits do not fit into shared memory). */
+int nsa_decode_step_supported(int batch, int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride,
+                              int block_size, int topk, int init_blocks, int local_blocks, int sparse_rows, int compress_rows,
+                              int sliding_rows, int dtype);
 
 /* Linear compression of the windows the coming decode step completes: taps[tap][b][key, value][h][:] = row `tap` of the
  * staged window (with the new token k, v appended; plus pe [Hkv, kernel_size, d] for keys, unless NULL) times its [d, d] slice of w_k / w_v [Hkv, kernel_size * d, d], for every

@@ -50,6 +50,7 @@ _SIGNATURES = {
     "nsa_pool_compress_decode_pair": [_P] * 8 + [_I, _I, _I, _I, _L, _L, _L, _I, _P],
     "nsa_pool_bias": [_P, _P, _P, _I, _I, _I, _I, _P],
     "nsa_linear_decode_taps": [_P] * 8 + [_I] * 5 + [_P, _I, _P],
+    "nsa_decode_step_supported": [_I] * 14,
     "nsa_decode_step": [_P] * 19 + [_F] + [_I] * 13 + [_P, _F, _I, _P],
     "nsa_decode_num_splits": [_I, _I, _I],
     "nsa_flash_attn_decode": [_P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P],

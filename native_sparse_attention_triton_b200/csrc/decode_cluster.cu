@@ -848,10 +848,12 @@ int run_compressed(Params p, cudaStream_t stream) {
   return launch<T, D, 4, kCompressed>(p, "decode_attn_compressed", stream);
 }
 
+// CTAs per cluster and logits per CTA of a step; kUnsupported where they do not fit into shared memory
+constexpr int kStepWarps = 8;
 template <typename T, int D>
-int run_step(Params p, cudaStream_t stream) {
-  constexpr int NW = 8;
-  const int half = NW / 2;
+int plan_step(Params* plan) {
+  Params& p = *plan;
+  const int half = kStepWarps / 2;
   // sub-tiles of the longest branch per warp that serves it
   int subtiles = (p.cmp.rows + kSub - 1) / kSub;
   const int win = (p.win.rows + kSub - 1) / kSub, sel = (p.topk_out * (p.block_size / kSub) + 1) / 2;
@@ -859,7 +861,31 @@ int run_step(Params p, cudaStream_t stream) {
   if (sel > subtiles) subtiles = sel;
   p.S = cluster_size((long long)p.B * p.Hkv, subtiles, half, 8);
   set_logit_slots(p, p.cmp.rows, half);
-  return launch<T, D, NW, kStep>(p, "decode_step", stream);
+  return smem_bytes<T, D, kStepWarps, kStep>(p) > kSmemLimit ? kUnsupported : kOk;
+}
+
+template <typename T, int D>
+int run_step(Params p, cudaStream_t stream) {
+  const int rc = plan_step<T, D>(&p);
+  return rc ? rc : launch<T, D, kStepWarps, kStep>(p, "decode_step", stream);
+}
+
+// The sizes of a step, checked
+int step_sizes(Params& p, int batch, int num_q_heads, int num_kv_heads, int kernel_size, int kernel_stride, int block_size, int topk,
+               int init_blocks, int local_blocks, int sparse_rows, int compress_rows, int sliding_rows) {
+  if (batch <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return kInvalid;
+  if (num_q_heads / num_kv_heads > 16) return kUnsupported;
+  if (kernel_size <= 0 || kernel_stride <= 0 || kernel_size % kernel_stride || block_size <= 0 || block_size % kernel_stride || topk < 1) return kInvalid;
+  if (topk < init_blocks + local_blocks || sparse_rows <= 0 || compress_rows <= 0 || sliding_rows <= 0) return kInvalid;
+  if (block_size % kSub) return kUnsupported;
+  p.B = batch; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.block_size = block_size; p.window = kernel_size;
+  p.stride = kernel_stride; p.init_blocks = init_blocks; p.local_blocks = local_blocks;
+  p.sel.rows = sparse_rows; p.cmp.rows = compress_rows; p.stage.rows = kernel_size; p.win.rows = sliding_rows;
+  const int max_blocks = (sparse_rows + block_size - 1) / block_size;
+  p.topk_out = topk < max_blocks ? topk : max_blocks;
+  p.nb_pad = (max_blocks + 31) & ~31;
+  if ((long long)p.topk_out * block_size > (long long)kMaxSelTiles * 64 || p.topk_out > kMaxSelTiles) return kUnsupported;
+  return kOk;
 }
 
 template <typename T, int D>
@@ -891,6 +917,17 @@ int decode_cluster_compressed(const DecodeOpArgs& a, cudaStream_t stream) {
 
 }  // namespace nsa
 
+extern "C" int nsa_decode_step_supported(int batch, int num_q_heads, int num_kv_heads, int head_dim, int kernel_size, int kernel_stride,
+                                         int block_size, int topk, int init_blocks, int local_blocks, int sparse_rows, int compress_rows,
+                                         int sliding_rows, int dtype) {
+  using namespace nsa;
+  Params p{};
+  const int rc = step_sizes(p, batch, num_q_heads, num_kv_heads, kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks,
+                            sparse_rows, compress_rows, sliding_rows);
+  if (rc) return rc;
+  return NSA_DISPATCH_T_D(dtype, head_dim, plan_step, &p);
+}
+
 // strides: q_b q_h | k_b k_h | v_b v_h | gate_b gate_h | out_b out_h | then (kv, sequence, row, head) of the selected-block,
 // compressed, staging and window caches: 26 entries, elements
 extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, const void* gate, void* out, void* sparse_cache, int* sparse_len,
@@ -901,16 +938,14 @@ extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, cons
                                int sparse_rows, int compress_rows, int sliding_rows, const long long* strides, float sm_scale, int dtype,
                                void* stream) {
   using namespace nsa;
-  if (!q || !k || !v || !gate || !out || !ticket || !inv_freq || !strides || batch <= 0 || num_kv_heads <= 0) return kInvalid;
-  if (num_q_heads % num_kv_heads) return kInvalid;
-  if (num_q_heads / num_kv_heads > 16) return kUnsupported;
-  if (kernel_size <= 0 || kernel_stride <= 0 || kernel_size % kernel_stride || block_size % kernel_stride || topk < 1) return kInvalid;
-  if (topk < init_blocks + local_blocks) return kInvalid;
-  if (block_size % kSub) return kUnsupported;
+  if (!q || !k || !v || !gate || !out || !ticket || !inv_freq || !strides) return kInvalid;
+  Params p{};
+  const int rc = step_sizes(p, batch, num_q_heads, num_kv_heads, kernel_size, kernel_stride, block_size, topk, init_blocks, local_blocks,
+                            sparse_rows, compress_rows, sliding_rows);
+  if (rc) return rc;
   for (int i = 0; i < 6; ++i)
     if (strides[i] % 8) return kInvalid;
   if (strides[8] % 8 || strides[9] % 8 || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out)) return kInvalid;
-  Params p{};
   p.q = q; p.k = k; p.v = v; p.gate = gate; p.o = out;
   p.q_sb = strides[0]; p.q_sh = strides[1]; p.k_sb = strides[2]; p.k_sh = strides[3]; p.v_sb = strides[4]; p.v_sh = strides[5];
   p.g_sb = strides[6]; p.g_sh = strides[7]; p.o_sb = strides[8]; p.o_sh = strides[9];
@@ -921,12 +956,6 @@ extern "C" int nsa_decode_step(const void* q, const void* k, const void* v, cons
   if (!cache_ok(p.sel) || !cache_ok(p.cmp) || !cache_ok(p.stage) || !cache_ok(p.win)) return kInvalid;
   p.ticket = ticket; p.w[0] = w_k; p.w[1] = w_v; p.pe = linear_taps ? nullptr : pe; p.partial = linear_taps; p.inv_freq = inv_freq;
   p.rope_scaling = attention_scaling;
-  p.B = batch; p.Hkv = num_kv_heads; p.G = num_q_heads / num_kv_heads; p.block_size = block_size; p.window = kernel_size;
-  p.stride = kernel_stride; p.init_blocks = init_blocks; p.local_blocks = local_blocks;
-  const int max_blocks = (sparse_rows + block_size - 1) / block_size;
-  p.topk_out = topk < max_blocks ? topk : max_blocks;
-  if ((long long)p.topk_out * block_size > (long long)kMaxSelTiles * 64 || p.topk_out > kMaxSelTiles) return kUnsupported;
-  p.nb_pad = (max_blocks + 31) & ~31;
   p.scale2 = sm_scale * kLog2e;
   p.st.word = status_word();
   return NSA_DISPATCH_T_D(dtype, head_dim, run_step, p, static_cast<cudaStream_t>(stream));

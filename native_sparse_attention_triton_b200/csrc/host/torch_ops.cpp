@@ -915,6 +915,10 @@ std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const 
   }
   const Tensor q = inner_contiguous(q_in), k = inner_contiguous(k_in), v = inner_contiguous(v_in), gate = gate_in.contiguous();
   Launch run(q);
+  const int fits = nsa_decode_step_supported((int)B, (int)Hq, (int)Hkv, (int)D, ks, st, block_size, topk, init_blocks, local_blocks,
+                                             (int)c.sel.size(2), (int)c.cmp.size(2), (int)c.win.size(2), dtype_code(q));
+  if (fits == -2) return std::nullopt;
+  check_rc(fits, "nsa_decode_step");
   Tensor pec;
   if (pe) pec = pe->contiguous();
   const auto p = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
@@ -935,13 +939,12 @@ std::optional<Tensor> decode_step(const Tensor& q_in, const Tensor& k_in, const 
   int n = 10;
   for (const Tensor* t : {&c.sel, &c.cmp, &c.stage, &c.win})
     for (int i = 0; i < 4; ++i) strides[n++] = t->stride(i);
-  const int rc = nsa_decode_step(ptr(q), ptr(k), ptr(v), ptr(gate), ptr(o), ptr(c.sel), ptr<int>(c.sel_len), ptr(c.cmp), ptr<int>(c.cmp_len),
-                                 ptr(c.stage), ptr<int>(c.stage_len), ptr(c.win), ptr<int>(c.win_len), ptr<int>(c.ticket), p(wk), p(wv),
-                                 p(pec), static_cast<float*>(p(taps)), ptr<float>(inv_freq), (float)rope_scaling, (int)B, (int)Hq, (int)Hkv,
-                                 (int)D, ks, st, block_size, topk, init_blocks, local_blocks, (int)c.sel.size(2), (int)c.cmp.size(2),
-                                 (int)c.win.size(2), strides, (float)default_scale(D), dtype_code(q), run.stream);
-  if (rc == -2) return std::nullopt;
-  check_rc(rc, "nsa_decode_step");
+  check_rc(nsa_decode_step(ptr(q), ptr(k), ptr(v), ptr(gate), ptr(o), ptr(c.sel), ptr<int>(c.sel_len), ptr(c.cmp), ptr<int>(c.cmp_len),
+                           ptr(c.stage), ptr<int>(c.stage_len), ptr(c.win), ptr<int>(c.win_len), ptr<int>(c.ticket), p(wk), p(wv),
+                           p(pec), static_cast<float*>(p(taps)), ptr<float>(inv_freq), (float)rope_scaling, (int)B, (int)Hq, (int)Hkv,
+                           (int)D, ks, st, block_size, topk, init_blocks, local_blocks, (int)c.sel.size(2), (int)c.cmp.size(2),
+                           (int)c.win.size(2), strides, (float)default_scale(D), dtype_code(q), run.stream),
+           "nsa_decode_step");
   return o;
 }
 

@@ -175,6 +175,41 @@ def test_a_first_step_can_be_captured():
     assert len(junk) == 200 and pkg.device_status() == 0
 
 
+def launches(run):
+    """Names of the library's launches during run()."""
+    import ctypes
+
+    from native_sparse_attention_triton_b200 import _lib
+    lib = _lib.lib()
+    lib.nsa_profile_enable(1)
+    try:
+        run()
+        buf = ctypes.create_string_buffer(1 << 16)
+        assert lib.nsa_profile_collect(buf, len(buf)) >= 0
+    finally:
+        lib.nsa_profile_enable(0)
+    return buf.value.decode()
+
+
+def test_a_refused_shape_costs_no_launch():
+    """A compressed cache whose scores do not fit into a cluster's shared memory: the step takes the operators, and the taps of the
+    fused step's linear compression are not launched for nothing."""
+    import native_sparse_attention_triton_b200 as pkg
+    s = Session("linear", "linear", max_length=70000)
+    assert pkg._lib.lib().nsa_decode_step_supported(2, HQ, HKV, D, KS, ST, BS, TOPK, 1, 2, 70000, s.cache.max_comp_length, W, 0) == 0
+    big = Session("linear", "linear", lens=(40,), max_length=400000)
+    assert pkg._lib.lib().nsa_decode_step_supported(1, HQ, HKV, D, KS, ST, BS, TOPK, 1, 2, 400000, big.cache.max_comp_length, W, 0) == -2
+    s.prefill()
+    rows = [t.cuda() for t in s.rows()]
+    names = launches(lambda: s.infer.nsa_infer(s.cu, 1, *rows, **s.args))
+    assert "linear_taps" in names and "decode_step" in names
+    big.prefill()
+    rows = [t.cuda() for t in big.rows()]
+    names = launches(lambda: big.infer._fused_decode_step(big.cache, *rows, big.args["rope"], big.args["compress_weight"],
+                                                          big.args["compress_func"], big.args["intra_block_pe"], BS, TOPK, 1, 2))
+    assert "linear_taps" not in names and "decode" not in names, names
+
+
 def test_a_graph_whose_cache_no_longer_fits_says_so():
     s = Session("weighted", "avg")
     s.prefill()
