@@ -220,3 +220,30 @@ def test_a_graph_whose_cache_no_longer_fits_says_so():
     s.cache.update_kv = lambda *a, **k: None
     with pytest.raises(RuntimeError):
         graph(*rows)
+
+
+def test_captured_graphs_replay():
+    """A step of separate operators, captured: two graphs alive on two sessions replay over the end of a compression window and give the
+    bits of eager steps from the same state; making a graph leaves the state as it was."""
+    import native_sparse_attention_triton_b200 as pkg
+    pairs, graphs = [(Session("linear", "avg"), Session("linear", "avg")), (Session("weighted", "linear"), Session("weighted", "linear"))], []
+    for a, b in pairs:
+        assert torch.equal(a.prefill(), b.prefill())
+        rows = [t.cuda() for t in a.rows()]
+        b.rows()
+        before = [t.clone() for t in a.infer.DecodeGraph._state(a.cache)]
+        graphs.append(a.infer.DecodeGraph(a.cu, *rows, **a.args))
+        assert graphs[-1].graph is not None
+        for x, y in zip(a.infer.DecodeGraph._state(a.cache), before):
+            assert torch.equal(x, y)
+    for step in range(1, 25):
+        for (a, b), graph in zip(pairs, graphs):
+            rows = a.rows()
+            gpu = [t.cuda() for t in rows]
+            out = graph(*gpu)
+            assert torch.equal(out, b.infer.nsa_infer(b.cu, step, *gpu, **b.args)), step
+            a.check(out, rows)
+    for a, b in pairs:
+        for x, y in zip(a.cache._tensors(), b.cache._tensors()):
+            assert torch.equal(x, y)
+    assert pkg.device_status() == 0

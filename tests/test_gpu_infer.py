@@ -1,6 +1,7 @@
 """Inference step on the device-side KV cache: prefill and a run of decode steps against the oracle, which restates what
 the reference's caches hold as a function of each sequence's token history; cache counters and the staged raw tokens are
-checked exactly; a CUDA-graph replay of the decode step must reproduce the eager launches bit for bit."""
+checked exactly; a DecodeGraph's step must reproduce the eager step bit for bit (here steps of the fused launch, which it launches
+directly; tests/test_gpu_decode_mixed.py has those it captures)."""
 import math
 
 import pytest
