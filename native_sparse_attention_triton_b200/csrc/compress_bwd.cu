@@ -445,7 +445,7 @@ extern "C" int nsa_linear_compress_bwd(const void* x, const void* w, const void*
   if (pe && (!dpe || !dbias_scratch)) return kInvalid;
   if (kernel_size <= 0 || kernel_stride <= 0 || kernel_size % kernel_stride || max_seqlen <= 0) return kInvalid;
   if (total_y > 0 && !dy) return kInvalid;
-  if ((x_stride_n | x_stride_h) % 8 || !aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(dw)) return kInvalid;
+  if ((x_stride_n | x_stride_h) % 8 || !aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(dw) || !aligned16(dy)) return kInvalid;
   LinBwdParams p;
   p.x = x; p.w = w; p.pe = pe; p.dy = dy; p.dbias = nullptr; p.dx = dx; p.dw = dw; p.cu = cu_seqlens; p.ycu = y_cu_seqlens;
   p.x_sn = x_stride_n; p.x_sh = x_stride_h; p.B = batch; p.H = num_heads; p.ks = kernel_size; p.stride = kernel_stride;
@@ -477,7 +477,7 @@ extern "C" int nsa_pool_compress_bwd(const void* x, const void* w, const void* p
   if (w && !dw) return kInvalid;
   if (kernel_size <= 0 || kernel_stride <= 0 || kernel_size % kernel_stride) return kInvalid;
   if (total_y > 0 && !dy) return kInvalid;
-  if ((x_stride_n | x_stride_h) % 8 || !aligned16(x) || !aligned16(dx)) return kInvalid;
+  if ((x_stride_n | x_stride_h) % 8 || !aligned16(x) || !aligned16(dx) || !aligned16(dy)) return kInvalid;
   PoolBwdParams p;
   p.x = x; p.w = w; p.pe = pe; p.dy = dy; p.dbias = nullptr; p.dx = dx; p.dw = w ? dw : nullptr; p.dpe = pe ? dpe : nullptr;
   p.cu = cu_seqlens; p.ycu = y_cu_seqlens; p.x_sn = x_stride_n; p.x_sh = x_stride_h;

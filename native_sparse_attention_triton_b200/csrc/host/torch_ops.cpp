@@ -270,7 +270,8 @@ struct CompressBackward final : SavingNode {
     at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor &x = s[0], &w = s[1], &pe = s[2], &cu = s[3], &ycu = s[4];
     const int64_t N = x.size(0), H = x.size(1), D = x.size(2);
-    const Tensor dy = grads[0].contiguous();
+    Tensor dy = grads[0].contiguous();
+    if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16) dy = dy.clone();  // a view of the caller's at an odd offset
     Tensor dx = empty({N, H, D}, x.scalar_type(), x.device()), dw, dpe;
     if (has_w) dw = empty(w.sizes(), w.scalar_type(), w.device());
     if (has_pe) dpe = empty(pe.sizes(), pe.scalar_type(), pe.device());
