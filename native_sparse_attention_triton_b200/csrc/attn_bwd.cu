@@ -926,6 +926,8 @@ static int varlen_attn_bwd_common(const void* q, const void* k, const void* v, c
   if (left >= 0 && (!causal || window != 1 || stride != 1)) return kUnsupported;
   for (int i = 0; i < 16; ++i)
     if (strides[i] % 8) return kInvalid;
+  for (const void* rows : {q, k, v, o, dout, (const void*)dq, (const void*)dk, (const void*)dv})  // read and written 16 bytes at a time
+    if (!aligned16(rows)) return kInvalid;
   if (workspace_bytes < (long long)dense_ws_bytes(total_q, total_k, num_q_heads, num_kv_heads, head_dim)) return kWorkspace;
   return NSA_DISPATCH_T_D(dtype, head_dim, run_dense_bwd, q, k, v, o, dout, lse, cu_seqlens_q, cu_seqlens_k, dq, dk, dv,
                           workspace, total_q, total_k, batch, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads, causal,
@@ -976,6 +978,8 @@ extern "C" int nsa_topk_sparse_attn_bwd(const void* q, const void* k, const void
   if (topk <= 0 || (long long)topk * (block_size / kKeyTile) > kMaxTilesBwd) return kUnsupported;
   for (int i = 0; i < 16; ++i)
     if (strides[i] % 8) return kInvalid;
+  for (const void* rows : {q, k, v, o, dout, (const void*)dq, (const void*)dk, (const void*)dv})  // read and written 16 bytes at a time
+    if (!aligned16(rows)) return kInvalid;
   if (workspace_bytes < (long long)sparse_ws_bytes(total_len, batch, num_q_heads, num_kv_heads, head_dim, topk, block_size))
     return kWorkspace;
   return NSA_DISPATCH_T_D(dtype, head_dim, run_sparse_bwd, q, k, v, o, dout, lse, topk_idx, cu_seqlens, dq, dk, dv,

@@ -96,6 +96,12 @@ Tensor inner_contiguous(const Tensor& t) {
   return ok ? t : t.contiguous();
 }
 
+// An output gradient as the kernels read it: also copied where it is a contiguous view at an odd offset.
+Tensor gradient_rows(const Tensor& t) {
+  const Tensor rows = inner_contiguous(t);
+  return reinterpret_cast<uintptr_t>(rows.data_ptr()) % 16 ? rows.clone() : rows;
+}
+
 // The tensors' device made current, and its current stream.
 struct Launch {
   c10::cuda::CUDAGuard guard;
@@ -270,8 +276,7 @@ struct CompressBackward final : SavingNode {
     at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor &x = s[0], &w = s[1], &pe = s[2], &cu = s[3], &ycu = s[4];
     const int64_t N = x.size(0), H = x.size(1), D = x.size(2);
-    Tensor dy = grads[0].contiguous();
-    if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16) dy = dy.clone();  // a view of the caller's at an odd offset
+    const Tensor dy = gradient_rows(grads[0].contiguous());
     Tensor dx = empty({N, H, D}, x.scalar_type(), x.device()), dw, dpe;
     if (has_w) dw = empty(w.sizes(), w.scalar_type(), w.device());
     if (has_pe) dpe = empty(pe.sizes(), pe.scalar_type(), pe.device());
@@ -425,7 +430,7 @@ struct DenseAttentionBackward final : SavingNode {
       out = {dq.zero_(), dk, dv};
       return out;
     }
-    const Tensor dout = inner_contiguous(grads[0]);
+    const Tensor dout = gradient_rows(grads[0]);
     const long long bytes = nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D);
     Tensor ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
     QkvStrides st;
@@ -549,7 +554,7 @@ struct SparseAttentionBackward final : SavingNode {
     const int batch = (int)cu.size(0) - 1;
     Tensor dq = empty({N, Hq, D}, q.scalar_type(), q.device()), dk = empty({N, Hkv, D}, q.scalar_type(), q.device()),
            dv = empty({N, Hkv, D}, q.scalar_type(), q.device());
-    const Tensor dout = inner_contiguous(grads[0]);
+    const Tensor dout = gradient_rows(grads[0]);
     const long long bytes = nsa_topk_sparse_attn_bwd_workspace((int)N, batch, (int)Hq, (int)Hkv, (int)D, (int)topk, block_size);
     Tensor ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
     QkvStrides st;
@@ -620,7 +625,7 @@ struct GateCombineBackward final : SavingNode {
     const auto s = unpack();
     at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor& gate = s[0];
-    const Tensor dout = inner_contiguous(grads[0]);
+    const Tensor dout = gradient_rows(grads[0]);
     for (int i = 0; i < 4; ++i) out[i] = empty_like_rows(s[i]);
     QkvStrides st;
     st.add(gate).add(s[1]).add(s[2]).add(s[3]).add(dout).add(out[0]).add(out[1]).add(out[2]).add(out[3]);
@@ -693,7 +698,7 @@ struct RopeBackward final : SavingNode {
     if (!grads[0].defined()) return out;
     const auto s = unpack();
     at::AutoDispatchBelowADInplaceOrView guard;
-    out[0] = rope_launch(inner_contiguous(grads[0]), s[0], s[1], m, 1);
+    out[0] = rope_launch(gradient_rows(grads[0]), s[0], s[1], m, 1);
     return out;
   }
 };

@@ -62,3 +62,21 @@ def test_dense(Hq, Hkv, lens, dtype, causal):
     pkg.ops.flash_attention_varlen(*dev, cu.cuda(), cu.cuda(), max(lens), max(lens), causal).backward(do.cuda())
     O.flash_attention_varlen(*ref, cu, cu, causal=causal).backward(do.float())
     check(dev, ref)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_gradient_at_an_odd_offset(d):
+    """A contiguous view whose address is no multiple of 16 bytes gives what its copy gives (up to the order of atomic sums)."""
+    import native_sparse_attention_triton_b200 as pkg
+    N, Hq, Hkv, bs = 300, 8, 2, 64
+    g = torch.Generator().manual_seed(4)
+    q, k, v = [torch.randn(N, h, d, generator=g).bfloat16().cuda().requires_grad_(True) for h in (Hq, Hkv, Hkv)]
+    cu = torch.tensor([0, N], dtype=torch.int32).cuda()
+    t = torch.arange(N)
+    idx = torch.stack([torch.zeros(N, dtype=torch.int64), torch.where(t < bs, -1, t // bs)], 1).int()[None].expand(Hkv, N, 2).contiguous().cuda()
+    odd = torch.randn(N * Hq * d + 1, generator=g).bfloat16().cuda()[1:].view(N, Hq, d)
+    assert odd.data_ptr() % 16 and odd.is_contiguous()
+    for o in (pkg.ops.topk_sparse_attention(q, k, v, idx, bs, cu), pkg.ops.flash_attention_varlen(q, k, v, cu, cu, N, N, causal=True)):
+        for a, b in zip(torch.autograd.grad(o, (q, k, v), odd, retain_graph=True), torch.autograd.grad(o, (q, k, v), odd.clone())):
+            assert float((a.float() - b.float()).norm()) <= 1e-3 * float(b.float().norm())
+    assert pkg.device_status() == 0
