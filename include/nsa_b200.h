@@ -37,7 +37,7 @@ int nsa_last_device_status(void* stream);
  * Replaces _topk_sparse_attention_fwd / forward_kernel,
  * native_sparse_attention/ops/triton/topk_sparse_attention.py:26-173,828-909.
  *   q [total_len, num_q_heads, d], k/v [total_len, num_kv_heads, d], o like q,
- *   topk_idx int32 [num_kv_heads, total_len, topk] (valid ids first, -1 padding),
+ *   topk_idx int32 [num_kv_heads, total_len, topk] (valid ids first, -1 padding; an id given twice counts twice),
  *   cu_seqlens int32 [batch+1], lse fp32 [total_len, num_q_heads] (base-2, scaled logits).
  *   strides[11] = {q_n, q_h, k_n, k_h, v_n, v_h, o_n, o_h, idx_h, idx_n, idx_k}. */
 int nsa_topk_sparse_attn_fwd(const void* q, const void* k, const void* v, const int* topk_idx,
@@ -126,8 +126,9 @@ int nsa_pool_bias(const void* pe, const void* w, void* bias, int num_heads, int 
  * be ZERO before the first call that uses a scratch buffer; every completed call leaves them zero again (they count with
  * wrap-around), so a buffer cleared once can be reused by any sequence of calls that do not overlap on the GPU -- except
  * that a call with MORE pairs than the previous call on the same buffer must clear its (longer) control region again,
- * because the previous call's partial results start right behind the shorter one.  One split of the flash / top-k
- * operators needs no scratch.  No counterpart in the reference. */
+ * because the previous call's partial results start right behind the shorter one.  One split of the flash operator, the top-k
+ * operator and all calls that the cluster kernels serve need no scratch; a call that needs it and has too little answers -3 before
+ * it launches anything.  No counterpart in the reference. */
 int nsa_decode_num_splits(int batch, int num_kv_heads, int max_tiles);
 long long nsa_decode_scratch_floats(int batch, int num_kv_heads, int head_dim, int num_splits);
 long long nsa_compressed_decode_scratch_floats(int batch, int num_kv_heads, int head_dim, int num_splits, int cache_len);
@@ -175,9 +176,10 @@ int nsa_topk_sparse_attn_decode(const void* q, const void* k, const void* v, con
  * Replaces compressed_attention_decode (about 15 ATen launches),
  * native_sparse_attention/ops/torch/compressed_attention_decode.py:21-153.
  *   topk_idx int32 [Hkv, B, min(topk, ceil(max_seqlen/block_size))] or NULL (output only).
- *   scratch: nsa_compressed_decode_scratch_floats(batch, num_kv_heads, head_dim, num_splits, cache_len) floats, always
- *   needed (-3 otherwise).  -2 when cache_len + ceil(max_seqlen/block_size) floats exceed two key tiles (about 8000 at
- *   head_dim 128: contexts beyond ~100 K tokens at stride 16). */
+ *   scratch: nsa_compressed_decode_scratch_floats(batch, num_kv_heads, head_dim, num_splits, cache_len) floats, needed beyond
+ *   three (sequence, KV head) pairs per SM or where a cluster's shared memory does not hold the scores (-3 otherwise).  There: -2
+ *   when cache_len + ceil(max_seqlen/block_size) floats exceed two key tiles (about 8000 at head_dim 128: contexts beyond ~100 K
+ *   tokens at stride 16). */
 int nsa_compressed_attn_decode(const void* q, const void* k, const void* v, const int* seqlens,
                                const int* compress_seqlens, void* o, int* topk_idx, float* scratch,
                                long long scratch_floats, int num_splits, int batch, int cache_len, int max_seqlen,

@@ -4,9 +4,11 @@
 native_sparse_attention/infer/nsa_inference.py:24-152 (with its helpers infer/inference_func.py:27-202): stage tokens for
 compression, compress, rotary embedding of query / compressed key / key, cache update, the three attention branches, the
 gated sum.  Differences, all on the decode path: positions and lengths come from the cache's device counters instead of
-the host-side ``step`` number, the staging buffers are compressed through the C interface with precomputed cu_seqlens,
-the compressed cache is passed whole (lengths mask it) instead of sliced to ``.max()``, and the sliding-window length is
-clamped on the device -- so one decode step is a fixed sequence of launches that ``DecodeGraph`` captures once and replays.
+the host-side ``step`` number, and nothing is read on the host.  With the library's own compression and rotary embedding a step
+is ONE launch (two with linear compression); with a caller's functions, a mixture of linear and pooling compression or a shape the
+fused kernel does not have it is a fixed sequence of launches, in which the staging buffers are compressed with precomputed
+cu_seqlens, the compressed cache is passed whole (lengths mask it) instead of sliced to ``.max()``, and the sliding-window length is
+clamped on the device.  ``DecodeGraph`` launches the first kind directly and captures and replays the second.
 """
 from typing import Callable, Optional, Tuple
 

@@ -5,8 +5,8 @@ Same constructor, attributes and methods as the reference's ``NSACache``
 values of the selected-block branch, of the compressed branch, the staging buffer of tokens not yet compressed, the
 sliding-window ring) with one int32 row counter each.  The reference fills them with a Triton kernel sized by
 ``.max().item()`` and updates them, per decode step, with ``torch.where`` and advanced-index assignments; here prefill is
-one copy kernel per cache and a decode step is two launches, all reading the counters on the device, so nothing
-synchronises with the host and a decode step can be replayed from a CUDA graph.
+one copy kernel per cache, and the bookkeeping of a decode step is part of the fused step's launch (``infer.py``) or two launches of
+its own, all reading the counters on the device, so nothing synchronises with the host and a decode step can be captured in a CUDA graph.
 """
 from typing import Union
 

@@ -13,6 +13,7 @@ than that is only ever taken from what the reference's kernels themselves score 
 import json
 import math
 import os
+import tempfile
 
 import pytest
 import torch
@@ -24,7 +25,7 @@ from oracle import nsa_oracle as O
 pytestmark = pytest.mark.gpu
 
 SLACK = 1.25
-REPORT = os.path.join(refbox.ROOT, os.environ.get("NSA_REPORT_DIR", "gpurun_out"), "parity_vs_triton.json")
+REPORT = os.path.join(refbox.ROOT, os.environ.get("NSA_REPORT_DIR", tempfile.gettempdir()), "parity_vs_triton.json")
 _report = {}
 
 
