@@ -161,8 +161,8 @@ def nsa_infer(cu_seqlens: torch.Tensor, step: int, query: torch.Tensor, key: tor
         mode_k, mode_v = _MODES.get(compress_func[0]), _MODES.get(compress_func[1])
         if mode_k is not None and mode_v is not None and type(rope) is RotaryEmbedding and _is_plain(cache):
             return _lib.host().prefill(cu_seqlens, query, key, value, gate_value, cache._tensors(), compress_weight[0], compress_weight[1],
-                                       intra_block_pe, mode_k, mode_v, rope.inv_freq, rope.attention_scaling, kernel_size, kernel_stride,
-                                       block_size, topk, init_blocks, local_blocks, window_size)
+                                       intra_block_pe, mode_k, mode_v, rope.inv_freq, rope.attention_scaling, cache.kernel_size,
+                                       cache.kernel_stride, block_size, topk, init_blocks, local_blocks, cache.window_size)
         cache.prepare_compress(cu_seqlens, 0, key, value)
         compress_key, compress_cu_seqlens = compress_func[0](key, compress_weight[0], cu_seqlens, kernel_size, kernel_stride,
                                                              intra_block_pe)

@@ -47,5 +47,6 @@ def compressed_attention(
     """
     if topk <= 0:
         warnings.warn("topk <= 0, returned topk_idx will be None")
+    max_seqlen_q, max_seqlen_k = (None if m is None else int(m) for m in (max_seqlen_q, max_seqlen_k))
     return _lib.host().compressed_attention(q, k, v, kernel_size, kernel_stride, block_size, topk, cu_seqlens_q, cu_seqlens_k,
                                             max_seqlen_q, max_seqlen_k, sm_scale, init_blocks, local_blocks)

@@ -28,7 +28,7 @@ def topk_sparse_attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tens
 
     topk_idx int32 [num_kv_heads, batch, topk], -1 padding.
     """
-    return _lib.host().topk_sparse_attention_decode(q, k, v, topk_idx, block_size, seqlens, sm_scale)
+    return _lib.host().topk_sparse_attention_decode(q, k, v, topk_idx, int(block_size), seqlens, sm_scale)
 
 
 def compressed_attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seqlens: torch.Tensor,

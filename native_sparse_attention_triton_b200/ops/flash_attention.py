@@ -16,4 +16,4 @@ def flash_attention_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu
     """Varlen GQA attention; causal means key j is visible to query i iff j <= i within a sequence."""
     if gqa_interleave:
         raise NotImplementedError("gqa_interleave=True is not supported")
-    return _lib.host().flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal, sm_scale)
+    return _lib.host().flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), bool(causal), sm_scale)

@@ -18,4 +18,4 @@ def rope(x: torch.Tensor, inv_freq: torch.Tensor, cu_seqlens: torch.Tensor, step
     """x [rows, heads, d] (d 64 or 128, bf16/fp16), inv_freq fp32 [d / 2], cu_seqlens int32 [batch + 1] -> rotated copy.
     With step > 0, rows == batch (one new token per sequence) and cu_seqlens holds the PREFILL lengths, as in the
     reference's decode loop."""
-    return _lib.host().rope(x, inv_freq, cu_seqlens, step, stride, attention_scaling)
+    return _lib.host().rope(x, inv_freq, cu_seqlens, int(step), int(stride), attention_scaling)

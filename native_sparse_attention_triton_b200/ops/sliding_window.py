@@ -17,4 +17,4 @@ def sliding_window_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     """q [total, Hq, d], k/v [total, Hkv, d] (self-attention: one cu_seqlens); key j is visible to query i of the same
     sequence iff i - window_size <= j <= i, i.e. window_size + 1 keys, as flash_attn's window_size=(window_size, -1) with
     causal=True gives."""
-    return _lib.host().sliding_window_attention(q, k, v, cu_seqlens, max_seqlen, window_size, sm_scale)
+    return _lib.host().sliding_window_attention(q, k, v, cu_seqlens, int(max_seqlen), int(window_size), sm_scale)

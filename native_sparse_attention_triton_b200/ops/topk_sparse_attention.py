@@ -24,4 +24,5 @@ def topk_sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, top
     Returns:
         attention output [total_len, num_q_heads, head_dim]
     """
-    return _lib.host().topk_sparse_attention(q, k, v, topk_idx, block_size, cu_seqlens, softmax_scale)
+    assert block_size in (32, 64, 128, 256), "block_size must be 32, 64, 128 or 256"
+    return _lib.host().topk_sparse_attention(q, k, v, topk_idx, int(block_size), cu_seqlens, softmax_scale)
