@@ -349,29 +349,53 @@ __global__ void __launch_bounds__(256) pool_dw_kernel(PoolBwdParams p) {
   }
 }
 
-// dw[h,k] from the streaming pass's partial rows (summed in slot order: deterministic) and dpe[h,k,:]
+// dw[h,k] and dpe[h,k,:] from the streaming pass's partial rows, summed in their order (deterministic).  Every CTA sums its head's
+// rows of dy's column sums for itself: 74 KB out of L2 for 144 rows, against a launch of its own.
 template <typename T>
-__global__ void __launch_bounds__(256) pool_dw_finish_kernel(PoolBwdParams p, const float* __restrict__ partial, int nslots) {
+__global__ void __launch_bounds__(256) pool_dw_finish_kernel(PoolBwdParams p, const float* __restrict__ partial, PoolBwdRows rows) {
+  constexpr int D = 128;
   __shared__ float red[8];
+  __shared__ float part[8][D];
+  __shared__ float dbias[D];
   const int h = blockIdx.x, k = blockIdx.y;
-  float acc = 0.f;
-  for (int s = threadIdx.x; s < nslots; s += blockDim.x) acc += partial[((size_t)s * p.H + h) * p.ks + k];
-  if (p.pe)
-    for (int n = threadIdx.x; n < p.D; n += blockDim.x)
-      acc += DT<T>::to_float(static_cast<const T*>(p.pe)[((size_t)h * p.ks + k) * p.D + n]) * p.dbias[h * p.D + n];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (p.pe && rows.bias) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 6
+    for (int r = warp; r < rows.ctas; r += 8)
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float tot = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red[i];
-    static_cast<T*>(p.dw)[h * p.ks + k] = DT<T>::from_float(tot);
+      for (int e = 0; e < 4; ++e) s[e] += __ldg(rows.bias + ((size_t)r * p.H + h) * D + e * 32 + lane);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) part[warp][e * 32 + lane] = s[e];
+    __syncthreads();
+    if (threadIdx.x < D) {
+      float t = 0.f;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) t += part[r][threadIdx.x];
+      dbias[threadIdx.x] = t;
+    }
+  } else if (p.pe && threadIdx.x < D) {
+    dbias[threadIdx.x] = p.dbias[h * D + threadIdx.x];
   }
-  if (p.dpe) {
-    const float wv = DT<T>::to_float(static_cast<const T*>(p.w)[h * p.ks + k]);
-    for (int n = threadIdx.x; n < p.D; n += blockDim.x)
-      static_cast<T*>(p.dpe)[((size_t)h * p.ks + k) * p.D + n] = DT<T>::from_float(wv * p.dbias[h * p.D + n]);
+  __syncthreads();
+  if (p.dw) {
+    float acc = 0.f;
+    for (int s = threadIdx.x; s < rows.slots; s += blockDim.x) acc += partial[((size_t)s * p.H + h) * p.ks + k];
+    if (p.pe && threadIdx.x < D)
+      acc += DT<T>::to_float(static_cast<const T*>(p.pe)[((size_t)h * p.ks + k) * D + threadIdx.x]) * dbias[threadIdx.x];
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float tot = 0.f;
+      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red[i];
+      static_cast<T*>(p.dw)[h * p.ks + k] = DT<T>::from_float(tot);
+    }
+  }
+  if (p.dpe && threadIdx.x < D) {
+    const float wv = p.w ? DT<T>::to_float(static_cast<const T*>(p.w)[h * p.ks + k]) : 1.f / (float)p.ks;
+    static_cast<T*>(p.dpe)[((size_t)h * p.ks + k) * D + threadIdx.x] = DT<T>::from_float(wv * dbias[threadIdx.x]);
   }
 }
 
@@ -405,27 +429,31 @@ static int run_linear_bwd(LinBwdParams p, void* dpe, float* dbias, int total_y, 
 template <typename T, int D>
 static int run_pool_bwd(PoolBwdParams p, float* dbias, float* partial, long long partial_floats, int total_y, int max_seqlen,
                         int dtype, cudaStream_t stream) {
-  if (p.pe) {
-    launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
-    p.dbias = dbias;
-  }
-  // long inputs: one streaming pass writes dx and (weighted pooling) the partial rows of dw
+  // long inputs: one streaming pass writes dx and the partial rows of dw (weighted pooling) and of dy's column sums (with pe)
   const long long need = pool_bwd_stream_partial_floats(p.H, D, p.N, p.B, max_seqlen, p.ks, p.stride);
-  if (total_y > 0 && need > 0 && (!p.dw || (partial && partial_floats >= need))) {
-    int nslots = 0;
-    const int rc = pool_bwd_stream(p.x, p.dw ? p.w : nullptr, p.dy, p.dx, p.dw ? partial : nullptr, &nslots, p.cu, p.ycu, p.B, p.N,
-                                   max_seqlen, p.H, D, p.ks, p.stride, p.x_sn, p.x_sh, dtype, stream);
+  const bool room = partial && partial_floats >= need;
+  bool summed = false;
+  if (total_y > 0 && need > 0 && (!p.dw || room)) {
+    if (p.pe && !room) {
+      launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
+      p.dbias = dbias;
+      summed = true;
+    }
+    PoolBwdRows rows;
+    const int rc = pool_bwd_stream(p.x, p.dw ? p.w : nullptr, p.dy, p.dx, room ? partial : nullptr, p.pe && room, &rows, p.cu, p.ycu, p.B,
+                                   p.N, max_seqlen, p.H, D, p.ks, p.stride, p.x_sn, p.x_sh, dtype, stream);
     if (rc != kInvalid && rc != kUnsupported) {
       if (rc) return rc;
-      if (p.dw) {
+      if (p.dw || p.dpe) {
         LaunchScope ls_("pool_dw_finish", stream);
-        pool_dw_finish_kernel<T><<<dim3(p.H, p.ks), 256, 0, stream>>>(p, partial, nslots);
-      } else if (p.dpe) {
-        LaunchScope ls_("pool_dw", stream);
-        pool_dw_kernel<T><<<dim3(p.H, p.ks), 256, 0, stream>>>(p);   // average pooling: only dpe is written
+        pool_dw_finish_kernel<T><<<dim3(p.H, p.ks), 256, 0, stream>>>(p, partial, rows);
       }
       return cuda_rc(cudaGetLastError());
     }
+  }
+  if (p.pe && !summed) {
+    launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
+    p.dbias = dbias;
   }
   const long long total = (long long)p.N * p.H * (D / 8);
   { LaunchScope ls_("pool_dx", stream); pool_dx_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(p); }

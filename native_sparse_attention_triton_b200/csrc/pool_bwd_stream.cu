@@ -8,6 +8,9 @@
 // consumer keeps the R gradient rows dy[c], ..., dy[c - R + 1] in registers (one new 16-byte load per chunk), writes the
 // chunk's dx rows, and accumulates the kernel_size partial dot products of its 8 columns in registers across its whole
 // sub-run; at the end they are summed over the 16 threads of a head and stored as one partial row per (CTA, group, head).
+// The column sums of dy that the position embedding's gradient needs come out of the same pass (every gradient row is the newest of
+// exactly one chunk): one partial row per CTA.  (As a kernel of their own in front of it they cost 23 us for 8 x 32 768 tokens, 4
+// heads: 17 MB read in 64-byte pieces by 128 CTAs.)
 // The caller adds the partial rows in a fixed order (deterministic, no floating-point atomics).
 #include <algorithm>
 
@@ -28,6 +31,7 @@ struct PoolBwdStreamParams {
   const void* dy;   // [M, H, D]
   void* dx;         // [N, H, D]
   float* partial;   // [slots][H][ks] or nullptr
+  float* bias;      // [slots / groups][H][D] or nullptr
   const int* cu;
   const int* ycu;
   int H, D, ks;
@@ -40,9 +44,15 @@ int pb_heads(int H) {
   while (hb * 2 <= H && hb < 8) hb *= 2;
   return hb;
 }
-int pb_run(int total_len, int stride, int groups) {
+// Chunks per CTA.  One CTA fits an SM (its ring), so the CTAs should fill whole waves: one wave while a CTA's run stays below 256
+// chunks, up to four beyond.  A sequence's last run is short, by half a run on average.  (8 x 32 768 tokens, 4 heads, weighted,
+// forward and backward: 195 us with runs of 128 chunks on 128 SMs and the column sums apart, 171 us with runs of 114 on 144.)
+int pb_run(int total_len, int batch, int stride, int groups, int head_blocks) {
   const int chunks = (total_len + stride - 1) / stride;
-  return std::max(32 * groups, (chunks + 148 * 4 - 1) / (148 * 4));
+  const int waves = std::min(4, std::max(1, (int)((long long)chunks * head_blocks / (148 * 128))));
+  const int ctas = 148 * waves / head_blocks;
+  const int full = std::max(std::max(1, ctas / 2), ctas - batch / 2);
+  return std::max(8 * groups, (chunks + full - 1) / full);
 }
 }  // namespace
 
@@ -55,13 +65,25 @@ __global__ void __launch_bounds__(kPbConsumers + 32, 1) pool_bwd_stream_kernel(c
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (DW ? (size_t)p.groups * p.slots * chunk_bytes : 0));
   uint64_t* empty = full + kPbMaxBars;
   float* wsm = reinterpret_cast<float*>(empty + kPbMaxBars);   // [hb][KS]
+  float* bias_sm = wsm + p.hb * KS;                            // [consumers][8], 16-byte aligned (hb and KS are multiples of two)
 
   const int b = blockIdx.y, h0 = blockIdx.z * p.hb;
   const int s0 = __ldg(p.cu + b), L = __ldg(p.cu + b + 1) - s0;
   const int y0 = __ldg(p.ycu + b), Mb = __ldg(p.ycu + b + 1) - y0;
   const int C = (L + S - 1) / S;
   const int c0 = blockIdx.x * p.run;
-  if (c0 >= C) return;
+  const int cta = blockIdx.y * gridDim.x + blockIdx.x;
+  if (c0 >= C) {  // nothing here: rows of zeros
+    const int heads = min(p.hb, p.H - h0);
+    if (DW)
+      for (int i = threadIdx.x; i < p.groups * heads * KS; i += blockDim.x) {
+        const int gg = i / (heads * KS);
+        p.partial[((size_t)(cta * p.groups + gg) * p.H + h0) * KS + (i - gg * heads * KS)] = 0.f;
+      }
+    if (p.bias)
+      for (int i = threadIdx.x; i < heads * p.D; i += blockDim.x) p.bias[((size_t)cta * p.H + h0) * p.D + i] = 0.f;
+    return;
+  }
   const int nch = min(p.run, C - c0);
   const int per_group = (nch + p.groups - 1) / p.groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -125,7 +147,6 @@ __global__ void __launch_bounds__(kPbConsumers + 32, 1) pool_bwd_stream_kernel(c
   const int g = threadIdx.x / items, col = threadIdx.x - g * items;
   const int hh = col / CH, cc = col - hh * CH;
   const int cg0 = g * per_group, cg1 = min(nch, cg0 + per_group);
-  if (cg1 <= cg0) return;
   const bool head_ok = h0 + hh < p.H;
   const int hq = head_ok ? h0 + hh : p.H - 1;   // a thread of a missing head reads a real row and stores nothing
   const T* dyp = static_cast<const T*>(p.dy) + ((size_t)y0 * p.H + hq) * p.D + cc * 8;
@@ -153,12 +174,16 @@ __global__ void __launch_bounds__(kPbConsumers + 32, 1) pool_bwd_stream_kernel(c
   const int row_bytes = p.hb * p.D * 2;
   T* dxp = static_cast<T*>(p.dx) + ((size_t)s0 * p.H + hq) * p.D + cc * 8;
 
+  float2 bsum[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   float2 dynext[4];   // the next chunk's new gradient row, fetched one chunk ahead
-  load_dy(c0 + cg0, dynext);
+  load_dy(cg0 < cg1 ? c0 + cg0 : -1, dynext);
   for (int i = 0; i < cg1 - cg0; ++i) {
     const int c = c0 + cg0 + i;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) dyr[0][e] = dynext[e];
+    for (int e = 0; e < 4; ++e) {
+      dyr[0][e] = dynext[e];
+      bsum[e] = fadd2(bsum[e], dynext[e]);
+    }
     load_dy(i + 1 < cg1 - cg0 ? c + 1 : -1, dynext);
     const uint8_t* rows = nullptr;
     if (DW) {
@@ -211,7 +236,7 @@ __global__ void __launch_bounds__(kPbConsumers + 32, 1) pool_bwd_stream_kernel(c
 
   if (DW) {
     // the 16 threads of a head (consecutive lanes) add their partial dot products; lane cc == 0 stores the row
-    const int slot = (blockIdx.y * gridDim.x + blockIdx.x) * p.groups + g;
+    const int slot = cta * p.groups + g;
     float* prow = p.partial + ((size_t)slot * p.H + hq) * KS;
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -222,6 +247,18 @@ __global__ void __launch_bounds__(kPbConsumers + 32, 1) pool_bwd_stream_kernel(c
         for (int off = 8; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if (cc == 0 && head_ok) prow[r * S + t] = v;
       }
+  }
+  if (p.bias) {  // the groups' sums, added in group order
+    float4* mine = reinterpret_cast<float4*>(bias_sm) + (size_t)threadIdx.x * 2;
+    mine[0] = make_float4(bsum[0].x, bsum[0].y, bsum[1].x, bsum[1].y);
+    mine[1] = make_float4(bsum[2].x, bsum[2].y, bsum[3].x, bsum[3].y);
+    asm volatile("bar.sync 1, %0;\n" ::"n"(kPbConsumers) : "memory");
+    const int heads = min(p.hb, p.H - h0);
+    for (int i = threadIdx.x; i < heads * p.D; i += kPbConsumers) {
+      float s = 0.f;
+      for (int gg = 0; gg < p.groups; ++gg) s += bias_sm[gg * items * 8 + i];
+      p.bias[((size_t)cta * p.H + h0) * p.D + i] = s;
+    }
   }
 }
 
@@ -243,32 +280,32 @@ long long pool_bwd_stream_partial_floats(int num_heads, int head_dim, int total_
   if (!pool_bwd_stream_eligible(num_heads, head_dim, total_len, kernel_size, kernel_stride)) return 0;
   const int hb = pb_heads(num_heads);
   const int groups = kPbConsumers / (hb * (head_dim / 8));
-  const int run = pb_run(total_len, kernel_stride, groups);
+  const int run = pb_run(total_len, batch, kernel_stride, groups, (num_heads + hb - 1) / hb);
   const long long ctas = (long long)(((max_seqlen + kernel_stride - 1) / kernel_stride + run - 1) / run) * batch;
-  return ctas * groups * num_heads * kernel_size;
+  return ctas * num_heads * ((long long)groups * kernel_size + head_dim);
 }
 
 template <typename T, int D>
-static int launch_pool_bwd_stream(const void* x, int* slots_out, int batch, int total_len, int max_seqlen, int stride,
+static int launch_pool_bwd_stream(const void* x, PoolBwdRows* rows_out, int batch, int total_len, int max_seqlen, int stride,
                                   long long x_sn, long long x_sh, PoolBwdStreamParams p, cudaStream_t stream) {
   p.hb = pb_heads(p.H);
   if (batch > 65535) return kUnsupported;   // the batch is a grid dimension here; the caller falls back
   const long long chunk = (long long)stride * p.hb * D * 2;
   p.groups = kPbConsumers / (p.hb * (D / 8));
   p.slots = (int)std::min<long long>(kPbMaxBars / p.groups, kPbRingBytes / chunk / p.groups);
-  p.run = pb_run(total_len, stride, p.groups);
+  p.run = pb_run(total_len, batch, stride, p.groups, (p.H + p.hb - 1) / p.hb);
   const bool dw = p.w != nullptr && p.partial != nullptr;
   CUtensorMap tmX;
   int rc = make_tmap_3d(&tmX, DT<T>::kTmapType, x, D, p.H, total_len, x_sh, x_sn, D, p.hb, stride);
   if (rc) return rc;
   const dim3 grid(((max_seqlen + stride - 1) / stride + p.run - 1) / p.run, batch, (p.H + p.hb - 1) / p.hb);
   const int nslots = (int)grid.x * batch * p.groups;
-  if (slots_out) *slots_out = nslots;
-  if (dw) {
-    cudaError_t e = cudaMemsetAsync(p.partial, 0, (size_t)nslots * p.H * p.ks * sizeof(float), stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-  }
-  const size_t smem = (dw ? (size_t)p.groups * p.slots * chunk : 0) + 2 * kPbMaxBars * sizeof(uint64_t) + (size_t)p.hb * p.ks * sizeof(float);
+  rows_out->slots = nslots;
+  rows_out->ctas = (int)grid.x * batch;
+  if (p.bias) p.bias += dw ? (size_t)nslots * p.H * p.ks : 0;  // behind the partial rows of dw
+  rows_out->bias = p.bias;
+  const size_t smem = (dw ? (size_t)p.groups * p.slots * chunk : 0) + 2 * kPbMaxBars * sizeof(uint64_t) + (size_t)p.hb * p.ks * sizeof(float) +
+                      (size_t)kPbConsumers * 8 * sizeof(float);
   auto launch = [&](auto kern) -> int {
     cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
@@ -287,14 +324,14 @@ static int launch_pool_bwd_stream(const void* x, int* slots_out, int batch, int 
   return kUnsupported;
 }
 
-int pool_bwd_stream(const void* x, const void* w, const void* dy, void* dx, float* partial, int* slots, const int* cu,
+int pool_bwd_stream(const void* x, const void* w, const void* dy, void* dx, float* partial, bool bias, PoolBwdRows* rows, const int* cu,
                     const int* ycu, int batch, int total_len, int max_seqlen, int num_heads, int head_dim, int kernel_size,
                     int kernel_stride, long long x_sn, long long x_sh, int dtype, cudaStream_t stream) {
   PoolBwdStreamParams p;
-  p.w = w; p.dy = dy; p.dx = dx; p.partial = partial; p.cu = cu; p.ycu = ycu; p.H = num_heads; p.D = head_dim; p.ks = kernel_size;
+  p.w = w; p.dy = dy; p.dx = dx; p.partial = w ? partial : nullptr; p.bias = bias ? partial : nullptr; p.cu = cu; p.ycu = ycu; p.H = num_heads; p.D = head_dim; p.ks = kernel_size;
   p.run = p.hb = p.groups = p.slots = 0;
   p.st.word = status_word();
-  return NSA_DISPATCH_T_D(dtype, head_dim, launch_pool_bwd_stream, x, slots, batch, total_len, max_seqlen, kernel_stride, x_sn,
+  return NSA_DISPATCH_T_D(dtype, head_dim, launch_pool_bwd_stream, x, rows, batch, total_len, max_seqlen, kernel_stride, x_sn,
                           x_sh, p, stream);
 }
 
