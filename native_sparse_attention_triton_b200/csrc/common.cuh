@@ -218,6 +218,12 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same asked by a whole warp.  The vote makes the answer, and with it the control flow behind it, warp-uniform for the compiler:
+// what an MMA-issuing warp counts then stays in uniform registers (a product of 8 instructions takes 900 clocks to issue otherwise).
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_test(bar, parity));
+}
+
 // Bounded wait: gives up after ~2^30 SM clocks (about half a second), raising kErrWaitTimeout.
 // Once any thread of the grid has given up, every later wait returns at once, so a broken
 // pipeline costs one timeout in total, not one per wait.  Returns false on timeout; the caller

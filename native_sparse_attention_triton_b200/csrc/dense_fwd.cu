@@ -27,7 +27,7 @@ struct DenseFwdParams {
 
 // tcgen05 implementation (dense_fwd_tc.cu)
 int varlen_attn_fwd_tc(const void* q, const void* k, const void* v, const int* cu_q, const int* cu_k, void* o, float* lse,
-                       int total_q, int total_k, int batch, int max_seqlen_q, int Hq, int Hkv, int head_dim, int causal,
+                       int total_q, int total_k, int batch, int Hq, int Hkv, int head_dim, int causal,
                        int window, int stride, int left, const long long* strides, float sm_scale, int dtype, cudaStream_t stream);
 
 }  // namespace nsa
@@ -59,7 +59,7 @@ static int varlen_attn_fwd_common(const void* q, const void* k, const void* v, c
   p.scale2 = sm_scale * kLog2e;
   p.st.word = status_word();
   if ((p.q_sn | p.q_sh | p.o_sn | p.o_sh) % 8 || !aligned16(q) || !aligned16(o)) return kInvalid;
-  return varlen_attn_fwd_tc(q, k, v, cu_seqlens_q, cu_seqlens_k, o, lse, total_q, total_k, batch, max_seqlen_q, num_q_heads,
+  return varlen_attn_fwd_tc(q, k, v, cu_seqlens_q, cu_seqlens_k, o, lse, total_q, total_k, batch, num_q_heads,
                             num_kv_heads, head_dim, causal, window, stride, left, strides, sm_scale, dtype,
                             static_cast<cudaStream_t>(stream));
 }
