@@ -233,7 +233,8 @@ extern "C" int nsa_compressed_attn_topk(const void* q, const void* k, const floa
   {
     // two row tiles per CTA when their block scores fit in shared memory, else one, else the mma.sync kernel: G < 4, folds wider
     // than 8 taps, and row tiles with more (token, block) pairs than the fold of the tcgen05 kernels holds (at kernel 32 / stride 16 /
-    // block 64 that is G of 4 and 8)
+    // block 64 that is G of 4; with G of 8, 16q/2kv, d 64, 7833 tokens, a forward and backward chain took 604 us on mma.sync, 582 on
+    // tcgen05)
     int rc = score_topk_pp_tc(q, k, strides[2], strides[3], total_q, total_k, max_seqlen_q, head_dim, dtype, p,
                               static_cast<cudaStream_t>(stream));
     if (rc == kUnsupported)

@@ -3,13 +3,16 @@
 // Same arithmetic as score_topk_tc.cu (logits produced TRANSPOSED, S^T = K Q^T, a thread owns one key and sums the G
 // heads of a token inside its own columns; key scores -> shared memory -> block scores -> warp top-k), but a CTA
 // works on TWO row tiles A and B of 128 rows = (128/G consecutive tokens) x (G heads) each, B right after A:
-//   warps 0..3 : tile A, one thread per key of the current 128-key tile, all 128 (token, head) columns of the tile
-//   warps 4..7 : tile B
-//   warp 8     : TMA producer (both Q tiles once, K tiles through a ring shared by the two row tiles)
-//   warp 9     : TMEM allocation and MMA issue, alternating between the row tiles
+//   warps 0..7  : tile A, two threads per key of the current 128-key tile, 64 of the tile's 128 (token, head) columns each
+//   warps 8..15 : tile B
+//   warp 16     : TMA producer (both Q tiles once, K tiles through a ring shared by the two row tiles)
+//   warp 17     : TMEM allocation and MMA issue, alternating between the row tiles
 // While one group exponentiates, the tensor pipe produces the other group's logits, and the two groups' barriers and
 // fold steps interleave instead of stalling all eight warps at once; each K tile is fetched once for 256 rows.
 // TMEM columns: tile g, buffer b at g*256 + b*128 (S^T is double-buffered per row tile).
+// What bounds it: the key-score threads' instruction stream (a key tile of both row tiles: 2048 clocks of exponentials without the
+// polynomial's share, 1024 of products, 4100 measured).  With one thread per key and two warps per scheduler 39 % of the issue slots
+// were used; with four warps per scheduler 64q/4kv, 8192 / 16 384 / 32 768 tokens: 160 / 435 / 1310 -> 141 / 390 / 1185 us.
 #include "attn_tile.cuh"
 #include "dispatch.h"
 #include "host_util.h"
@@ -28,11 +31,16 @@ namespace {
 constexpr int kPpKeyTile = 128;
 constexpr int kPpStages = 2;
 
-__device__ __forceinline__ void bar_sync_group(int g) { asm volatile("bar.sync %0, 128;\n" ::"r"(1 + g) : "memory"); }
+constexpr int kPpWarps = 16;                          // 8 per row tile
+constexpr int kPpThreads = (kPpWarps + 2) * 32;
+constexpr int kPpGroup = kPpWarps / 2 * 32;           // threads of a row tile
+constexpr int kPpRounds = 3;                          // (token, block) pairs a thread folds per key tile
+
+__device__ __forceinline__ void bar_sync_group(int g) { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + g), "n"(kPpGroup) : "memory"); }
 }  // namespace
 
 template <typename T, int D, int LOGG>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kPpThreads, 1)
 score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, ScoreParams p) {
   constexpr int PANELS = D / 64;
   constexpr int PANEL_BYTES = 128 * 128;
@@ -40,6 +48,8 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   constexpr int K_BYTES = kPpKeyTile * D * 2;
   constexpr int GG = 1 << LOGG;
   constexpr int TPT = 128 >> LOGG;  // tokens per row tile
+  // groups of 16 only: the small groups' scores come from as exact exponentials as on the mma.sync kernel they share the work with
+  constexpr int POLY_EVERY = LOGG == 4 ? kScorePolyEvery : 1 << 20;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_sm = smem;                              // [2] row tiles
   uint8_t* k_sm = q_sm + 2 * Q_BYTES;
@@ -77,7 +87,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     }
     for (int s = 0; s < 4; ++s) {
       mbar_init(s_full + s, 1);
-      mbar_init(s_empty + s, 4);
+      mbar_init(s_empty + s, kPpWarps / 2);
     }
     fence_barrier_init();
   }
@@ -88,7 +98,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     lse_sh[col] = t < Lq ? __ldg(p.lse + (long long)(qs + t) * p.Hq + h * p.G + (col & (GG - 1))) : INFINITY;
   }
   for (int i = threadIdx.x; i < 2 * TPT * p.nb_pad; i += blockDim.x) bsc[i] = 0.f;
-  if (warp == 9) {
+  if (warp == kPpWarps + 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -97,7 +107,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   tc_fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
-  if (warp == 8) {
+  if (warp == kPpWarps) {
     // ===================== TMA producer =====================
     if (lane == 0 && ntiles > 0) {
       mbar_expect_tx(q_full, 2 * Q_BYTES);
@@ -115,7 +125,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           tma_load_3d(k_sm + s * K_BYTES + pn * PANEL_BYTES, &tmK, k_full + s, pn * 64, h, ksq + i * kPpKeyTile);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == kPpWarps + 1) {
     // ===================== MMA issuer: converged warp, one elected lane issues (see tc5.cuh) =====================
     if (ntiles > 0) {
       const uint32_t idesc = umma_idesc<T>(128, 128, false, false);
@@ -140,10 +150,11 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
     }
   } else {
-    // ===================== key-score threads: group g (tile A: warps 0..3, tile B: warps 4..7), one thread per key ==========
-    const int g = warp >> 2;
-    const int key_l = threadIdx.x & 127;
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 256);
+    // ===================== key-score threads: group g (tile A: warps 0..7, tile B: warps 8..15), two threads per key ==========
+    const int g = warp >> 3, half = (warp >> 2) & 1;
+    const int key_l = (warp & 3) * 32 + lane;
+    const int tid_g = threadIdx.x & (kPpGroup - 1);
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 256 + half * 64);
     const int a = p.window / p.stride, c = p.block_size / p.stride;
     const int tq0 = q0 + g * TPT;  // first token of the group's row tile
     float* ks_g = keysc + g * 2 * TPT * kPpKeyTile;
@@ -151,13 +162,12 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const float4* lse4 = reinterpret_cast<const float4*>(lse_sh + g * 128);
     // this thread's (token, relative block) pairs of the fold step; the same for every tile
     const int nblk = kPpKeyTile / c + (a - 1 + c - 1) / c;  // blocks touched by one key tile
-    int ftok[3], fbrel[3], fk0[3];
+    int ftok[kPpRounds], fbrel[kPpRounds];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const int idx = key_l + 128 * r;
+    for (int r = 0; r < kPpRounds; ++r) {
+      const int idx = tid_g + kPpGroup * r;
       ftok[r] = idx < TPT * nblk ? idx / nblk : -1;
       fbrel[r] = idx - (idx / nblk) * nblk;
-      fk0[r] = fbrel[r] * c - (a - 1);
     }
     for (int i = 0; i < ntiles; ++i) {
       const int bsel = i & 1;
@@ -169,10 +179,9 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       mbar_wait(s_full + g * 2 + bsel, (i >> 1) & 1, p.st);
       tc_fence_after_sync();
 #pragma unroll
-      for (int hc = 0; hc < 2; ++hc) {  // 64 columns at a time
-        uint32_t su[2][32];
-        tmem_ld32(lane_base + bsel * 128 + hc * 64, su[0]);
-        tmem_ld32(lane_base + bsel * 128 + hc * 64 + 32, su[1]);
+      for (int hc = 0; hc < 2; ++hc) {  // 32 columns at a time
+        uint32_t su[32];
+        tmem_ld32(lane_base + bsel * 128 + hc * 32, su);
         tmem_ld_wait();
         if (hc == 1) {  // the logits of this buffer are in registers: the next product may overwrite it
           tc_fence_before_sync();
@@ -181,46 +190,41 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         // sums over the G heads of each token; a token's sum is kept or dropped as a whole (visible tokens are a suffix)
 #pragma unroll
-        for (int tk = 0; tk < 64 / GG; ++tk) {
-          float e[GG];
+        for (int tk = 0; tk < 32 / GG; ++tk) {
+          float2 e[GG / 2];
 #pragma unroll
           for (int q4 = 0; q4 < GG / 4; ++q4) {
-            const int col = tk * GG + q4 * 4;  // within the 64
-            const float4 l4 = lse4[(hc * 64 + col) >> 2];
+            const int col = tk * GG + q4 * 4;  // within the 32
+            const float4 l4 = lse4[(half * 64 + hc * 32 + col) >> 2];
             const float2 sc2 = make_float2(p.scale2, p.scale2);
-            const float2 x01 = ffma2(make_float2(__uint_as_float(su[col >> 5][(col + 0) & 31]), __uint_as_float(su[col >> 5][(col + 1) & 31])),
-                                     sc2, make_float2(-l4.x, -l4.y));
-            const float2 x23 = ffma2(make_float2(__uint_as_float(su[col >> 5][(col + 2) & 31]), __uint_as_float(su[col >> 5][(col + 3) & 31])),
-                                     sc2, make_float2(-l4.z, -l4.w));
+            const float2 x01 = ffma2(make_float2(__uint_as_float(su[col + 0]), __uint_as_float(su[col + 1])), sc2, make_float2(-l4.x, -l4.y));
+            const float2 x23 = ffma2(make_float2(__uint_as_float(su[col + 2]), __uint_as_float(su[col + 3])), sc2, make_float2(-l4.z, -l4.w));
             // a share of the exponentials runs as a polynomial on the FMA pipe (the other unit bounds this pass)
             const int pair0 = (tk * (GG / 4) + q4) * 2;
-            const float2 e01 = (pair0 % kScorePolyEvery == kScorePolyEvery - 1) ? exp2_poly2(x01) : make_float2(fast_exp2(x01.x), fast_exp2(x01.y));
-            const float2 e23 = ((pair0 + 1) % kScorePolyEvery == kScorePolyEvery - 1) ? exp2_poly2(x23) : make_float2(fast_exp2(x23.x), fast_exp2(x23.y));
-            e[q4 * 4 + 0] = e01.x;
-            e[q4 * 4 + 1] = e01.y;
-            e[q4 * 4 + 2] = e23.x;
-            e[q4 * 4 + 3] = e23.y;
+            e[q4 * 2] = (pair0 % POLY_EVERY == POLY_EVERY - 1) ? exp2_poly2(x01) : make_float2(fast_exp2(x01.x), fast_exp2(x01.y));
+            e[q4 * 2 + 1] = ((pair0 + 1) % POLY_EVERY == POLY_EVERY - 1) ? exp2_poly2(x23) : make_float2(fast_exp2(x23.x), fast_exp2(x23.y));
           }
 #pragma unroll
-          for (int w = GG / 2; w >= 1; w >>= 1)
+          for (int w = GG / 4; w >= 1; w >>= 1)
 #pragma unroll
-            for (int gg = 0; gg < w; ++gg) e[gg] += e[gg + w];
-          const int tok = hc * (64 / GG) + tk;
-          ks_t[tok * kPpKeyTile + key_l] = tok >= tok_min ? e[0] : 0.f;
+            for (int gg = 0; gg < w; ++gg) e[gg] = fadd2(e[gg], e[gg + w]);
+          const int tok = half * (64 / GG) + hc * (32 / GG) + tk;
+          ks_t[tok * kPpKeyTile + key_l] = tok >= tok_min ? e[0].x + e[0].y : 0.f;
         }
       }
       bar_sync_group(g);  // key scores of this tile are complete
       // fold: block b_lo + brel reads tile-local keys fk0 .. fk0 + a + c - 2 (the layout repeats every tile: c divides 128)
       const int b_lo = i * (kPpKeyTile / c);
 #pragma unroll
-      for (int r = 0; r < 3; ++r) {
+      for (int r = 0; r < kPpRounds; ++r) {
         const int bb = b_lo + fbrel[r];
         if (ftok[r] < 0 || bb >= p.nb_pad) continue;
-        const float* src = ks_t + ftok[r] * kPpKeyTile + fk0[r];
+        const int k0 = fbrel[r] * c - (a - 1);
+        const float* src = ks_t + ftok[r] * kPpKeyTile + k0;
         float part[8];
 #pragma unroll
         for (int o = 0; o < 8; ++o) {   // a + c - 1 <= 8 offsets (checked on the host); loads are independent
-          const bool ok = o <= a + c - 2 && fk0[r] + o >= 0 && fk0[r] + o < kPpKeyTile;
+          const bool ok = o <= a + c - 2 && k0 + o >= 0 && k0 + o < kPpKeyTile;
           part[o] = ok ? (float)fold_weight(o, a, c) * src[o] : 0.f;
         }
         const float accb = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
@@ -228,8 +232,8 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
     }
     bar_sync_group(g);  // every block score of the group is final before its warps start selecting
-    // ---- selection: the tokens of the row tile are dealt to the group's four warps ----
-    for (int tok = warp & 3; tok < TPT; tok += 4) {
+    // ---- selection: the tokens of the row tile are dealt to the group's eight warps ----
+    for (int tok = warp & 7; tok < TPT; tok += 8) {
       const int t = tq0 + tok;
       if (t >= Lq) break;
       warp_select_topk(bsc_g + (size_t)tok * p.nb_pad, t / p.block_size, p.topk_out, p.init_blocks, p.local_blocks,
@@ -238,7 +242,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem, 512);
+  if (warp == kPpWarps + 1) tmem_dealloc(tmem, 512);
 }
 
 template <typename T, int D>
@@ -257,17 +261,17 @@ static int launch_score_topk_pp_tc(const void* q, const void* k, long long k_sn,
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_seqlen_q + 2 * TPT - 1) / (2 * TPT), p.B, p.Hkv);
-  { LaunchScope ls_("score_topk_tc", stream); kern<<<grid, 320, smem, stream>>>(tmQ, tmK, p); }
+  { LaunchScope ls_("score_topk_tc", stream); kern<<<grid, kPpThreads, smem, stream>>>(tmQ, tmK, p); }
   return cuda_rc(cudaGetLastError());
 }
 
 // Returns kUnsupported when the block scores of two row tiles do not fit in shared memory (very long sequences) or the
-// fold geometry needs more than 3 (token, block) pairs per thread; the caller then uses the one-tile kernel.
+// fold geometry needs more than kPpRounds (token, block) pairs per thread; the caller then uses the one-tile kernel.
 int score_topk_pp_tc(const void* q, const void* k, long long k_sn, long long k_sh, int Nq, int Nk, int max_seqlen_q, int head_dim,
                      int dtype, ScoreParams p, cudaStream_t stream) {
   if (p.G < 4 || p.G > 16) return kUnsupported;
   const int a = p.window / p.stride, c = p.block_size / p.stride;
-  if (c <= 0 || kPpKeyTile % c || a + c - 1 > 8 || (128 / p.G) * (kPpKeyTile / c + (a - 1 + c - 1) / c) > 3 * 128) return kUnsupported;
+  if (c <= 0 || kPpKeyTile % c || a + c - 1 > 8 || (128 / p.G) * (kPpKeyTile / c + (a - 1 + c - 1) / c) > kPpRounds * kPpGroup) return kUnsupported;
   return NSA_DISPATCH_T_D(dtype, head_dim, launch_score_topk_pp_tc, q, k, k_sn, k_sh, Nq, Nk, max_seqlen_q, p, stream);
 }
 
