@@ -218,8 +218,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// The same asked by a whole warp.  The vote makes the answer, and with it the control flow behind it, warp-uniform for the compiler:
-// what an MMA-issuing warp counts then stays in uniform registers (a product of 8 instructions takes 900 clocks to issue otherwise).
+// The same asked by a whole warp, with one answer for all its lanes.
 __device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_test(bar, parity));
 }
