@@ -95,8 +95,10 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* s_full = v_empty + kTcStages;    // [2] per row tile
   uint64_t* p_full = s_full + 2;             // [2]
   uint64_t* pv_done = p_full + 2;            // [2]
-  uint64_t* o_full = pv_done + 2;            // [2] the output is in the Q buffer
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  // Per Q buffer, not per row tile: a buffer is not filled again before its output was handled, so a phase cannot be overtaken by the
+  // next one while the warp that stores the outputs has yet to look at it.
+  uint64_t* o_full = pv_done + 2;            // the output is in the Q buffer
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + kTcQBufs);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (smem_u32(smem) & 1023u) {  // the swizzled operand tiles need a 1024-byte aligned base
@@ -107,6 +109,7 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int s = 0; s < kTcQBufs; ++s) {
       mbar_init(q_full + s, 1);
       mbar_init(q_empty + s, 1);
+      mbar_init(o_full + s, kTcSoftWarps / 2);
     }
     for (int s = 0; s < kTcStages; ++s) {
       mbar_init(k_full + s, 1);
@@ -118,7 +121,6 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(s_full + s, 1);
       mbar_init(p_full + s, kTcSoftWarps / 2);
       mbar_init(pv_done + s, 1);
-      mbar_init(o_full + s, kTcSoftWarps / 2);
     }
     items_init(ring, steal, kTcSoftWarps + 2);
     fence_barrier_init();
@@ -271,8 +273,8 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int taken = 0; item_take(ring, taken, w, p.st); ++taken) {
       if (w.ntiles == 0) continue;
       for (int g = 0; g < 2; ++g, ++rt) {
-        mbar_wait(o_full + g, (rt >> 1) & 1, p.st);
         const int qb = rt % kTcQBufs;
+        mbar_wait(o_full + qb, (rt / kTcQBufs) & 1, p.st);
         if (lane == 0) {
           if (w.q0 + g * QT + QT <= w.Lq) {
 #pragma unroll
@@ -484,7 +486,7 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (ntiles > 0) {
         if (staged) fence_proxy_async();  // the TMA engine reads the tile through the async proxy
         __syncwarp();
-        if (lane == 0) mbar_arrive(o_full + g);
+        if (lane == 0) mbar_arrive(o_full + qb);
       }
       kt += ntiles;
       if (ntiles > 0) rt += 2;
