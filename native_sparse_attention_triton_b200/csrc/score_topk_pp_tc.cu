@@ -35,11 +35,16 @@ constexpr int kPpWarps = 16;                          // 8 per row tile
 constexpr int kPpThreads = (kPpWarps + 2) * 32;
 constexpr int kPpGroup = kPpWarps / 2 * 32;           // threads of a row tile
 constexpr int kPpRounds = 3;                          // (token, block) pairs a thread folds per key tile
+constexpr int kPpCubicPairs = 384;                    // most pairs of a row tile whose scores may come from cubics
+
+// (token, block) pairs that the fold of one row tile and key tile adds to; a = window / stride, c = block_size / stride
+int pp_pairs(int G, int a, int c) { return (128 / G) * (kPpKeyTile / c + (a - 1 + c - 1) / c); }
 
 __device__ __forceinline__ void bar_sync_group(int g) { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + g), "n"(kPpGroup) : "memory"); }
 }  // namespace
 
-template <typename T, int D, int LOGG>
+// CUBIC: a share of the exponentials runs as a polynomial (see the launch)
+template <typename T, int D, int LOGG, bool CUBIC>
 __global__ void __launch_bounds__(kPpThreads, 1)
 score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, ScoreParams p) {
   constexpr int PANELS = D / 64;
@@ -48,8 +53,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   constexpr int K_BYTES = kPpKeyTile * D * 2;
   constexpr int GG = 1 << LOGG;
   constexpr int TPT = 128 >> LOGG;  // tokens per row tile
-  // groups of 16 only: the small groups' scores come from as exact exponentials as on the mma.sync kernel they share the work with
-  constexpr int POLY_EVERY = LOGG == 4 ? kScorePolyEvery : 1 << 20;
+  constexpr int POLY_EVERY = CUBIC ? kScorePolyEvery : 1 << 20;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_sm = smem;                              // [2] row tiles
   uint8_t* k_sm = q_sm + 2 * Q_BYTES;
@@ -257,7 +261,15 @@ static int launch_score_topk_pp_tc(const void* q, const void* k, long long k_sn,
   if (rc) return rc;
   rc = make_tmap_3d(&tmK, DT<T>::kTmapType, k, D, p.Hkv, Nk, k_sh, k_sn, 64, 1, kPpKeyTile);
   if (rc) return rc;
-  auto kern = p.logG == 4 ? score_topk_pp_tc_kernel<T, D, 4> : (p.logG == 3 ? score_topk_pp_tc_kernel<T, D, 3> : score_topk_pp_tc_kernel<T, D, 2>);
+  // Cubics (relative error 7.5e-5) only for groups of 16 with at most kPpCubicPairs pairs.  Other layouts, groups of 8 at kernel 32 /
+  // stride 16 / block 64 and groups of 16 at 64 / 32 / 64 among them, came here from kernels (mma.sync, one row tile) that take every
+  // exponential from the exponential unit, and keep that: the largest gap between a block left out and one taken, 8192 tokens, 64 / 32 / 64,
+  // is 3.5e-5 of its score with cubics and below 1e-6 without.  64q/4kv at 32 768 tokens, compressed attention with selection: 3226 us on
+  // mma.sync, 1543 to 1580 here with cubics, 1541 to 1584 without.
+  const bool cubic = p.G == 16 && pp_pairs(p.G, p.window / p.stride, p.block_size / p.stride) <= kPpCubicPairs;
+  auto kern = cubic ? score_topk_pp_tc_kernel<T, D, 4, true>
+                    : (p.logG == 4 ? score_topk_pp_tc_kernel<T, D, 4, false>
+                                   : (p.logG == 3 ? score_topk_pp_tc_kernel<T, D, 3, false> : score_topk_pp_tc_kernel<T, D, 2, false>));
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
   dim3 grid((max_seqlen_q + 2 * TPT - 1) / (2 * TPT), p.B, p.Hkv);
@@ -271,7 +283,7 @@ int score_topk_pp_tc(const void* q, const void* k, long long k_sn, long long k_s
                      int dtype, ScoreParams p, cudaStream_t stream) {
   if (p.G < 4 || p.G > 16) return kUnsupported;
   const int a = p.window / p.stride, c = p.block_size / p.stride;
-  if (c <= 0 || kPpKeyTile % c || a + c - 1 > 8 || (128 / p.G) * (kPpKeyTile / c + (a - 1 + c - 1) / c) > kPpRounds * kPpGroup) return kUnsupported;
+  if (c <= 0 || kPpKeyTile % c || a + c - 1 > 8 || pp_pairs(p.G, a, c) > kPpRounds * kPpGroup) return kUnsupported;
   return NSA_DISPATCH_T_D(dtype, head_dim, launch_score_topk_pp_tc, q, k, k_sn, k_sh, Nq, Nk, max_seqlen_q, p, stream);
 }
 
