@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) pool_dw_kernel(PoolBwdParams p) {
 }
 
 // dw[h,k] and dpe[h,k,:] from the streaming pass's partial rows, summed in their order (deterministic).  Every CTA sums its head's
-// rows of dy's column sums for itself: 74 KB out of L2 for 144 rows, against a launch of its own.
+// rows of dy's column sums for itself: 74 KB out of L2 for 144 rows, against a launch of its own (pool_bwd_stream_sums on how many).
 template <typename T>
 __global__ void __launch_bounds__(256) pool_dw_finish_kernel(PoolBwdParams p, const float* __restrict__ partial, PoolBwdRows rows) {
   constexpr int D = 128;
@@ -432,15 +432,16 @@ static int run_pool_bwd(PoolBwdParams p, float* dbias, float* partial, long long
   // long inputs: one streaming pass writes dx and the partial rows of dw (weighted pooling) and of dy's column sums (with pe)
   const long long need = pool_bwd_stream_partial_floats(p.H, D, p.N, p.B, max_seqlen, p.ks, p.stride);
   const bool room = partial && partial_floats >= need;
+  const bool bias_rows = p.pe && room && need > 0 && pool_bwd_stream_sums(p.H, D, p.N, p.B, max_seqlen, p.stride);
   bool summed = false;
   if (total_y > 0 && need > 0 && (!p.dw || room)) {
-    if (p.pe && !room) {
+    if (p.pe && !bias_rows) {
       launch_colsum<T>(p.dy, dbias, total_y, p.H, D, stream);
       p.dbias = dbias;
       summed = true;
     }
     PoolBwdRows rows;
-    const int rc = pool_bwd_stream(p.x, p.dw ? p.w : nullptr, p.dy, p.dx, room ? partial : nullptr, p.pe && room, &rows, p.cu, p.ycu, p.B,
+    const int rc = pool_bwd_stream(p.x, p.dw ? p.w : nullptr, p.dy, p.dx, room ? partial : nullptr, bias_rows, &rows, p.cu, p.ycu, p.B,
                                    p.N, max_seqlen, p.H, D, p.ks, p.stride, p.x_sn, p.x_sh, dtype, stream);
     if (rc != kInvalid && rc != kUnsupported) {
       if (rc) return rc;

@@ -54,6 +54,11 @@ int pb_run(int total_len, int batch, int stride, int groups, int head_blocks) {
   const int full = std::max(std::max(1, ctas / 2), ctas - batch / 2);
   return std::max(8 * groups, (chunks + full - 1) / full);
 }
+// CTAs per head block, those beyond a sequence's end among them
+long long pb_ctas(int total_len, int batch, int max_seqlen, int stride, int groups, int head_blocks) {
+  const int run = pb_run(total_len, batch, stride, groups, head_blocks);
+  return (long long)(((max_seqlen + stride - 1) / stride + run - 1) / run) * batch;
+}
 }  // namespace
 
 template <typename T, int R, int S, bool DW>
@@ -280,9 +285,19 @@ long long pool_bwd_stream_partial_floats(int num_heads, int head_dim, int total_
   if (!pool_bwd_stream_eligible(num_heads, head_dim, total_len, kernel_size, kernel_stride)) return 0;
   const int hb = pb_heads(num_heads);
   const int groups = kPbConsumers / (hb * (head_dim / 8));
-  const int run = pb_run(total_len, batch, kernel_stride, groups, (num_heads + hb - 1) / hb);
-  const long long ctas = (long long)(((max_seqlen + kernel_stride - 1) / kernel_stride + run - 1) / run) * batch;
-  return ctas * num_heads * ((long long)groups * kernel_size + head_dim);
+  const bool sums = pool_bwd_stream_sums(num_heads, head_dim, total_len, batch, max_seqlen, kernel_stride);
+  return pb_ctas(total_len, batch, max_seqlen, kernel_stride, groups, (num_heads + hb - 1) / hb) * num_heads *
+         ((long long)groups * kernel_size + (sums ? head_dim : 0));
+}
+
+// Every CTA of the finishing kernel adds up its head's rows, which batches of many or very uneven sequences have one of per sequence and
+// run of the longest: past a row for 32 chunks of the input a pass of its own over dy costs less.  4 heads, weighted, 262 144 tokens in
+// all, backward, rows / own pass: 512 sequences of 512 tokens (512 rows) 143 / 154 us, 1024 of 256 (1024 rows) 172 / 157, one of 131 072
+// and 64 of 2048 (3770 rows) 347 / 199; 8192 of 64 778 / 449.
+bool pool_bwd_stream_sums(int num_heads, int head_dim, int total_len, int batch, int max_seqlen, int kernel_stride) {
+  const int hb = pb_heads(num_heads);
+  const int groups = kPbConsumers / (hb * (head_dim / 8));
+  return pb_ctas(total_len, batch, max_seqlen, kernel_stride, groups, (num_heads + hb - 1) / hb) * 32 <= (total_len + kernel_stride - 1) / kernel_stride;
 }
 
 template <typename T, int D>

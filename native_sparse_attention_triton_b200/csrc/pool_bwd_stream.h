@@ -10,6 +10,9 @@ bool pool_bwd_stream_eligible(int num_heads, int head_dim, int total_len, int ke
 long long pool_bwd_stream_partial_floats(int num_heads, int head_dim, int total_len, int batch, int max_seqlen,
                                          int kernel_size, int kernel_stride);
 
+// Whether the pass can sum dy's columns as well; else they are better left to a pass of their own
+bool pool_bwd_stream_sums(int num_heads, int head_dim, int total_len, int batch, int max_seqlen, int kernel_stride);
+
 struct PoolBwdRows {
   int slots = 0;                // partial rows of dw, [slots][H][ks] at the workspace's start
   int ctas = 0;                 // partial rows of the column sums of dy, [ctas][H][128] at `bias`
