@@ -28,8 +28,6 @@
 // start -> now: window 512 over 32 768 tokens 946 -> 720 us, window 128 673 -> 433; compressed keys of 8192 tokens 168 -> 138,
 // of 16 384 425 -> 344, of 32 768 1214 -> 1070; 32 full key tiles per item 483 -> 495 (two K stages for three).
 // Two threads per row instead of one: 2.05 us a step against 1.7, the exponentials of A and B then coincide.
-#include <limits.h>
-
 #include <type_traits>
 
 #include "attn_tile.cuh"
@@ -142,7 +140,7 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     auto lookup = [&](uint3 blk, AttnItem& w) {
       int b, tile;
       // long rows first
-      if (!find_row_tile(p.cu_q, p.B, 2 * QT, (int)gridDim.x - 1 - (int)blk.x, INT_MAX, b, w.qs, w.Lq, tile)) return false;
+      if (!find_row_tile(p.cu_q, p.B, 8 - p.logG, (int)gridDim.x - 1 - (int)blk.x, b, w.qs, w.Lq, tile)) return false;
       w.head = blk.y;
       w.ksq = __ldg(p.cu_k + b);
       w.Lk = __ldg(p.cu_k + b + 1) - w.ksq;
@@ -515,7 +513,7 @@ static int launch_dense_fwd_tc(const void* q, const void* k, const void* v, cons
   auto kern = dense_fwd_tc_kernel<T, D>;
   cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return cuda_rc(e);
-  const dim3 grid(Nq / (2 * QT) + p.B, p.Hkv);
+  const dim3 grid((unsigned)row_tile_slots(Nq, p.B, 8 - p.logG), p.Hkv);
   { LaunchScope ls_("dense_fwd_tc", stream); kern<<<grid, kTcThreads, smem, stream>>>(tmQ, tmK, tmV, tmO, p); }
   return cuda_rc(cudaGetLastError());
 }

@@ -27,8 +27,9 @@ def _exact(q, k, v, cq, ck, visible):
 
 
 # row tiles of 128 rows, two per item: lengths around 128 / G and 256 / G tokens; runs of sequences without a compressed key (shorter
-# than 32), longer than the ring of items; more items than SMs
-LENS = [[17], [7, 8, 9, 15, 16, 17, 31, 32, 33], [3] * 70 + [40] * 9, [200] + [5] * 12 + [1111, 64, 129, 2000], [0, 300, 0, 0, 47]]
+# than 32), longer than the ring of items; more items than SMs; more sequences than two turns of the search for an item (1024)
+LENS = [[17], [7, 8, 9, 15, 16, 17, 31, 32, 33], [3] * 70 + [40] * 9, [200] + [5] * 12 + [1111, 64, 129, 2000], [0, 300, 0, 0, 47],
+        [1 + i * 37 % 23 if i % 7 else 0 for i in range(1100)]]
 
 
 @pytest.mark.parametrize("lens", LENS)
