@@ -22,11 +22,12 @@
 // overwrite P(i) before it has been read.
 // TMEM columns: [0,128) S/P of A, [128,256) S/P of B, [256,256+D) O of A, [384,384+D) O of B.
 //
-// What bounds it: a key tile of both row tiles takes 3200 clocks (2048 of products, 1366 of exponentials): softmax of a row tile,
+// What bounds it: a key tile of both row tiles takes about 3100 clocks (2048 of products, 1366 of exponentials): softmax of a row tile,
 // the hand-over to the issuing warp, its P V and next S, and the hand-over back are a chain.  A CTA of its own per item cost 12 000
 // clocks more each, of which set-up, the first loads and the output now run beside the neighbouring items.  64q/4kv, bf16, d 128,
-// start -> now: window 512 over 32 768 tokens 946 -> 720 us, window 128 673 -> 433; compressed keys of 8192 tokens 168 -> 138,
-// of 16 384 425 -> 344, of 32 768 1214 -> 1070; 32 full key tiles per item 483 -> 495 (two K stages for three).
+// this kernel alone, a CTA per item -> persistent: window 512 over 32 768 tokens 999 -> 763 us, window 128 694 -> 454; compressed keys
+// of 8192 tokens 180 -> 147, of 16 384 451 -> 371, of 32 768 1276 -> 1102; 4096 keys, none masked, 467 -> 454, 8192 1696 -> 1659;
+// 8192 tokens, causal, 938 -> 914; 300 sequences of 200 (32q/2kv) 519 -> 476.
 // Two threads per row instead of one: 2.05 us a step against 1.7, the exponentials of A and B then coincide.
 #include <type_traits>
 
@@ -188,32 +189,34 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // The whole warp runs the control flow converged; one elected lane issues (see tc5.cuh on why).
     const uint32_t idesc_qk = umma_idesc<T>(128, kTcKeyTile, false, false);
     const uint32_t idesc_pv = umma_idesc<T>(128, D, false, true);
-    // S of row tile g, held by Q buffer qb, for key tile c (counted over all items); the second row tile's product releases the K stage
-    auto issue_qk = [&](int c, int g, int qb) {
-      const uint32_t k_addr = smem_u32(k_sm + (c % kTcStages) * KV_BYTES), q_addr = smem_u32(q_sm + qb * Q_BYTES);
+    const uint32_t q_base = smem_u32(q_sm), k_base = smem_u32(k_sm), v_base = smem_u32(v_sm);
+    // S of row tile g from the Q at q_addr for the key tile in stage st; the second row tile's product releases the K stage
+    auto issue_qk = [&](unsigned st, int g, uint32_t q_addr) {
+      const uint32_t k_addr = k_base + st * KV_BYTES;
       if (elect_one()) {
         umma_block_ss<D / 16, PANEL_BYTES>(tmem + (uint32_t)(g * 128), q_addr, k_addr, idesc_qk);
         umma_commit(s_full + g);
-        if (g == 1) umma_commit(k_empty + (c % kTcStages));
+        if (g == 1) umma_commit(k_empty + st);
       }
       __syncwarp();
     };
-    auto issue_pv = [&](int c, int g, bool first) {
-      const uint32_t v_addr = smem_u32(v_sm + (c % kTcStages) * KV_BYTES);
+    auto issue_pv = [&](unsigned st, int g, bool first) {
+      const uint32_t v_addr = v_base + st * KV_BYTES;
       const uint32_t p_tmem = tmem + (uint32_t)(g * 128);  // P overwrote the first 64 columns of the tile's S
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < kTcKeyTile / 16; ++kk)
           umma_ts(tmem + 256 + g * 128, p_tmem + kk * 8, umma_desc_mnmajor(v_addr + kk * 2048, PANEL_BYTES), idesc_pv, !first || kk > 0);
         umma_commit(pv_done + g);
-        if (g == 1) umma_commit(v_empty + (c % kTcStages));
+        if (g == 1) umma_commit(v_empty + st);
       }
       __syncwarp();
     };
     // Items without key tiles are passed over.  While products of the present item are still to be issued the next one is only
     // looked for, not waited for: it may depend on the softmax warps getting on with the present one.
     AttnItem w;
-    int taken = 0, rt = 0, kt = 0;  // items taken, row tiles and key tiles of the items before the present one
+    int taken = 0;
+    unsigned rt = 0, kt = 0;  // row tiles and key tiles of the items before the present one
     auto next_item = [&](bool wait) {  // 1: w is the next item, 0: there is none left, -1: not known yet
       for (;;) {
         if (!wait && !item_ready(ring, taken)) return -1;
@@ -221,45 +224,54 @@ dense_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (w.ntiles > 0) return 1;
       }
     };
-    auto start = [&](int c, int t, int g) {  // the first product of row tile t, the item's tile g
-      if (g == 0) mbar_wait(k_full + (c % kTcStages), (c / kTcStages) & 1, p.st);
+    auto q_tile = [&](unsigned t) { return q_base + t % kTcQBufs * Q_BYTES; };
+    // S of tile x of the item that starts at row tile t, for its first key tile c
+    auto start = [&](unsigned c, unsigned t, int x) {
+      if (x == 0) mbar_wait(k_full + c % kTcStages, (c / kTcStages) & 1, p.st);
+      t += x;
       mbar_wait(q_full + t % kTcQBufs, (t / kTcQBufs) & 1, p.st);
       tc_fence_after_sync();
-      issue_qk(c, g, t % kTcQBufs);
+      issue_qk(c % kTcStages, x, q_tile(t));
     };
     int have = next_item(true);
     if (have == 1) {
-      start(0, 0, 0);
-      start(0, 1, 1);
+#pragma unroll 1
+      for (int x = 0; x < 2; ++x) start(0, 0, x);
     }
     while (have == 1) {
       const int ntiles = w.ntiles;
-      for (int i = 0; i < ntiles; ++i) {
-        const int c = kt + i;
+      unsigned c = kt;
+      const uint32_t q_addr[2] = {q_tile(rt), q_tile(rt + 1)};
+      // A product's issue is a link of the chain that bounds a step.  What it needs besides P is waited for in front of P: V of this tile
+      // and K of the next one, asked for when the stages of the tile before became free.  (With the waits, the choice of the next
+      // item and the addresses between the products a step took 3300 clocks: 32 full key tiles per item 471 us instead of 450.)
+      for (int i = 0; i + 1 < ntiles; ++i, ++c) {
+        const unsigned n = c + 1;
+        mbar_wait(v_full + c % kTcStages, (c / kTcStages) & 1, p.st);
+        mbar_wait(k_full + n % kTcStages, (n / kTcStages) & 1, p.st);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           // P(c) is written (for an item's first tile this also says that O of the item before it has been read)
           mbar_wait(p_full + g, c & 1, p.st);
-          if (g == 0) mbar_wait(v_full + (c % kTcStages), (c / kTcStages) & 1, p.st);
           tc_fence_after_sync();
-          issue_pv(c, g, i == 0);
-          if (i + 1 < ntiles) {
-            if (g == 0) {
-              mbar_wait(k_full + ((c + 1) % kTcStages), ((c + 1) / kTcStages) & 1, p.st);
-              tc_fence_after_sync();
-            }
-            issue_qk(c + 1, g, (rt + g) % kTcQBufs);
-          } else if (g == 0) {
-            have = next_item(false);
-            if (have == 1) start(c + 1, rt + 2, 0);
-          } else {
-            if (have < 0) {
-              have = next_item(true);
-              if (have == 1) start(c + 1, rt + 2, 0);
-            }
-            if (have == 1) start(c + 1, rt + 3, 1);
-          }
+          issue_pv(c % kTcStages, g, i == 0);
+          issue_qk(n % kTcStages, g, q_addr[g]);
         }
+      }
+      // The last key tile: the next item's first products take the place of the next tile's.  In as little code as it can be: items of
+      // one or two key tiles come by here as often as by the loop above (unrolled, 1024 sequences of 64 tokens 678 us instead of 659).
+      have = -1;
+      int begun = 0;  // row tiles of the next item whose first product is issued
+#pragma unroll 1
+      for (int g = 0; g < 2; ++g) {
+        mbar_wait(p_full + g, c & 1, p.st);
+        if (g == 0) mbar_wait(v_full + c % kTcStages, (c / kTcStages) & 1, p.st);
+        tc_fence_after_sync();
+        issue_pv(c % kTcStages, g, ntiles == 1);
+        if (have < 0) have = next_item(g == 1);
+        if (have == 1)
+#pragma unroll 1
+          for (; begun <= g; ++begun) start(c + 1, rt + 2, begun);
       }
       kt += ntiles;
       rt += 2;
