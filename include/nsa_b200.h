@@ -251,9 +251,10 @@ int nsa_linear_compress_bwd(const void* x, const void* w, const void* pe, const 
  * Replaces sliding_pool_dxdw_kernel + dw.sum(1) and the autograd of the bias,
  * native_sparse_attention/ops/triton/weighted_pool.py:88-179,241-298,320-324,357-362.
  *   workspace: fp32, nsa_pool_compress_bwd_workspace_floats(...) words: the column sums of dy ([H, d], needed iff pe) followed
- *   by the partial rows of dw and of the column sums that the one-pass kernel for long inputs (131 072 tokens or more, head_dim
- *   128, kernel_size <= 32) leaves per CTA; a workspace of only H * d words (or NULL without pe) is accepted and keeps long
- *   inputs on the per-thread kernels.  max_seqlen is the longest input sequence. */
+ *   by the partial rows of dw and, unless sequences are many, of the column sums that the one-pass kernel for long inputs (131 072
+ *   tokens or more, head_dim 128, kernel_size <= 32) leaves per CTA; a workspace of only H * d words (or NULL without pe) is
+ *   accepted: weighted pooling of long inputs then stays on the per-thread kernels, average pooling takes its column sums from a
+ *   kernel of their own.  max_seqlen is the longest input sequence. */
 long long nsa_pool_compress_bwd_workspace_floats(int total_len, int batch, int max_seqlen, int num_heads, int head_dim,
                                                  int kernel_size, int kernel_stride);
 int nsa_pool_compress_bwd(const void* x, const void* w, const void* pe, const void* dy, const int* cu_seqlens,

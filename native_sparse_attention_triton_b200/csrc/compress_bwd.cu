@@ -496,8 +496,8 @@ extern "C" int nsa_pool_compress_bwd(const void* x, const void* w, const void* p
                                      long long x_stride_h, int dtype, void* stream) {
   using namespace nsa;
   if (!x || !cu_seqlens || !y_cu_seqlens || !dx || batch <= 0 || num_heads <= 0 || total_len <= 0 || max_seqlen <= 0) return kInvalid;
-  // workspace: [H, d] column sums of dy (needed iff pe), then the partial rows of dw of the streaming pass (optional: without
-  // them long inputs run on the per-thread kernels)
+  // workspace: [H, d] column sums of dy (needed iff pe), then the partial rows of the streaming pass (optional: without them weighted
+  // pooling runs on the per-thread kernels)
   const long long dbias_floats = (long long)num_heads * head_dim;
   float* dbias_scratch = workspace && workspace_floats >= dbias_floats ? workspace : nullptr;
   float* partial = workspace && workspace_floats > dbias_floats ? workspace + dbias_floats : nullptr;

@@ -12,19 +12,6 @@
 
 namespace nsa {
 
-struct DenseFwdParams {
-  const void* q;
-  void* o;
-  float* lse;  // [Nq, Hq]
-  const int* cu_q;
-  const int* cu_k;
-  long long q_sn, q_sh, o_sn, o_sh;
-  int B, Hq, Hkv, G, logG;
-  int window, stride, causal;
-  float scale2;
-  Status st;
-};
-
 // tcgen05 implementation (dense_fwd_tc.cu)
 int varlen_attn_fwd_tc(const void* q, const void* k, const void* v, const int* cu_q, const int* cu_k, void* o, float* lse,
                        int total_q, int total_k, int batch, int Hq, int Hkv, int head_dim, int causal,
@@ -49,16 +36,8 @@ static int varlen_attn_fwd_common(const void* q, const void* k, const void* v, c
     return kOk;
   }
   if (!k || !v) return kInvalid;
-  DenseFwdParams p;
-  p.q = q; p.o = o; p.lse = lse; p.cu_q = cu_seqlens_q; p.cu_k = cu_seqlens_k;
-  p.q_sn = strides[0]; p.q_sh = strides[1]; p.o_sn = strides[6]; p.o_sh = strides[7];
-  p.B = batch; p.Hq = num_q_heads; p.Hkv = num_kv_heads; p.G = G;
-  p.logG = 0;
-  while ((1 << p.logG) < G) ++p.logG;
-  p.window = window; p.stride = stride; p.causal = causal;
-  p.scale2 = sm_scale * kLog2e;
-  p.st.word = status_word();
-  if ((p.q_sn | p.q_sh | p.o_sn | p.o_sh) % 8 || !aligned16(q) || !aligned16(o)) return kInvalid;
+  // strides: q_n q_h k_n k_h v_n v_h o_n o_h (those of k and v are checked with their tensor maps)
+  if ((strides[0] | strides[1] | strides[6] | strides[7]) % 8 || !aligned16(q) || !aligned16(o)) return kInvalid;
   return varlen_attn_fwd_tc(q, k, v, cu_seqlens_q, cu_seqlens_k, o, lse, total_q, total_k, batch, num_q_heads,
                             num_kv_heads, head_dim, causal, window, stride, left, strides, sm_scale, dtype,
                             static_cast<cudaStream_t>(stream));

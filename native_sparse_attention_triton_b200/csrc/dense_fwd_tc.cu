@@ -22,7 +22,7 @@
 // overwrite P(i) before it has been read.
 // TMEM columns: [0,128) S/P of A, [128,256) S/P of B, [256,256+D) O of A, [384,384+D) O of B.
 //
-// What bounds it: a key tile of both row tiles takes about 3100 clocks (2048 of products, 1366 of exponentials): softmax of a row tile,
+// What bounds it: a key tile of both row tiles takes 2930 clocks (2048 of products, 1366 of exponentials): softmax of a row tile,
 // the hand-over to the issuing warp, its P V and next S, and the hand-over back are a chain.  A CTA of its own per item cost 12 000
 // clocks more each, of which set-up, the first loads and the output now run beside the neighbouring items.  64q/4kv, bf16, d 128,
 // this kernel alone, a CTA per item -> persistent: window 512 over 32 768 tokens 999 -> 763 us, window 128 694 -> 454; compressed keys

@@ -290,7 +290,7 @@ struct CompressBackward final : SavingNode {
                                        x.stride(0), x.stride(1), dtype_code(x), run.stream),
                "nsa_linear_compress_bwd");
     } else {
-      // column sums of dy, then the partial rows of dw
+      // column sums of dy, then the streaming pass's partial rows
       const long long n = nsa_pool_compress_bwd_workspace_floats((int)N, m.batch, m.longest_x, (int)H, (int)D, m.ks, m.st);
       Tensor ws = empty({n}, at::kFloat, x.device());
       check_rc(nsa_pool_compress_bwd(p(x), p(w), p(pe), p(dy), ptr<int>(cu), ptr<int>(ycu), p(dx), p(dw), p(dpe), ptr<float>(ws), n,

@@ -232,9 +232,10 @@ extern "C" int nsa_compressed_attn_topk(const void* q, const void* k, const floa
   if ((p.q_sn | p.q_sh) % 8 || !aligned16(q)) return kInvalid;
   {
     // two row tiles per CTA when their block scores fit in shared memory, else one, else the mma.sync kernel: G < 4, folds wider
-    // than 8 taps, and row tiles with more (token, block) pairs than the fold of the tcgen05 kernels holds (at kernel 32 / stride 16 /
-    // block 64 that is G of 4; with G of 8, 16q/2kv, d 64, 7833 tokens, a forward and backward chain took 604 us on mma.sync, 582 on
-    // tcgen05)
+    // than 8 taps, and row tiles with more (token, block) pairs than the fold of the tcgen05 kernels holds: 768 with two row tiles, 512
+    // with one.  At kernel 32 / stride 16 / block 64 that is G of 4 (1056), and, since one row tile does not hold its 528, G of 8 beyond
+    // 32 768 tokens (head_dim 64: 65 536); at 64 / 32 / 64 G of 16 (520) beyond 81 920 (147 456).  (16q/2kv, d 64, 7833 tokens, a forward and
+    // backward chain took 604 us with the scores on mma.sync, 582 on tcgen05.)
     int rc = score_topk_pp_tc(q, k, strides[2], strides[3], total_q, total_k, max_seqlen_q, head_dim, dtype, p,
                               static_cast<cudaStream_t>(stream));
     if (rc == kUnsupported)

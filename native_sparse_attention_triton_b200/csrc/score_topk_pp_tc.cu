@@ -8,7 +8,7 @@
 //   warp 16     : TMA producer (both Q tiles once, K tiles through a ring shared by the two row tiles)
 //   warp 17     : TMEM allocation and MMA issue, alternating between the row tiles
 // While one group exponentiates, the tensor pipe produces the other group's logits, and the two groups' barriers and
-// fold steps interleave instead of stalling all eight warps at once; each K tile is fetched once for 256 rows.
+// fold steps interleave instead of stalling all warps at once; each K tile is fetched once for 256 rows.
 // TMEM columns: tile g, buffer b at g*256 + b*128 (S^T is double-buffered per row tile).
 // What bounds it: the key-score threads' instruction stream (a key tile of both row tiles: 2048 clocks of exponentials without the
 // polynomial's share, 1024 of products, 4100 measured).  With one thread per key and two warps per scheduler 39 % of the issue slots
@@ -217,7 +217,7 @@ score_topk_pp_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
       }
       bar_sync_group(g);  // key scores of this tile are complete
-      // fold: block b_lo + brel reads tile-local keys fk0 .. fk0 + a + c - 2 (the layout repeats every tile: c divides 128)
+      // fold: block b_lo + brel reads tile-local keys k0 .. k0 + a + c - 2 (the layout repeats every tile: c divides 128)
       const int b_lo = i * (kPpKeyTile / c);
 #pragma unroll
       for (int r = 0; r < kPpRounds; ++r) {
@@ -263,9 +263,9 @@ static int launch_score_topk_pp_tc(const void* q, const void* k, long long k_sn,
   if (rc) return rc;
   // Cubics (relative error 7.5e-5) only for groups of 16 with at most kPpCubicPairs pairs.  Other layouts, groups of 8 at kernel 32 /
   // stride 16 / block 64 and groups of 16 at 64 / 32 / 64 among them, came here from kernels (mma.sync, one row tile) that take every
-  // exponential from the exponential unit, and keep that: the largest gap between a block left out and one taken, 8192 tokens, 64 / 32 / 64,
-  // is 3.5e-5 of its score with cubics and below 1e-6 without.  64q/4kv at 32 768 tokens, compressed attention with selection: 3226 us on
-  // mma.sync, 1543 to 1580 here with cubics, 1541 to 1584 without.
+  // exponential from the exponential unit, and keep that: over 8192 tokens, 64 / 32 / 64, a block left out scores up to 3.5e-5 of itself
+  // more than one taken with cubics, and never without.  64q/4kv at 32 768 tokens, compressed attention with selection: 3226 us on mma.sync,
+  // 1543 to 1580 here with cubics, 1541 to 1584 without.
   const bool cubic = p.G == 16 && pp_pairs(p.G, p.window / p.stride, p.block_size / p.stride) <= kPpCubicPairs;
   auto kern = cubic ? score_topk_pp_tc_kernel<T, D, 4, true>
                     : (p.logG == 4 ? score_topk_pp_tc_kernel<T, D, 4, false>

@@ -193,7 +193,7 @@ score_topk_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
     }
     bar_sync_softmax();  // every block score is final before any warp starts selecting
-    // ---- selection: the tokens of the CTA are dealt to the four warps ----
+    // ---- selection: the tokens of the CTA are dealt to the eight warps ----
     for (int tok = warp; tok < TPT; tok += 8) {
       const int t = q0 + tok;
       if (t >= Lq) break;
@@ -230,7 +230,7 @@ int score_topk_tc(const void* q, const void* k, long long k_sn, long long k_sh, 
                   int dtype, ScoreParams p, cudaStream_t stream) {
   if (p.G < 4 || p.G > 16) return kUnsupported;  // 8 to 32 tokens per CTA
   const int a = p.window / p.stride, c = p.block_size / p.stride;
-  // the fold step assumes that the block layout repeats every 128-key tile and that 3 (token, block) pairs per thread suffice
+  // the fold step assumes that the block layout repeats every 128-key tile and that 2 (token, block) pairs per thread suffice
   if (c <= 0 || kScKeyTile % c || a + c - 1 > 8 || (128 / p.G) * (kScKeyTile / c + (a - 1 + c - 1) / c) > 2 * 256) return kUnsupported;
   return NSA_DISPATCH_T_D(dtype, head_dim, launch_score_topk_tc, q, k, k_sn, k_sh, Nq, Nk, max_seqlen_q, p, stream);
 }

@@ -455,14 +455,15 @@ sparse_fwd_union_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // T - 3 free choices as uniform over the nb blocks before it (neighbours that agree more only make the union smaller), 2 QT tokens
 // touch U = 3 + nb (1 - (1 - (T - 3) / nb)^(2 QT)) of them; the union wins while U * (clocks per union tile) < 2 QT * T * (clocks per
 // private tile).  Measured with such selections, all tokens private / all in unions / split by this rule, us:
-//   32q/2kv d128 top-8   1024 tokens: 43 / 40 / 40    4096: 150 / 161 / 149    8192: 290 / 388 / 292
-//   64q/4kv d128 top-16  1024: 99 / 56 / 56   4096: 459 / 359 / 359   8192: 934 / 1033 / 882   16384: 1886 / 2882 / 1848
-//   32q/8kv d128 top-16  1024: 167 / 42 / 42  4096: 860 / 239 / 239   8192: 1775 / 656 / 656   16384: 3618 / 2217 / 2217
-//   16q/2kv d64  top-8   1024: 31 / 34 / 34   4096: 94 / 87 / 91      8192: 176 / 230 / 179
-// From the increments between the lengths: about 2150 clocks per union tile (64 keys, both row tiles) against 530 per private one at
-// head_dim 128, 1950 against 370 at 64.  The rule counts 1850 at 128: the second kernel's start and its last wave count against a
-// division that leaves it few tokens (with 2150 32q/2kv 2048 tokens: 79 us against 67, 64q/4kv 4096: 384 against 359, 8192: 876
-// against 882).
+//   32q/2kv d128 top-8   1024 tokens: 43 / 38 / 38    4096: 148 / 153 / 144    8192: 285 / 372 / 286
+//   64q/4kv d128 top-16  1024: 96 / 54 / 54   4096: 455 / 341 / 341   8192: 930 / 999 / 859   16384: 1884 / 2822 / 1830
+//   32q/8kv d128 top-16  1024: 162 / 44 / 42  4096: 857 / 238 / 228   8192: 1774 / 648 / 638  16384: 3619 / 2159 / 2158
+//   16q/2kv d64  top-8   1024: 31 / 34 / 34   4096: 90 / 83 / 89      8192: 172 / 222 / 175
+//   32q/2kv d64  top-8   1024: 31 / 34 / 34   4096: 92 / 130 / 104    8192: 178 / 312 / 185
+// From the increments between the lengths: about 2100 clocks per union tile (64 keys, both row tiles) against 530 per private one at
+// head_dim 128.  The rule counts 1850 there: the second kernel's start and its last wave count against a division that leaves it few
+// tokens.  At head_dim 64 it counts 1950 against 370 for groups of 8 and 16 alike, which gives groups of 16 too many tokens to the unions
+// (the last line).
 int union_limit(int G, int T, int block_size, int head_dim) {
   const double union_clocks = head_dim == 128 ? 1850. : 1950., private_clocks = head_dim == 128 ? 530. : 370.;
   const int tokens = 2 * (128 / G), nsub = block_size / 64, mw = (tokens + 31) / 32;
