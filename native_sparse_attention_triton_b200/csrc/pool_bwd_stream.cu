@@ -291,9 +291,9 @@ long long pool_bwd_stream_partial_floats(int num_heads, int head_dim, int total_
 }
 
 // Every CTA of the finishing kernel adds up its head's rows, which batches of many or very uneven sequences have one of per sequence and
-// run of the longest: past a row for 32 chunks of the input a pass of its own over dy costs less.  4 heads, weighted, 262 144 tokens in
-// all, backward, rows / own pass: 512 sequences of 512 tokens (512 rows) 143 / 154 us, 1024 of 256 (1024 rows) 172 / 157, one of 131 072
-// and 64 of 2048 (3770 rows) 347 / 199; 8192 of 64 778 / 449.
+// run of the longest: past a row for 32 chunks of the input a pass of its own over dy costs less.  4 heads, weighted, backward, rows / own
+// pass: 512 sequences of 512 tokens (512 rows) 141 / 147 us, 1024 of 256 (1024 rows) 178 / 151, one of 131 072 and 64 of 2048 (3770
+// rows) 352 / 205, 8192 of 64 (8192 rows) 775 / 435.
 bool pool_bwd_stream_sums(int num_heads, int head_dim, int total_len, int batch, int max_seqlen, int kernel_stride) {
   const int hb = pb_heads(num_heads);
   const int groups = kPbConsumers / (hb * (head_dim / 8));
