@@ -768,11 +768,14 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   return cv.run<T>(stream);
 }
 
-// Tokens of one block's list per work item.  512 where there is work enough (an item carries its block's K/V tile and the read-out
-// of its dK/dV sums); fewer where that would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads
-// x top-8 are 30 items of up to 64 tiles (148 us) at 512, 244 of 8 (see the figures in sparse_dkdv_tc.cu) at 64.
-static int sparse_chunk(int N, int Hkv, int topk) {
-  int chunk = 512;
+// Tokens of one block's list per work item.  Up to 32 row tiles of 128 / G tokens where there is work enough: the lists of long
+// sequences are shorter anyway, and where they are not, 64 tiles (150 us) leave a last wave that is nearly empty (1024 + 7168 + 8192
+// tokens, 64q/4kv, top-16: 2045 us with 64 tiles, 1832 with 32, 1811 with 16, 1965 with 8; 32 768 tokens, top-8: 2475, 2272, 2364,
+// 2447).  At most 512 tokens for the smaller groups (7097 tokens, 32q/8kv: 488 us with 16 tiles, 518 with 8).  Fewer where that
+// would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads x top-8 are 30 items of up to 64 tiles
+// (148 us) at 512 tokens, 244 of 8 (see the figures in sparse_dkdv_tc.cu) at 64.
+static int sparse_chunk(int N, int Hkv, int G, int topk) {
+  int chunk = std::min(512, 32 * (128 / G));
   while (chunk > 64 && (long long)Hkv * N * topk / chunk < 4 * 148) chunk >>= 1;
   return chunk;
 }
@@ -794,7 +797,7 @@ static size_t sparse_ws_bytes(int N, int batch, int Hq, int Hkv, int D, int topk
   const size_t x = (size_t)Hkv * sparse_windows(N, Hq / Hkv, D).second * TB + 1;
   return align_up((size_t)N * Hq * sizeof(float2), 256) + 2 * align_up((size_t)N * Hkv * D * sizeof(float), 256) +
          4 * align_up(x * sizeof(int), 256) + align_up((size_t)Hkv * N * topk * sizeof(int), 256) +
-         align_up(((size_t)Hkv * N * topk / sparse_chunk(N, Hkv, topk) + x) * sizeof(int), 256) +
+         align_up(((size_t)Hkv * N * topk / sparse_chunk(N, Hkv, Hq / Hkv, topk) + x) * sizeof(int), 256) +
          (sparse_fused_dq(Hq / Hkv) ? align_up((size_t)N * Hq * D * sizeof(float), 256) : 0);
 }
 
@@ -807,7 +810,7 @@ static int run_sparse_bwd(const void* q, const void* k, const void* v, const voi
   const int G = Hq / Hkv;
   const int TB = N / block_size + batch;
   const auto [W, NW] = sparse_windows(N, G, D);
-  const int chunk = sparse_chunk(N, Hkv, topk);
+  const int chunk = sparse_chunk(N, Hkv, G, topk);
   const size_t X = (size_t)Hkv * NW * TB + 1;
   uint8_t* w = static_cast<uint8_t*>(ws);
   float2* ld = reinterpret_cast<float2*>(w);
