@@ -190,6 +190,10 @@ int nsa_compressed_attn_decode(const void* q, const void* k, const void* v, cons
 /* Bytes of scratch nsa_varlen_attn_bwd needs.  No counterpart in the reference (it allocates
  * [G, total_k, Hkv, d] per-head buffers inside _compressed_attention_bwd, compressed_attention.py:664-669). */
 long long nsa_varlen_attn_bwd_workspace(int total_q, int total_k, int num_q_heads, int num_kv_heads, int head_dim);
+/* The bytes with which it makes dq beside dk and dv in one pass, where that is the faster way (long keys, head_dim 128): an fp32
+ * accumulator of dq more.  The same as above where it is not. */
+long long nsa_varlen_attn_bwd_workspace_one_pass(int total_q, int total_k, int batch, int max_seqlen_k, int num_q_heads,
+                                                 int num_kv_heads, int head_dim);
 
 /* Backward of nsa_varlen_attn_fwd: dq, dk, dv from (q, k, v, o, do, lse).
  * Replaces _compressed_attention_bwd (backward_sum_o_do, backward_dkdv, backward_dq and the .sum(0) over heads),

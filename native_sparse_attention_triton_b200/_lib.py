@@ -65,6 +65,7 @@ _SIGNATURES = {
 _SIZE_QUERIES = {
     "nsa_pool_compress_bwd_workspace_floats": [_I] * 7,
     "nsa_varlen_attn_bwd_workspace": [_I, _I, _I, _I, _I],
+    "nsa_varlen_attn_bwd_workspace_one_pass": [_I, _I, _I, _I, _I, _I, _I],
     "nsa_topk_sparse_attn_bwd_workspace": [_I, _I, _I, _I, _I, _I, _I],
     "nsa_launch_count": [],
     "nsa_flash_attn_decode_static_capacity": [],

@@ -663,6 +663,12 @@ __device__ __forceinline__ void row_stats(const T* __restrict__ o, const T* __re
   if (row < rows && sub == 0) ld[row] = make_float2(__ldg(lse + row), acc);
 }
 
+template <typename T, int D>
+__global__ void __launch_bounds__(128) row_stats_kernel(DenseBwdParams p, int total_q) {
+  row_stats<T, D>(static_cast<const T*>(p.o), static_cast<const T*>(p.dout), p.lse, p.ld, (long long)total_q * p.Hq, p.Hq, p.o_sn, p.o_sh, p.do_sn,
+                  p.do_sh, (long long)blockIdx.x * 128 + threadIdx.x);
+}
+
 // The histogram of the inverted index and the row statistics in one launch: they depend on nothing the other makes.
 template <typename T, int D>
 __global__ void __launch_bounds__(128) index_count_stats_kernel(IndexParams ip, unsigned count_blocks, SparseBwdParams p) {
@@ -721,10 +727,21 @@ static size_t dense_ws_bytes(int total_q, int total_k, int Hq, int Hkv, int D) {
   return align_up((size_t)total_q * Hq * sizeof(float2), 256) + 2 * align_up((size_t)total_k * Hkv * D * sizeof(float), 256);
 }
 
+// dQ, dK and dV in one pass (dense_bwd_tc.cu) or a dQ pass and a dK/dV pass.  One pass forms five products a tile and two passes
+// seven, but dQ then needs a zeroed fp32 accumulator, a conversion and its row statistics in a launch of their own (1.4 ms for 65 536
+// tokens of 64 heads), so what counts is how many key tiles a query sees.  Forward and backward, us, two passes -> one: 8192 tokens
+// 64q/4kv, causal 4441 -> 4157, 32q/8kv 2421 -> 2146; 2 x 3072 1405 -> 1274; 4 x 2048 1264 -> 1275; backward alone, 4095 keys
+// compressed from 65 536 tokens 14 298 -> 14 246, 2047 from 32 768 4078 -> 4748.  The longest sequence stands for the others only
+// where these are not much shorter.  Windows see few tiles.
+static bool dense_one_pass(int total_k, int batch, int max_k, int D) {
+  return D == 128 && max_k >= 3072 && 2ll * total_k >= (long long)batch * max_k;
+}
+static size_t dense_dq_bytes(int total_q, int Hq, int D) { return align_up((size_t)total_q * Hq * D * sizeof(float), 256); }
+
 template <typename T, int D>
 static int run_dense_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
-                         const int* cu_q, const int* cu_k, void* dq, void* dk, void* dv, void* ws, int total_q, int total_k,
-                         int batch, int max_q, int max_k, int Hq, int Hkv, int causal, int window, int stride, int left,
+                         const int* cu_q, const int* cu_k, void* dq, void* dk, void* dv, void* ws, long long ws_bytes, int total_q,
+                         int total_k, int batch, int max_q, int max_k, int Hq, int Hkv, int causal, int window, int stride, int left,
                          const long long* S, float sm_scale, cudaStream_t stream) {
   // S: q_n q_h k_n k_h v_n v_h o_n o_h do_n do_h dq_n dq_h dk_n dk_h dv_n dv_h
   const int G = Hq / Hkv;
@@ -734,7 +751,12 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   float* dk32 = reinterpret_cast<float*>(w);
   w += align_up((size_t)total_k * Hkv * D * sizeof(float), 256);
   float* dv32 = reinterpret_cast<float*>(w);
-  cudaError_t e = cudaMemsetAsync(dk32, 0, 2 * align_up((size_t)total_k * Hkv * D * sizeof(float), 256), stream);
+  w += align_up((size_t)total_k * Hkv * D * sizeof(float), 256);
+  const bool one_pass = left < 0 && dense_one_pass(total_k, batch, max_k, D) &&
+                        ws_bytes >= (long long)(dense_ws_bytes(total_q, total_k, Hq, Hkv, D) + dense_dq_bytes(total_q, Hq, D));
+  float* dq32 = one_pass ? reinterpret_cast<float*>(w) : nullptr;
+  if (one_pass) w += dense_dq_bytes(total_q, Hq, D);
+  cudaError_t e = cudaMemsetAsync(dk32, 0, w - reinterpret_cast<uint8_t*>(dk32), stream);
   if (e != cudaSuccess) return cuda_rc(e);
 
   DenseBwdParams p;
@@ -747,7 +769,11 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   p.scale2 = sm_scale * kLog2e; p.sm_scale = sm_scale;
   p.st.word = status_word();
   if (left >= 0 && D != 128) return kUnsupported;  // the sliding window is built for head_dim 128
-  {
+  if (one_pass) {
+    const unsigned blocks = (unsigned)(((long long)total_q * Hq * 16 + 127) / 128);
+    LaunchScope ls_("row_stats", stream);
+    row_stats_kernel<T, D><<<blocks, 128, 0, stream>>>(p, total_q);
+  } else {
     const int dt = DT<T>::kTmapType == CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 ? NSA_DTYPE_BF16 : NSA_DTYPE_FP16;
     const int rc = dense_dq_tc(k, v, S[2], S[3], S[4], S[5], total_q, total_k, max_q, D, dt, p, stream);
     if (rc) return rc;
@@ -760,9 +786,12 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   d.window = window; d.stride = stride; d.causal = causal; d.left = left;
   d.scale2 = p.scale2; d.sm_scale = sm_scale; d.st = p.st;
   const long long ds[8] = {S[0], S[1], S[2], S[3], S[4], S[5], S[8], S[9]};
-  const int rc = launch_dense_dkdv_tc<T, D>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream);
+  d.dq32 = dq32;
+  const int rc = one_pass ? launch_dense_bwd_tc<T>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream)
+                          : launch_dense_dkdv_tc<T, D>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream);
   if (rc) return rc;
   Converter cv;
+  if (one_pass) cv.add(dq32, dq, total_q, Hq, D, S[10], S[11]);
   cv.add(dk32, dk, total_k, Hkv, D, S[12], S[13]);
   cv.add(dv32, dv, total_k, Hkv, D, S[14], S[15]);
   return cv.run<T>(stream);
@@ -913,6 +942,12 @@ extern "C" long long nsa_varlen_attn_bwd_workspace(int total_q, int total_k, int
   return (long long)nsa::dense_ws_bytes(total_q, total_k, num_q_heads, num_kv_heads, head_dim);
 }
 
+extern "C" long long nsa_varlen_attn_bwd_workspace_one_pass(int total_q, int total_k, int batch, int max_seqlen_k, int num_q_heads,
+                                                            int num_kv_heads, int head_dim) {
+  return (long long)(nsa::dense_ws_bytes(total_q, total_k, num_q_heads, num_kv_heads, head_dim) +
+                     (nsa::dense_one_pass(total_k, batch, max_seqlen_k, head_dim) ? nsa::dense_dq_bytes(total_q, num_q_heads, head_dim) : 0));
+}
+
 static int varlen_attn_bwd_common(const void* q, const void* k, const void* v, const void* o, const void* dout,
                                   const float* lse, const int* cu_seqlens_q, const int* cu_seqlens_k, void* dq, void* dk,
                                   void* dv, void* workspace, long long workspace_bytes, int total_q, int total_k, int batch,
@@ -933,8 +968,8 @@ static int varlen_attn_bwd_common(const void* q, const void* k, const void* v, c
     if (!aligned16(rows)) return kInvalid;
   if (workspace_bytes < (long long)dense_ws_bytes(total_q, total_k, num_q_heads, num_kv_heads, head_dim)) return kWorkspace;
   return NSA_DISPATCH_T_D(dtype, head_dim, run_dense_bwd, q, k, v, o, dout, lse, cu_seqlens_q, cu_seqlens_k, dq, dk, dv,
-                          workspace, total_q, total_k, batch, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads, causal,
-                          window, stride, left, strides, sm_scale, static_cast<cudaStream_t>(stream));
+                          workspace, workspace_bytes, total_q, total_k, batch, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads,
+                          causal, window, stride, left, strides, sm_scale, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nsa_varlen_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,

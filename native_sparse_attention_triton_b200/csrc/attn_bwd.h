@@ -25,7 +25,7 @@ struct DkdvParams {
   const float2* ld;    // [Nq, Hq]
   float* dk32;         // [Nk, Hkv, D] fp32 accumulators (zeroed)
   float* dv32;
-  float* dq32 = nullptr;  // sparse tcgen05 pass only: [Nq, Hq, D] fp32 accumulator (zeroed)
+  float* dq32 = nullptr;  // sparse tcgen05 pass and the dense pass that also makes dQ: [Nq, Hq, D] fp32 accumulator (zeroed)
   const int* cu_q;
   const int* cu_k;      // dense: compressed cu; sparse: same as cu_q
   // sparse
@@ -77,5 +77,11 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
 template <typename T, int D>
 int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk,
                          int max_q, int max_k, int batch, DkdvParams p, cudaStream_t stream);
+
+// dQ, dK and dV of the dense attention in one pass (dense_bwd_tc.cu); head_dim 128, group size a power of two <= 16.
+// p.chunk = tokens per CTA; p.dq32 zeroed like p.dk32 and p.dv32.
+template <typename T>
+int launch_dense_bwd_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk, int max_q,
+                        int max_k, int batch, DkdvParams p, cudaStream_t stream);
 
 }  // namespace nsa

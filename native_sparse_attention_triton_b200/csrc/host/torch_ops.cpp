@@ -431,11 +431,12 @@ struct DenseAttentionBackward final : SavingNode {
       return out;
     }
     const Tensor dout = gradient_rows(grads[0]);
-    const long long bytes = nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D);
+    const int batch = (int)cu_q.size(0) - 1;
+    const long long bytes = m.left >= 0 ? nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D)
+                                        : nsa_varlen_attn_bwd_workspace_one_pass((int)N, (int)Nk, batch, m.max_k, (int)Hq, (int)Hkv, (int)D);
     Tensor ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
     QkvStrides st;
     st.add(q).add(k).add(v).add(o).add(dout).add(dq).add(dk).add(dv);
-    const int batch = (int)cu_q.size(0) - 1;
     Launch run(q);
     if (m.left >= 0)
       check_rc(nsa_window_attn_bwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(dout), ptr<float>(lse), ptr<int>(cu_q), ptr(dq), ptr(dk), ptr(dv),
