@@ -216,6 +216,7 @@ def kernel_work(name, f, fused_dq=True):
         "score_topk": ("tensor", cmp_f / 2),       # S recomputed once for the scores (selection overhead)
         "dense_dq": ("tensor", cmp_f),             # 2 of the 5 backward GEMM units
         "dense_dkdv": ("tensor", 1.5 * cmp_f),     # 3 of the 5 backward GEMM units
+        "dense_bwd": ("tensor", 2.5 * cmp_f),      # all five, where one pass makes dQ, dK and dV
         "sparse_fwd": ("tensor", sel_f),
         "sparse_dq": ("tensor", sel_f),
         "sparse_dkdv": ("tensor", (2.5 if fused_dq else 1.5) * sel_f),
