@@ -79,3 +79,34 @@ def test_compressed_keys_and_the_smaller_workspace():
     for a, b in zip(*grads):
         assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("Hq,Hkv,lens_q,lens_k,dtype", [
+    (16, 1, [200, 5], [3500, 3100], torch.bfloat16),   # fewer queries than keys
+    (8, 4, [4000, 0, 1], [3072, 3300, 3200], torch.float16),  # a sequence without queries, one with a single one
+])
+def test_other_lengths_and_strides(Hq, Hkv, lens_q, lens_k, dtype):
+    """No mask, queries and keys of different lengths, all inputs and the gradient strided views."""
+    import native_sparse_attention_triton_b200 as pkg
+    d, Nq, Nk = 128, sum(lens_q), sum(lens_k)
+    g = torch.Generator(device="cuda").manual_seed(Nq)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    q = rnd(Hq, Nq, d).transpose(0, 1)              # heads outermost
+    k, v = rnd(Nk, 2, Hkv, d).unbind(1)             # packed pairs
+    do = rnd(Nq, Hq + 1, d + 8)[:, 1:, :d]          # padded rows
+    leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+    cu = [torch.tensor([0] + torch.tensor(n).cumsum(0).tolist(), dtype=torch.int32, device="cuda") for n in (lens_q, lens_k)]
+    assert pkg._lib.lib().nsa_varlen_attn_bwd_workspace_one_pass(Nq, Nk, len(lens_k), max(lens_k), Hq, Hkv, d) > \
+        pkg._lib.lib().nsa_varlen_attn_bwd_workspace(Nq, Nk, Hq, Hkv, d)
+    pkg.ops.flash_attention_varlen(*leaves, *cu, max(lens_q), max(lens_k), causal=False).backward(do)
+    ref = [t.detach().float().requires_grad_(True) for t in (q, k, v)]
+    outs, aq, ak = [], 0, 0
+    for nq, nk in zip(lens_q, lens_k):
+        qs, ks, vs = ref[0][aq:aq + nq], ref[1][ak:ak + nk], ref[2][ak:ak + nk]
+        s = torch.einsum("qhgd,khd->hgqk", qs.reshape(nq, Hkv, Hq // Hkv, d), ks) / math.sqrt(d)
+        outs.append(torch.einsum("hgqk,khd->qhgd", s.softmax(-1), vs).reshape(nq, Hq, d))
+        aq, ak = aq + nq, ak + nk
+    torch.cat(outs).backward(do.float())
+    for name, a, b in zip(("dq", "dk", "dv"), leaves, ref):
+        assert_close_16bit(a.grad, b.grad.cpu(), name, grad_tol(name, False), MEAN_TOL)
+    assert pkg.device_status() == 0
