@@ -805,10 +805,13 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
 // tokens, 64q/4kv, top-16: 2045 us with 64 tiles, 1832 with 32, 1811 with 16, 1965 with 8; 32 768 tokens, top-8: 2475, 2272, 2364,
 // 2447).  At most 512 tokens for the smaller groups (7097 tokens, 32q/8kv: 488 us with 16 tiles, 518 with 8).  Fewer where that
 // would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads x top-8 are 30 items of up to 64 tiles
-// (148 us) at 512 tokens, 244 of 8 (see the figures in sparse_dkdv_tc.cu) at 64.
+// (148 us) at 512 tokens, 244 of 8 at 64.  Down to four row tiles where even those are less than two for every SM: 977 tokens x 2 heads
+// x top-8 48 -> 43 us, 512 tokens 29 -> 23; with more of them an item's K and V tile and read-out cost more than that gives (2000 tokens
+// x 1 head x top-16, 500 items of 8 tiles, 70 us; 78 with 4).
 static int sparse_chunk(int N, int Hkv, int G, int topk) {
   int chunk = std::min(512, 32 * (128 / G));
   while (chunk > 64 && (long long)Hkv * N * topk / chunk < 4 * 148) chunk >>= 1;
+  if (chunk > 4 * (128 / G) && (long long)Hkv * N * topk / chunk < 2 * 148) chunk >>= 1;
   return chunk;
 }
 
