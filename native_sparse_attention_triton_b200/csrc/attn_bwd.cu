@@ -800,25 +800,29 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   return cv.run<T>(stream);
 }
 
-// Tokens of one block's list per work item.  Up to 32 row tiles of 128 / G tokens where there is work enough: the lists of long
-// sequences are shorter anyway, and where they are not, 64 tiles (150 us) leave a last wave that is nearly empty (1024 + 7168 + 8192
-// tokens, 64q/4kv, top-16: 2045 us with 64 tiles, 1832 with 32, 1811 with 16, 1965 with 8; 32 768 tokens, top-8: 2475, 2272, 2364,
-// 2447).  At most 512 tokens for the smaller groups (7097 tokens, 32q/8kv: 488 us with 16 tiles, 518 with 8).  Fewer where that
-// would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads x top-8 are 30 items of up to 64 tiles
-// (148 us) at 512 tokens, 244 of 8 at 64.  Down to four row tiles where even those are less than two for every SM: 977 tokens x 2 heads
-// x top-8 48 -> 43 us, 512 tokens 29 -> 23; with more of them an item's K and V tile and read-out cost more than that gives (2000 tokens
-// x 1 head x top-16, 500 items of 8 tiles, 70 us; 78 with 4).
+// dQ comes out of the tcgen05 dK/dV pass for these groups; the others have the mma.sync passes.
+static bool sparse_fused_dq(int G) { return G >= 4 && (G & (G - 1)) == 0; }
+
+// Tokens of one block's list per work item.  tcgen05 pass: up to 32 row tiles of 128 / G tokens where there is work enough: the lists of
+// long sequences are shorter anyway, and where they are not, 64 tiles (150 us) leave a last wave that is nearly empty (whole backward,
+// 1024 + 7168 + 8192 tokens, 64q/4kv, top-16: 2600 us with 64 tiles, 2494 with 32, 2556 with 16, 2733 with 8; 32 768 tokens, top-8: 3448,
+// 3319, 3437, 3580).  At most 512 tokens for the smaller groups (7097 tokens, 32q/8kv: 678 us with 16 tiles, 693 with 8).  Fewer where
+// that would leave SMs without an item or with one long chain of row tiles: 977 tokens x 2 heads x top-8 are 30 items of up to 64 tiles
+// at 512 tokens (176 us), 244 of 8 at 64 (86).  Down to four row tiles where even those are less than two for every SM: 81 us there; with
+// more of them an item's K and V tile and read-out cost more than that gives (2000 tokens x 1 head x top-16, 500 items of 8 tiles,
+// 112 us; 119 with 4).
+// mma.sync pass: 512 tokens, halved down to 64 while there are less than four items for every SM.  It has no tiles of 128 rows: items
+// counted in those took 977 tokens, 24q/2kv, top-8 from 117 to 128 us and 6000 tokens, 20q/2kv, top-16 from 1144 to 1177.
 static int sparse_chunk(int N, int Hkv, int G, int topk) {
-  int chunk = std::min(512, 32 * (128 / G));
+  const int tile = sparse_fused_dq(G) ? 128 / G : 16;  // 16: 512 tokens at most, 64 at least
+  int chunk = std::min(512, 32 * tile);
   while (chunk > 64 && (long long)Hkv * N * topk / chunk < 4 * 148) chunk >>= 1;
-  if (chunk > 4 * (128 / G) && (long long)Hkv * N * topk / chunk < 2 * 148) chunk >>= 1;
+  if (chunk > 4 * tile && (long long)Hkv * N * topk / chunk < 2 * 148) chunk >>= 1;
   return chunk;
 }
 
 // Token windows of the inverted index: as many tokens as keep the Q and dO rows of one KV-head group (G heads) within
 // about half of the L2 cache, a power of two, at least 1024.  Returns (tokens per window, windows).
-static bool sparse_fused_dq(int G) { return G >= 4 && (G & (G - 1)) == 0; }
-
 static std::pair<int, int> sparse_windows(int N, int G, int D) {
   // Q and dO rows (16-bit) and, where the tcgen05 pass also produces dQ, the fp32 dQ accumulator rows it reduces into
   const long long bytes_per_token = 2ll * G * D * 2 + (sparse_fused_dq(G) ? 4ll * G * D : 0);
