@@ -99,12 +99,6 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int tok_end = p.left >= 0 ? min(min(c_lo + p.chunk, Lq), kpos + kvalid + p.left) : min(c_lo + p.chunk, Lq);
   if (tok_end <= tok_begin) return;
   const int ntiles = (tok_end - tok_begin + TPT - 1) / TPT;
-  // The key tiles of a token chunk run side by side and add to the same dQ rows: each begins its round over the chunk's row tiles
-  // at a place of its own, so that not all of them add to the same lines at one time (64 KB of reductions: 2890 clocks when they do,
-  // 2720 otherwise).
-  const int first = (int)((unsigned)blockIdx.x * ntiles / gridDim.x);
-  // in-sequence position of the first token of the i-th tile of the round
-  auto tile_token = [&](int i) { return tok_begin + (first + i < ntiles ? first + i : first + i - ntiles) * TPT; };
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -149,7 +143,7 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
     for (int i = 0; i < ntiles; ++i) {
-      const int tok0 = tile_token(i);
+      const int tok0 = tok_begin + i * TPT;
       const int s = i % kStages;
       const uint32_t before = ((i / kStages) - 1) & 1;
       if (lane == 0) {
@@ -262,7 +256,7 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     };
     for (int i = 0; i < ntiles; ++i) {
-      const int tok0 = tile_token(i);
+      const int tok0 = tok_begin + i * TPT;
       const int nrows = min(TPT, tok_end - tok0) << logG;
       float* tile = p.dq32 + ((long long)(qs + tok0) * p.Hq + h * p.G) * D + (warp & 3) * 32 + lane;
       if (!mbar_wait(dq_full, i & 1, p.st)) break;
@@ -294,7 +288,7 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const bool key_ok = key < kvalid;
     for (int i = 0; i < ntiles; ++i) {
       const int ms = i & 1;
-      const int tok0 = tile_token(i);
+      const int tok0 = tok_begin + i * TPT;
       // visible columns of this thread: [clo, chi) in tile columns, shifted to the thread's own 64
       const int clo = max(0, thr - tok0) << logG;
       int chi = key_ok ? (min(TPT, tok_end - tok0) << logG) : 0;
