@@ -729,13 +729,31 @@ static size_t dense_ws_bytes(int total_q, int total_k, int Hq, int Hkv, int D) {
 
 // dQ, dK and dV in one pass (dense_bwd_tc.cu) or a dQ pass and a dK/dV pass.  One pass forms five products a tile and two passes
 // seven, but dQ then needs a zeroed fp32 accumulator, a conversion and its row statistics in a launch of their own (1.4 ms for 65 536
-// tokens of 64 heads), so what counts is how many key tiles a query sees.  Forward and backward, us, two passes -> one: 8192 tokens
-// 64q/4kv, causal 4441 -> 4157, 32q/8kv 2421 -> 2146; 2 x 3072 1405 -> 1274; 4 x 2048 1264 -> 1275; backward alone, 4095 keys
-// compressed from 65 536 tokens 14 298 -> 14 246, 2047 from 32 768 4078 -> 4748.  The longest sequence stands for the others only
-// where these are not much shorter.  Windows see few tiles.
+// tokens of 64 heads), so what counts is how many key tiles a query sees.  Backward alone, us, both forms in turn, two passes -> one:
+// 3072 tokens, causal, 64q/4kv 564 -> 547, 16q/1kv 186 -> 183, 8q/8kv 173 -> 128; 4 x 3072 tokens 64q/4kv 2190 -> 2096; 8192 tokens 64q/4kv
+// 3345 -> 3167, 32q/8kv 1906 -> 1622; 3072 keys compressed from 12 296 tokens 2141 -> 2137, from 49 168 8242 -> 8084 (16q/1kv 2228 -> 2095), 4095
+// from 65 536 14 465 -> 13 747 (32q/8kv 7495 -> 6595); 200 queries of 3500 keys 90 -> 62.  The longest sequence stands for the others only
+// where these are not much shorter (3072 and three of 1100: 878 -> 842).  Windows see few tiles.
 static bool dense_one_pass(int total_k, int batch, int max_k, int D) {
   return D == 128 && max_k >= 3072 && 2ll * total_k >= (long long)batch * max_k;
 }
+
+// Tokens per CTA of the one pass.  A CTA's loads, ramp and the read-out of dK and dV cost as much as 2.4 row tiles (16 384 tokens 8q/8kv:
+// 2852 us with 4 tiles, 2324 with 8, 2047 with 16, 1887 with 32, 1829 with 64), and at the end an SM waits for half a CTA on average: of W row
+// tiles an SM takes W (1 + 2.4 / t) + t / 2 of time, which is least at t = sqrt(4.8 W).  The power of two next to it, us, against half and
+// twice as many: 3072 tokens 8q/8kv (W 15) 8 tiles 128, 16 136; 3072 tokens 16q/8kv 16 tiles 183, 8 190, 32 201; 4096 tokens 64q/4kv (W 220) 32
+// tiles 924, 64 916, 16 979; 8192 tokens 64q/4kv (W 890) 64 tiles 3270, 32 3392, 128 3308; 16 384 tokens 64q/4kv (W 3540) 128 tiles 12 014, 64
+// 12 311; 20 000 tokens 32q/2kv 8891, 9138.  Lengths in tokens, as the dK/dV pass has them, gave small groups CTAs of 2 to 8 tiles: 3072 tokens
+// 8q/8kv 175 us, 4 x 3072 622 (411 now), slower than the two passes.
+static int one_pass_chunk(int total_k, int batch, int max_q, int Hkv, int G, int causal) {
+  // (key tile, head) pairs times the row tiles that see one, half of them under the causal mask
+  const double row_tiles = (double)max_q * G / (causal ? 256 : 128);
+  const double per_sm = ((double)total_k / 128 + batch) * Hkv * row_tiles / 148;
+  int tiles = 128;
+  while (tiles > 8 && (double)tiles * tiles > 10 * per_sm) tiles >>= 1;
+  return tiles * (128 / G);
+}
+
 static size_t dense_dq_bytes(int total_q, int Hq, int D) { return align_up((size_t)total_q * Hq * D * sizeof(float), 256); }
 
 template <typename T, int D>
@@ -782,13 +800,10 @@ static int run_dense_bwd(const void* q, const void* k, const void* v, const void
   d.ld = ld; d.dk32 = dk32; d.dv32 = dv32; d.cu_q = cu_q; d.cu_k = cu_k;
   d.offsets = nullptr; d.item_base = nullptr; d.item_bin = nullptr; d.item_counter = nullptr; d.list = nullptr;
   d.B = batch; d.Hq = Hq; d.Hkv = Hkv; d.G = G; d.TB = 0; d.NW = 1; d.block_size = kKeyTile;
-  d.chunk = dense_chunk(max_q, max_k, batch * Hkv, G, left);
+  d.chunk = one_pass ? one_pass_chunk(total_k, batch, max_q, Hkv, G, causal) : dense_chunk(max_q, max_k, batch * Hkv, G, left);
   d.window = window; d.stride = stride; d.causal = causal; d.left = left;
   d.scale2 = p.scale2; d.sm_scale = sm_scale; d.st = p.st;
   const long long ds[8] = {S[0], S[1], S[2], S[3], S[4], S[5], S[8], S[9]};
-  // One pass: at most 64 row tiles (170 us) a CTA, so that the last wave is not long: 64q/4kv, forward and backward, 8192 tokens causal
-  // 4180 us with 128 tiles, 4100 with 64, 4260 with 32; 4096 all visible 2083, 2013, 2031; 16q/1kv, 8192 tokens 1095, 1029, 1045.
-  if (one_pass) d.chunk = std::min(d.chunk, 64 * (128 / G));
   d.dq32 = dq32;
   const int rc = one_pass ? launch_dense_bwd_tc<T>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream)
                           : launch_dense_dkdv_tc<T, D>(q, dout, k, v, ds, total_q, total_k, max_q, max_k, batch, d, stream);

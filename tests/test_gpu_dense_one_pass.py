@@ -53,32 +53,96 @@ def test_gradients(Hq, Hkv, lens, causal, dtype):
     assert pkg.device_status() == 0
 
 
-def test_compressed_keys_and_the_smaller_workspace():
-    """Strided causal mask: 3073 keys of 16 tokens each; the two-pass kernels, chosen by the workspace, give the same gradients.
-    Both round fp32 sums to 16 bits once: they differ by single roundings (2^-8 of a value) where the sums' order does."""
+def both_forms(lens_q, lens_k, Hq, Hkv, causal, window, stride):
+    """The backward as a call that takes one pass, and one that takes two: chosen by the workspace.  Returns (call, its gradients) each
+    and the inputs."""
     import native_sparse_attention_triton_b200 as pkg
     lib = pkg._lib.lib()
-    N, m, Hq, Hkv, d = 3073 * 16 + 5, 3073, 8, 2, 128
+    N, m, B, d = sum(lens_q), sum(lens_k), len(lens_q), 128
     g = torch.Generator(device="cuda").manual_seed(3)
     q, k, v, do = [torch.randn(n, h, d, generator=g, device="cuda").bfloat16() for n, h in ((N, Hq), (m, Hkv), (m, Hkv), (N, Hq))]
-    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device="cuda") for n in (N, m))
+    cu_q, cu_k = (torch.tensor([0] + torch.tensor(n).cumsum(0).tolist(), dtype=torch.int32, device="cuda") for n in (lens_q, lens_k))
     o, lse = torch.empty_like(q), torch.empty(N, Hq, device="cuda")
     P, scale = lambda t: t.data_ptr(), 1 / math.sqrt(d)
     rows, kv = [Hq * d, d], [Hkv * d, d]
     fwd = pkg._lib.strides_array(*rows, *kv, *kv, *rows)
-    assert lib.nsa_varlen_attn_fwd(P(q), P(k), P(v), P(cu_q), P(cu_k), P(o), P(lse), N, m, 1, N, Hq, Hkv, d, 1, 16, 16, fwd, scale, 0, None) == 0
+    assert lib.nsa_varlen_attn_fwd(P(q), P(k), P(v), P(cu_q), P(cu_k), P(o), P(lse), N, m, B, max(lens_q), Hq, Hkv, d, causal, window, stride, fwd, scale,
+                                   0, None) == 0
     bwd = pkg._lib.strides_array(*rows, *kv, *kv, *rows, *rows, *rows, *kv, *kv)
-    grads = []
-    for size in (lib.nsa_varlen_attn_bwd_workspace_one_pass(N, m, 1, m, Hq, Hkv, d), lib.nsa_varlen_attn_bwd_workspace(N, m, Hq, Hkv, d)):
+    sizes = lib.nsa_varlen_attn_bwd_workspace_one_pass(N, m, B, max(lens_k), Hq, Hkv, d), lib.nsa_varlen_attn_bwd_workspace(N, m, Hq, Hkv, d)
+    assert sizes[0] > sizes[1]
+
+    def form(size):
         out = [torch.empty_like(t) for t in (q, k, v)]
         ws = torch.empty(size, dtype=torch.uint8, device="cuda")
-        assert lib.nsa_varlen_attn_bwd(P(q), P(k), P(v), P(o), P(do), P(lse), P(cu_q), P(cu_k), *(P(t) for t in out), P(ws), size, N, m, 1, N, m,
-                                       Hq, Hkv, d, 1, 16, 16, bwd, scale, 0, None) == 0
-        torch.cuda.synchronize()
-        grads.append(out)
-    for a, b in zip(*grads):
-        assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
+
+        def call():
+            assert lib.nsa_varlen_attn_bwd(P(q), P(k), P(v), P(o), P(do), P(lse), P(cu_q), P(cu_k), *(P(t) for t in out), P(ws), size, N, m, B, max(lens_q),
+                                           max(lens_k), Hq, Hkv, d, causal, window, stride, bwd, scale, 0, torch.cuda.current_stream().cuda_stream) == 0
+        return call, out
+    return form(sizes[0]), form(sizes[1]), (q, k, v, do)
+
+
+def test_compressed_keys_and_the_smaller_workspace():
+    """Strided causal mask: 3073 keys of 16 tokens each, against fp32 sums over every key; the two-pass kernels, chosen by the workspace,
+    give the same gradients.  Both round fp32 sums to 16 bits once: they differ by single roundings (2^-8 of a value) where the sums'
+    order does."""
+    import native_sparse_attention_triton_b200 as pkg
+    N, m, Hq, Hkv = 3073 * 16 + 5, 3073, 8, 2
+    (one, a), (two, b), (q, k, v, do) = both_forms([N], [m], Hq, Hkv, 1, 16, 16)
+    one(), two()
+    for x, y in zip(a, b):
+        assert (x.float() - y.float()).norm() <= 2 ** -8 * y.float().norm()
+    # fp32, a block of queries and a head at a time: key j is seen from token 16 j + 15 on
+    ref = [torch.zeros(t.shape, device="cuda") for t in (q, k, v)]
+    first = torch.arange(m, device="cuda") * 16 + 15
+    for at in range(0, N, 8192):
+        t = slice(at, min(N, at + 8192))
+        hidden = first[None, :] > torch.arange(at, t.stop, device="cuda")[:, None]
+        for h in range(Hq):
+            leaves = [x.float().requires_grad_(True) for x in (q[t, h], k[:, h // (Hq // Hkv)], v[:, h // (Hq // Hkv)])]
+            s = (leaves[0] @ leaves[1].T / math.sqrt(128)).masked_fill(hidden, float("-inf"))
+            p = s.softmax(-1).nan_to_num(0.0)  # the first 15 tokens see no key
+            gq, gk, gv = torch.autograd.grad([p @ leaves[2]], leaves, [do[t, h].float()])
+            ref[0][t, h] = gq.nan_to_num(0.0)
+            ref[1][:, h // (Hq // Hkv)] += gk.nan_to_num(0.0)
+            ref[2][:, h // (Hq // Hkv)] += gv
+    for name, x, r in zip(("dq", "dk", "dv"), a, ref):
+        assert_close_16bit(x, r.cpu(), name, grad_tol(name, False), MEAN_TOL)
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("Hq,Hkv,lens,causal", [
+    (2, 2, [3072], 1),           # CTAs of 8 row tiles, the least
+    (8, 8, [3072] * 4, 1),       # 16
+    (4, 1, [5000, 3071], 1),     # 16
+    (16, 1, [6100], 1),          # 32
+    (16, 1, [9000], 0),          # 64
+    (16, 1, [24600], 1),         # 128, the most
+])
+def test_cta_lengths(Hq, Hkv, lens, causal):
+    """One pass against two, as above, with CTAs of every length."""
+    import native_sparse_attention_triton_b200 as pkg
+    (one, a), (two, b), _ = both_forms(lens, lens, Hq, Hkv, causal, 1, 1)
+    one(), two()
+    for x, y in zip(a, b):
+        assert (x.float() - y.float()).norm() <= 2 ** -8 * y.float().norm()
+    assert pkg.device_status() == 0
+
+
+def test_one_query_head_per_key_head_is_not_slower():
+    """Groups of one, whose row tiles are 128 tokens: in turn with the two passes, where CTAs of few row tiles took 1.07 of their time
+    (as long as the CTAs should be: 0.71)."""
+    (one, _), (two, _), _ = both_forms([3072] * 4, [3072] * 4, 8, 8, 1, 1, 1)
+    times = [[], []]
+    for i in range(20):
+        for call, ts in zip((one, two), times):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record(), call(), end.record()
+            end.synchronize()
+            ts.append(start.elapsed_time(end))
+    one_ms, two_ms = (sorted(ts)[len(ts) // 2] for ts in times)
+    assert one_ms < two_ms
 
 
 @pytest.mark.parametrize("Hq,Hkv,lens_q,lens_k,dtype", [
