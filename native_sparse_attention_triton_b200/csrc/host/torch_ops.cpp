@@ -432,9 +432,17 @@ struct DenseAttentionBackward final : SavingNode {
     }
     const Tensor dout = gradient_rows(grads[0]);
     const int batch = (int)cu_q.size(0) - 1;
-    const long long bytes = m.left >= 0 ? nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D)
-                                        : nsa_varlen_attn_bwd_workspace_one_pass((int)N, (int)Nk, batch, m.max_k, (int)Hq, (int)Hkv, (int)D);
-    Tensor ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
+    const long long least = nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D);
+    long long bytes = m.left >= 0 ? least : nsa_varlen_attn_bwd_workspace_one_pass((int)N, (int)Nk, batch, m.max_k, (int)Hq, (int)Hkv, (int)D);
+    Tensor ws;
+    try {
+      ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
+    } catch (const c10::OutOfMemoryError&) {
+      // one pass asks for an fp32 dq more (2.1 GB for 65 536 tokens of 64 heads): where that does not fit, two passes are the way
+      if (bytes == least) throw;
+      bytes = least;
+      ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());
+    }
     QkvStrides st;
     st.add(q).add(k).add(v).add(o).add(dout).add(dq).add(dk).add(dv);
     Launch run(q);

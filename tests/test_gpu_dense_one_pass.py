@@ -174,3 +174,49 @@ def test_other_lengths_and_strides(Hq, Hkv, lens_q, lens_k, dtype):
     for name, a, b in zip(("dq", "dk", "dv"), leaves, ref):
         assert_close_16bit(a.grad, b.grad.cpu(), name, grad_tol(name, False), MEAN_TOL)
     assert pkg.device_status() == 0
+
+
+def kernels(call):
+    """Names of the kernels that a call launches."""
+    import native_sparse_attention_triton_b200 as pkg
+    pkg._lib.profile(True)
+    try:
+        call()
+        torch.cuda.synchronize()
+        return set(pkg._lib.profile_collect())
+    finally:
+        pkg._lib.profile(False)
+
+
+def test_two_passes_where_the_larger_workspace_does_not_fit():
+    import native_sparse_attention_triton_b200 as pkg
+    N, Hq, Hkv, d = 3072, 64, 4, 128
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v, do = [torch.randn(N, h, d, generator=g, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv, Hq)]
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    cu = torch.tensor([0, N], dtype=torch.int32, device="cuda")
+    grads = lambda: torch.autograd.grad([pkg.ops.flash_attention_varlen(*leaves, cu, cu, N, N, causal=True)], leaves, [do])
+    want = []
+    assert "dense_bwd_tc" in kernels(lambda: want.extend(t.cpu() for t in grads()))
+    o = pkg.ops.flash_attention_varlen(*leaves, cu, cu, N, N, causal=True)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total, held = torch.cuda.get_device_properties(0).total_memory, torch.cuda.memory_reserved()
+    filler, got = [], []
+    try:
+        torch.cuda.set_per_process_memory_fraction(held / total)
+        for size in (32 << 20, 4 << 20, 2 << 20):  # room in the pieces that the process holds
+            try:
+                while True:
+                    filler.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        # 100 MiB more are enough for dq, dk and dv (48 + 3 + 3) and the smaller workspace (14); the larger one is 110
+        torch.cuda.set_per_process_memory_fraction((held + (100 << 20)) / total)
+        ran = kernels(lambda: got.extend(torch.autograd.grad([o], leaves, [do])))
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert "dense_dq_tc" in ran and "dense_bwd_tc" not in ran
+    for x, y in zip((t.cpu() for t in got), want):
+        assert (x.float() - y.float()).norm() <= 2 ** -8 * y.float().norm()
+    assert pkg.device_status() == 0
