@@ -191,7 +191,8 @@ int nsa_compressed_attn_decode(const void* q, const void* k, const void* v, cons
  * [G, total_k, Hkv, d] per-head buffers inside _compressed_attention_bwd, compressed_attention.py:664-669). */
 long long nsa_varlen_attn_bwd_workspace(int total_q, int total_k, int num_q_heads, int num_kv_heads, int head_dim);
 /* The bytes with which it makes dq beside dk and dv in one pass, where that is the faster way (long keys, head_dim 128): an fp32
- * accumulator of dq more.  The same as above where it is not. */
+ * accumulator of dq more.  The same as above where it is not.  dq is then a sum of fp32 atomic adds like dk and dv; with less
+ * workspace it is summed in a fixed order and is the same from run to run. */
 long long nsa_varlen_attn_bwd_workspace_one_pass(int total_q, int total_k, int batch, int max_seqlen_k, int num_q_heads,
                                                  int num_kv_heads, int head_dim);
 
@@ -201,7 +202,7 @@ long long nsa_varlen_attn_bwd_workspace_one_pass(int total_q, int total_k, int b
  * native_sparse_attention/ops/triton/flash_attention.py:168-560,660-822.
  *   strides[16] = {q_n,q_h, k_n,k_h, v_n,v_h, o_n,o_h, do_n,do_h, dq_n,dq_h, dk_n,dk_h, dv_n,dv_h}.
  *   dk/dv partial sums of CTAs sharing a key tile are combined with fp32 atomic adds (run-to-run
- *   differences at fp32 rounding level, as in the reference's atomic-based kernels). */
+ *   differences at fp32 rounding level, as in the reference's atomic-based kernels); dq's too, in one pass (above). */
 int nsa_varlen_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
                         const float* lse, const int* cu_seqlens_q, const int* cu_seqlens_k, void* dq, void* dk,
                         void* dv, void* workspace, long long workspace_bytes, int total_q, int total_k, int batch,

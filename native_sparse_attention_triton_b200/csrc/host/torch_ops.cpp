@@ -433,7 +433,10 @@ struct DenseAttentionBackward final : SavingNode {
     const Tensor dout = gradient_rows(grads[0]);
     const int batch = (int)cu_q.size(0) - 1;
     const long long least = nsa_varlen_attn_bwd_workspace((int)N, (int)Nk, (int)Hq, (int)Hkv, (int)D);
-    long long bytes = m.left >= 0 ? least : nsa_varlen_attn_bwd_workspace_one_pass((int)N, (int)Nk, batch, m.max_k, (int)Hq, (int)Hkv, (int)D);
+    // one pass adds dQ up in the order in which CTAs arrive, the dQ pass in a fixed one
+    long long bytes = m.left >= 0 || at::globalContext().deterministicAlgorithms()
+                          ? least
+                          : nsa_varlen_attn_bwd_workspace_one_pass((int)N, (int)Nk, batch, m.max_k, (int)Hq, (int)Hkv, (int)D);
     Tensor ws;
     try {
       ws = empty({std::max<long long>(bytes, 16)}, at::kByte, q.device());

@@ -220,3 +220,21 @@ def test_two_passes_where_the_larger_workspace_does_not_fit():
     for x, y in zip((t.cpu() for t in got), want):
         assert (x.float() - y.float()).norm() <= 2 ** -8 * y.float().norm()
     assert pkg.device_status() == 0
+
+
+def test_dq_repeats_itself_where_that_is_asked_for():
+    import native_sparse_attention_triton_b200 as pkg
+    N, Hq, Hkv, d = 3500, 32, 2, 128
+    g = torch.Generator(device="cuda").manual_seed(10)
+    q, k, v, do = [torch.randn(N, h, d, generator=g, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv, Hq)]
+    cu = torch.tensor([0, N], dtype=torch.int32, device="cuda")
+    o = pkg.ops.flash_attention_varlen(q.requires_grad_(True), k, v, cu, cu, N, N, causal=True)
+    got = []
+    torch.use_deterministic_algorithms(True)
+    try:
+        ran = kernels(lambda: got.extend(torch.autograd.grad([o], [q], [do], retain_graph=True)[0] for _ in range(3)))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert "dense_bwd_tc" not in ran
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert "dense_bwd_tc" in kernels(lambda: torch.autograd.grad([o], [q], [do]))
