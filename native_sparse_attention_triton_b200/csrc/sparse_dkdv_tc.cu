@@ -26,13 +26,13 @@
 //
 // The rows of a tile are scattered tokens (4 KB of Q and of dO each at G = 16); a token's G heads are one TMA box per panel of
 // 64 d.  Boxes of 2 KB arrive at 26 bytes a clock and SM, cp.async at more than 60, but cp.async shares the load/store path with
-// the reductions, which hold it for 2700 clocks of every tile, and four warps issue it.  Rows that cannot be described to TMA still
-// come that way.  The Q ring has three stages (a Q tile lives from its S product to its dK product), the dO ring two.
+// the reductions, which hold it for 2700 clocks of every tile, and takes four warps to issue.  The Q ring has three stages (a Q
+// tile lives from its S product to its dK product), the dO ring two.
 //   warps 0..7  : two threads per row (32 of the 64 key columns each).  P phase (after S): P = exp2(S*scale - lse)
 //                 -> 16-bit SMEM tile; dS phase (after dP): dS = P (dP - delta) scale -> SMEM tile.  The per-row
 //                 (lse, delta) come straight from global memory, fetched one tile ahead.  At the end they drain
 //                 dV / dK from TMEM
-//   warps 8, 9  : Q and dO rows (cp.async: warps 8,9 even tiles; 10,11 odd tiles)
+//   warps 8, 9  : Q and dO rows (warps 10, 11: idle)
 //   warp 12     : S and dP products (converged warp, one elected lane issues)
 //   warps 13..16: dQ drain: warp w owns the TMEM lanes (= d) of quarter w % 4 and adds the 128 rows of
 //                 every tile's dQ^T to the fp32 accumulator
@@ -93,18 +93,17 @@ struct alignas(16) SpItem {
   int ntiles;  // 0: nothing to do (past the end of the sequence, or an empty chunk); in a queue entry -1: no more items
 };
 
-template <typename T, int LOGG, int D, bool BOXES>
+template <typename T, int LOGG, int D>
 __global__ void __launch_bounds__(kSpThreads, 1)
 sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ,
-                      const __grid_constant__ CUtensorMap tmDO, const T* __restrict__ q,
-                      const T* __restrict__ dout, long long q_sn, long long q_sh, long long do_sn, long long do_sh, DkdvParams p) {
+                      const __grid_constant__ CUtensorMap tmDO, DkdvParams p) {
   constexpr int logG = LOGG;
   constexpr int G = 1 << LOGG;
   constexpr int KT = 64;
   using C = SpCfg<D>;
   constexpr int PANELS = C::kPanels, NB = C::kPdBufs;
-  constexpr int kLoaders = BOXES ? 2 : 4;             // loader warps
-  constexpr int kItemReaders = kSpWarps - 5 + kLoaders;  // warps that read an entry of the item queue: all in use but the one that writes it
+  constexpr int kLoaders = 2;                         // loader warps
+  constexpr int kItemReaders = kSpWarps - 3;          // warps that read an entry of the item queue: all but the one that writes it and two idle ones
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* k_sm = smem;
   uint8_t* v_sm = k_sm + C::kKvBytes;
@@ -185,11 +184,11 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     mbar_init(kv_empty, 1);
     mbar_init(kv_empty + 1, 1);
     for (int s = 0; s < C::kQStages; ++s) {
-      mbar_init(q_full + s, BOXES ? 1 : 64);
+      mbar_init(q_full + s, 1);
       mbar_init(q_empty + s, 1);
     }
     for (int s = 0; s < C::kDoStages; ++s) {
-      mbar_init(do_full + s, BOXES ? 1 : 64);
+      mbar_init(do_full + s, 1);
       mbar_init(do_empty + s, D == 128 ? 2 : 1);  // read by dP and dV, which come from two warps (head_dim 64: see issue_pair)
     }
     mbar_init(s_full, 1);
@@ -240,131 +239,46 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   };
 
   // every role walks the same list of items; `gt` is the number of tiles of the items before the current one
-  if (BOXES && warp >= 8 && warp < 12) {
+  if (warp == 8 || warp == 9) {
     // ===================== loaders: warp 8 the Q rows, warp 9 the dO rows; a token's heads are one TMA box per panel =====================
-    if (warp < 10) {
-      const bool is_q = warp == 8;
-      const CUtensorMap* tm = is_q ? &tmQ : &tmDO;
-      uint64_t* full = is_q ? q_full : do_full;
-      uint64_t* empty = is_q ? q_empty : do_empty;
-      uint8_t* ring = is_q ? q_ring : do_ring;
-      const int stages = is_q ? C::kQStages : C::kDoStages;
-      // a lane's boxes: one token of the tile (32 is a multiple of their number), every kPnStep-th panel
-      constexpr int kPnStep = G / 4;
-      const int pn0 = lane >> (7 - LOGG), slot = lane & (TPT - 1);
-      const uint32_t off = slot * (G * 128);
-      int s = 0;
-      uint32_t round = 0;  // parity of the ring's round
-      bool first = true;
-      for (int k = 0;; ++k) {
-        const SpItem cur = take(k);
-        if (cur.ntiles < 0) break;
-        if (lane == 0) mbar_arrive(iq_begun);
-        auto token_of = [&](int i) {
-          const int ti = i * TPT + slot;
-          return ti < cur.tok_count ? __ldg(p.list + cur.tok_begin + ti) : -1;  // a missing token: out of range, zero fill
-        };
-        int n = token_of(0);
-        for (int i = 0; i < cur.ntiles; ++i) {
-          const int next_n = token_of(i + 1);
-          if (!first) mbar_wait(empty + s, round ^ 1u, p.st);
-          if (lane == 0) mbar_expect_tx(full + s, C::kRowBytes);
-          __syncwarp();
-#pragma unroll
-          for (int pb = 0; pb < PANELS; pb += kPnStep) {
-            const int pn = pb + pn0;
-            if (pn < PANELS) tma_load_3d(ring + s * C::kQStride + off + pn * kSpRowPanel, tm, full + s, pn * 64, cur.h * G, n);
-          }
-          n = next_n;
-          if (++s == stages) {
-            s = 0;
-            round ^= 1u;
-            first = false;
-          }
-        }
-      }
-    }
-  } else if (warp >= 8 && warp < 12) {
-    // ===================== loaders: group 0 (warps 8,9) tiles with even j, group 1 (warps 10,11) odd j =====================
-    const int grp = (warp - 8) >> 1;
-    const int tl = threadIdx.x - (8 + 2 * grp) * 32;  // 0..63
-    const int chunk16 = tl % (D / 8);                 // which 16 bytes of the row
-    const int row_in_step = tl / (D / 8);             // 4 rows per step (head_dim 64: 8)
-    const uint32_t pn_off = (chunk16 >> 3) * kSpRowPanel;
-    const int c8 = chunk16 & 7;
-    int gt = 0;
+    const bool is_q = warp == 8;
+    const CUtensorMap* tm = is_q ? &tmQ : &tmDO;
+    uint64_t* full = is_q ? q_full : do_full;
+    uint64_t* empty = is_q ? q_empty : do_empty;
+    uint8_t* ring = is_q ? q_ring : do_ring;
+    const int stages = is_q ? C::kQStages : C::kDoStages;
+    // a lane's boxes: one token of the tile (32 is a multiple of their number), every kPnStep-th panel
+    constexpr int kPnStep = G / 4;
+    const int pn0 = lane >> (7 - LOGG), slot = lane & (TPT - 1);
+    const uint32_t off = slot * (G * 128);
+    int s = 0;
+    uint32_t round = 0;  // parity of the ring's round
+    bool first = true;
     for (int k = 0;; ++k) {
       const SpItem cur = take(k);
       if (cur.ntiles < 0) break;
       if (lane == 0) mbar_arrive(iq_begun);
-      {
-        const int ntiles = cur.ntiles, tok_begin = cur.tok_begin, tok_count = cur.tok_count, h = cur.h;
-        // token ids of a tile: lane t of every loader warp holds the id of the tile's t-th token (at most 32 tokens per
-        // tile), fetched one round ahead so that the gather itself has no dependent global load in front of it
-        auto tile_tokens = [&](int i) {
-          const int ti = i * TPT + lane;
-          return (i < ntiles && lane < TPT && ti < tok_count) ? __ldg(p.list + tok_begin + ti) : -1;
-        };
-        const long long q_row0 = (long long)(h * p.G) * q_sh + chunk16 * 8, do_row0 = (long long)(h * p.G) * do_sh + chunk16 * 8;
-        const int i0 = ((gt & 1) == grp) ? 0 : 1;
-        int my_n = tile_tokens(i0);
-        for (int i = i0; i < ntiles; i += 2) {
-          const int j = gt + i;
-          const int next_n = tile_tokens(i + 2);
-          // Row r = slot * G + 4 * jj + row_in_step of the tile comes from token `slot`, head r % G.  Everything that does
-          // not depend on the token is folded into constants so that a copy costs a handful of instructions.
-          auto gather = [&](const T* src, long long sn, long long sh, long long row0, uint32_t dst_base) {
-            const uint32_t dst0 = dst_base + pn_off + row_in_step * 128;
-            if constexpr (D == 64) {
-              const uint32_t sw = (uint32_t)((c8 ^ row_in_step) << 4);
-#pragma unroll 4
-              for (int st = 0; st < 16; ++st) {
-                const int r = st * 8 + row_in_step;
-                const int n = __shfl_sync(0xffffffffu, my_n, r >> LOGG);
-                const bool ok = n >= 0;
-                cp_async16(dst0 + st * 1024 + sw, src + row0 + (long long)(ok ? n : 0) * sn + (long long)(r & (G - 1)) * sh, ok);
-              }
-            } else {
-              const uint32_t sw0 = (uint32_t)((c8 ^ row_in_step) << 4), sw1 = (uint32_t)((c8 ^ (row_in_step + 4)) << 4);
-              const T* src0 = src + row0 + (long long)row_in_step * sh;
-#pragma unroll 4
-              for (int slot = 0; slot < (128 >> LOGG); ++slot) {
-                const int n = __shfl_sync(0xffffffffu, my_n, slot);
-                const bool ok = n >= 0;
-                const T* g = src0 + (long long)(ok ? n : 0) * sn;
+      auto token_of = [&](int i) {
+        const int ti = i * TPT + slot;
+        return ti < cur.tok_count ? __ldg(p.list + cur.tok_begin + ti) : -1;  // a missing token: out of range, zero fill
+      };
+      int n = token_of(0);
+      for (int i = 0; i < cur.ntiles; ++i) {
+        const int next_n = token_of(i + 1);
+        if (!first) mbar_wait(empty + s, round ^ 1u, p.st);
+        if (lane == 0) mbar_expect_tx(full + s, C::kRowBytes);
+        __syncwarp();
 #pragma unroll
-                for (int jj = 0; jj < G / 4; ++jj) {
-                  const int jr = slot * (G / 4) + jj;  // r = 4 jr + row_in_step; r & 7 = row_in_step + 4 (jr & 1)
-                  cp_async16(dst0 + jr * 512 + ((jr & 1) ? sw1 : sw0), g + (long long)(4 * jj) * sh, ok);  // missing tokens: zero fill
-                }
-              }
-            }
-          };
-          const int sq = j % C::kQStages, sd = j % C::kDoStages;
-          if (j >= C::kQStages) mbar_wait(q_empty + sq, ((j / C::kQStages) - 1) & 1, p.st);
-          gather(q, q_sn, q_sh, q_row0, smem_u32(q_ring + sq * C::kQStride));
-          cp_async_commit();
-          // S needs the Q rows alone: they are not held back while the dO stage is still in use
-          const bool do_free = j < C::kDoStages || __all_sync(0xffffffffu, mbar_test(do_empty + sd, ((j / C::kDoStages) - 1) & 1));
-          if (!do_free) {
-            cp_async_wait<0>();
-            fence_proxy_async();
-            mbar_arrive(q_full + sq);
-            mbar_wait(do_empty + sd, ((j / C::kDoStages) - 1) & 1, p.st);
-          }
-          gather(dout, do_sn, do_sh, do_row0, smem_u32(do_ring + sd * C::kDoStride));
-          cp_async_commit();
-          if (do_free) {
-            cp_async_wait<1>();
-            fence_proxy_async();  // the tensor pipe reads these bytes through the async proxy
-            mbar_arrive(q_full + sq);
-          }
-          cp_async_wait<0>();
-          fence_proxy_async();
-          mbar_arrive(do_full + sd);
-          my_n = next_n;
+        for (int pb = 0; pb < PANELS; pb += kPnStep) {
+          const int pn = pb + pn0;
+          if (pn < PANELS) tma_load_3d(ring + s * C::kQStride + off + pn * kSpRowPanel, tm, full + s, pn * 64, cur.h * G, n);
         }
-        gt += ntiles;
+        n = next_n;
+        if (++s == stages) {
+          s = 0;
+          round ^= 1u;
+          first = false;
+        }
       }
     }
   } else if (warp == 18) {
@@ -591,7 +505,7 @@ sparse_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       for (int k = 0; take(k).ntiles >= 0; ++k) {
       }
     }
-  } else {
+  } else if (warp < 8) {
     // ===================== softmax / dS threads: two threads per row (32 of the 64 key columns each) =====================
     const int half = warp >> 2;
     const int row = (warp & 3) * 32 + lane;
@@ -751,10 +665,12 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
   rc = make_tmap_3d(&tmV, DT<T>::kTmapType, v, D, p.Hkv, Nk, strides[5], strides[4], 64, 1, 64);
   if (rc) return rc;
   const size_t smem = SpCfg<D>::kSmem;
-  // a token's rows as TMA boxes, where the rows can be described to TMA: an expanded gradient (stride 0) need not be
-  CUtensorMap tmQ = tmK, tmDO = tmK;
-  const bool boxes = make_tmap_3d(&tmQ, DT<T>::kTmapType, q, D, p.Hq, Nk, strides[1], strides[0], 64, p.G, 1) == kOk &&
-                     make_tmap_3d(&tmDO, DT<T>::kTmapType, dout, D, p.Hq, Nk, strides[7], strides[6], 64, p.G, 1) == kOk;
+  // a token's rows as TMA boxes; an expanded gradient's strides of 0 are multiples of 16 bytes like any others
+  CUtensorMap tmQ, tmDO;
+  rc = make_tmap_3d(&tmQ, DT<T>::kTmapType, q, D, p.Hq, Nk, strides[1], strides[0], 64, p.G, 1);
+  if (rc) return rc;
+  rc = make_tmap_3d(&tmDO, DT<T>::kTmapType, dout, D, p.Hq, Nk, strides[7], strides[6], 64, p.G, 1);
+  if (rc) return rc;
   auto launch = [&](auto kern) -> int {
     cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_rc(e);
@@ -764,14 +680,13 @@ int launch_sparse_dkdv_tc(const void* q, const void* dout, const void* k, const 
     const int sms = num_sms();
     const unsigned long long bound = (unsigned long long)grid.x * grid.y;   // (list entries) x (tiles per block)
     grid = dim3((unsigned)std::min<unsigned long long>(bound, (unsigned long long)sms), 1, 1);
-    kern<<<grid, kSpThreads, smem, stream>>>(tmK, tmV, tmQ, tmDO, static_cast<const T*>(q), static_cast<const T*>(dout), strides[0],
-                                             strides[1], strides[6], strides[7], p);
+    kern<<<grid, kSpThreads, smem, stream>>>(tmK, tmV, tmQ, tmDO, p);
     return cuda_rc(cudaGetLastError());
   };
   switch (logG) {
-    case 2: return boxes ? launch(sparse_dkdv_tc_kernel<T, 2, D, true>) : launch(sparse_dkdv_tc_kernel<T, 2, D, false>);
-    case 3: return boxes ? launch(sparse_dkdv_tc_kernel<T, 3, D, true>) : launch(sparse_dkdv_tc_kernel<T, 3, D, false>);
-    case 4: return boxes ? launch(sparse_dkdv_tc_kernel<T, 4, D, true>) : launch(sparse_dkdv_tc_kernel<T, 4, D, false>);
+    case 2: return launch(sparse_dkdv_tc_kernel<T, 2, D>);
+    case 3: return launch(sparse_dkdv_tc_kernel<T, 3, D>);
+    case 4: return launch(sparse_dkdv_tc_kernel<T, 4, D>);
     default: return kUnsupported;
   }
 }

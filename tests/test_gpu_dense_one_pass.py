@@ -176,6 +176,24 @@ def test_other_lengths_and_strides(Hq, Hkv, lens_q, lens_k, dtype):
     assert pkg.device_status() == 0
 
 
+@pytest.mark.parametrize("lens", [[3100], [1500, 700]])  # one pass, two passes
+@pytest.mark.parametrize("expanded", ["tokens", "tokens and heads"])
+def test_expanded_gradient(lens, expanded):
+    """The gradient of a sum over tokens, or over tokens and heads: strides of 0."""
+    import native_sparse_attention_triton_b200 as pkg
+    N, Hq, Hkv, d = sum(lens), 8, 2, 128
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v = [torch.randn(N, h, d, generator=g, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv)]
+    w = torch.randn(1, 1 if expanded == "tokens and heads" else Hq, d, generator=g, device="cuda").bfloat16()
+    do = w.expand(N, Hq, d)
+    leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    pkg.ops.flash_attention_varlen(*leaves, cu, cu, max(lens), max(lens), causal=True).backward(do)
+    for name, t, ref in zip(("dq", "dk", "dv"), leaves, reference(q, k, v, do, lens, True)):
+        assert_close_16bit(t.grad, ref.cpu(), name, grad_tol(name, False), MEAN_TOL)
+    assert pkg.device_status() == 0
+
+
 def kernels(call):
     """Names of the kernels that a call launches."""
     import native_sparse_attention_triton_b200 as pkg

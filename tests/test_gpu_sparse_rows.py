@@ -1,5 +1,5 @@
-"""Backward of the selected-block attention with output gradients of other strides: rows that TMA can describe come as boxes, others
-(an expanded gradient) by cp.async.  Gradients against autograd over the fp32 oracle, for every group size of the tcgen05 pass, lists
+"""Backward of the selected-block attention with output gradients of other strides, down to an expanded gradient's strides of 0: a
+token's rows come as TMA boxes.  Gradients against autograd over the fp32 oracle, for every group size of the tcgen05 pass, lists
 of one token, of a row tile and one more, and longer than a work item; one KV head's items are one CTA's, many or few."""
 import pytest
 import torch
