@@ -38,7 +38,7 @@ struct DkdvParams {
   int NW;  // sparse: token windows per KV head; bin x = (head * NW + window) * TB + block
 
   int window, stride, causal;
-  int left;  // dense pass only; >= 0: sliding window (key >= t - left, plain causal mask), < 0: none
+  int left;  // dense dK/dV pass only; >= 0: sliding window (key >= t - left, plain causal mask), < 0: none
   float scale2, sm_scale;
   Status st;
 };
@@ -79,7 +79,7 @@ int launch_dense_dkdv_tc(const void* q, const void* dout, const void* k, const v
                          int max_q, int max_k, int batch, DkdvParams p, cudaStream_t stream);
 
 // dQ, dK and dV of the dense attention in one pass (dense_bwd_tc.cu); head_dim 128, group size a power of two <= 16.
-// p.chunk = tokens per CTA; p.dq32 zeroed like p.dk32 and p.dv32.
+// p.chunk = tokens per CTA; p.dq32 zeroed like p.dk32 and p.dv32.  No sliding window: p.left is not read.
 template <typename T>
 int launch_dense_bwd_tc(const void* q, const void* dout, const void* k, const void* v, const long long* strides, int Nq, int Nk, int max_q,
                         int max_k, int batch, DkdvParams p, cudaStream_t stream);
