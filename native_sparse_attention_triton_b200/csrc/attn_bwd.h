@@ -21,6 +21,11 @@ __device__ __forceinline__ int find_block_sequence(const int* __restrict__ cu, i
   return lo;
 }
 
+// One fp32 value (its bits) added to an accumulator in global memory.
+__device__ __forceinline__ void red_add1(float* dst, uint32_t v) {
+  asm volatile("red.global.add.f32 [%0], %1;\n" ::"l"(dst), "f"(__uint_as_float(v)) : "memory");
+}
+
 struct DkdvParams {
   const float2* ld;    // [Nq, Hq]
   float* dk32;         // [Nk, Hkv, D] fp32 accumulators (zeroed)

@@ -21,9 +21,8 @@
 // tile), and waits of 500 for each of S and dP: 4650 a tile.  The two passes it replaces take 3.2-3.5 ms there, this one 2.7-3.1
 // (both move with the clock under the power cap), and its launches around it 0.2 ms more; where it is taken: attn_bwd.cu.
 // TMEM columns: dV [0,128)  dK [128,256)  S^T / P^T [256,384)  dP^T / dQ^T [384,512).
-#include "attn_bwd.h"
+#include "dense_bwd_tile.cuh"
 #include "host_util.h"
-#include "tc5.cuh"
 
 namespace nsa {
 namespace {
@@ -33,13 +32,6 @@ constexpr int kTile = 2 * kPanel;   // [128][128]
 constexpr int kThreads = 16 * 32;
 constexpr int kColDv = 0, kColDk = 128, kColS = 256, kColDp = 384;
 constexpr size_t kSmem = (size_t)(2 + 2 * kStages + 1) * kTile + 4 * 128 * sizeof(float) + 28 * sizeof(uint64_t) + 16;
-
-__device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-__device__ __forceinline__ void red_add1(float* dst, uint32_t v) {
-  asm volatile("red.global.add.f32 [%0], %1;\n" ::"l"(dst), "f"(__uint_as_float(v)) : "memory");
-}
 }  // namespace
 
 template <typename T, int LOGG>
@@ -154,15 +146,7 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       {
         const int m = i & 1;
         if (i >= 2) mbar_wait(meta_empty + m, ((i >> 1) - 1) & 1, p.st);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = lane + 32 * j;
-          const int tok = tok0 + (r >> logG);
-          float2 ldv = make_float2(INFINITY, 0.f);
-          if (tok < tok_end) ldv = __ldg(p.ld + (long long)(qs + tok) * p.Hq + h * p.G + (r & (p.G - 1)));
-          nlse_sh[m * 128 + r] = -ldv.x;
-          dsc_sh[m * 128 + r] = ldv.y * p.sm_scale;
-        }
+        fill_row_table(nlse_sh + m * 128, dsc_sh + m * 128, p, logG, h, qs, tok0, tok_end, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(meta_full + m);
       }
@@ -302,37 +286,11 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       float pf[64];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        uint32_t su[32];
-        tmem_ld32(lane_base + kColS + half * 64 + c * 32, su);
+        uint32_t su[1][32];
+        tmem_ld32(lane_base + kColS + half * 64 + c * 32, su[0]);
         tmem_ld_wait();
-        const float4* nl4 = reinterpret_cast<const float4*>(nlse_sh + ms * 128 + half * 64 + c * 32);
-        if (full) {
-#pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 nl = nl4[j4];
-            const int j = 4 * j4;
-            const float2 sc2 = make_float2(p.scale2, p.scale2);
-            const float2 x01 = ffma2(make_float2(__uint_as_float(su[j]), __uint_as_float(su[j + 1])), sc2, make_float2(nl.x, nl.y));
-            const float2 x23 = ffma2(make_float2(__uint_as_float(su[j + 2]), __uint_as_float(su[j + 3])), sc2, make_float2(nl.z, nl.w));
-            pf[c * 32 + j + 0] = fast_exp2(x01.x);
-            pf[c * 32 + j + 1] = fast_exp2(x01.y);
-            pf[c * 32 + j + 2] = fast_exp2(x23.x);
-            pf[c * 32 + j + 3] = fast_exp2(x23.y);
-          }
-        } else {
-#pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 nl = nl4[j4];
-            const int j = 4 * j4, col = c * 32 + j;
-            pf[col + 0] = masked_exp2((unsigned)(col + 0 - clo_rel) < span, fmaf(__uint_as_float(su[j + 0]), p.scale2, nl.x));
-            pf[col + 1] = masked_exp2((unsigned)(col + 1 - clo_rel) < span, fmaf(__uint_as_float(su[j + 1]), p.scale2, nl.y));
-            pf[col + 2] = masked_exp2((unsigned)(col + 2 - clo_rel) < span, fmaf(__uint_as_float(su[j + 2]), p.scale2, nl.z));
-            pf[col + 3] = masked_exp2((unsigned)(col + 3 - clo_rel) < span, fmaf(__uint_as_float(su[j + 3]), p.scale2, nl.w));
-          }
-        }
         uint32_t pk[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) pk[j] = DT<T>::pack(pf[c * 32 + 2 * j], pf[c * 32 + 2 * j + 1]);
+        probabilities<T, 1>(su, nlse_sh + ms * 128 + half * 64 + c * 32, p.scale2, full, clo_rel - c * 32, span, pf + c * 32, pk);
         tmem_st16(lane_base + kColS + half * 64 + c * 16, pk);  // over logits of this thread's that are in registers by now
       }
       tmem_st_wait();
@@ -345,23 +303,11 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (i > 0) mbar_wait(ds_empty, (i - 1) & 1, p.st);  // dQ and dK of the tile before have read the dS tile
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        uint32_t du[32];
-        tmem_ld32(lane_base + kColDp + half * 64 + c * 32, du);
+        uint32_t du[1][32];
+        tmem_ld32(lane_base + kColDp + half * 64 + c * 32, du[0]);
         tmem_ld_wait();
-        const float4* dl4 = reinterpret_cast<const float4*>(dsc_sh + ms * 128 + half * 64 + c * 32);
         uint32_t pk[16];
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 dl = dl4[j4];
-          const int j = 4 * j4;
-          const float2 sm2 = make_float2(p.sm_scale, p.sm_scale);
-          const float2 t01 = ffma2(make_float2(__uint_as_float(du[j]), __uint_as_float(du[j + 1])), sm2, make_float2(-dl.x, -dl.y));
-          const float2 t23 = ffma2(make_float2(__uint_as_float(du[j + 2]), __uint_as_float(du[j + 3])), sm2, make_float2(-dl.z, -dl.w));
-          const float2 d01 = fmul2(make_float2(pf[c * 32 + j], pf[c * 32 + j + 1]), t01);
-          const float2 d23 = fmul2(make_float2(pf[c * 32 + j + 2], pf[c * 32 + j + 3]), t23);
-          pk[2 * j4] = DT<T>::pack(d01.x, d01.y);
-          pk[2 * j4 + 1] = DT<T>::pack(d23.x, d23.y);
-        }
+        ds_columns<T, 1>(du, dsc_sh + ms * 128 + half * 64 + c * 32, p.sm_scale, pf + c * 32, pk);
 #pragma unroll
         for (int c4 = 0; c4 < 4; ++c4)
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(ds_row + (((c * 4 + c4) ^ (key & 7)) << 4)), "r"(pk[c4 * 4]),
@@ -375,25 +321,11 @@ dense_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mbar_arrive(meta_empty + ms);
       }
     }
-    // ---- thread (key, half) adds half of the d columns of its key's dV and dK rows ----
+    // ---- read-out ----
     mbar_wait(all_done, 0, p.st);
     tc_fence_after_sync();
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      float* dst = (which == 0 ? p.dv32 : p.dk32) + ((size_t)(krow0 + key) * p.Hkv + h) * D + half * (D / 2);
-#pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t r[32];
-        tmem_ld32(lane_base + (which == 0 ? kColDv : kColDk) + half * (D / 2) + c * 32, r);
-        tmem_ld_wait();
-        if (key_ok) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            red_add_v4(dst + c * 32 + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                       __uint_as_float(r[j + 3]));
-        }
-      }
-    }
+    static_assert(kColDk == kColDv + 128);
+    add_key_rows<D>(p, lane_base + kColDv, (size_t)(krow0 + key) * p.Hkv + h, half, key_ok);
   }
   tc_fence_before_sync();
   __syncthreads();

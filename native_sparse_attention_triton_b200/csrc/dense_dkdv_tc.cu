@@ -18,19 +18,14 @@
 //   warp 8     : TMA producer (Q ring of 3 tiles, dO ring of 2) and the per-row table
 //   warp 9     : TMEM allocation, MMA issue (one thread polls four queues: S, dP, dV, dK)
 // TMEM columns: dV [0,128)  dK [128,256)  S^T / P^T [256,384)  dP^T / dS^T [384,512).
-#include "attn_bwd.h"
+#include "dense_bwd_tile.cuh"
 #include "host_util.h"
-#include "tc5.cuh"
 
 namespace nsa {
 namespace {
 constexpr int kQStages = 3;
 constexpr int kDoStages = 2;
 constexpr int kPanelBytes = 128 * 128;  // [128][64] 16-bit elements; an operand tile of 128 x D is D / 64 of them
-
-__device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 }  // namespace
 
 template <typename T, int D>
@@ -141,15 +136,7 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       {
         const int s = i & 1;
         if (i >= 2) mbar_wait(meta_empty + s, ((i >> 1) - 1) & 1, p.st);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = lane + 32 * j;
-          const int tok = tok0 + (r >> logG);
-          float2 ldv = make_float2(INFINITY, 0.f);
-          if (tok < tok_end) ldv = __ldg(p.ld + (long long)(qs + tok) * p.Hq + h * p.G + (r & (p.G - 1)));
-          nlse_sh[s * 128 + r] = -ldv.x;
-          dsc_sh[s * 128 + r] = ldv.y * p.sm_scale;
-        }
+        fill_row_table(nlse_sh + s * 128, dsc_sh + s * 128, p, logG, h, qs, tok0, tok_end, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(meta_full + s);
       }
@@ -258,37 +245,10 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tmem_ld32(lane_base + 256 + half * 64, su[0]);
         tmem_ld32(lane_base + 256 + half * 64 + 32, su[1]);
         tmem_ld_wait();
-        const float4* nl4 = reinterpret_cast<const float4*>(nlse_sh + ms * 128 + half * 64);
         // tiles every key of the warp sees in full (all but those on the mask's edge) skip the mask instructions
-        if (__all_sync(0xffffffffu, clo == 0 && chi == 128)) {
-#pragma unroll
-          for (int j4 = 0; j4 < 16; ++j4) {
-            const float4 nl = nl4[j4];
-            const int j = 4 * j4;
-            const float2 sc2 = make_float2(p.scale2, p.scale2);
-            const float2 x01 = ffma2(make_float2(__uint_as_float(su[j >> 5][(j + 0) & 31]), __uint_as_float(su[j >> 5][(j + 1) & 31])), sc2,
-                                     make_float2(nl.x, nl.y));
-            const float2 x23 = ffma2(make_float2(__uint_as_float(su[j >> 5][(j + 2) & 31]), __uint_as_float(su[j >> 5][(j + 3) & 31])), sc2,
-                                     make_float2(nl.z, nl.w));
-            pf[j + 0] = fast_exp2(x01.x);
-            pf[j + 1] = fast_exp2(x01.y);
-            pf[j + 2] = fast_exp2(x23.x);
-            pf[j + 3] = fast_exp2(x23.y);
-          }
-        } else {
-#pragma unroll
-          for (int j4 = 0; j4 < 16; ++j4) {
-            const float4 nl = nl4[j4];
-            const int j = 4 * j4;
-            pf[j + 0] = masked_exp2((unsigned)(j + 0 - clo_rel) < span, fmaf(__uint_as_float(su[j >> 5][(j + 0) & 31]), p.scale2, nl.x));
-            pf[j + 1] = masked_exp2((unsigned)(j + 1 - clo_rel) < span, fmaf(__uint_as_float(su[j >> 5][(j + 1) & 31]), p.scale2, nl.y));
-            pf[j + 2] = masked_exp2((unsigned)(j + 2 - clo_rel) < span, fmaf(__uint_as_float(su[j >> 5][(j + 2) & 31]), p.scale2, nl.z));
-            pf[j + 3] = masked_exp2((unsigned)(j + 3 - clo_rel) < span, fmaf(__uint_as_float(su[j >> 5][(j + 3) & 31]), p.scale2, nl.w));
-          }
-        }
+        const bool full = __all_sync(0xffffffffu, clo == 0 && chi == 128);
         uint32_t pk[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) pk[j] = DT<T>::pack(pf[2 * j], pf[2 * j + 1]);
+        probabilities<T, 2>(su, nlse_sh + ms * 128 + half * 64, p.scale2, full, clo_rel, span, pf, pk);
         tmem_st32(lane_base + 256 + half * 64, pk);  // over this thread's own logits
         tmem_st_wait();
       }
@@ -303,22 +263,8 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tmem_ld32(lane_base + 384 + half * 64, du[0]);
         tmem_ld32(lane_base + 384 + half * 64 + 32, du[1]);
         tmem_ld_wait();
-        const float4* dl4 = reinterpret_cast<const float4*>(dsc_sh + ms * 128 + half * 64);
         uint32_t pk[32];
-#pragma unroll
-        for (int j4 = 0; j4 < 16; ++j4) {
-          const float4 dl = dl4[j4];
-          const int j = 4 * j4;
-          const float2 sm2 = make_float2(p.sm_scale, p.sm_scale);
-          const float2 t01 = ffma2(make_float2(__uint_as_float(du[j >> 5][(j + 0) & 31]), __uint_as_float(du[j >> 5][(j + 1) & 31])), sm2,
-                                   make_float2(-dl.x, -dl.y));
-          const float2 t23 = ffma2(make_float2(__uint_as_float(du[j >> 5][(j + 2) & 31]), __uint_as_float(du[j >> 5][(j + 3) & 31])), sm2,
-                                   make_float2(-dl.z, -dl.w));
-          const float2 d01 = fmul2(make_float2(pf[j + 0], pf[j + 1]), t01);
-          const float2 d23 = fmul2(make_float2(pf[j + 2], pf[j + 3]), t23);
-          pk[2 * j4] = DT<T>::pack(d01.x, d01.y);
-          pk[2 * j4 + 1] = DT<T>::pack(d23.x, d23.y);
-        }
+        ds_columns<T, 2>(du, dsc_sh + ms * 128 + half * 64, p.sm_scale, pf, pk);
         tmem_st32(lane_base + 384 + half * 64, pk);
         tmem_st_wait();
       }
@@ -329,25 +275,10 @@ dense_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         mbar_arrive(meta_empty + ms);
       }
     }
-    // ---- drain: thread (key, half) adds half of the d columns of its key's dV and dK rows ----
+    // ---- drain ----
     mbar_wait(all_done, 0, p.st);
     tc_fence_after_sync();
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      float* dst = (which == 0 ? p.dv32 : p.dk32) + ((size_t)(krow0 + key) * p.Hkv + h) * D + half * (D / 2);
-#pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t r[32];
-        tmem_ld32(lane_base + which * 128 + half * (D / 2) + c * 32, r);
-        tmem_ld_wait();
-        if (key_ok) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            red_add_v4(dst + c * 32 + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                       __uint_as_float(r[j + 3]));
-        }
-      }
-    }
+    add_key_rows<D>(p, lane_base, (size_t)(krow0 + key) * p.Hkv + h, half, key_ok);
   }
   tc_fence_before_sync();
   __syncthreads();

@@ -81,10 +81,6 @@ struct SpCfg {
 };
 constexpr int kTmS = 0, kTmDp = 64, kTmAcc = 128, kTmDq = 256;  // TMEM columns: logits, dP, dV and dK (64 each), two buffers for dQ
 constexpr int kSpWarps = 19, kSpThreads = kSpWarps * 32;
-
-__device__ __forceinline__ void red_add1(float* dst, uint32_t v) {
-  asm volatile("red.global.add.f32 [%0], %1;\n" ::"l"(dst), "f"(__uint_as_float(v)) : "memory");
-}
 }  // namespace
 
 // One work item: a 64-key tile of a selected block and (a chunk of) the list of tokens that selected the block.
