@@ -196,17 +196,18 @@ def config_record():
                 l2_policy="inputs (q alone is 1.07 GB) exceed the 126 MB L2; no explicit flush")
 
 
-# kernel -> (bound, algorithmic work per launch as a function of the useful-FLOP model of oracle.nsa_oracle.useful_flops)
 # DRAM bytes (read + write) per launch measured by ncu on a 16384-token case.
 # These kernels' DRAM traffic is their linear-in-tokens streams (Q, O, dO, dQ rows; K/V re-reads hit L2), so the figure is
-# scaled by tokens / 16384 for the workload at hand.
+# scaled by tokens / 16384 for the workload at hand.  dense_bwd_tc, which takes 3072 keys and more, was captured with one of the
+# workload's four KV heads instead: 65536 tokens, 16q/1kv, 4095 compressed keys, the same bytes as a quarter of the tokens with all four.
 NCU_DRAM_BYTES_16K = {
     "dense_fwd_tc": 0.271e9 + 226.9e6, "score_topk_tc": 0.275e9 + 6.3e6, "sparse_fwd": 0.306e9 + 241.0e6,
     "sparse_dq": 0.851e9 + 259.3e6, "sparse_dkdv_tc": 3.242e9 + 1.889e9, "dense_dq_tc": 0.815e9 + 253.8e6,
-    "dense_dkdv_tc": 0.553e9 + 7.3e6,
+    "dense_dkdv_tc": 0.553e9 + 7.3e6, "dense_bwd_tc": 1.115e9 + 515.9e6,
 }
 
 
+# kernel -> (bound, algorithmic work per launch as a function of the useful-FLOP model of oracle.nsa_oracle.useful_flops)
 def kernel_work(name, f, fused_dq=True):
     """fused_dq: the sparse dK/dV pass also produces dQ (no separate sparse_dq launch), so it is credited all five
     backward GEMM units of the selected-block attention."""
@@ -1182,7 +1183,8 @@ def main():
             traffic = NCU_DRAM_BYTES_16K.get(dom)
             roofline = dict(kernel=dom, bound=work[0], achieved=achieved, peak=pk["tc_sustained"], unit="TFLOP/s",
                             frac=achieved / pk["tc_sustained"], traffic=None if traffic is None else traffic * N / 16384,
-                            traffic_unit="bytes of DRAM read+write per launch (ncu capture at 16384 tokens, scaled by tokens)",
+                            traffic_unit="bytes of DRAM read+write per launch (ncu capture of a quarter of the work: 16384 tokens, scaled by tokens; "
+                                         "dense_bwd_tc: one of four KV heads)",
                             launch_ms=avg_ms, peak_source=pk["source"],
                             note="peak = sustained cuBLAS bf16 figure (kernel timed inside a long step)")
         else:

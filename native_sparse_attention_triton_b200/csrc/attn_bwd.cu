@@ -15,6 +15,7 @@
 //               share a key tile are added with fp32 red.global into a zeroed accumulator and
 //               converted to the storage type at the end.
 #include <algorithm>
+#include <cmath>
 #include <utility>
 
 #include "attn_tile.cuh"
@@ -730,27 +731,32 @@ static size_t dense_ws_bytes(int total_q, int total_k, int Hq, int Hkv, int D) {
 // dQ, dK and dV in one pass (dense_bwd_tc.cu) or a dQ pass and a dK/dV pass.  One pass forms five products a tile and two passes
 // seven, but dQ then needs a zeroed fp32 accumulator, a conversion and its row statistics in a launch of their own (1.4 ms for 65 536
 // tokens of 64 heads), so what counts is how many key tiles a query sees.  Backward alone, us, both forms in turn, two passes -> one:
-// 3072 tokens, causal, 64q/4kv 564 -> 547, 16q/1kv 186 -> 183, 8q/8kv 173 -> 128; 4 x 3072 tokens 64q/4kv 2190 -> 2096; 8192 tokens 64q/4kv
-// 3345 -> 3167, 32q/8kv 1906 -> 1622; 3072 keys compressed from 12 296 tokens 2141 -> 2137, from 49 168 8242 -> 8084 (16q/1kv 2228 -> 2095), 4095
-// from 65 536 14 465 -> 13 747 (32q/8kv 7495 -> 6595); 200 queries of 3500 keys 90 -> 62.  The longest sequence stands for the others only
-// where these are not much shorter (3072 and three of 1100: 878 -> 842).  Windows see few tiles.
+// 3072 tokens, causal, 64q/4kv 555 -> 545, 16q/1kv 184 -> 183, 8q/8kv 173 -> 127; 4 x 3072 tokens 64q/4kv 2122 -> 2060; 8192 tokens 64q/4kv
+// 3298 -> 3150, 32q/8kv 1898 -> 1657; 3072 keys compressed from 12 296 tokens 2100 -> 2096, from 49 168 8159 -> 7870 (16q/1kv 2198 -> 2075), 4095
+// from 65 536 13 693 -> 13 302 (32q/8kv 7412 -> 6789); 200 queries of 3500 keys 87 -> 52.  The longest sequence stands for the others only
+// where these are not much shorter (3072 and three of 1100: 854 -> 827).  Windows see few tiles.
 static bool dense_one_pass(int total_k, int batch, int max_k, int D) {
   return D == 128 && max_k >= 3072 && 2ll * total_k >= (long long)batch * max_k;
 }
 
 // Tokens per CTA of the one pass.  A CTA's loads, ramp and the read-out of dK and dV cost as much as 2.4 row tiles (16 384 tokens 8q/8kv:
-// 2852 us with 4 tiles, 2324 with 8, 2047 with 16, 1887 with 32, 1829 with 64), and at the end an SM waits for half a CTA on average: of W row
-// tiles an SM takes W (1 + 2.4 / t) + t / 2 of time, which is least at t = sqrt(4.8 W).  The power of two next to it, us, against half and
-// twice as many: 3072 tokens 8q/8kv (W 15) 8 tiles 128, 16 136; 3072 tokens 16q/8kv 16 tiles 183, 8 190, 32 201; 4096 tokens 64q/4kv (W 220) 32
-// tiles 924, 64 916, 16 979; 8192 tokens 64q/4kv (W 890) 64 tiles 3270, 32 3392, 128 3308; 16 384 tokens 64q/4kv (W 3540) 128 tiles 12 014, 64
-// 12 311; 20 000 tokens 32q/2kv 8891, 9138.  Lengths in tokens, as the dK/dV pass has them, gave small groups CTAs of 2 to 8 tiles: 3072 tokens
-// 8q/8kv 175 us, 4 x 3072 622 (411 now), slower than the two passes.
+// 2307 us with 8 tiles, 2041 with 16, 1901 with 32, 1859 with 64), and at the end SMs wait for a CTA that has just begun: of W row tiles an SM
+// takes W (1 + 2.4 / t) and a part of t of time, which is least at a multiple of sqrt(W).  Taken is the power of two up to 5.3 sqrt(W), us, against
+// half and twice as many: 3072 tokens 64q/4kv (W 130) 32 tiles 551, 16 594, 64 571; 7000 tokens 32q/2kv at stride 2 (W 167) 64 tiles 696, 32 722;
+// 8192 tokens 64q/4kv (W 890) 64 tiles 3270, 32 3392, 128 3308.  Fewer where that leaves less than two CTAs for every SM, for then the last
+// wave counts: 3500 tokens 16q/1kv 16 tiles 189, 32 217; 3072 tokens 8q/8kv 8 tiles 128, 16 135.  Lengths in tokens alone, as the dK/dV pass has
+// them, gave small groups CTAs of 2 to 8 tiles: 3072 tokens 8q/8kv 175 us, 4 x 3072 622 (411 now), slower than the two passes.
+// At most 32 tiles, 16 for groups of one and two, and up to 64 where the dK/dV pass's CTAs (256 tokens, 512 past 4096, 1024 past 8192) are
+// as long: the tensor pipe's fp32 sums are cut off at every step, so dK and dV get further from 64 bits with their length (fp16, error of
+// dK's sums: 8192 tokens 16q/1kv 2.211e-4 with 16 tiles, 2.212e-4 with 32, 2.214e-4 with 64, 2.224e-4 with 128, 2.270e-4 with 256; 2q/2kv 2.233e-4
+// with 4, 2.235e-4 with 16, 2.238e-4 with 32), for little time (16 384 tokens 64q/4kv 12 311 us with 64, 12 014 with 128).
 static int one_pass_chunk(int total_k, int batch, int max_q, int Hkv, int G, int causal) {
-  // (key tile, head) pairs times the row tiles that see one, half of them under the causal mask
-  const double row_tiles = (double)max_q * G / (causal ? 256 : 128);
-  const double per_sm = ((double)total_k / 128 + batch) * Hkv * row_tiles / 148;
-  int tiles = 128;
-  while (tiles > 8 && (double)tiles * tiles > 10 * per_sm) tiles >>= 1;
+  // (key tile, head) pairs, and the tokens that see one, half of them under the causal mask
+  const double pairs = ((double)total_k / 128 + batch) * Hkv, span = causal ? 0.5 * max_q : max_q;
+  const double per_sm = pairs * span * G / 128 / 148;  // row tiles
+  const int tokens = max_q > 8192 ? 1024 : max_q > 4096 ? 512 : 256;
+  int tiles = std::min(64, std::max(G >= 4 ? 32 : 16, tokens * G / 128));
+  while (tiles > 8 && ((double)tiles * tiles > 28 * per_sm || pairs * std::ceil(span / (tiles * (128 / G))) < 2 * 148)) tiles >>= 1;
   return tiles * (128 / G);
 }
 

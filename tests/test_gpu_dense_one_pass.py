@@ -114,11 +114,11 @@ def test_compressed_keys_and_the_smaller_workspace():
 
 @pytest.mark.parametrize("Hq,Hkv,lens,causal", [
     (2, 2, [3072], 1),           # CTAs of 8 row tiles, the least
-    (8, 8, [3072] * 4, 1),       # 16
+    (8, 8, [3072] * 4, 1),       # 16, the most for groups of one and two
     (4, 1, [5000, 3071], 1),     # 16
     (16, 1, [6100], 1),          # 32
-    (16, 1, [9000], 0),          # 64
-    (16, 1, [24600], 1),         # 128, the most
+    (16, 1, [9000], 0),          # 64, the most
+    (16, 1, [24600], 1),
 ])
 def test_cta_lengths(Hq, Hkv, lens, causal):
     """One pass against two, as above, with CTAs of every length."""
